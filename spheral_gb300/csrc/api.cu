@@ -7,6 +7,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <numeric>
 #include <stdexcept>
@@ -137,6 +138,7 @@ struct sphgpu_ctx {
   long permVersion = 0;      // bumped whenever the internal order changes
   long invVersion = -1;      // permVersion the inverse was built for
   DBuf posh, velm, thermo;   // FP32 mirrors of the pair-loop inputs
+  DBuf pk;                   // isotropic pair loop: per-node inputs (mixed SPH)
   DBuf hten;                 // ASPH: FP32 mirror of tensor H (2 float4 per node)
   DBuf vol32, rkc32;         // CRKSPH, mixed mode: FP32 mirrors of the RK volume and corrections
   double kernelExtent = 2.0; // extent of the configured base kernel (BSpline 2, NBSpline (order+1)/2)
@@ -147,20 +149,23 @@ struct sphgpu_ctx {
   sphgpu_exchange_fn xfn = nullptr;
   void* xuser = nullptr;
   DBuf xstage, xidx;         // exchange rows and caller indices
-  DBuf v12;                  // half-step velocities + DepsDt0 of the mixed-mode energy sweep
+  DBuf v12;                  // half-step velocities + DepsDt0 of the energy sweep
+  DBuf rec64;                // FP64 isotropic SPH: node records of the sweeps
   int cur = 0;
   long cap = 0;
   // neighbour build
   Grid grid{};
-  DBuf keys, vals, keysAlt, valsAlt, sortWs, cellStart, cellEnd, counts, nbrStart, nbr, scanWs, pacc;
+  DBuf keys, vals, keysAlt, valsAlt, sortWs, cellRange, counts, nbr, pacc;
   size_t cellSpace = 0;
   long long nnbr = 0;
   int nbCap = 0;             // slots per node of the warp-interleaved neighbour lists (0: not sized yet)
   int nbCapNext = 0;         // smaller capacity to adopt at the next build (0: keep)
-  DBuf itemFlag, items;      // work items of the warp-cooperative neighbour search
+  DBuf items;                // work items of the warp-cooperative neighbour search
   bool haveNeighbors = false;
   // scratch
   DBuf scratch, small;
+  DBuf stepScratch;           // StepScratch of the handle's kernels
+  StepScratch* hstep = nullptr;   // its pinned copy
   double* hsmall = nullptr;   // pinned
   // integrator
   double time = 0.0, lastDt = 1e-5, dtMultiplier = 1.0;
@@ -185,8 +190,7 @@ struct sphgpu_ctx {
   long pairEvals = 0, pairRetuneAt = -1;
   long energyEvals = 0, energyRetuneAt = -1;
   long widthTunedN = 0;      // node count it was tuned at
-  DBuf itemCount;            // device: number of work items
-  bool capCheckPending = false, totalPending = false;
+  bool capCheckPending = false;
   double cachedBounds[kBoundsVals] = {};   // min h^-1, min x y z, max x y z, tensor extents of the current state
   bool boundsValid = false;      // cachedBounds describe the current state
   int pairVariant = -1;      // autotuned FP32 pair-kernel variant (-1: not tuned yet)
@@ -221,6 +225,9 @@ struct sphgpu_ctx {
     t.p32b = reinterpret_cast<const float2*>(b32 + 2 * nc + 4 * (nc / 3));
     return t;
   }
+  StepScratch* step() { return stepScratch.as<StepScratch>(); }
+  int* cellStart() { return cellRange.as<int>(); }
+  int* cellEnd() { return cellRange.as<int>() + cellSpace; }
   NeighborLists nl() { return NeighborLists{nbr.as<uint32_t>(), counts.as<int>(), nbCap, cellp()}; }
   size_t nbSlots() const { return (size_t)((n + 31) / 32) * 32 * (size_t)nbCap; }
   Fields32 f32() {
@@ -228,6 +235,7 @@ struct sphgpu_ctx {
     p.posh = posh.as<float4>();
     p.velm = velm.as<float4>();
     p.thermo = thermo.as<float4>();
+    p.pk = pk.as<float4>();
     p.cell = cellp();
     p.dvq = dvq.p ? dvq.as<float4>() : nullptr;
     p.hten = cfg.smoothing_scale != SPHGPU_SMOOTHING_SPH ? hten.as<float4>() : nullptr;
@@ -235,6 +243,8 @@ struct sphgpu_ctx {
     p.rkc = rkc32.p ? rkc32.as<float4>() : nullptr;
     return p;
   }
+  // FP64 sweeps with isotropic H (hydro64.cu)
+  bool iso64() const { return !fp32() && cfg.smoothing_scale == SPHGPU_SMOOTHING_SPH; }
   bool fp32() const { return cfg.precision != SPHGPU_PRECISION_FP64; }   // FP32 sweeps (compensated or plain)
   void check() { CUDA_OK(cudaGetLastError()); }
 };
@@ -252,6 +262,10 @@ void ensureCapacity(sphgpu_ctx* c, long n) {
   c->posh.release(); c->posh.ensure(n * sizeof(float4));
   c->velm.release(); c->velm.ensure(n * sizeof(float4));
   c->thermo.release(); c->thermo.ensure(n * sizeof(float4));
+  c->pk.release();
+  c->rec64.release();
+  if (c->iso64()) c->rec64.ensure(n * nodeRecordBytes64());
+  if (c->fp32()) c->pk.ensure(n * sizeof(float4));
   c->hten.release();
   if (c->cfg.smoothing_scale != SPHGPU_SMOOTHING_SPH) c->hten.ensure(2 * n * sizeof(float4));
   c->vol32.release();
@@ -267,8 +281,11 @@ void ensureCapacity(sphgpu_ctx* c, long n) {
   }
 }
 
+// cubic: the table is the built-in cubic B-spline's with at least 400 points
+// (interpolation error below 4e-9): the FP32 sweeps evaluate that kernel in
+// registers instead.
 void setTable(sphgpu_ctx* c, const double* w, const double* g, const double* g2, const double* nperh,
-              const double* wsum, const double* meta) {
+              const double* wsum, const double* meta, bool cubic) {
   const int N1 = (int)meta[0];
   const int nh = (int)meta[2];
   if (N1 < 1 || 3 * (N1 + 1) > kMaxTable || nh < 3) throw Error(SPHGPU_E_ARG, "kernel table size out of range");
@@ -301,6 +318,7 @@ void setTable(sphgpu_ctx* c, const double* w, const double* g, const double* g2,
                      h32.size() * sizeof(float), cudaMemcpyHostToDevice));
   // Derived constants
   auto& hp = c->hp;
+  hp.cubicSpline = cubic ? 1 : 0;
   hp.tableN1 = N1;
   hp.tableXstep = meta[1];
   hp.extent = c->kernelExtent;
@@ -470,35 +488,35 @@ void buildGrid(sphgpu_ctx* c) {
 }
 
 int capFor(int m) { return std::max(32, ((m + m / 8 + 16 + 31) / 32) * 32); }
-int* maxCountPtr(sphgpu_ctx* c) { return reinterpret_cast<int*>(c->small.as<double>() + 40); }
+// The kernels' scratch values, read back in stream order (valid after the
+// next synchronisation).
+void fetchScratch(sphgpu_ctx* c) {
+  CUDA_OK(cudaMemcpyAsync(c->hstep, c->step(), sizeof(StepScratch), cudaMemcpyDeviceToHost, c->stream));
+}
 int readMaxCount(sphgpu_ctx* c) {
-  CUDA_OK(cudaMemcpyAsync(c->hsmall + 40, maxCountPtr(c), sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  fetchScratch(c);
   CUDA_OK(cudaStreamSynchronize(c->stream));
-  int m;
-  std::memcpy(&m, c->hsmall + 40, sizeof(int));
-  return m;
+  if (c->hstep->sortTimeout) throw Error(SPHGPU_E_TIMEOUT, "a wait inside the node sort ran out");
+  return c->hstep->maxCount;
 }
-// Write pass of the neighbour search into lists of capacity nbCap; the
-// largest count lands in the maxCount slot.
-void writeLists(sphgpu_ctx* c) {
+void searchLists(sphgpu_ctx* c, bool write) {
+  launchNeighborsWarp(c->F, c->f32(), c->n, c->items.as<int>(), c->itemBound, c->step(), c->itemWidth, c->grid,
+                      c->cellStart(), c->cellEnd(), c->counts.as<int>(), write ? c->nbr.as<uint32_t>() : nullptr,
+                      write ? c->nbCap : 0, c->hp.extent * c->hp.extent, c->hp.asph != 0, c->itemBox.as<float4>(),
+                      c->chunkOf.as<int>(), c->stream, &c->lc);
+  c->check();
+}
+// A search clears its counters first unless the node keys have just done so.
+void clearCounts(sphgpu_ctx* c) {
+  CUDA_OK(cudaMemsetAsync(&c->step()->maxCount, 0, sizeof(int), c->stream));
+  CUDA_OK(cudaMemsetAsync(c->step()->entries, 0, sizeof(c->hstep->entries), c->stream));
+}
+// Write pass of the neighbour search into lists of capacity nbCap.
+void writeLists(sphgpu_ctx* c, bool fresh) {
   c->nbr.ensure(std::max<size_t>(1, c->nbSlots()) * sizeof(uint32_t));
-  CUDA_OK(cudaMemsetAsync(maxCountPtr(c), 0, sizeof(int), c->stream));
+  if (!fresh) clearCounts(c);
   Scope sc(c->prof, "neighbors");
-  launchNeighborsWarp(c->F, c->f32(), c->n, c->items.as<int>(), c->itemBound, c->itemCount.as<long long>(),
-                      c->itemWidth, c->grid, c->cellStart.as<int>(), c->cellEnd.as<int>(), c->counts.as<int>(),
-                      maxCountPtr(c), c->nbr.as<uint32_t>(), c->nbCap, c->hp.extent * c->hp.extent, c->hp.asph != 0,
-                      c->itemBox.as<float4>(), c->chunkOf.as<int>(), c->stream, &c->lc);
-  c->check();
-}
-// CSR offsets of the lists (caller-order transfers) and their total, read
-// back without a synchronisation.
-void scanTotals(sphgpu_ctx* c) {
-  const long n = c->n;
-  long long* dTot = c->nbrStart.as<long long>() + n;
-  scanExclusive<int>(c->counts.as<int>(), c->nbrStart.as<long long>(), n, c->scanWs.p, dTot, c->stream, &c->lc);
-  c->check();
-  CUDA_OK(cudaMemcpyAsync(c->hsmall + 42, dTot, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-  c->totalPending = true;
+  searchLists(c, true);
 }
 bool resolveNeighbors(sphgpu_ctx* c);
 
@@ -510,15 +528,25 @@ bool resolveNeighbors(sphgpu_ctx* c);
 // to the step's dt synchronisation and only the carried fields are permuted
 // (the step rewrites the others before it returns).
 void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
-  const bool deferCheck = inStep;
   const long n = c->n;
   buildGrid(c);
-  int bitsAxis = 0;
-  while ((1 << bitsAxis) < std::max(c->grid.nc[0], std::max(c->grid.nc[1], c->grid.nc[2]))) ++bitsAxis;
-  // one sub-cell Morton level in the sort key while it fits 30 bits
-  c->grid.subShift = bitsAxis <= 9 ? 3 : 0;
+  // Key layout: as many Morton levels as the narrowest axis has bits, the
+  // wider axes' remaining bits above them (no key space for cells that an
+  // elongated grid does not have), one sub-cell level below while it fits.
+  {
+    int bits[3], low = 10, at;
+    for (int a = 0; a < 3; ++a) {
+      bits[a] = 0;
+      while ((1 << bits[a]) < c->grid.nc[a]) ++bits[a];
+      low = std::min(low, bits[a]);
+    }
+    c->grid.keyBits = low;
+    at = 3 * low;
+    for (int a = 0; a < 3; ++a) { c->grid.keyHigh[a] = at; at += bits[a] - low; }
+    c->grid.subShift = at <= 27 ? 3 : 0;
+  }
   const Grid& g = c->grid;
-  const int keyBits = std::max(1, 3 * bitsAxis);            // bits of the cell key
+  const int keyBits = std::max(1, g.keyHigh[2] + [&] { int b = 0; while ((1 << b) < g.nc[2]) ++b; return b - g.keyBits; }());
   const int sortBits = keyBits + g.subShift;                // bits of the sort key
   c->keys.ensure(n * sizeof(uint32_t));
   c->keysAlt.ensure(n * sizeof(uint32_t));
@@ -527,7 +555,7 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   c->sortWs.ensure(radixSortWorkspaceBytes(n));
   {
     Scope sc(c->prof, "cell_keys");
-    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->stream, &c->lc);
+    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->step(), c->stream, &c->lc);
   }
   uint32_t* k = c->keys.as<uint32_t>();
   int* v = c->vals.as<int>();
@@ -535,85 +563,69 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   int* va = c->valsAlt.as<int>();
   {
     Scope sc(c->prof, "radix_sort");
-    radixSortPairs(k, v, ka, va, n, ((sortBits + 7) / 8) * 8, c->sortWs.p, c->stream, &c->lc);
+    radixSortPairs(k, v, ka, va, n, sortBits, c->sortWs.p, &c->step()->sortTimeout, c->stream, &c->lc);
   }
   c->check();
+  const size_t space = (size_t)1 << keyBits;
+  if (space > c->cellSpace) {
+    c->cellRange.release();
+    c->cellRange.ensure(2 * space * sizeof(int));
+    c->cellSpace = space;
+  }
+  CUDA_OK(cudaMemsetAsync(c->cellStart(), 0, (c->cellSpace + space) * sizeof(int), c->stream));
   {
     Scope sc(c->prof, "permute");
     const int nx = 1 - c->cur;
+    Fields32 m = c->f32();
+    m.cell = c->cellc[nx].as<uint32_t>();
     launchPermute(c->F, c->Falt, v, c->orig[c->cur].as<int>(), c->orig[nx].as<int>(), c->list[c->cur].as<int>(),
                   c->list[nx].as<int>(), c->cellc[c->cur].as<uint32_t>(), c->cellc[nx].as<uint32_t>(), n,
-                  inStep, c->hp.asph != 0, c->hp.crk != 0, c->stream, &c->lc);
+                  inStep, c->hp.asph != 0, c->hp.crk != 0, m, g, c->fp32(), k, (uint32_t)space, c->cellStart(),
+                  c->cellEnd(), c->stream, &c->lc);
     std::swap(c->bankA, c->bankB);
     std::swap(c->F, c->Falt);
     c->cur = nx;
     ++c->permVersion;
   }
   c->check();
-  const size_t space = (size_t)1 << keyBits;
-  if (space > c->cellSpace) {
-    c->cellStart.release(); c->cellEnd.release();
-    c->cellStart.ensure(space * sizeof(int));
-    c->cellEnd.ensure(space * sizeof(int));
-    c->cellSpace = space;
-  }
-  CUDA_OK(cudaMemsetAsync(c->cellStart.p, 0, space * sizeof(int), c->stream));
-  CUDA_OK(cudaMemsetAsync(c->cellEnd.p, 0, space * sizeof(int), c->stream));
-  {
-    Scope sc(c->prof, "cell_ranges");
-    launchCellRanges(k, n, g.subShift, c->cellStart.as<int>(), c->cellEnd.as<int>(), c->stream, &c->lc);
-  }
-  {
-    Scope sc(c->prof, "prepare_fp32");
-    launchPrepareFP32(c->F, c->f32(), n, g, c->stream, &c->lc);
-  }
   c->counts.ensure(n * sizeof(int));
-  c->nbrStart.ensure((n + 1) * sizeof(long long));
-  c->scanWs.ensure(scanWorkspaceBytes(n) + 64);
-  c->itemCount.ensure(sizeof(long long));
   // work items: first node of every chunk of up to `width` nodes of a cell.
   // The first guess of the group width follows the mean occupancy of the
   // cells so that few lanes of a group idle; the autotuner below then times
   // the widths once per problem size.
   const double cellsTotal = (double)g.nc[0] * g.nc[1] * g.nc[2];
   const double occupancy = (double)n / cellsTotal;
-  const int guess = occupancy >= 24.0 ? 32 : (occupancy >= 12.0 ? 16 : 8);
+  // The isotropic search runs 32 lanes per item at any width, so 32 it is.
+  const int guess = (!c->hp.asph || occupancy >= 24.0) ? 32 : (occupancy >= 12.0 ? 16 : 8);
   ++c->listBuilds;
   const bool retuneWidth = c->widthRetuneAt >= 0 && c->listBuilds >= c->widthRetuneAt;
-  const bool tuned = c->pinnedWidth > 0 ||
+  if (!c->hp.asph) c->tunedWidth = guess, c->widthTunedN = n;
+  const bool tuned = c->pinnedWidth > 0 || !c->hp.asph ||
                      (!retuneWidth && c->tunedWidth > 0 && std::labs(n - c->widthTunedN) <= c->widthTunedN / 8);
-  c->itemFlag.ensure(n * sizeof(int));
   c->items.ensure(n * sizeof(int));
   c->itemBox.ensure(2 * (size_t)n * sizeof(float4));
   c->chunkOf.ensure(n * sizeof(int));
-  auto makeItems = [&](int width) {
+  auto makeItems = [&](int width, bool fresh) {
     c->itemWidth = width;
     // every non-empty cell adds at most one partial chunk
     c->itemBound = (int)std::min<double>((double)n, (double)(n / width) + cellsTotal);
+    if (!fresh) CUDA_OK(cudaMemsetAsync(&c->step()->items, 0, sizeof(int), c->stream));
     Scope sc(c->prof, "neighbor_items");
-    long long* pos = c->nbrStart.as<long long>();
-    launchItemFlags(k, n, g.subShift, c->cellStart.as<int>(), width, c->itemFlag.as<int>(), c->stream, &c->lc);
-    scanExclusive<int>(c->itemFlag.as<int>(), pos, n, c->scanWs.p, c->itemCount.as<long long>(), c->stream, &c->lc);
-    launchItemFill(c->itemFlag.as<int>(), pos, n, c->items.as<int>(), c->stream, &c->lc);
-    launchItemBoxes(c->items.as<int>(), c->itemCount.as<long long>(), c->itemBound, n, width, c->f32(),
-                    c->itemBox.as<float4>(), c->chunkOf.as<int>(), c->stream, &c->lc);
+    launchItems(k, n, g.subShift, (uint32_t)space, c->cellEnd(), width, c->itemBound, c->f32(), c->items.as<int>(),
+                c->chunkOf.as<int>(), c->itemBox.as<float4>(), c->step(), c->stream, &c->lc);
     c->check();
   };
-  makeItems(c->pinnedWidth > 0 ? c->pinnedWidth : (tuned ? c->tunedWidth : guess));
+  makeItems(c->pinnedWidth > 0 ? c->pinnedWidth : (tuned ? c->tunedWidth : guess), true);
   if (c->nbCapNext > 0) {   // adopt a smaller capacity decided at the previous build
     c->nbCap = c->nbCapNext;
     c->nbCapNext = 0;
   }
+  bool fresh = true;   // the counters of the search are clear
   if (c->nbCap == 0) {   // first build: size the lists with a counting pass
-    int* dMax = maxCountPtr(c);
-    CUDA_OK(cudaMemsetAsync(dMax, 0, sizeof(int), c->stream));
     Scope sc(c->prof, "neighbor_count");
-    launchNeighborsWarp(c->F, c->f32(), n, c->items.as<int>(), c->itemBound, c->itemCount.as<long long>(),
-                        c->itemWidth, g, c->cellStart.as<int>(), c->cellEnd.as<int>(), c->counts.as<int>(), dMax,
-                        nullptr, 0, c->hp.extent * c->hp.extent, c->hp.asph != 0, c->itemBox.as<float4>(),
-                        c->chunkOf.as<int>(), c->stream, &c->lc);
-    c->check();
+    searchLists(c, false);
     c->nbCap = capFor(readMaxCount(c));
+    fresh = false;
   }
   if (!tuned) {
     // Autotuner: the lists do not depend on the group width (the candidate
@@ -628,9 +640,9 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
     int bestW = guess;
     for (int round = 0; round < 2; ++round)
       for (const int w : {8, 16, 32}) {
-        if (w != c->itemWidth) makeItems(w);
+        if (w != c->itemWidth) makeItems(w, false);
         CUDA_OK(cudaEventRecord(e0, c->stream));
-        writeLists(c);
+        writeLists(c, false);
         CUDA_OK(cudaEventRecord(e1, c->stream));
         CUDA_OK(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -642,56 +654,37 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
     c->tunedWidth = bestW;
     c->widthTunedN = n;
     c->widthRetuneAt = retuneWidth ? -1 : c->listBuilds + kRetuneAfter;
-    if (bestW != c->itemWidth) makeItems(bestW);
+    if (bestW != c->itemWidth) makeItems(bestW, false);
+    fresh = false;
   }
-  writeLists(c);
-  if (deferCheck) {
-    // The capacity check and the entry total are read at the caller's next
-    // stream synchronisation (resolveNeighbors).
-    CUDA_OK(cudaMemcpyAsync(c->hsmall + 40, maxCountPtr(c), sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    c->capCheckPending = true;
-  } else {
-    while (true) {
-      const int m = readMaxCount(c);
-      if (m <= c->nbCap) {
-        if (capFor(m) * 2 < c->nbCap) c->nbCapNext = capFor(m);   // shrink at the next build, not now
-        break;
-      }
-      c->nbCap = capFor(m);   // overflow: enlarge and rewrite
-      writeLists(c);
-    }
-  }
-  scanTotals(c);
+  writeLists(c, fresh);
+  c->capCheckPending = true;   // read at the caller's next stream synchronisation (resolveNeighbors)
   c->haveNeighbors = true;
-  if (!deferCheck) resolveNeighbors(c);
+  if (!inStep) {
+    readMaxCount(c);
+    resolveNeighbors(c);
+  }
 }
 
-// Reads the deferred capacity check and entry total after a stream
-// synchronisation.  Returns true when the lists overflowed and were rewritten
-// with a larger capacity (the caller must redo sweeps that used them).
+// Settles the capacity check and the entry total of the last build from the
+// scratch values read back at a synchronisation since.  Returns true when the
+// lists overflowed and were rewritten with a larger capacity (the caller must
+// redo sweeps that used them).
 bool resolveNeighbors(sphgpu_ctx* c) {
+  if (!c->capCheckPending) return false;
+  c->capCheckPending = false;
+  if (c->hstep->sortTimeout) throw Error(SPHGPU_E_TIMEOUT, "a wait inside the node sort ran out");
+  int m = c->hstep->maxCount;
   bool regrown = false;
-  if (c->capCheckPending) {
-    c->capCheckPending = false;
-    int m;
-    std::memcpy(&m, c->hsmall + 40, sizeof(int));
-    if (m > c->nbCap) {
-      do {
-        c->nbCap = capFor(m);
-        writeLists(c);
-        m = readMaxCount(c);
-      } while (m > c->nbCap);
-      scanTotals(c);
-      regrown = true;
-    } else if (capFor(m) * 2 < c->nbCap) {
-      c->nbCapNext = capFor(m);
-    }
+  while (m > c->nbCap) {   // overflow: enlarge and rewrite
+    c->nbCap = capFor(m);
+    writeLists(c, false);
+    m = readMaxCount(c);
+    regrown = true;
   }
-  if (c->totalPending) {
-    CUDA_OK(cudaStreamSynchronize(c->stream));
-    std::memcpy(&c->nnbr, c->hsmall + 42, sizeof(long long));
-    c->totalPending = false;
-  }
+  if (!regrown && capFor(m) * 2 < c->nbCap) c->nbCapNext = capFor(m);   // shrink at the next build, not now
+  c->nnbr = 0;
+  for (const auto e : c->hstep->entries) c->nnbr += (long long)e;
   return regrown;
 }
 
@@ -723,6 +716,9 @@ void sumDensity(sphgpu_ctx* c) {
     launchCRKDensity(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   else if (c->fp32())
     launchSumDensityFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
+  else if (c->iso64())
+    launchDensityDt64(c->F, c->rec64.p, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, true, false,
+                      c->maxNperh(), nullptr, nullptr, c->stream, &c->lc);
   else
     launchSumDensity(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   c->check();
@@ -731,6 +727,8 @@ void gradh(sphgpu_ctx* c) {
   Scope sc(c->prof, "gradh");
   if (c->fp32())
     launchGradhFP32(c->F, c->f32(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
+  else if (c->iso64())
+    launchGradh64(c->F, c->rec64.p, c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   else
     launchGradh(c->F, c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   c->check();
@@ -745,8 +743,10 @@ void evalDerivs(sphgpu_ctx* c) {
   ensurePacc(c);
   if (c->fp32() && c->hp.limitedQ) {   // FP32 mirror of the Q's DvDx in the current node order
     c->dvq.ensure((size_t)c->n * 3 * sizeof(float4));
-    launchQGradient32(c->F, c->dvq.as<float4>(), c->n, c->stream, &c->lc);
-    c->check();
+    if (c->hp.asph || c->hp.crk) {   // the isotropic SPH sweep writes its own form
+      launchQGradient32(c->F, c->dvq.as<float4>(), c->n, c->stream, &c->lc);
+      c->check();
+    }
   }
   // Autotuner of the mixed pair kernels: time each variant (register budget,
   // loop form) twice per problem size and again two uses later (the kernel
@@ -811,8 +811,12 @@ void evalDerivs(sphgpu_ctx* c) {
                   &c->lc);
   } else {
     Scope sc(c->prof, "pair_fp64");
-    launchPairFP64(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->pacc.as<double>(),
-                   128, c->stream, &c->lc);
+    if (c->iso64())
+      launchPair64(c->F, c->rec64.p, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->pacc.as<double>(),
+                   c->stream, &c->lc);
+    else
+      launchPairFP64(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->pacc.as<double>(), c->stream,
+                     &c->lc);
   }
   c->check();
   if (c->cfg.gravity) {
@@ -839,24 +843,40 @@ void setGhostParams(sphgpu_ctx* c) {
   c->hp.nOwn = c->n - c->nGhost;
 }
 
+// Blocks of a vote sweep at most (up to 8 lanes per node in the FP64 sweep).
+long voteBlocks(long n) { return (8 * n + 127) / 128; }
+
+// The vote of the mixed sweeps: the value with its low bits as the reason.
+void readVote(const StepScratch& h, double& v, int& reason) {
+  if (h.voteKey == ~0ULL) { v = std::numeric_limits<double>::max(); reason = -1; return; }
+  const unsigned long long b = h.voteKey & ~7ULL;
+  std::memcpy(&v, &b, sizeof v);
+  reason = (int)(h.voteKey & 7ULL);
+}
+
 double packageDt(sphgpu_ctx* c, int* reason, bool fusedDone = false) {
   Scope sc(c->prof, "dt");
   setGhostParams(c);
-  const long nb = (c->n + 127) / 128;
+  const long nb = voteBlocks(c->n);
   c->scratch.ensure(std::max<size_t>(2 * nb * sizeof(double), 7 * sizeof(double) * 4096));
   double* d = c->small.as<double>();
   if (fusedDone) {
   } else if (c->fp32())
-    launchDtFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->hp, c->maxNperh(),
-                 c->scratch.as<double>(), (int)(2 * nb), d, c->stream, &c->lc);
+    launchDtFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->hp, c->maxNperh(), c->step(), c->stream, &c->lc);
+  else if (c->iso64())
+    launchDensityDt64(c->F, c->rec64.p, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, false, true,
+                      c->maxNperh(), c->scratch.as<double>(), d, c->stream, &c->lc);
   else
     launchDt(c->F, c->listp(), c->n, c->grid, c->nl(), c->hp, c->maxNperh(), c->scratch.as<double>(),
              (int)(2 * nb), d, c->stream, &c->lc);
   c->check();
-  CUDA_OK(cudaMemcpyAsync(c->hsmall, d, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  fetchScratch(c);
+  if (!c->fp32()) CUDA_OK(cudaMemcpyAsync(c->hsmall, d, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CUDA_OK(cudaStreamSynchronize(c->stream));
-  double dt = c->hsmall[0] * c->cfg.cfl;
+  double dt = c->hsmall[0];
   int r = (int)c->hsmall[1];
+  if (c->fp32()) readVote(*c->hstep, dt, r);
+  dt *= c->cfg.cfl;
   if (c->cfg.gravity) {
     const double gdt = c->cfg.ftimestep * c->dtMinAcc;
     if (gdt < dt) { dt = gdt; r = 6; }
@@ -876,22 +896,22 @@ double selectDt(sphgpu_ctx* c, double dtMin, double dtMax, bool fusedDone = fals
   return dt;
 }
 
-// The end-of-step check also takes the bounds the next neighbour build needs
-// (min h^-1, bounding box), read back in the same synchronisation.
-void checkState(sphgpu_ctx* c, const char* where) {
-  int* flag = reinterpret_cast<int*>(c->small.as<double>() + 30);
-  CUDA_OK(cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
-  launchCheckState(c->F, c->n, flag, c->stream, &c->lc);
-  double* b = c->small.as<double>() + 20;
-  c->scratch.ensure(kBoundsVals * sizeof(double) * 4096);
-  launchBounds(c->F, c->n, c->hp.asph != 0, c->scratch.as<double>(), kBoundsVals * 4096, b, c->stream, &c->lc);
-  CUDA_OK(cudaMemcpyAsync(c->hsmall + 20, b, kBoundsVals * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_OK(cudaMemcpyAsync(c->hsmall + 30, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+// The end of the step in one pass: walls, the state check and the bounds the
+// next neighbour build needs, read back in one synchronisation.
+void endStep(sphgpu_ctx* c) {
+  {
+    Scope sc(c->prof, "enforce");
+    launchEndStep(c->F, c->n, c->grid, c->hp.asph != 0, c->step(), c->stream, &c->lc);
+  }
+  c->check();
+  fetchScratch(c);
   CUDA_OK(cudaStreamSynchronize(c->stream));
-  int h;
-  std::memcpy(&h, c->hsmall + 30, sizeof(int));
-  if (h) throw Error(SPHGPU_E_NAN, std::string("non-finite or non-positive state after ") + where);
-  std::memcpy(c->cachedBounds, c->hsmall + 20, sizeof(c->cachedBounds));
+  if (c->hstep->bad) throw Error(SPHGPU_E_NAN, "non-finite or non-positive state after the step");
+  for (int k = 0; k < kBoundsVals; ++k) {   // order keys back to doubles
+    long long b = c->hstep->bounds[k];
+    if (b < 0) b ^= 0x7fffffffffffffffLL;
+    std::memcpy(&c->cachedBounds[k], &b, sizeof b);
+  }
   c->boundsValid = true;
 }
 
@@ -912,7 +932,7 @@ double step(sphgpu_ctx* c, double maxTime) {
   refreshParams(c);
   buildNeighbors(c, true);                           // Integrator::setGhostNodes + connectivity
   bool fused = false;
-  auto preStep = [&]() {
+  auto preStep = [&](bool again) {
     if (c->hp.radialOnly) launchRadius0(c->F, c->n, c->stream, &c->lc);   // SmoothingScaleBase::preStepInitialize
     if (c->hp.crk) {   // RKCorrections::preStepInitialize: the RK volumes
       Scope sc(c->prof, "rk_volume");
@@ -921,14 +941,17 @@ double step(sphgpu_ctx* c, double maxTime) {
       else
         launchRKVolumes(c->F, c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
     }
-    if (c->cfg.density_update == SPHGPU_DENSITY_RIGOROUS_SUM) {   // preStepInitialize (+ dt vote when mixed SPH)
-      if (c->fp32() && !c->hp.crk) {
+    if (c->cfg.density_update == SPHGPU_DENSITY_RIGOROUS_SUM) {   // preStepInitialize (+ dt vote in the fused sweeps)
+      if (!c->hp.crk && (c->fp32() || c->iso64())) {
         Scope sc(c->prof, "density_dt");
-        const long nb = (c->n + 127) / 128;
+        const long nb = voteBlocks(c->n);
         c->scratch.ensure(std::max<size_t>(2 * nb * sizeof(double), 7 * sizeof(double) * 4096));
         setGhostParams(c);
-        launchDensityDtFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp,
+        if (c->iso64())
+          launchDensityDt64(c->F, c->rec64.p, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, true, true,
                             c->maxNperh(), c->scratch.as<double>(), c->small.as<double>(), c->stream, &c->lc);
+        else launchDensityDtFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp,
+                            c->maxNperh(), c->step(), again, c->stream, &c->lc);
         c->check();
         fused = true;
       } else {
@@ -936,14 +959,14 @@ double step(sphgpu_ctx* c, double maxTime) {
       }
     }
   };
-  preStep();
+  preStep(false);
   const double t = c->time;
   double dt = selectDt(c, std::min(c->cfg.dt_min, maxTime - t), std::min(c->cfg.dt_max, maxTime - t), fused);
   // The dt read synchronised the stream: settle the deferred list check.  A
   // list that overflowed its capacity was rewritten larger; redo the sweeps
   // that read it.
   if (resolveNeighbors(c)) {
-    preStep();
+    preStep(true);
     dt = selectDt(c, std::min(c->cfg.dt_min, maxTime - t), std::min(c->cfg.dt_max, maxTime - t), fused);
   }
   if (c->xfn) {
@@ -966,10 +989,6 @@ double step(sphgpu_ctx* c, double maxTime) {
   if (c->cfg.gradh_correction) exchangePoint(c, SPHGPU_EXCHANGE_OMEGA);
   evalDerivs(c);                                     // derivs.Zero(); evaluateDerivatives(t + dt/2)
   exchangePoint(c, SPHGPU_EXCHANGE_DERIVS);          // the halo's accelerations and energy rates
-  {
-    Scope sc(c->prof, "update");
-    launchRestoreState0(c->F, c->n, c->hp.asph != 0, c->hp.crk != 0, c->stream, &c->lc);
-  }
   if (c->cfg.compatible_energy) {
     Scope sc(c->prof, "energy");
     if (c->fp32()) {
@@ -1007,8 +1026,10 @@ double step(sphgpu_ctx* c, double maxTime) {
       launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(),
                                  c->v12.as<float4>() + c->n, dt, c->energyVariant, c->stream, &c->lc);
     }
-    else
-      launchCompatibleEnergy(c->F, c->n, c->grid, c->nl(), c->pacc.as<double>(), nullptr, dt, c->stream, &c->lc);
+    else {
+      c->v12.ensure(c->n * 4 * sizeof(double));
+      launchEnergy64(c->F, c->v12.p, c->n, c->grid, c->nl(), c->pacc.as<double>(), dt, c->stream, &c->lc);
+    }
   }
   {
     Scope sc(c->prof, "update");
@@ -1041,12 +1062,7 @@ double step(sphgpu_ctx* c, double maxTime) {
                   c->stream, &c->lc);
     c->check();
   }
-  {
-    Scope sc(c->prof, "enforce");
-    launchEnforce(c->F, c->n, c->grid, c->hp.asph != 0, c->stream, &c->lc);
-  }
-  c->check();
-  checkState(c, "the step");
+  endStep(c);
   c->cycle += 1;
   c->lastDt = dt;
   return dt;
@@ -1244,6 +1260,8 @@ int sphgpu_create(const sphgpu_config* cfg, sphgpu_handle* out) {
     c->prof.s = c->stream;
     c->small.ensure(64 * sizeof(double));
     CUDA_OK(cudaMallocHost(&c->hsmall, 64 * sizeof(double)));
+    c->stepScratch.ensure(sizeof(StepScratch));
+    CUDA_OK(cudaMallocHost(&c->hstep, sizeof(StepScratch)));
     c->time = cfg->time;
     c->lastDt = cfg->last_dt;
     for (int k = 0; k < kMaxNodeLists; ++k)
@@ -1264,7 +1282,8 @@ int sphgpu_create(const sphgpu_config* cfg, sphgpu_handle* out) {
                                 ws.data(), meta.data()) != 0)
       throw Error(SPHGPU_E_ARG, "bad num_table_points");
     c->kernelExtent = meta[9];
-    setTable(c, w.data(), g.data(), g2.data(), nh.data(), ws.data(), meta.data());
+    setTable(c, w.data(), g.data(), g2.data(), nh.data(), ws.data(), meta.data(),
+             cfg->kernel == SPHGPU_KERNEL_BSPLINE && np >= 400);
     refreshParams(c);
   } catch (const Error& e) {
     const int code = e.code;
@@ -1284,16 +1303,17 @@ int sphgpu_destroy(sphgpu_handle c) {
   c->prof.on = false;
   for (auto& r : c->prof.pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   DBuf* bufs[] = {&c->dTable, &c->bankA, &c->bankB, &c->keys, &c->vals, &c->keysAlt, &c->valsAlt, &c->sortWs,
-                  &c->cellStart, &c->cellEnd, &c->counts, &c->nbrStart, &c->nbr, &c->scanWs, &c->pacc,
-                  &c->scratch, &c->small, &c->posh, &c->velm, &c->thermo, &c->hten, &c->stage, &c->v12, &c->itemFlag,
+                  &c->cellRange, &c->counts, &c->nbr, &c->stepScratch, &c->pacc,
+                  &c->scratch, &c->small, &c->posh, &c->velm, &c->thermo, &c->pk, &c->rec64, &c->hten, &c->stage, &c->v12,
                   &c->items, &c->dLists, &c->dvq, &c->inv, &c->vol32, &c->rkc32, &c->xstage, &c->xidx,
-                  &c->itemBox, &c->chunkOf, &c->itemCount};
+                  &c->itemBox, &c->chunkOf};
   for (auto* b : bufs) b->release();
   for (int k = 0; k < 2; ++k) { c->orig[k].release(); c->list[k].release(); c->cellc[k].release(); }
   if (c->grav) gravityDestroy(c->grav);
   if (c->tA) cudaEventDestroy(c->tA);
   if (c->tB) cudaEventDestroy(c->tB);
   if (c->hsmall) cudaFreeHost(c->hsmall);
+  if (c->hstep) cudaFreeHost(c->hstep);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return SPHGPU_OK;
@@ -1320,7 +1340,11 @@ int sphgpu_set_kernel_table(sphgpu_handle c, const double* w, const double* grad
                             const double* nperh, const double* wsum, const double* meta) {
   API_BEGIN(c)
   if (!w || !grad || !grad2 || !nperh || !wsum || !meta) throw Error(SPHGPU_E_ARG, "null table pointer");
-  setTable(c, w, grad, grad2, nperh, wsum, meta);
+  // the installed cubic B-spline set again stays the cubic B-spline
+  const size_t nc = meta[0] >= 1.0 && meta[0] < kMaxTable ? 3 * ((size_t)meta[0] + 1) : 0;
+  const bool same = c->hp.cubicSpline && nc == c->tw.size() && std::equal(w, w + nc, c->tw.begin()) &&
+                    std::equal(grad, grad + nc, c->tg.begin());
+  setTable(c, w, grad, grad2, nperh, wsum, meta, same);
   refreshParams(c);
   API_END(c)
 }
@@ -1644,7 +1668,7 @@ int sphgpu_advance(sphgpu_handle c, int nsteps, double max_time) {
 
 int sphgpu_set_pair_variant(sphgpu_handle c, int variant) {
   API_BEGIN(c)
-  if (variant < -1 || variant >= kPairVariants) throw Error(SPHGPU_E_ARG, "pair variant out of range");
+  if (variant < -1 || variant >= kPairVariantsMax) throw Error(SPHGPU_E_ARG, "pair variant out of range");
   c->pairVariant = variant;
   c->pinnedVariant = variant >= 0;
   API_END(c)

@@ -30,6 +30,10 @@ struct Grid {
   float cellf[3];      // cell edges rounded to FP32 (set on the host: no device conversions)
   float ext2f;         // kernel extent squared, FP32
   int subShift;        // 3: sort keys carry one sub-cell Morton level below the cell key; 0: none
+  // cell key: the low keyBits of every axis interleaved (Morton), the
+  // remaining bits of the longer axes above them
+  int keyBits;
+  int keyHigh[3];      // position of each axis' remaining bits in the cell key
 };
 
 struct NodeListParams {
@@ -49,6 +53,7 @@ struct HydroParams {
   int tableN1;        // N1 of the quadratic table
   double tableXstep;  // interval of the quadratic table
   double extent;      // kernel extent
+  int cubicSpline;    // the table is the built-in cubic B-spline's (fine enough for FP32)
   int hermN;          // Hermite knots of the nperh lookup
   double hermXmin, hermXmax, hermXstep;
   const NodeListParams* lists;   // device table of the NodeLists (kMaxNodeLists entries)
@@ -111,6 +116,16 @@ __host__ __device__ __forceinline__ uint32_t spreadBits10(uint32_t v) {
 }
 __host__ __device__ __forceinline__ uint32_t morton3(uint32_t x, uint32_t y, uint32_t z) {
   return spreadBits10(x) | (spreadBits10(y) << 1) | (spreadBits10(z) << 2);
+}
+
+// Key of cell (x, y, z); with half-cell coordinates and one more bit per axis
+// (extra = 1) the key's low three bits are the octant inside the cell and its
+// upper bits the cell's key.
+__host__ __device__ __forceinline__ uint32_t cellKey(const Grid& g, uint32_t x, uint32_t y, uint32_t z, int extra) {
+  const int b = g.keyBits + extra;
+  const uint32_t m = (1u << b) - 1u;
+  return morton3(x & m, y & m, z & m) | ((x >> b) << (g.keyHigh[0] + 3 * extra)) |
+         ((y >> b) << (g.keyHigh[1] + 3 * extra)) | ((z >> b) << (g.keyHigh[2] + 3 * extra));
 }
 
 }  // namespace sph

@@ -443,9 +443,10 @@ __global__ void __launch_bounds__(128) pairKernelCRK(Fields F, const int* __rest
     dvy -= ay;
     dvz -= az;
     if (COMPAT) {
-      pacc[3 * slot] = -ax;
-      pacc[3 * slot + 1] = -ay;
-      pacc[3 * slot + 2] = -az;
+      double* out = pacc + paccSlot(slot);
+      out[0] = -ax;
+      out[32] = -ay;
+      out[64] = -az;
     }
     deps += f * (Pj * (vijx * dgx + vijy * dgy + vijz * dgz) + workQi) * invMi;
     if (XSPH && lj == li) {

@@ -120,10 +120,7 @@ __global__ void __launch_bounds__(128) rkSumVolume32(Fields F, Fields32 P, long 
                                                      TableDev t, HydroParams hp) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
   const Tab32 T = loadTab32(ta, tb, t, hp);
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
-  __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int ci[3];
@@ -138,7 +135,7 @@ __global__ void __launch_bounds__(128) rkSumVolume32(Fields F, Fields32 P, long 
     const uint32_t ent = nl.nbr[nbSlot(i, q, nl.cap)];
     const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
     float rx, ry, rz;
-    relSepTab(pi, P.posh[j], dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
+    relSepEntry(pi, P.posh[j], ent, mm, cx, cy, cz, rx, ry, rz);
     float e2, re;
     const float em = etaMag(ai * rx, ai * ry, ai * rz, e2, re);
     float W, G;
@@ -161,10 +158,7 @@ __global__ void __launch_bounds__(128) crkDensity32(Fields F, Fields32 P, const 
                                                     Grid g, NeighborLists nl, TableDev t, HydroParams hp) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
   const Tab32 T = loadTab32(ta, tb, t, hp);
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
-  __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int ci[3];
@@ -182,7 +176,7 @@ __global__ void __launch_bounds__(128) crkDensity32(Fields F, Fields32 P, const 
     if (multi && list[j] != li) continue;
     const float4 pj = P.posh[j];
     float rx, ry, rz;
-    relSepTab(pi, pj, dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
+    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
     const float aj = pj.w;
     float e2, re;
     const float em = etaMag(aj * rx, aj * ry, aj * rz, e2, re);
@@ -218,10 +212,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
                                                        TableDev t, HydroParams hp) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
   const Tab32 T = loadTab32(ta, tb, t, hp);
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
-  __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int ci[3];
@@ -259,7 +250,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
     const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
     const float4 pj = P.posh[j];
     float rx, ry, rz;
-    relSepTab(pi, pj, dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
+    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
     const float aj = pj.w;
     const float ex = aj * rx, ey = aj * ry, ez = aj * rz;
     float e2, re;
@@ -360,10 +351,7 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
                                                        float* __restrict__ pacc) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
   const Tab32 T = loadTab32(ta, tb, t, hp);
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
-  __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int ci[3];
@@ -400,7 +388,7 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
     const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
     const uint32_t mq = (uint32_t)dcode & mm;
     float rx, ry, rz;
-    relSepTab(pi, pj, dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
+    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
     float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
     mirrorVel(mq, vxj, vyj, vzj);
     const float aj = pj.w, mj = vj4.w, rhoj = thj.x, Pj = thj.y, csj = thj.z;
@@ -477,9 +465,10 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
     kahanAdd(sdy, cdy, -ay);
     kahanAdd(sdz, cdz, -az);
     if (COMPAT) {
-      pacc[3 * slot] = -ax;
-      pacc[3 * slot + 1] = -ay;
-      pacc[3 * slot + 2] = -az;
+      float* out = pacc + paccSlot(slot);
+      out[0] = -ax;
+      out[32] = -ay;
+      out[64] = -az;
     }
     // DepsDt_i += V_i V_j / 2 (P_j + rho_j e_j) v_ij . (gradW_j - gradW_i) / m_i
     const float vdg = __fmaf_rn(vz, dgz, __fmaf_rn(vy, dgy, __fmul_rn(vx, dgx)));

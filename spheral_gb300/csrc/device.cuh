@@ -29,6 +29,76 @@ __device__ __forceinline__ void sumAdd(float& s, float& c, float x, int plain) {
 // its eta_i and eta_j; the density/dt and grad-h sweeps use it too.
 __device__ __forceinline__ float etaFromSq(float e2) { return __fmul_rn(e2, rsqrtf(fmaxf(e2, 1.0e-30f))); }
 
+//------------------------------------------------------------------------------
+// Lanes per node of the mixed-mode sweeps.  L consecutive lanes of a warp
+// share one node: lane l takes the list slots l, l + L, ..., and the partial
+// sums are combined by shuffles.
+//------------------------------------------------------------------------------
+template <int L>
+__device__ __forceinline__ float laneSum(float v) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int L>
+__device__ __forceinline__ float laneMax(float v) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// Compensated partial sums s - c: the rounding error of every addition of
+// two partial sums goes into the compensation (TwoSum), so the total keeps
+// the accuracy of the parts.
+template <int L>
+__device__ __forceinline__ void laneSumKahan(float& s, float& c) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) {
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), c2 = __shfl_xor_sync(0xffffffffu, c, o);
+    const float t = __fadd_rn(s, s2);
+    const float b = __fsub_rn(t, s);
+    const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(s2, b));
+    c = __fsub_rn(__fadd_rn(c, c2), err);
+    s = t;
+  }
+}
+
+// The cubic B-spline and its derivative in registers, without the volume
+// normalisation A = 1/pi (kSplineA), which the sweeps apply once per node so
+// that the rounding of A does not bias every term:
+//   eta < 1: W/A = 1 - 3/2 eta^2 + 3/4 eta^3,  W'/A = -(3 - 9/4 eta) eta
+//   eta < 2: W/A = 1/4 (2 - eta)^3,            W'/A = -3/4 (2 - eta)^2
+// The interpolation table of this kernel (500 intervals) agrees with it to
+// ~1e-9, far below FP32 rounding, and costs two shared-memory gathers with
+// bank conflicts per lookup; the other kernels and caller tables use the
+// packed table.
+constexpr double kSplineA = 0.31830988618379067154;
+__device__ __forceinline__ float bsplineGrad(float eta) {
+  const float d = fmaxf(2.0f - eta, 0.0f);
+  const float in = __fmul_rn(eta, __fmaf_rn(2.25f, eta, -3.0f));
+  const float out = __fmul_rn(d, __fmul_rn(-0.75f, d));
+  return eta < 1.0f ? in : out;
+}
+__device__ __forceinline__ float bsplineW(float eta) {
+  const float d = fmaxf(2.0f - eta, 0.0f);
+  const float in = __fmaf_rn(__fmul_rn(eta, eta), __fmaf_rn(0.75f, eta, -1.5f), 1.0f);
+  const float out = __fmul_rn(__fmul_rn(d, d), __fmul_rn(0.25f, d));
+  return eta < 1.0f ? in : out;
+}
+// x times A for one FP32 value per node (A as an unevaluated float pair).
+__device__ __forceinline__ float timesSplineA(float x) {
+  constexpr float hi = (float)kSplineA, lo = (float)(kSplineA - (double)(float)kSplineA);
+  return __fmaf_rn(x, hi, __fmul_rn(x, lo));
+}
+
+__device__ __forceinline__ void resetScratch(StepScratch* sc) {
+  for (int k = 0; k < 4; ++k) sc->bounds[k] = 0x7fffffffffffffffLL;
+  for (int k = 4; k < 10; ++k) sc->bounds[k] = k < 7 ? (long long)0x8000000000000000ULL : 0LL;
+  sc->bad = sc->sortTimeout = sc->maxCount = sc->items = 0;
+  for (int k = 0; k < kEntrySums; ++k) sc->entries[k] = 0ULL;
+  sc->voteKey = ~0ULL;
+  sc->voteEst = 0x7f7fffffu;   // FLT_MAX
+}
+
 // Velocity of a mirror image: the components along the mirrored axes flip
 // (mir: per-axis bits of the entry's cell-offset code that cross a wall).
 __device__ __forceinline__ void mirrorVel(uint32_t mir, float& vx, float& vy, float& vz) {
@@ -44,6 +114,49 @@ __device__ __forceinline__ void mirrorVel(uint32_t mir, float& vx, float& vy, fl
 // touches one contiguous 128-byte line.
 __device__ __forceinline__ long long nbSlot(long i, int q, int cap) {
   return ((long long)(i >> 5) * cap + q) * 32 + (i & 31);
+}
+
+// FP32 pair accelerations: the three components of a list slot sit in three
+// 32-wide planes per slot row, so a warp writing (reading) one component of
+// slot q of its 32 nodes touches one 128-byte line.  paccSlot(nbSlot(..)) is
+// the x component; y is 32 floats further, z 64.
+__device__ __forceinline__ long long paccSlot(long long slot) { return (slot >> 5) * 96 + (slot & 31); }
+
+// Walk the list slots of node i that belong to lane `sub` of its L lanes, in
+// list order, U slots per iteration: load(j, rec) gathers a neighbour's
+// record, slot(entry, rec) evaluates it.  The U gathers of an iteration are
+// issued together and the next iteration's entries are loaded before they are
+// used.
+template <int L, int U, class Rec, class Load, class Slot>
+__device__ __forceinline__ void laneSlots(const NeighborLists& nl, long i, int sub, int cnt, Load load, Slot slot) {
+  constexpr int ST = 32 * L;
+  const int mine = (cnt - sub + L - 1) / L;
+  const uint32_t* __restrict__ nb = nl.nbr + nbSlot(i, 0, nl.cap) + 32 * sub;
+  uint32_t nx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) nx[u] = u < mine ? nb[u * ST] : 0u;
+  int q = 0;
+  for (; q + U <= mine; q += U) {
+    uint32_t e[U];
+    Rec rec[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = nx[u];
+#pragma unroll
+    for (int u = 0; u < U; ++u) load(e[u] & kIndexMask, rec[u]);
+    nb += U * ST;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (q + U + u < mine) nx[u] = nb[u * ST];
+#pragma unroll
+    for (int u = 0; u < U; ++u) slot(e[u], rec[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U - 1; ++u)
+    if (q + u < mine) {
+      Rec rec;
+      load(nx[u] & kIndexMask, rec);
+      slot(nx[u], rec);
+    }
 }
 
 __device__ __forceinline__ void unpackCell(uint32_t cc, int c[3]) {
@@ -84,7 +197,7 @@ __device__ __forceinline__ void forEachCandidate(const Grid& g, uint32_t cc, con
           cell[a] = nn;
         }
         if (!ok) continue;
-        const uint32_t key = morton3((uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2]);
+        const uint32_t key = cellKey(g, (uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2], 0);
         const int s = cellStart[key], e = cellEnd[key];
         for (int k = s; k < e; ++k) fn(k, dcode);
       }
@@ -115,6 +228,37 @@ __device__ __forceinline__ uint32_t mirrorMask(const Grid& g, const int c[3]) {
   return m;
 }
 
+// Whether any wall of the grid reflects (host): the sweeps' forms without
+// mirror images serve every other grid.
+inline bool hasMirrors(const Grid& g) {
+  for (int a = 0; a < 3; ++a)
+    if (g.kindLo[a] == AXIS_REFLECT || g.kindHi[a] == AXIS_REFLECT) return true;
+  return false;
+}
+
+// FP32 mirrors of the node stored at F.f[.][i], into slot k.  The conversions
+// take the integer pipe (the FP64 pipe bounds the callers otherwise) and
+// omega / (omega^2 + 1e-30) is formed in FP32.  full false: only what the
+// neighbour search reads.
+__device__ __forceinline__ void writeMirrors(const Fields& F, long i, const Fields32& P, long k, uint32_t cell,
+                                             const Grid& g, bool full) {
+  int c[3];
+  unpackCell(cell, c);
+  const double ox = g.lo[0] + smallIntToDouble(c[0]) * g.cell[0];
+  const double oy = g.lo[1] + smallIntToDouble(c[1]) * g.cell[1];
+  const double oz = g.lo[2] + smallIntToDouble(c[2]) * g.cell[2];
+  P.posh[k] = make_float4(toFloatRN(F.f[F_X][i] - ox), toFloatRN(F.f[F_Y][i] - oy), toFloatRN(F.f[F_Z][i] - oz),
+                          toFloatRN(F.f[F_HINV][i]));
+  if (P.hten) writeTensorMirror(F, i, P, k);
+  if (!full) return;
+  P.velm[k] = make_float4(toFloatRN(F.f[F_VX][i]), toFloatRN(F.f[F_VY][i]), toFloatRN(F.f[F_VZ][i]),
+                          toFloatRN(F.f[F_MASS][i]));
+  const float om = toFloatRN(F.f[F_OMEGA][i]);
+  P.thermo[k] = make_float4(toFloatRN(F.f[F_RHO][i]), toFloatRN(F.f[F_P][i]), toFloatRN(F.f[F_CS][i]),
+                            om / (om * om + 1.0e-30f));
+  if (P.vol) P.vol[k] = toFloatRN(F.f[F_VOL][i]);
+}
+
 // FP32 separation r_i - r_j' on cell-relative coordinates: r = (x_i - x_j')
 // - d cell per axis, with x_j' = cell - x_j for a mirror image.  Periodic
 // images need no box arithmetic: the cell offset d carries the wrap.
@@ -136,31 +280,30 @@ __device__ __forceinline__ void relSep(const float4& pi, const float4& pj, int d
   rz = __fadd_rn(__fsub_rn(pi.z, zj), oz);
 }
 
-// The cell offset (ox, oy, oz) of each of the 64 cell-offset codes of a
-// neighbour entry, staged once per block: relSepTab then reads it with one
-// shared load instead of decoding the code per pair.
-__device__ __forceinline__ void fillCellOffsets(float4* sOff, float cx, float cy, float cz) {
-  for (int t = threadIdx.x; t < 64; t += blockDim.x) {
-    const int d0 = t & 3, d1 = (t >> 2) & 3, d2 = (t >> 4) & 3;
-    sOff[t] = make_float4(d0 == 1 ? cx : (d0 == 2 ? -cx : 0.0f), d1 == 1 ? cy : (d1 == 2 ? -cy : 0.0f),
-                          d2 == 1 ? cz : (d2 == 2 ? -cz : 0.0f), 0.0f);
-  }
+// relSep from a list entry (bitwise the same result), the cell offset per axis
+// (0, +c, -c for codes 0, 1, 2) by integer selection: the sweeps are bound by
+// shared-memory / L1 wavefronts (~11 per 16-byte gather), so a table of the
+// offsets in shared memory costs more than these instructions.
+// MIR false: no wall of the grid reflects, so no entry is a mirror image.
+__device__ __forceinline__ float cellOffset(uint32_t ent, int axis, float c) {
+  const uint32_t f = (ent >> (kIndexBits + 2 * axis)) & 3u;
+  return __uint_as_float((f ? __float_as_uint(c) : 0u) ^ ((f & 2u) << 30));
 }
-// relSep with the offsets from the staged table (bitwise the same result).
-__device__ __forceinline__ void relSepTab(const float4& pi, const float4& pj, int dcode, uint32_t mm, float cx,
-                                          float cy, float cz, const float4* __restrict__ sOff, float& rx, float& ry,
-                                          float& rz) {
+template <bool MIR = true>
+__device__ __forceinline__ void relSepEntry(const float4& pi, const float4& pj, uint32_t ent, uint32_t mm, float cx,
+                                            float cy, float cz, float& rx, float& ry, float& rz) {
   float xj = pj.x, yj = pj.y, zj = pj.z;
-  const uint32_t mir = (uint32_t)dcode & mm;
-  if (mir) {
-    if (mir & 3u) xj = cx - xj;
-    if (mir & 12u) yj = cy - yj;
-    if (mir & 48u) zj = cz - zj;
+  if (MIR) {
+    const uint32_t mir = (ent >> kIndexBits) & mm;
+    if (mir) {
+      if (mir & 3u) xj = cx - xj;
+      if (mir & 12u) yj = cy - yj;
+      if (mir & 48u) zj = cz - zj;
+    }
   }
-  const float4 o = sOff[dcode];
-  rx = __fadd_rn(__fsub_rn(pi.x, xj), o.x);
-  ry = __fadd_rn(__fsub_rn(pi.y, yj), o.y);
-  rz = __fadd_rn(__fsub_rn(pi.z, zj), o.z);
+  rx = __fadd_rn(__fsub_rn(pi.x, xj), cellOffset(ent, 0, cx));
+  ry = __fadd_rn(__fsub_rn(pi.y, yj), cellOffset(ent, 1, cy));
+  rz = __fadd_rn(__fsub_rn(pi.z, zj), cellOffset(ent, 2, cz));
 }
 
 __device__ __forceinline__ void imagePos(const Grid& g, int code, double& x, double& y, double& z) {
@@ -495,6 +638,102 @@ __device__ __forceinline__ void finalizeNode32(Fields& F, long i, int li, const 
   const float s = fminf(4.0f, fmaxf(0.25f, nPerh / (cur + 1.0e-30f)));
   const float aa = s < 1.0f ? 0.4f * (1.0f + s * s) : 0.4f * (1.0f + 1.0f / (s * s * s));
   const double hid = (double)(ai / (1.0f - aa + aa * s));
+  F.f[F_HIDEAL][i] = fmin(L.hminInv, fmax(L.hmaxInv, hid));
+}
+
+// Node completion of the isotropic mixed pair loop: finalizeNode32 in terms
+// of the loop's reduced sums.  The FP32 results go into the FP64 fields by
+// integer conversions (the FP64 pipe is ~1/64 of the FP32 rate).
+struct PairSums32 {
+  float w, mw, ve, g0, m1x, m1y, m1z;      // sum w, m w, (V/2) e w, |g|, |g| r
+  float D[9], M[6], gx, gy, gz, maxE;      // sum u v r^T, u r r^T (xx xy xz yy yz zz), u (rho_j - rho_i) r; max e
+  float xw, xdx, xdy, xdz;                 // XSPH
+  double dvx, dvy, dvz, deps;
+};
+// SPLINE: the sums carry W/A and W'/A of the cubic B-spline (the energy rate
+// one factor of A already).
+template <bool SPLINE>
+__device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSums32& a, float ai, float mi,
+                                               float rhoi, int numNb, const HydroParams& hp,
+                                               const double* __restrict__ herm) {
+  auto put = [&](int f, float v) { F.f[f][i] = toDouble(v); };
+  const float Hdeti = (ai * ai) * ai, W0 = (float)hp.W0;
+  const float irho = 1.0f / rhoi;
+  if (SPLINE) {
+    a.w = timesSplineA(a.w); a.mw = timesSplineA(a.mw); a.g0 = timesSplineA(a.g0);
+    a.m1x = timesSplineA(a.m1x); a.m1y = timesSplineA(a.m1y); a.m1z = timesSplineA(a.m1z);
+  }
+  put(F_RHOSUM, Hdeti * (a.mw + mi * W0));
+  put(F_NORM, mi * irho * Hdeti * (a.w + W0));
+  // gradW_i = a_i^4 g_i r / |r|: the sums carry g_i r / |r|
+  const float f = SPLINE ? -timesSplineA(Hdeti * ai) : -(Hdeti * ai);
+  float D[9], Mm[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) D[k] = f * a.D[k];
+  Mm[0] = f * a.M[0]; Mm[1] = f * a.M[1]; Mm[2] = f * a.M[2];
+  Mm[3] = Mm[1];      Mm[4] = f * a.M[3]; Mm[5] = f * a.M[4];
+  Mm[6] = Mm[2];      Mm[7] = Mm[5];      Mm[8] = f * a.M[5];
+  const float detM = (Mm[0] * Mm[4] * Mm[8] + Mm[1] * Mm[5] * Mm[6] + Mm[2] * Mm[3] * Mm[7] -
+                      Mm[0] * Mm[5] * Mm[7] - Mm[1] * Mm[3] * Mm[8] - Mm[2] * Mm[4] * Mm[6]);
+  if (hp.correctVelGrad && fabsf(detM) > 1.0e-10f && numNb > 8) {
+    const float id = 1.0f / detM;
+    const float inv[9] = {(Mm[4] * Mm[8] - Mm[5] * Mm[7]) * id, (Mm[2] * Mm[7] - Mm[1] * Mm[8]) * id,
+                          (Mm[1] * Mm[5] - Mm[2] * Mm[4]) * id, (Mm[5] * Mm[6] - Mm[3] * Mm[8]) * id,
+                          (Mm[0] * Mm[8] - Mm[2] * Mm[6]) * id, (Mm[2] * Mm[3] - Mm[0] * Mm[5]) * id,
+                          (Mm[3] * Mm[7] - Mm[4] * Mm[6]) * id, (Mm[1] * Mm[6] - Mm[0] * Mm[7]) * id,
+                          (Mm[0] * Mm[4] - Mm[1] * Mm[3]) * id};
+    float R[9];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        R[3 * r + c] = D[3 * r] * inv[c] + D[3 * r + 1] * inv[3 + c] + D[3 * r + 2] * inv[6 + c];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) { D[k] = R[k]; Mm[k] = inv[k]; }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) D[k] *= irho;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { put(F_DVDX_XX + k, D[k]); put(F_M_XX + k, Mm[k]); }
+  const float fr = -f * irho;
+  put(F_GRADRHO_X, fr * a.gx); put(F_GRADRHO_Y, fr * a.gy); put(F_GRADRHO_Z, fr * a.gz);
+  const float trace = D[0] + D[4] + D[8];
+  put(F_DRHODT, -rhoi * trace);
+  const double vxi = F.f[F_VX][i], vyi = F.f[F_VY][i], vzi = F.f[F_VZ][i];
+  F.f[F_DVDT_X][i] = a.dvx;
+  F.f[F_DVDT_Y][i] = a.dvy;
+  F.f[F_DVDT_Z][i] = a.dvz;
+  const double deps = a.deps * toDouble(Hdeti * ai);
+  F.f[F_DEPSDT][i] =
+      hp.totalEnergy ? toDouble(mi) * ((vxi * a.dvx + vyi * a.dvy + vzi * a.dvz) + deps) : deps;
+  put(F_MAXQ, rhoi * a.maxE);
+  put(F_EFFQ, 2.0f * rhoi * Hdeti * a.ve);
+  float xw = a.xw;
+  if (hp.xsph) {
+    xw += Hdeti * mi * irho * W0;
+    const float ws = fmaxf(1.0e-30f, xw);
+    F.f[F_DXDT_X][i] = vxi + toDouble(a.xdx / ws);
+    F.f[F_DXDT_Y][i] = vyi + toDouble(a.xdy / ws);
+    F.f[F_DXDT_Z][i] = vzi + toDouble(a.xdz / ws);
+  } else {
+    F.f[F_DXDT_X][i] = vxi;
+    F.f[F_DXDT_Y][i] = vyi;
+    F.f[F_DXDT_Z][i] = vzi;
+  }
+  put(F_XSPHW, xw);
+  put(F_XSPHDV_X, a.xdx); put(F_XSPHDV_Y, a.xdy); put(F_XSPHDV_Z, a.xdz);
+  const NodeListParams L = hp.lists[li];
+  const float m0 = cbrtf(fmaxf(0.0f, a.g0));
+  put(F_M0, m0);
+  put(F_M1_X, -ai * a.m1x); put(F_M1_Y, -ai * a.m1y); put(F_M1_Z, -ai * a.m1z);
+  put(F_DHDT, -(ai * (1.0f / 3.0f)) * trace);
+  const float nPerh = (float)L.nPerh;
+  const bool iso = fabsf(m0) <= 1.0e-15f * fmaxf(1.0f, fabsf(m0));
+  const float cur = iso ? 0.5f * nPerh : fmaxf(0.0f, hermiteLookup32(herm, hp, m0));
+  const float s = fminf(4.0f, fmaxf(0.25f, nPerh / (cur + 1.0e-30f)));
+  const float aa = s < 1.0f ? 0.4f * (1.0f + s * s) : 0.4f * (1.0f + 1.0f / (s * s * s));
+  const double hid = toDouble(ai / (1.0f - aa + aa * s));
   F.f[F_HIDEAL][i] = fmin(L.hminInv, fmax(L.hmaxInv, hid));
 }
 

@@ -64,8 +64,10 @@ struct Fields32 {
   float4* posh;     // (x - cell origin, y - ..., z - ..., hinv)
   float4* velm;     // (vx, vy, vz, m)
   float4* thermo;   // (rho, P/rho^2 * Omega^-1, cs, unused)
+  float4* pk;       // isotropic SPH pair loop: (rho, Omega^-1 P / rho^2, -Cl c, 1 / (2 rho))
   uint32_t* cell;   // packed cell coordinates (10 bits per axis)
-  float4* dvq;      // limited Q: DvDx of the Q as 3 float4 per node (xx xy xz yx | yy yz zx zy | zz - - -)
+  float4* dvq;      // limited Q: DvDx of the Q as 3 float4 per node (xx xy xz yx | yy yz zx zy | zz - - -);
+                    // isotropic SPH: its symmetric part, 2 per node (xx yy zz xy | xz yz - -)
   float4* hten;     // ASPH: tensor H as 2 float4 per node (xx xy xz yy | yz zz det(H) lambda_max)
   float* vol;       // CRKSPH: RK volume
   float4* rkc;      // CRKSPH: LinearOrder corrections, 4 float4 per node (C | dC/dx | dC/dy | dC/dz)

@@ -208,10 +208,10 @@ __global__ void boxFinalKernel(const double* __restrict__ part, int nb, double o
 }
 
 //------------------------------------------------------------------------------
-// Morton keys of the level-20 cell coordinates; sort by (hi 30, lo 30) bits.
+// Morton keys of the level-20 cell coordinates (60 bits).
 //------------------------------------------------------------------------------
 __global__ void treeKeyKernel(Fields F, long n, const double* __restrict__ box, uint64_t* __restrict__ key64,
-                              uint32_t* __restrict__ lo, int* __restrict__ vals) {
+                              int* __restrict__ vals) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double L = box[3];
@@ -223,25 +223,16 @@ __global__ void treeKeyKernel(Fields F, long n, const double* __restrict__ box, 
     key = spread3(ix) | (spread3(iy) << 1) | (spread3(iz) << 2);
   }
   key64[i] = key;
-  lo[i] = (uint32_t)(key & 0x3FFFFFFFull);
   vals[i] = (int)i;
 }
 
-__global__ void gatherHiKernel(const uint64_t* __restrict__ key64, const int* __restrict__ vals, long n,
-                               uint32_t* __restrict__ hi) {
-  const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  hi[k] = (uint32_t)(key64[vals[k]] >> 30);
-}
-
-// Tree-ordered node data and the shared-level count cpl(k).
-__global__ void treeNodesKernel(Fields F, const uint64_t* __restrict__ key64, const int* __restrict__ vals, long n,
-                                uint64_t* __restrict__ skey, TreeNode* __restrict__ tpos,
+// Tree-ordered node data.  Indices of a sort that gave up waiting stay in
+// range; the evaluation then fails on the sort's flag.
+__global__ void treeNodesKernel(Fields F, const int* __restrict__ vals, long n, TreeNode* __restrict__ tpos,
                                 TreeNode32* __restrict__ tpos32) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const int i = vals[k];
-  skey[k] = key64[i];
+  const int i = (int)min((unsigned)vals[k], (unsigned)(n - 1));
   const double x = F.f[F_X][i], y = F.f[F_Y][i], z = F.f[F_Z][i], m = F.f[F_MASS][i];
   tpos[k] = TreeNode{x, y, z, m};
   if (tpos32) {
@@ -632,7 +623,7 @@ __global__ void zeroGravityKernel(Fields F, long n, double G, double* __restrict
 }  // namespace
 
 struct GravityWork {
-  GBuf part, box, thr, dtBits, key64, lo, lo2, vals, vals2, sortWs, skey, tpos, nc, off, scanWs, total, cells, mx,
+  GBuf part, box, thr, dtBits, key64, timeout, vals, vals2, sortWs, skey, tpos, nc, off, scanWs, total, cells, mx,
       energy, tpos32, cells32;
   long long* hTotal = nullptr;
   long long lastCells = 0;
@@ -640,13 +631,13 @@ struct GravityWork {
 
 GravityWork* gravityCreate() {
   GravityWork* w = new GravityWork();
-  if (cudaMallocHost(&w->hTotal, sizeof(long long)) != cudaSuccess) w->hTotal = nullptr;
+  if (cudaMallocHost(&w->hTotal, 2 * sizeof(long long)) != cudaSuccess) w->hTotal = nullptr;
   return w;
 }
 
 void gravityDestroy(GravityWork* w) {
   if (!w) return;
-  GBuf* all[] = {&w->part, &w->box, &w->thr, &w->dtBits, &w->key64, &w->lo, &w->lo2, &w->vals, &w->vals2,
+  GBuf* all[] = {&w->part, &w->box, &w->thr, &w->dtBits, &w->key64, &w->timeout, &w->vals, &w->vals2,
                  &w->sortWs, &w->skey, &w->tpos, &w->nc, &w->off, &w->scanWs, &w->total, &w->cells, &w->mx,
                  &w->energy, &w->tpos32, &w->cells32};
   for (GBuf* b : all) b->release();
@@ -685,8 +676,7 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   GCHK(w->dtBits.ensure(sizeof(unsigned long long)));
   GCHK(w->key64.ensure(n * sizeof(uint64_t)));
   GCHK(w->skey.ensure(n * sizeof(uint64_t)));
-  GCHK(w->lo.ensure(n * sizeof(uint32_t)));
-  GCHK(w->lo2.ensure(n * sizeof(uint32_t)));
+  GCHK(w->timeout.ensure(sizeof(int)));
   GCHK(w->vals.ensure(n * sizeof(int)));
   GCHK(w->vals2.ensure(n * sizeof(int)));
   GCHK(w->sortWs.ensure(radixSortWorkspaceBytes(n)));
@@ -703,25 +693,27 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   boxFinalKernel<<<1, 32, 0, s>>>(w->part.as<double>(), nbBox, opening, w->box.as<double>(), w->thr.as<double>(),
                                  w->dtBits.as<unsigned long long>());
   treeKeyKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, n, w->box.as<double>(), w->key64.as<uint64_t>(),
-                                                           w->lo.as<uint32_t>(), w->vals.as<int>());
+                                                           w->vals.as<int>());
   lc->add(3);
-  uint32_t* keys = w->lo.as<uint32_t>();
-  uint32_t* keysAlt = w->lo2.as<uint32_t>();
+  uint64_t* skey = w->key64.as<uint64_t>();
+  uint64_t* skeyAlt = w->skey.as<uint64_t>();
   int* vals = w->vals.as<int>();
   int* valsAlt = w->vals2.as<int>();
-  radixSortPairs(keys, vals, keysAlt, valsAlt, n, 30, w->sortWs.p, s, lc);
-  gatherHiKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(w->key64.as<uint64_t>(), vals, n, keys);
-  lc->add(1);
-  radixSortPairs(keys, vals, keysAlt, valsAlt, n, 30, w->sortWs.p, s, lc);
-  treeNodesKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, w->key64.as<uint64_t>(), vals, n,
-                                                             w->skey.as<uint64_t>(), w->tpos.as<TreeNode>(),
+  GCHK(cudaMemsetAsync(w->timeout.p, 0, sizeof(int), s));
+  radixSortPairs(skey, vals, skeyAlt, valsAlt, n, 3 * kMaxLevel, w->sortWs.p, w->timeout.as<int>(), s, lc);
+  treeNodesKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, vals, n, w->tpos.as<TreeNode>(),
                                                              mixed ? w->tpos32.as<TreeNode32>() : nullptr);
-  chainCountKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(w->skey.as<uint64_t>(), n, w->nc.as<int>());
+  chainCountKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(skey, n, w->nc.as<int>());
   lc->add(2);
   scanExclusive<int>(w->nc.as<int>(), w->off.as<long long>(), n, w->scanWs.p, w->total.as<long long>(), s, lc);
   GCHK(cudaMemcpyAsync(w->hTotal, w->total.p, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  GCHK(cudaMemcpyAsync(w->hTotal + 1, w->timeout.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   GCHK(cudaStreamSynchronize(s));
   const long long numCells = *w->hTotal;
+  if (*reinterpret_cast<const int*>(w->hTotal + 1)) {
+    std::snprintf(err, errlen, "a wait inside the octree sort ran out");
+    return SPHGPU_E_TIMEOUT;
+  }
   if (numCells <= 0 || numCells > 0x7FFFFFFFll) {
     std::snprintf(err, errlen, "octree cell count %lld out of range", numCells);
     return SPHGPU_E_OVERFLOW;
@@ -730,12 +722,12 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   GCHK(w->cells.ensure(numCells * sizeof(TreeCell)));
   GCHK(w->mx.ensure(numCells * 3 * sizeof(double)));
   TreeCell* cells = w->cells.as<TreeCell>();
-  cellBuildKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(w->skey.as<uint64_t>(), n, w->off.as<long long>(),
+  cellBuildKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(skey, n, w->off.as<long long>(),
                                                              numCells, cells);
   lc->add(1);
   const int nbCells = (int)((numCells + kThreads - 1) / kThreads);
   for (int l = kMaxLevel; l >= 0; --l) {
-    momentKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, l, w->tpos.as<TreeNode>(), w->skey.as<uint64_t>(),
+    momentKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, l, w->tpos.as<TreeNode>(), skey,
                                               w->box.as<double>(), w->mx.as<double>());
   }
   lc->add(kMaxLevel + 1);

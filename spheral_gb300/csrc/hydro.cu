@@ -12,6 +12,8 @@
 // entry carries a 6-bit image code and the neighbour's coordinates are mapped
 // with the reference's own plane formula (imageCoord).
 #include "device.cuh"
+#include <algorithm>
+#include <climits>
 
 namespace sph {
 namespace {
@@ -61,8 +63,9 @@ __global__ void boundsFinalKernel(const double* __restrict__ part, int nb, doubl
 // Neighbour build.
 //------------------------------------------------------------------------------
 __global__ void cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ keys, int* __restrict__ vals,
-                              uint32_t* __restrict__ cellc) {
+                              uint32_t* __restrict__ cellc, StepScratch* __restrict__ sc) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i == 0) resetScratch(sc);
   if (i >= n) return;
   const double p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
   uint32_t c[3], f[3];
@@ -86,33 +89,36 @@ __global__ void cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ k
   // top bits are the cell's Morton key: nodes stay grouped by cell and within
   // a cell they are ordered by octant, so consecutive nodes of a cell (a work
   // chunk or a candidate batch of the neighbour search) sit close together.
-  keys[i] = g.subShift ? morton3(f[0], f[1], f[2]) : morton3(c[0], c[1], c[2]);
+  keys[i] = g.subShift ? cellKey(g, f[0], f[1], f[2], 1) : cellKey(g, c[0], c[1], c[2], 0);
   vals[i] = (int)i;
   cellc[i] = c[0] | (c[1] << 10) | (c[2] << 20);
 }
 
+// Gather of the carried fields into the new order, with what the same pass can
+// take along: the cells' node ranges (from the sorted keys) and the FP32
+// mirrors of the new order.  Indices and keys of a sort that gave up waiting
+// stay in range; the step then fails on the sort's flag.
 __global__ void permuteKernel(Fields Fin, Fields Fout, const int* __restrict__ perm, const int* __restrict__ origIn,
                               int* __restrict__ origOut, const int* __restrict__ listIn, int* __restrict__ listOut,
                               const uint32_t* __restrict__ cellIn, uint32_t* __restrict__ cellOut, long n,
-                              FieldRanges sel) {
+                              FieldRanges sel, Fields32 P, Grid g, int mirrors, const uint32_t* __restrict__ keys,
+                              uint32_t space, int* __restrict__ cellStart, int* __restrict__ cellEnd) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const int p = perm[k];
+  const int p = (int)min((unsigned)perm[k], (unsigned)(n - 1));
   for (int r = 0; r < sel.n; ++r)
 #pragma unroll 4
     for (int f = sel.first[r]; f < sel.last[r]; ++f) Fout.f[f][k] = Fin.f[f][p];
   origOut[k] = origIn[p];
   listOut[k] = listIn[p];
-  cellOut[k] = cellIn[p];
-}
-
-__global__ void cellRangeKernel(const uint32_t* __restrict__ keys, long n, int shift, int* __restrict__ cellStart,
-                                int* __restrict__ cellEnd) {
-  const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const uint32_t key = keys[k] >> shift;
-  if (k == 0 || (keys[k - 1] >> shift) != key) cellStart[key] = (int)k;
-  if (k == n - 1 || (keys[k + 1] >> shift) != key) cellEnd[key] = (int)(k + 1);
+  const uint32_t cell = cellIn[p];
+  cellOut[k] = cell;
+  const uint32_t key = keys[k] >> g.subShift;
+  if (key < space) {
+    if (k == 0 || (keys[k - 1] >> g.subShift) != key) cellStart[key] = (int)k;
+    if (k == n - 1 || (keys[k + 1] >> g.subShift) != key) cellEnd[key] = (int)(k + 1);
+  }
+  writeMirrors(Fin, p, P, k, cell, g, mirrors != 0);
 }
 
 // Pair criterion of ConnectivityMap::computeConnectivity
@@ -173,8 +179,7 @@ __global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, 
                                                           int nItems, Grid g, const int* __restrict__ cellStart,
                                                           const int* __restrict__ cellEnd, int* __restrict__ counts,
                                                           uint32_t* __restrict__ nbr, double ext2, float bandA,
-                                                          float bandB, int cap, int* __restrict__ maxCount,
-                                                          const long long* __restrict__ dItems,
+                                                          float bandB, int cap, StepScratch* __restrict__ sc,
                                                           const float4* __restrict__ box,
                                                           const int* __restrict__ chunkOf) {
   constexpr int G = 128 / W;             // groups per 128-thread block
@@ -193,7 +198,7 @@ __global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, 
   // lanes of this group within the warp
   const unsigned gmask = (W == 32) ? 0xffffffffu : (((1u << W) - 1u) << ((threadIdx.x & 31) / W * W));
   // the grid is sized for an upper bound; the item count itself is on the device
-  if (item >= min((long long)nItems, *dItems)) return;   // group-uniform
+  if (item >= min(nItems, sc->items)) return;   // group-uniform
   const int k0 = items[item];
   const uint32_t cc = P.cell[k0];
   int hc[3];
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, 
                       ((d2 == 0 ? 1 : (d2 == 2 ? 2 : 0)) << 4);
     int4 r = make_int4(0, 0, 0, dcode);
     if (ok) {
-      const uint32_t key = morton3((uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2]);
+      const uint32_t key = cellKey(g, (uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2], 0);
       r.x = cellStart[key];
       r.y = cellEnd[key];
       if (r.x < r.y) r.z = chunkOf[r.x];
@@ -497,51 +502,415 @@ __global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, 
   if (active) counts[i] = WRITE ? min(cnt, cap) : cnt;
   // one atomic per group: a per-node atomic on a single address serialises
   const int gmax = __reduce_max_sync(gmask, active ? cnt : 0);
-  if (lane == 0) atomicMax(maxCount, gmax);
+  const int gsum = __reduce_add_sync(gmask, active ? cnt : 0);
+  if (lane == 0) {
+    if (gmax > *(volatile int*)&sc->maxCount) atomicMax(&sc->maxCount, gmax);
+    atomicAdd(&sc->entries[blockIdx.x & (kEntrySums - 1)], (unsigned long long)gsum);
+  }
 }
 
-// Items of the warp search: the first node of every chunk of up to 32 nodes
-// of a cell.  flag pass + scan + fill.
-__global__ void itemFlagKernel(const uint32_t* __restrict__ keys, long n, int shift,
-                               const int* __restrict__ cellStart, int width, int* __restrict__ flag) {
-  const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  flag[k] = ((k - cellStart[keys[k] >> shift]) % width == 0) ? 1 : 0;
+//------------------------------------------------------------------------------
+// Isotropic search.  A warp (CW = 1) or the block's four warps (CW = 4) own one
+// work item: up to 32 consecutive nodes of a cell, one per lane.
+//
+//  1. The chunks of the 27 candidate cells (in cell order, up to kTile at a
+//     time) are listed and culled lane-parallel: a chunk whose bounding box is
+//     farther from the item's box than the item's largest FP32 band edge
+//     allows holds no neighbour of any lane.
+//  2. Each surviving chunk (a batch of up to 32 candidates) is staged and
+//     tested two candidates per packed FP32 operation; the lane's hits up to
+//     the top of its guard band form a 32-bit mask.  A lane whose largest hit
+//     lies inside the band forms the mask of that batch again with the exact
+//     FP64 criterion.  (CW = 4: the warps take the batches in turn.)
+//  3. The masks are written out as list entries, the q-th hit of every lane in
+//     the same iteration, so a row of the warp-interleaved list is one 128-byte
+//     store.  (CW = 4: the warps take a quarter of the batches each.)
+//
+// Every list is in candidate order, whatever the item width and CW.
+//
+// What bounds it: instruction issue.  Testing and storing candidate by
+// candidate took ~36 warp instructions per candidate of a group (predicated
+// store, list pointer, counter and band flag per candidate); the masks take
+// ~9 for the test and ~3 for the writing.
+//------------------------------------------------------------------------------
+constexpr int kTile = 32;   // batches listed at a time
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-// Bounding box of every work chunk (up to `width` consecutive nodes of one
-// cell) in its cell's FP32 coordinates, with the smallest and largest h^-1:
-// box[2k] = (min x, min y, min z, min a), box[2k+1] = (max x, max y, max z,
-// max a).  chunkOf[first node of the chunk] = k.
-__global__ void itemBoxKernel(const int* __restrict__ items, const long long* __restrict__ dItems, long n,
-                              int width, Fields32 P, float4* __restrict__ box, int* __restrict__ chunkOf) {
-  const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= *dItems) return;
-  const int s = items[k];
-  const uint32_t cell = P.cell[s];
-  float4 lo = P.posh[s], hi = lo;
-  for (int j = s + 1; j < s + width && j < n && P.cell[j] == cell; ++j) {
-    const float4 q = P.posh[j];
-    lo = make_float4(fminf(lo.x, q.x), fminf(lo.y, q.y), fminf(lo.z, q.z), fminf(lo.w, q.w));
-    hi = make_float4(fmaxf(hi.x, q.x), fmaxf(hi.y, q.y), fmaxf(hi.z, q.z), fmaxf(hi.w, q.w));
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// min(a, |b|, |c|) for a >= 0
+__device__ __forceinline__ float minAbs3(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// The 27 candidate cells of home cell hc, one per lane (lanes 0..26): node
+// range, first work chunk, offset code and offset.
+struct CandidateCell {
+  int start, end, chunk, dcode;
+  float ox, oy, oz;
+};
+__device__ __forceinline__ CandidateCell candidateCell(int t, const int* hc, const Grid& g,
+                                                       const int* __restrict__ cellStart,
+                                                       const int* __restrict__ cellEnd,
+                                                       const int* __restrict__ chunkOf) {
+  CandidateCell r{0, 0, 0, 0, 0.f, 0.f, 0.f};
+  const int d[3] = {t % 3, (t / 3) % 3, t / 9};   // 0, 1, 2 for -1, 0, +1
+  int cell[3];
+  bool ok = t < 27;
+  float o[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    int nn = hc[a] + d[a] - 1;
+    if (nn < 0) {
+      if (g.kindLo[a] == AXIS_PERIODIC) nn = g.nc[a] - 1;
+      else if (g.kindLo[a] == AXIS_REFLECT) nn = 0;
+      else ok = false;
+    } else if (nn >= g.nc[a]) {
+      if (g.kindHi[a] == AXIS_PERIODIC) nn = 0;
+      else if (g.kindHi[a] == AXIS_REFLECT) nn = g.nc[a] - 1;
+      else ok = false;
+    }
+    cell[a] = nn;
+    r.dcode |= (d[a] == 0 ? 1 : (d[a] == 2 ? 2 : 0)) << (2 * a);
+    o[a] = d[a] == 0 ? g.cellf[a] : (d[a] == 2 ? -g.cellf[a] : 0.0f);
   }
-  box[2 * k] = lo;
-  box[2 * k + 1] = hi;
-  chunkOf[s] = (int)k;
+  r.ox = o[0]; r.oy = o[1]; r.oz = o[2];
+  if (ok) {
+    const uint32_t key = cellKey(g, (uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2], 0);
+    r.start = cellStart[key];
+    r.end = cellEnd[key];
+    if (r.start < r.end) r.chunk = chunkOf[r.start];
+  }
+  return r;
 }
-__global__ void itemFillKernel(const int* __restrict__ flag, const long long* __restrict__ pos, long n,
-                               int* __restrict__ items) {
+
+template <bool WRITE, int CW>
+__global__ void __launch_bounds__(128, 6) neighborMaskKernel(Fields F, Fields32 P, const int* __restrict__ items,
+                                                          int nItems, int width, Grid g,
+                                                          const int* __restrict__ cellStart,
+                                                          const int* __restrict__ cellEnd, int* __restrict__ counts,
+                                                          uint32_t* __restrict__ nbr, double ext2, float bandA,
+                                                          float bandB, int cap, StepScratch* __restrict__ sc,
+                                                          const float4* __restrict__ box,
+                                                          const int* __restrict__ chunkOf) {
+  constexpr int G = 4 / CW;                          // items per block
+  __shared__ __align__(16) float stage[4][4][32];    // per warp: -x, -y, -z, (h^-1)^2 of a batch
+  __shared__ int2 desc[G][kTile];                    // kept batches: entry of the first node, size
+  __shared__ float4 offs[G][kTile];                  // and the cell offset
+  __shared__ uint32_t masks[G][kTile][32];
+  __shared__ int part[CW == 4 ? 4 : 1][32];          // CW = 4: hits per lane of each warp's batches
+  __shared__ int keptCount[G];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = CW == 4 ? 0 : warp, sub = CW == 4 ? warp : 0;
+  const int item = blockIdx.x * G + grp;
+  if (item >= min(nItems, sc->items)) return;   // uniform over the item's warps
+  auto groupSync = [] {
+    if (CW == 4) __syncthreads();
+    else __syncwarp();
+  };
+  const int k0 = items[item];
+  int hc[3];
+  unpackCell(P.cell[k0], hc);
+  const CandidateCell cc = candidateCell(lane, hc, g, cellStart, cellEnd, chunkOf);
+  const int k1 = min(k0 + width, __shfl_sync(0xffffffffu, cc.end, 13));   // cell 13 is the home cell
+  const long i = k0 + lane;
+  const bool active = i < k1;
+  const float4 pi = active ? P.posh[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float ai2 = pi.w * pi.w;
+  const float del = __fmaf_rn(bandA, pi.w, bandB);   // per-node band half-width (relative)
+  const float e2t = g.ext2f;
+  const float bandLo = del < 0.5f ? e2t * (1.0f - del) : -1.0f;
+  const float bandHi = del < 0.5f ? e2t * (1.0f + del) : FLT_MAX;
+  // a candidate whose e2 is farther than this from bandHi is outside the band
+  // on one side or the other (with room for the rounding of the difference)
+  const float bandGap = del < 0.5f ? 1.01f * (bandHi - bandLo) + 4.0e-7f * bandHi : FLT_MAX;
+  const f32x2 nhi2 = pack2(-bandHi, -bandHi);
+  const uint32_t mm = mirrorMask(g, hc);
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
+  const float4 gLo = box[2 * item], gHi = box[2 * item + 1];
+  const float delMax = __fmaf_rn(bandA, gHi.w, bandB);
+  const bool cull = delMax < 0.5f;
+  const float cullThr = e2t * (1.0f + delMax) * 1.0001f;
+  // batches of each candidate cell, and how many come before them
+  const int nb = (cc.end - cc.start + width - 1) / width;
+  int before = nb;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += y;
+  }
+  const int batches = __shfl_sync(0xffffffffu, before, 31);
+  before -= nb;
+
+  int cnt = 0;   // this lane's hits so far
+  for (int tile = 0; tile < batches; tile += kTile) {
+    const int inTile = min(kTile, batches - tile);
+    if (sub == 0) {
+      // list and cull the tile's batches, one per lane
+      {
+        const int b = tile + lane;
+        // the cell of batch b: the last one that starts at or before it
+        int t = 0;
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1) {
+          const int c = __shfl_sync(0xffffffffu, before, min(t + st, 26));
+          if (t + st <= 26 && c <= b) t += st;
+        }
+        const int cs = __shfl_sync(0xffffffffu, cc.start, t), ce = __shfl_sync(0xffffffffu, cc.end, t);
+        const int cb = b - __shfl_sync(0xffffffffu, before, t);
+        const int chunk = __shfl_sync(0xffffffffu, cc.chunk, t) + cb;
+        const int dcode = __shfl_sync(0xffffffffu, cc.dcode, t);
+        const float ox = __shfl_sync(0xffffffffu, cc.ox, t), oy = __shfl_sync(0xffffffffu, cc.oy, t);
+        const float oz = __shfl_sync(0xffffffffu, cc.oz, t);
+        bool keep = lane < inTile;
+        if (keep && cull) {
+          // the batch's box in the frame of the item's cell: a candidate at q
+          // (mirrored where the entry crosses a wall) sits at q - o there
+          const float4 bLo = box[2 * chunk], bHi = box[2 * chunk + 1];
+          const uint32_t mir = (uint32_t)dcode & mm;
+          float lx = bLo.x, hx = bHi.x, ly = bLo.y, hy = bHi.y, lz = bLo.z, hz = bHi.z;
+          if (mir & 3u) { lx = cx - bHi.x; hx = cx - bLo.x; }
+          if (mir & 12u) { ly = cy - bHi.y; hy = cy - bLo.y; }
+          if (mir & 48u) { lz = cz - bHi.z; hz = cz - bLo.z; }
+          const float gx = fmaxf(0.0f, fmaxf((lx - ox) - gHi.x, gLo.x - (hx - ox)));
+          const float gy = fmaxf(0.0f, fmaxf((ly - oy) - gHi.y, gLo.y - (hy - oy)));
+          const float gz = fmaxf(0.0f, fmaxf((lz - oz) - gHi.z, gLo.z - (hz - oz)));
+          const float am = fminf(gLo.w, bLo.w);
+          keep = !((am * am) * (gx * gx + gy * gy + gz * gz) > cullThr);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int first = cs + cb * width;
+          const int at = __popc(m & ((1u << lane) - 1u));
+          desc[grp][at] = make_int2(first | (int)((uint32_t)dcode << kIndexBits), min(width, ce - first));
+          offs[grp][at] = make_float4(ox, oy, oz, 0.0f);
+        }
+        if (lane == 0) keptCount[grp] = __popc(m);
+      }
+    }
+    groupSync();
+    const int kept = keptCount[grp];
+    // masks of this warp's batches (candidates of the next one loaded ahead)
+    // nonempty: the kept batches that hold hits of this lane
+    uint32_t nonempty = 0u;
+    int hits = 0;
+    float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (sub < kept && lane < desc[grp][sub].y) qn = P.posh[(desc[grp][sub].x & kIndexMask) + lane];
+    for (int b = sub; b < kept; b += CW) {
+      const int2 ds = desc[grp][b];
+      const int base = ds.x & kIndexMask, nval = ds.y, dcode = (int)((uint32_t)ds.x >> kIndexBits);
+      float4 q = qn;
+      if (b + CW < kept) {
+        const int2 dn = desc[grp][b + CW];
+        if (lane < dn.y) qn = P.posh[(dn.x & kIndexMask) + lane];
+      }
+      const uint32_t mir = (uint32_t)dcode & mm;
+      if (mir) {
+        if (mir & 3u) q.x = cx - q.x;
+        if (mir & 12u) q.y = cy - q.y;
+        if (mir & 48u) q.z = cz - q.z;
+      }
+      const float4 o = offs[grp][b];
+      // empty slots of the batch hold NaN: every comparison with them is false
+      stage[warp][0][lane] = lane < nval ? -q.x : __int_as_float(0x7fffffff);
+      stage[warp][1][lane] = -q.y;
+      stage[warp][2][lane] = -q.z;
+      stage[warp][3][lane] = q.w * q.w;
+      __syncwarp();
+      const float px = __fadd_rn(pi.x, o.x), py = __fadd_rn(pi.y, o.y), pz = __fadd_rn(pi.z, o.z);
+      const f32x2 px2 = pack2(px, px), py2 = pack2(py, py), pz2 = pack2(pz, pz);
+      // e2 - bandHi: its sign bits, shifted in one by one, are the mask (bit
+      // order reversed), and its smallest magnitude tells whether a candidate
+      // may lie inside the band
+      uint32_t mask = 0u;
+      float near = FLT_MAX;
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) {
+        if (u >= nval) { mask <<= 32 - u; break; }   // uniform
+        const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&stage[warp][0][u]);
+        const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&stage[warp][1][u]);
+        const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&stage[warp][2][u]);
+        const float4 A = *reinterpret_cast<const float4*>(&stage[warp][3][u]);
+        const f32x2 rx0 = add2(px2, X.x), ry0 = add2(py2, Y.x), rz0 = add2(pz2, Z.x);
+        const f32x2 rx1 = add2(px2, X.y), ry1 = add2(py2, Y.y), rz1 = add2(pz2, Z.y);
+        const f32x2 s0 = fma2(fma2(rz0, rz0, fma2(ry0, ry0, mul2(rx0, rx0))), pack2(fminf(ai2, A.x), fminf(ai2, A.y)), nhi2);
+        const f32x2 s1 = fma2(fma2(rz1, rz1, fma2(ry1, ry1, mul2(rx1, rx1))), pack2(fminf(ai2, A.z), fminf(ai2, A.w)), nhi2);
+        float e[4];
+        unpack2(s0, e[0], e[1]);
+        unpack2(s1, e[2], e[3]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) mask = __funnelshift_l(__float_as_uint(e[v]), mask, 1);
+        near = minAbs3(minAbs3(near, e[0], e[1]), e[2], e[3]);
+      }
+      mask = __brev(mask);
+      if (nval < 32) mask &= (1u << nval) - 1u;
+      if (dcode == 0 && base == k0) mask &= ~(1u << lane);   // the item's own batch: candidate `lane` is node i
+      if (active && near <= bandGap) {   // guard band: this lane's mask again, band candidates by the exact FP64 criterion
+        mask = 0u;
+        for (int u = 0; u < nval; ++u) {
+          const float rx = __fadd_rn(px, stage[warp][0][u]), ry = __fadd_rn(py, stage[warp][1][u]),
+                      rz = __fadd_rn(pz, stage[warp][2][u]);
+          const float e2 = fminf(ai2, stage[warp][3][u]) * (rx * rx + ry * ry + rz * rz);
+          if (e2 > bandHi || (dcode == 0 && base + u == i)) continue;
+          bool in = e2 < bandLo;
+          if (!in) {
+            const int j = base + u;
+            double xjd = F.f[F_X][j], yjd = F.f[F_Y][j], zjd = F.f[F_Z][j];
+            imagePos(g, imageCode(g, hc, dcode), xjd, yjd, zjd);
+            const double qx = __dsub_rn(F.f[F_X][i], xjd), qy = __dsub_rn(F.f[F_Y][i], yjd),
+                         qz = __dsub_rn(F.f[F_Z][i], zjd);
+            in = eta2Exact(F.f[F_HINV][i], qx, qy, qz) <= ext2 || eta2Exact(F.f[F_HINV][j], qx, qy, qz) <= ext2;
+          }
+          if (in) mask |= 1u << u;
+        }
+      }
+      if (!active) mask = 0u;
+      masks[grp][b][lane] = mask;
+      if (CW == 1) {
+        if (mask) nonempty |= 1u << b;
+        hits += __popc(mask);
+      }
+      __syncwarp();
+    }
+    groupSync();
+    // entries: the nonempty batches of this warp (CW = 4: of its quarter of the
+    // batches), from the lane's hit `at`
+    int at = cnt;
+    if (CW == 4) {
+      for (int b = sub * kept / 4; b < (sub + 1) * kept / 4; ++b) {
+        const uint32_t m = masks[grp][b][lane];
+        if (m) nonempty |= 1u << b;
+        hits += __popc(m);
+      }
+      part[sub][lane] = hits;
+      __syncthreads();
+      int all = 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        if (w < sub) at += part[w][lane];
+        all += part[w][lane];
+      }
+      cnt += all;
+    } else {
+      cnt += hits;
+    }
+    if (WRITE) {
+      uint32_t* out = nbr + nbSlot(active ? i : k0, 0, cap) + (size_t)at * 32;
+      const int stored = min(hits, cap - at);
+      const int most = __reduce_max_sync(0xffffffffu, stored);
+      uint32_t m = 0u;
+      int first = 0;
+      for (int h = 0; h < most; ++h, out += 32)
+        if (h < stored) {
+          if (m == 0u) {
+            const int b = __ffs(nonempty) - 1;
+            nonempty &= nonempty - 1u;
+            m = masks[grp][b][lane];
+            first = desc[grp][b].x;
+          }
+          *out = (uint32_t)(first + __ffs(m) - 1);
+          m &= m - 1u;
+        }
+    }
+    groupSync();   // the next tile overwrites desc, masks and part
+  }
+  if (sub != 0) return;
+  // The stored count never exceeds the capacity: sweeps that run before an
+  // overflow is noticed read only written slots.  The true maximum goes to
+  // maxCount (the overflow signal).
+  if (active) counts[i] = WRITE ? min(cnt, cap) : cnt;
+  const int gmax = __reduce_max_sync(0xffffffffu, active ? cnt : 0);
+  const int gsum = __reduce_add_sync(0xffffffffu, active ? cnt : 0);
+  if (lane == 0) {
+    if (gmax > *(volatile int*)&sc->maxCount) atomicMax(&sc->maxCount, gmax);
+    atomicAdd(&sc->entries[blockIdx.x & (kEntrySums - 1)], (unsigned long long)gsum);
+  }
+}
+
+// Work items of the search: every chunk of up to `width` consecutive nodes of
+// a cell, in items[], the chunks of one cell consecutive (their order among
+// cells is free); chunkOf[first node of the cell] = its first chunk.
+__global__ void itemsKernel(const uint32_t* __restrict__ keys, long n, int shift, uint32_t space,
+                            const int* __restrict__ cellEnd, int width, int* __restrict__ items,
+                            int* __restrict__ chunkOf, StepScratch* __restrict__ sc) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  if (flag[k]) items[pos[k]] = (int)k;
+  const int lane = threadIdx.x & 31;
+  int chunks = 0, first = 0;
+  if (k < n) {
+    const uint32_t key = keys[k] >> shift;
+    if (key < space && (k == 0 || (keys[k - 1] >> shift) != key)) {
+      chunks = (cellEnd[key] - (int)k + width - 1) / width;
+      first = (int)k;
+    }
+  }
+  int incl = chunks;   // warp prefix: one atomic per warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int base = 0;
+  if (lane == 31 && incl > 0) base = atomicAdd(&sc->items, incl);
+  base = __shfl_sync(0xffffffffu, base, 31) + incl - chunks;
+  if (chunks > 0) chunkOf[first] = base;
+  for (int c = 0; c < chunks; ++c) items[base + c] = first + c * width;
+}
+// Bounding box of every work chunk in its cell's FP32 coordinates, with the
+// smallest and largest h^-1, W lanes per chunk: box[2k] = (min x, min y,
+// min z, min a), box[2k+1] = (max x, max y, max z, max a).
+template <int W>
+__global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ items, const StepScratch* __restrict__ sc,
+                                                     long n, Fields32 P, float4* __restrict__ box) {
+  const int k = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) / W);
+  const int lane = threadIdx.x % W;
+  const bool live = k < sc->items;
+  const int s = live ? items[k] : 0;
+  const long j = (long)s + lane;
+  const bool in = live && j < n && P.cell[j] == P.cell[s];
+  const float4 q = P.posh[in ? j : s];
+  float lo[4] = {q.x, q.y, q.z, q.w}, hi[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+    }
+  if (live && lane == 0) {
+    box[2 * k] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    box[2 * k + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+  }
 }
 
 //------------------------------------------------------------------------------
 // computeSPHSumMassDensity (src/SPH/computeSPHSumMassDensity.cc:15-87),
 // gathered: rho_i = m_i W(0) Hdet_i + sum_j m W(|Hj ri - Hj rj|, Hdet_j) with
-// m = m_j for the same NodeList and m_i otherwise.  TENSOR: H_j a symmetric
-// tensor (ASPH), seen through the image of the entry.
+// m = m_j for the same NodeList and m_i otherwise.  Tensor H_j (ASPH), seen
+// through the image of the entry.
 //------------------------------------------------------------------------------
-template <bool TENSOR>
 __global__ void __launch_bounds__(128) sumDensityKernel(Fields F, const int* __restrict__ list, long n, Grid g,
                                                         NeighborLists nl, TableDev t, HydroParams hp) {
   extern __shared__ double smem[];
@@ -555,11 +924,10 @@ __global__ void __launch_bounds__(128) sumDensityKernel(Fields F, const int* __r
   const double* __restrict__ X = F.f[F_X];
   const double* __restrict__ Y = F.f[F_Y];
   const double* __restrict__ Z = F.f[F_Z];
-  const double* __restrict__ A = F.f[F_HINV];
   const double* __restrict__ Ms = F.f[F_MASS];
-  const double xi = X[i], yi = Y[i], zi = Z[i], ai = A[i], mi = Ms[i];
+  const double xi = X[i], yi = Y[i], zi = Z[i], mi = Ms[i];
   const int li = list[i];
-  const double Hdeti = TENSOR ? symDet(loadSym(F, F_HT_XX, i)) : (ai * ai) * ai;
+  const double Hdeti = symDet(loadSym(F, F_HT_XX, i));
   const double self = mi * (Hdeti * smem[0]);
   double sum = 0.0;
   const int cnt = nl.count[i];
@@ -570,7 +938,7 @@ __global__ void __launch_bounds__(128) sumDensityKernel(Fields F, const int* __r
     double xj = X[j], yj = Y[j], zj = Z[j];
     imagePos(g, code, xj, yj, zj);
     double dx, dy, dz, Hdetj;
-    if (TENSOR) {   // |Hj ri - Hj rj|
+    {   // |Hj ri - Hj rj|
       Sym Hj = loadSym(F, F_HT_XX, j);
       imageSym(g, code, Hj);
       double ax, ay, az, bx, by, bz;
@@ -578,12 +946,6 @@ __global__ void __launch_bounds__(128) sumDensityKernel(Fields F, const int* __r
       symDot(Hj, xj, yj, zj, bx, by, bz);
       dx = ax - bx; dy = ay - by; dz = az - bz;
       Hdetj = symDet(Hj);
-    } else {
-      const double aj = A[j];
-      dx = __dsub_rn(__dmul_rn(aj, xi), __dmul_rn(aj, xj));
-      dy = __dsub_rn(__dmul_rn(aj, yi), __dmul_rn(aj, yj));
-      dz = __dsub_rn(__dmul_rn(aj, zi), __dmul_rn(aj, zj));
-      Hdetj = (aj * aj) * aj;
     }
     const double eta = sqrt(dx * dx + dy * dy + dz * dz);
     if (eta < hp.extent) {
@@ -598,7 +960,6 @@ __global__ void __launch_bounds__(128) sumDensityKernel(Fields F, const int* __r
 //------------------------------------------------------------------------------
 // computeSPHOmegaGradhCorrection (src/SPH/computeSPHOmegaGradhCorrection.cc:15-116).
 //------------------------------------------------------------------------------
-template <bool TENSOR>
 __global__ void __launch_bounds__(128) gradhKernel(Fields F, long n, Grid g, NeighborLists nl, TableDev t,
                                                    HydroParams hp) {
   extern __shared__ double smem[];
@@ -612,10 +973,9 @@ __global__ void __launch_bounds__(128) gradhKernel(Fields F, long n, Grid g, Nei
   const double* __restrict__ X = F.f[F_X];
   const double* __restrict__ Y = F.f[F_Y];
   const double* __restrict__ Z = F.f[F_Z];
-  const double xi = X[i], yi = Y[i], zi = Z[i], ai = F.f[F_HINV][i];
-  Sym Hi{};
-  if (TENSOR) Hi = loadSym(F, F_HT_XX, i);
-  const double Hdeti = TENSOR ? symDet(Hi) : (ai * ai) * ai;
+  const double xi = X[i], yi = Y[i], zi = Z[i];
+  const Sym Hi = loadSym(F, F_HT_XX, i);
+  const double Hdeti = symDet(Hi);
   double wsum = 0.0, gsum = 0.0;
   const int cnt = nl.count[i];
   for (int q = 0; q < cnt; ++q) {
@@ -626,8 +986,7 @@ __global__ void __launch_bounds__(128) gradhKernel(Fields F, long n, Grid g, Nei
     imagePos(g, code, xj, yj, zj);
     const double rx = xi - xj, ry = yi - yj, rz = zi - zj;
     double ex, ey, ez;
-    if (TENSOR) symDot(Hi, rx, ry, rz, ex, ey, ez);
-    else { ex = ai * rx; ey = ai * ry; ez = ai * rz; }
+    symDot(Hi, rx, ry, rz, ex, ey, ez);
     const double eta = sqrt(ex * ex + ey * ey + ez * ez);
     if (eta < hp.extent) {
       const int i0 = tableIndex(eta, hp.tableN1, hp.tableXstep);
@@ -646,9 +1005,9 @@ __global__ void __launch_bounds__(128) gradhKernel(Fields F, long n, Grid g, Nei
 // MonaghanGingoldViscosity::QPiij (MonaghanGingoldViscosity.cc:41-101) and the
 // SPHSmoothingScale moments + IdealH (SPHSmoothingScale.cc:154-272), FP64.
 //------------------------------------------------------------------------------
-// TENSOR: ASPH -- symmetric-tensor H_i, H_j (eta = H r, grad W = gW H eta^),
-// the ASPHClassicSmoothingScale second moment and its finalize.
-template <bool XSPH, bool COMPAT, bool TENSOR>
+// ASPH: symmetric-tensor H_i, H_j (eta = H r, grad W = gW H eta^), the
+// ASPHClassicSmoothingScale second moment and its finalize.
+template <bool XSPH, bool COMPAT>
 __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __restrict__ list, long n, Grid g,
                                                       NeighborLists nl, TableDev t, HydroParams hp,
                                                       double* __restrict__ pacc) {
@@ -671,16 +1030,14 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
   const double* __restrict__ PP = F.f[F_P];
   const double* __restrict__ CS = F.f[F_CS];
   const double* __restrict__ OM = F.f[F_OMEGA];
-  const double* __restrict__ A = F.f[F_HINV];
   const double* __restrict__ tw = smem;
   const double* __restrict__ tg = smem + ntab;
 
   const double xi = X[i], yi = Y[i], zi = Z[i], vxi = VX[i], vyi = VY[i], vzi = VZ[i];
-  const double mi = Ms[i], rhoi = RHO[i], Pi = PP[i], ci = CS[i], omi = OM[i], ai = A[i];
+  const double mi = Ms[i], rhoi = RHO[i], Pi = PP[i], ci = CS[i], omi = OM[i];
   const int li = list[i];
-  Sym Hi{};
-  if (TENSOR) Hi = loadSym(F, F_HT_XX, i);
-  const double Hdeti = TENSOR ? symDet(Hi) : (ai * ai) * ai;
+  const Sym Hi = loadSym(F, F_HT_XX, i);
+  const double Hdeti = symDet(Hi);
   const double safeOmegai = omi / (omi * omi + kTiny30);
   const double tiny = kTiny30;
   const double Clij = 0.5 * (1.0 + 1.0) * 1.0 * hp.Cl;
@@ -705,25 +1062,17 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
     double xj = X[j], yj = Y[j], zj = Z[j], vxj = VX[j], vyj = VY[j], vzj = VZ[j];
     imagePos(g, code, xj, yj, zj);
     imageVec(g, code, vxj, vyj, vzj);
-    const double mj = Ms[j], rhoj = RHO[j], Pj = PP[j], cj = CS[j], omj = OM[j], aj = A[j];
+    const double mj = Ms[j], rhoj = RHO[j], Pj = PP[j], cj = CS[j], omj = OM[j];
     const int lj = list[j];
-    Sym Hj{};
-    if (TENSOR) {
-      Hj = loadSym(F, F_HT_XX, j);
-      imageSym(g, code, Hj);
-    }
-    const double Hdetj = TENSOR ? symDet(Hj) : (aj * aj) * aj;
+    Sym Hj = loadSym(F, F_HT_XX, j);
+    imageSym(g, code, Hj);
+    const double Hdetj = symDet(Hj);
     const double safeOmegaj = omj / (omj * omj + kTiny30);
 
     const double rx = xi - xj, ry = yi - yj, rz = zi - zj;
     double eix, eiy, eiz, ejx, ejy, ejz;
-    if (TENSOR) {
-      symDot(Hi, rx, ry, rz, eix, eiy, eiz);
-      symDot(Hj, rx, ry, rz, ejx, ejy, ejz);
-    } else {
-      eix = ai * rx; eiy = ai * ry; eiz = ai * rz;
-      ejx = aj * rx; ejy = aj * ry; ejz = aj * rz;
-    }
+    symDot(Hi, rx, ry, rz, eix, eiy, eiz);
+    symDot(Hj, rx, ry, rz, ejx, ejy, ejz);
     const double etaMag2i = eix * eix + eiy * eiy + eiz * eiz;
     const double etaMag2j = ejx * ejx + ejy * ejy + ejz * ejz;
     const double etaMagi = sqrt(etaMag2i), etaMagj = sqrt(etaMag2j);
@@ -745,16 +1094,12 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
     Wi *= Hdeti; Wj *= Hdetj;
     const double gWi = Hdeti * gi, gWj = Hdetj * gj;
     double gwix, gwiy, gwiz, gwjx, gwjy, gwjz;
-    if (TENSOR) {   // gW H eta^
+    {   // gW H eta^
       double hx, hy, hz;
       symDot(Hi, uix, uiy, uiz, hx, hy, hz);
       gwix = gWi * hx; gwiy = gWi * hy; gwiz = gWi * hz;
       symDot(Hj, ujx, ujy, ujz, hx, hy, hz);
       gwjx = gWj * hx; gwjy = gWj * hy; gwjz = gWj * hz;
-    } else {
-      const double gHi = gWi * ai, gHj = gWj * aj;
-      gwix = gHi * uix; gwiy = gHi * uiy; gwiz = gHi * uiz;
-      gwjx = gHj * ujx; gwjy = gHj * ujy; gwjz = gHj * ujz;
     }
 
     if (lj == li) {
@@ -823,9 +1168,10 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
     a.dvy -= mj * ddy;
     a.dvz -= mj * ddz;
     if (COMPAT) {
-      pacc[3 * k] = -mj * ddx;
-      pacc[3 * k + 1] = -mj * ddy;
-      pacc[3 * k + 2] = -mj * ddz;
+      double* out = pacc + paccSlot(k);
+      out[0] = -mj * ddx;
+      out[32] = -mj * ddy;
+      out[64] = -mj * ddz;
     }
     a.deps += mj * (Prhoi * (vijx * gwix + vijy * gwiy + vijz * gwiz) + workQi);
     const double mvx = mj * vijx, mvy = mj * vijy, mvz = mj * vijz;
@@ -848,7 +1194,7 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
     a.m0 += fw * WSPHi;
     const double fwW = fw * WSPHi;
     a.m1x -= fwW * eix; a.m1y -= fwW * eiy; a.m1z -= fwW * eiz;
-    if (TENSOR) {   // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
+    {   // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
       const double rm = sqrt(rx * rx + ry * ry + rz * rz);
       const double f5 = 1.0 / fmax(kTiny30, rm * rm * rm * rm * rm);
       const double w2 = fwW * WSPHi;
@@ -856,8 +1202,7 @@ __global__ void __launch_bounds__(128) pairKernelFP64(Fields F, const int* __res
       a.m2[3] += w2 * (ry * ry * f5); a.m2[4] += w2 * (ry * rz * f5); a.m2[5] += w2 * (rz * rz * f5);
     }
   }
-  if (TENSOR) finalizeNodeASPH(F, i, li, a, Hi, mi, rhoi, vxi, vyi, vzi, cnt, hp, t.herm);
-  else finalizeNode(F, i, li, a, mi, rhoi, vxi, vyi, vzi, ai, cnt, hp, t.herm);
+  finalizeNodeASPH(F, i, li, a, Hi, mi, rhoi, vxi, vyi, vzi, cnt, hp, t.herm);
 }
 
 //------------------------------------------------------------------------------
@@ -948,53 +1293,6 @@ __global__ void dtFinalKernel(const double* __restrict__ part, int nb, double* _
 }
 
 //------------------------------------------------------------------------------
-// SpecificThermalEnergyPolicy::update (src/Hydro/SpecificThermalEnergyPolicy.cc:110-173),
-// gathered: node i takes its own share w_i du_ij of every pair, with the pair
-// acceleration stored per ordered slot by the pair loop.
-//------------------------------------------------------------------------------
-template <bool F32PACC>
-__global__ void __launch_bounds__(128) energyKernel(Fields F, long n, Grid g, NeighborLists nl,
-                                                    const double* __restrict__ pacc, const float* __restrict__ pacc32,
-                                                    double dt) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int hc[3];
-  unpackCell(nl.cell[i], hc);
-  const double hdt = 0.5 * dt;
-  const double* __restrict__ VX = F.f[F_VX];
-  const double* __restrict__ VY = F.f[F_VY];
-  const double* __restrict__ VZ = F.f[F_VZ];
-  const double* __restrict__ AX = F.f[F_DVDT_X];
-  const double* __restrict__ AY = F.f[F_DVDT_Y];
-  const double* __restrict__ AZ = F.f[F_DVDT_Z];
-  const double* __restrict__ D0 = F.f[F_DEPSDT];
-  const double vxi = VX[i] + AX[i] * hdt, vyi = VY[i] + AY[i] * hdt, vzi = VZ[i] + AZ[i] * hdt;
-  const double d0i = D0[i];
-  double sum = 0.0;
-  const int cnt = nl.count[i];
-  for (int q = 0; q < cnt; ++q) {
-    const long long k = nbSlot(i, q, nl.cap);
-    const uint32_t ent = nl.nbr[k];
-    const int j = (int)(ent & kIndexMask), code = imageCode(g, hc, (int)(ent >> kIndexBits));
-    double vxj = VX[j], vyj = VY[j], vzj = VZ[j], axj = AX[j], ayj = AY[j], azj = AZ[j];
-    imageVec(g, code, vxj, vyj, vzj);
-    imageVec(g, code, axj, ayj, azj);
-    const double wx = vxj + axj * hdt - vxi, wy = vyj + ayj * hdt - vyi, wz = vzj + azj * hdt - vzi;
-    double px, py, pz;
-    if (F32PACC) { px = pacc32[3 * k]; py = pacc32[3 * k + 1]; pz = pacc32[3 * k + 2]; }
-    else { px = pacc[3 * k]; py = pacc[3 * k + 1]; pz = pacc[3 * k + 2]; }
-    const double du = wx * px + wy * py + wz * pz;
-    const double sg = du < 0.0 ? -1.0 : 1.0;
-    const double weighti = fmax(DBL_EPSILON, d0i * sg);
-    const double weightj = fmax(DBL_EPSILON, D0[j] * sg);
-    const double wi = weighti / (weighti + weightj);
-    sum += wi * du;
-  }
-  F.f[F_DEPS_COMPAT][i] = sum;
-  F.f[F_EPS][i] += sum * dt;
-}
-
-//------------------------------------------------------------------------------
 // State updates (State::update with IncrementState / IncrementBoundedState /
 // ReplaceBoundedState, PressurePolicy, SoundSpeedPolicy) and GammaLawGas.
 //------------------------------------------------------------------------------
@@ -1004,18 +1302,6 @@ __device__ __forceinline__ void eosNode(Fields& F, long i, const NodeListParams&
   p = p < L.minP ? L.minP : (p > L.maxP ? L.maxP : p);
   F.f[F_P][i] = p;
   F.f[F_CS][i] = sqrt(fmax(0.0, L.gamma * (L.gamma - 1.0) * eps));
-}
-
-__global__ void restoreState0Kernel(Fields F, long n, int tensor, int crk) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  F.f[F_X][i] = F.f[F_X0][i]; F.f[F_Y][i] = F.f[F_Y0][i]; F.f[F_Z][i] = F.f[F_Z0][i];
-  F.f[F_VX][i] = F.f[F_VX0][i]; F.f[F_VY][i] = F.f[F_VY0][i]; F.f[F_VZ][i] = F.f[F_VZ0][i];
-  F.f[F_RHO][i] = F.f[F_RHO0][i]; F.f[F_EPS][i] = F.f[F_EPS0][i]; F.f[F_HINV][i] = F.f[F_HINV0][i];
-  if (tensor)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) F.f[F_HT_XX + k][i] = F.f[F_HT0_XX + k][i];
-  if (crk) F.f[F_VOL][i] = F.f[F_VOL0][i];
 }
 
 // Extent of tensor H (ASPH): smallest eigenvalue -> F_HINV (cell size,
@@ -1107,7 +1393,7 @@ __global__ void __launch_bounds__(128) asphEndKernel(Fields F, Fields32 P, const
   if (P.posh) {
     storeExtent32(F, i, Hn);
     P.posh[i].w = (float)F.f[F_HINV][i];
-    writeTensorMirror(F, P, i);
+    writeTensorMirror(F, i, P, i);
   } else {
     storeExtent(F, i, Hn);
   }
@@ -1119,6 +1405,10 @@ __global__ void tensorExtentKernel(Fields F, long n) {
   storeExtent(F, i, loadSym(F, F_HT_XX, i));
 }
 
+// The half-step update (mid) advances the current state and keeps its
+// beginning-of-step copy (state0); the full update advances state0 itself
+// (State::update after the reference's state.assign(state0)), eps already
+// advanced by the compatible-energy sweep when compatible.
 // P != nullptr (mixed mode): the FP32 mirrors of the new state are written
 // here as well (the prepare pass folded into the update).
 // tensor (ASPH): H is the symmetric tensor, bounded on its eigenvalues
@@ -1134,45 +1424,50 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const NodeListParams L = lists[list[i]];
+  // state the update starts from
+  const int bx = mid ? F_X : F_X0, bvx = mid ? F_VX : F_VX0;
   // the position before this update (the radial direction of radialOnly:
   // State::update applies the "H" policy before the "position" one)
-  const double xOld = F.f[F_X][i], yOld = F.f[F_Y][i], zOld = F.f[F_Z][i];
-  // the half-step update first takes the beginning-of-step copy (state0)
-  if (mid) {
-    F.f[F_X0][i] = F.f[F_X][i]; F.f[F_Y0][i] = F.f[F_Y][i]; F.f[F_Z0][i] = F.f[F_Z][i];
-    F.f[F_VX0][i] = F.f[F_VX][i]; F.f[F_VY0][i] = F.f[F_VY][i]; F.f[F_VZ0][i] = F.f[F_VZ][i];
-    F.f[F_RHO0][i] = F.f[F_RHO][i]; F.f[F_EPS0][i] = F.f[F_EPS][i]; F.f[F_HINV0][i] = F.f[F_HINV][i];
-    if (TENSOR)
-#pragma unroll
-      for (int k = 0; k < 6; ++k) F.f[F_HT0_XX + k][i] = F.f[F_HT_XX + k][i];
-    if (crk) F.f[F_VOL0][i] = F.f[F_VOL][i];
+  const double xOld = F.f[bx][i], yOld = F.f[bx + 1][i], zOld = F.f[bx + 2][i];
+  const double vxOld = F.f[bvx][i], vyOld = F.f[bvx + 1][i], vzOld = F.f[bvx + 2][i];
+  const double rhoOld = F.f[mid ? F_RHO : F_RHO0][i], hOld = F.f[mid ? F_HINV : F_HINV0][i];
+  const double volOld = crk ? F.f[mid ? F_VOL : F_VOL0][i] : 0.0;
+  Sym HOld{};
+  if (TENSOR) HOld = loadSym(F, mid ? F_HT_XX : F_HT0_XX, i);
+  double eps = F.f[mid || !epsIncrement ? F_EPS : F_EPS0][i];
+  if (mid) {   // state0
+    F.f[F_X0][i] = xOld; F.f[F_Y0][i] = yOld; F.f[F_Z0][i] = zOld;
+    F.f[F_VX0][i] = vxOld; F.f[F_VY0][i] = vyOld; F.f[F_VZ0][i] = vzOld;
+    F.f[F_RHO0][i] = rhoOld; F.f[F_EPS0][i] = eps; F.f[F_HINV0][i] = hOld;
+    if (TENSOR) storeSym(F, F_HT0_XX, i, HOld);
+    if (crk) F.f[F_VOL0][i] = volOld;
   }
+  const double ax = F.f[F_DVDT_X][i], ay = F.f[F_DVDT_Y][i], az = F.f[F_DVDT_Z][i];
   if (epsIncrement) {
     if (totalEnergy) {
       // SpecificFromTotalThermalEnergyPolicy::update: eps from the total
       // energy m (v^2/2 + eps) advanced by DEDt, with the hydro acceleration
       // for the new kinetic part (it fires before the velocity update)
       const double mi = F.f[F_MASS][i];
-      const double v0x = F.f[F_VX][i], v0y = F.f[F_VY][i], v0z = F.f[F_VZ][i];
-      const double v1x = v0x + mult * F.f[F_DVDT_X][i], v1y = v0y + mult * F.f[F_DVDT_Y][i],
-                   v1z = v0z + mult * F.f[F_DVDT_Z][i];
-      const double E0 = mi * (0.5 * (v0x * v0x + v0y * v0y + v0z * v0z) + F.f[F_EPS][i]);
+      const double v1x = vxOld + mult * ax, v1y = vyOld + mult * ay, v1z = vzOld + mult * az;
+      const double E0 = mi * (0.5 * (vxOld * vxOld + vyOld * vyOld + vzOld * vzOld) + eps);
       const double E1 = E0 + mult * F.f[F_DEPSDT][i];
-      F.f[F_EPS][i] = E1 / mi - 0.5 * (v1x * v1x + v1y * v1y + v1z * v1z);
+      eps = E1 / mi - 0.5 * (v1x * v1x + v1y * v1y + v1z * v1z);
     } else {
-      F.f[F_EPS][i] += mult * F.f[F_DEPSDT][i];
+      eps += mult * F.f[F_DEPSDT][i];
     }
+    F.f[F_EPS][i] = eps;
   }
-  const double x = F.f[F_X][i] + mult * F.f[F_DXDT_X][i];
-  const double y = F.f[F_Y][i] + mult * F.f[F_DXDT_Y][i];
-  const double z = F.f[F_Z][i] + mult * F.f[F_DXDT_Z][i];
+  const double x = xOld + mult * F.f[F_DXDT_X][i];
+  const double y = yOld + mult * F.f[F_DXDT_Y][i];
+  const double z = zOld + mult * F.f[F_DXDT_Z][i];
   F.f[F_X][i] = x;
   F.f[F_Y][i] = y;
   F.f[F_Z][i] = z;
   // velocity: "delta velocity hydro" sorts before "delta velocity" (gravity)
-  double vx = F.f[F_VX][i] + mult * F.f[F_DVDT_X][i];
-  double vy = F.f[F_VY][i] + mult * F.f[F_DVDT_Y][i];
-  double vz = F.f[F_VZ][i] + mult * F.f[F_DVDT_Z][i];
+  double vx = vxOld + mult * ax;
+  double vy = vyOld + mult * ay;
+  double vz = vzOld + mult * az;
   if (gravity) {
     vx += mult * F.f[F_GRAV_X][i];
     vy += mult * F.f[F_GRAV_Y][i];
@@ -1181,16 +1476,16 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
   F.f[F_VX][i] = vx;
   F.f[F_VY][i] = vy;
   F.f[F_VZ][i] = vz;
-  const double rho = fmin(L.rhoMax, fmax(L.rhoMin, F.f[F_RHO][i] + mult * F.f[F_DRHODT][i]));
+  const double rho = fmin(L.rhoMax, fmax(L.rhoMin, rhoOld + mult * F.f[F_DRHODT][i]));
   F.f[F_RHO][i] = rho;
   const double hminInv = L.hminInv, hmaxInv = L.hmaxInv;
   double h;
   const bool increment = mid || hUpdate == 1;
-  if (hUpdate == 2) {
-    h = F.f[F_HINV][i];
+  if (hUpdate == 2) {   // FixedH: both copies hold the same H
+    h = hOld;
   } else if (TENSOR && asphEnd) {
-    const Sym t = incrementASPHHtensor(loadSym(F, F_HT_XX, i), loadSym(F, F_DHDTT_XX, i), mult, xOld, yOld, zOld,
-                                       fixShape != 0, radialOnly != 0, hminInv, hmaxInv, L.hminratio);
+    const Sym t = incrementASPHHtensor(HOld, loadSym(F, F_DHDTT_XX, i), mult, xOld, yOld, zOld, fixShape != 0,
+                                       radialOnly != 0, hminInv, hmaxInv, L.hminratio);
     storeSym(F, F_HT_XX, i, t);
     if (P.posh) storeExtent32(F, i, t);
     else storeExtent(F, i, t);
@@ -1198,10 +1493,9 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
   } else if (TENSOR) {
     Sym t;
     if (increment) {
-      t = loadSym(F, F_HT_XX, i);
       const Sym d = loadSym(F, F_DHDTT_XX, i);
-      t = Sym{t.xx + mult * d.xx, t.xy + mult * d.xy, t.xz + mult * d.xz, t.yy + mult * d.yy, t.yz + mult * d.yz,
-              t.zz + mult * d.zz};
+      t = Sym{HOld.xx + mult * d.xx, HOld.xy + mult * d.xy, HOld.xz + mult * d.xz, HOld.yy + mult * d.yy,
+              HOld.yz + mult * d.yz, HOld.zz + mult * d.zz};
     } else {
       t = loadSym(F, F_HIDEALT_XX, i);
     }
@@ -1211,7 +1505,7 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     else storeExtent(F, i, t);
     h = F.f[F_HINV][i];
   } else {
-    h = increment ? F.f[F_HINV][i] + mult * F.f[F_DHDT][i] : F.f[F_HIDEAL][i];
+    h = increment ? hOld + mult * F.f[F_DHDT][i] : F.f[F_HIDEAL][i];
     if (h < hmaxInv) h = hmaxInv;
     if (h > hminInv) h = hminInv;
     F.f[F_HINV][i] = h;
@@ -1223,7 +1517,7 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     const double volMin = 0.5 * mi * safeInvVarD(rho);
     const double volMax = 4.0 * 3.141592653589793 / (3.0 * ((h * h) * h));
     const double dVdt = -mi * safeInvVarD(rho * rho) * F.f[F_DRHODT][i];
-    F.f[F_VOL][i] = fmax(volMin, fmin(volMax, F.f[F_VOL][i] + mult * dVdt));
+    F.f[F_VOL][i] = fmax(volMin, fmin(volMax, volOld + mult * dVdt));
   }
   if (P.posh) {
     // Mixed mode.  The sound speed feeds only FP32 sweeps (Q, dt vote), so it
@@ -1231,7 +1525,6 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     // the integer pipe (convert.cuh) and the cell origins an integer-built
     // index: GB300's FP64 pipe, which runs FP64 arithmetic and the
     // conversion instructions at ~1/64 of the FP32 rate, bounds this kernel.
-    const double eps = F.f[F_EPS][i];
     double p = L.gm1 * rho * eps;
     p = p < L.minP ? L.minP : (p > L.maxP ? L.maxP : p);
     F.f[F_P][i] = p;
@@ -1246,7 +1539,7 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     P.velm[i] = make_float4(toFloatRN(vx), toFloatRN(vy), toFloatRN(vz), toFloatRN(F.f[F_MASS][i]));
     const float om = toFloatRN(F.f[F_OMEGA][i]);
     P.thermo[i] = make_float4(toFloatRN(rho), toFloatRN(p), cs, om / (om * om + 1.0e-30f));
-    if (TENSOR) writeTensorMirror(F, P, i);
+    if (TENSOR) writeTensorMirror(F, i, P, i);
     if (crk && P.vol) P.vol[i] = toFloatRN(F.f[F_VOL][i]);
   } else {
     eosNode(F, i, L);
@@ -1272,9 +1565,7 @@ __device__ __forceinline__ long long orderKey(double x) {
 // tensor: the H of a node mapped back through a reflecting wall is reflected
 // too (PlanarBoundary::updateViolationNodes -> enforceBoundary(Hfield),
 // (R H R).Symmetric()).
-__global__ void enforceKernel(Fields F, long n, Grid g, int tensor) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ void enforceNode(Fields& F, long i, const Grid& g, int tensor) {
   auto reflectH = [&](int a) {
     if (!tensor) return;
     if (a == 0) { F.f[F_HT_XY][i] = -F.f[F_HT_XY][i]; F.f[F_HT_XZ][i] = -F.f[F_HT_XZ][i]; }
@@ -1314,6 +1605,66 @@ __global__ void enforceKernel(Fields F, long n, Grid g, int tensor) {
   }
 }
 
+// Bit tests of the end-of-step check (integer pipe).
+__device__ __forceinline__ bool finiteBits(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+__device__ __forceinline__ bool positiveBits(double x) {   // x > 0 and finite
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b < 0x7ff0000000000000LL;
+}
+
+// End of the step in one pass: nodes outside a wall are mapped back, the state
+// is checked (finite, positive) and the bounds the next neighbour build needs
+// are taken (as boundsKernel; the comparisons on order keys).
+__global__ void __launch_bounds__(256) endStepKernel(Fields F, long n, Grid g, int tensor, StepScratch* __restrict__ sc) {
+  long long mn[4] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MAX};
+  long long mx[6] = {LLONG_MIN, LLONG_MIN, LLONG_MIN, 0, 0, 0};
+  bool bad = false;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    enforceNode(F, i, g, tensor);
+    const double a = F.f[F_HINV][i], p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
+    bad |= !positiveBits(F.f[F_MASS][i]) | !positiveBits(F.f[F_RHO][i]) | !positiveBits(a) | !finiteBits(F.f[F_EPS][i]) |
+           !finiteBits(p[0]) | !finiteBits(p[1]) | !finiteBits(p[2]) | !finiteBits(F.f[F_VX][i]) |
+           !finiteBits(F.f[F_VY][i]) | !finiteBits(F.f[F_VZ][i]);
+    mn[0] = min(mn[0], orderKey(a));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const long long o = orderKey(p[k]);
+      mn[1 + k] = min(mn[1 + k], o);
+      mx[k] = max(mx[k], o);
+    }
+    if (tensor) {
+      const Sym w = symInverse(loadSym(F, F_HT_XX, i));
+      mx[3] = max(mx[3], orderKey(sqrt(w.xx * w.xx + w.xy * w.xy + w.xz * w.xz)));
+      mx[4] = max(mx[4], orderKey(sqrt(w.xy * w.xy + w.yy * w.yy + w.yz * w.yz)));
+      mx[5] = max(mx[5], orderKey(sqrt(w.xz * w.xz + w.yz * w.yz + w.zz * w.zz)));
+    }
+  }
+  __shared__ long long sm[8][10];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 10; ++k) {
+    if (k >= 7 && !tensor) break;
+    long long v = k < 4 ? mn[k] : mx[k - 4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long w = __shfl_xor_sync(0xffffffffu, v, o);
+      v = k < 4 ? min(v, w) : max(v, w);
+    }
+    if (lane == 0) sm[warp][k] = v;
+  }
+  if (bad) atomicExch(&sc->bad, 1);
+  __syncthreads();
+  if (threadIdx.x < (tensor ? 10 : 7)) {
+    const int k = threadIdx.x;
+    long long v = sm[0][k];
+    for (int w = 1; w < 8; ++w) v = k < 4 ? min(v, sm[w][k]) : max(v, sm[w][k]);
+    if (k < 4) atomicMin(&sc->bounds[k], v);
+    else atomicMax(&sc->bounds[k], v);
+  }
+}
+
 // SpheralConservation totals (SpheralConservation.py:54-150) in FP64:
 // mass, momentum, kinetic, thermal, gravitational (1/2 m phi).
 __global__ void conservationKernel(Fields F, long n, int gravity, double* __restrict__ part) {
@@ -1342,17 +1693,6 @@ __global__ void conservationFinalKernel(const double* __restrict__ part, int nb,
     if (threadIdx.x == 0) out[k] = r;
   }
   if (threadIdx.x == 0) out[7] = out[4] + out[5] + out[6];
-}
-
-__global__ void checkStateKernel(Fields F, long n, int* __restrict__ flag) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double m = F.f[F_MASS][i], rho = F.f[F_RHO][i], a = F.f[F_HINV][i], eps = F.f[F_EPS][i];
-  const double x = F.f[F_X][i], y = F.f[F_Y][i], z = F.f[F_Z][i];
-  const double vx = F.f[F_VX][i], vy = F.f[F_VY][i], vz = F.f[F_VZ][i];
-  const bool bad = !(m > 0.0) || !(rho > 0.0) || !(a > 0.0) || !isfinite(eps) || !isfinite(x) || !isfinite(y) ||
-                   !isfinite(z) || !isfinite(vx) || !isfinite(vy) || !isfinite(vz) || !isfinite(rho) || !isfinite(a);
-  if (bad) atomicExch(flag, 1);
 }
 
 // Caller-order transfers: stage[orig[k] * stride + c] <-> F[first + c][k].
@@ -1457,9 +1797,9 @@ void launchBounds(const Fields& F, long n, bool tensor, double* dScratch, int nS
   boundsFinalKernel<<<1, 256, 0, s>>>(dScratch, nb, dOut);
   lc->add(2);
 }
-void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, cudaStream_t s,
-                    LaunchCounter* lc) {
-  cellKeyKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, keys, vals, cellc);
+void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
+                    cudaStream_t s, LaunchCounter* lc) {
+  cellKeyKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, keys, vals, cellc, sc);
   lc->add(1);
 }
 // ArtificialViscosityHandle::postStateUpdate: the Q's DvDx = the hydro DvDx.
@@ -1490,7 +1830,9 @@ void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCoun
 }
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
-                   bool carriedOnly, bool tensor, bool crk, cudaStream_t s, LaunchCounter* lc) {
+                   bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
+                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, cudaStream_t s,
+                   LaunchCounter* lc) {
   // the tensor-H fields (the end of the carried block and of the permuted
   // block) move only in ASPH mode, the RK volume and corrections (the end of
   // the permuted block) only in CRKSPH mode
@@ -1502,18 +1844,18 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
     if (crk) add(F_VOL, F_NUM_PERMUTED);
   }
   permuteKernel<<<gridFor(n, 256), 256, 0, s>>>(Fin, Fout, perm, origIn, origOut, listIn, listOut, cellIn, cellOut, n,
-                                                sel);
+                                                sel, P, g, mirrors ? 1 : 0, sortedKeys, space, cellStart, cellEnd);
   lc->add(1);
 }
-void launchCellRanges(const uint32_t* sortedKeys, long n, int shift, int* cellStart, int* cellEnd, cudaStream_t s,
-                      LaunchCounter* lc) {
-  cellRangeKernel<<<gridFor(n, 256), 256, 0, s>>>(sortedKeys, n, shift, cellStart, cellEnd);
-  lc->add(1);
-}
-void launchItemBoxes(const int* items, const long long* dItems, int nItemsBound, long n, int width, Fields32 P,
-                     float4* box, int* chunkOf, cudaStream_t s, LaunchCounter* lc) {
-  itemBoxKernel<<<gridFor(std::max(1, nItemsBound), 256), 256, 0, s>>>(items, dItems, n, width, P, box, chunkOf);
-  lc->add(1);
+void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
+                 int nItemsBound, Fields32 P, int* items, int* chunkOf, float4* box, StepScratch* sc, cudaStream_t s,
+                 LaunchCounter* lc) {
+  itemsKernel<<<gridFor(n, 256), 256, 0, s>>>(sortedKeys, n, shift, space, cellEnd, width, items, chunkOf, sc);
+  const unsigned gb = gridFor((long)nItemsBound * width, 128);
+  if (width == 8) itemBoxKernel<8><<<gb, 128, 0, s>>>(items, sc, n, P, box);
+  else if (width == 16) itemBoxKernel<16><<<gb, 128, 0, s>>>(items, sc, n, P, box);
+  else itemBoxKernel<32><<<gb, 128, 0, s>>>(items, sc, n, P, box);
+  lc->add(2);
 }
 // Band of the FP32 pre-filter on e2 = min(a_i, a_j)^2 r^2 around ext^2
 // (a = 1/h).  Every cell-relative coordinate is within about one cell size C
@@ -1524,6 +1866,7 @@ void launchItemBoxes(const int* items, const long long* dItems, int nItemsBound,
 // band used is four times that bound, evaluated with a = a_i >= min(a_i, a_j):
 // delta_i = bandA a_i + bandB.  A node whose delta reaches 1/2 takes the exact
 // test on every candidate.
+constexpr int kWideItems = 2400;   // items below which four warps share one
 static void neighborBand(const Grid& g, double ext2, float& bandA, float& bandB) {
   const double u = 1.0 / 16777216.0;
   const double cmax = std::max(g.cell[0], std::max(g.cell[1], g.cell[2]));
@@ -1531,36 +1874,28 @@ static void neighborBand(const Grid& g, double ext2, float& bandA, float& bandB)
   bandA = (float)(4.0 * 20.0 * std::sqrt(3.0) * u * cmax / ext);
   bandB = (float)(4.0 * 7.0 * u);
 }
+// Tensor H (ASPH); the isotropic FP64 sweeps are in hydro64.cu.
 void launchSumDensity(Fields F, const int* list, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                       cudaStream_t s, LaunchCounter* lc) {
   const size_t sm = sizeof(double) * 3 * (hp.tableN1 + 1);
-  if (hp.asph) sumDensityKernel<true><<<gridFor(n, 128), 128, sm, s>>>(F, list, n, g, nl, t, hp);
-  else sumDensityKernel<false><<<gridFor(n, 128), 128, sm, s>>>(F, list, n, g, nl, t, hp);
+  sumDensityKernel<<<gridFor(n, 128), 128, sm, s>>>(F, list, n, g, nl, t, hp);
   lc->add(1);
 }
 void launchGradh(Fields F, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp, cudaStream_t s,
                  LaunchCounter* lc) {
   const size_t sm = sizeof(double) * 6 * (hp.tableN1 + 1);
-  if (hp.asph) gradhKernel<true><<<gridFor(n, 128), 128, sm, s>>>(F, n, g, nl, t, hp);
-  else gradhKernel<false><<<gridFor(n, 128), 128, sm, s>>>(F, n, g, nl, t, hp);
+  gradhKernel<<<gridFor(n, 128), 128, sm, s>>>(F, n, g, nl, t, hp);
   lc->add(1);
 }
 void launchPairFP64(Fields F, const int* list, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                    double* pacc, int blockSize, cudaStream_t s, LaunchCounter* lc) {
+                    double* pacc, cudaStream_t s, LaunchCounter* lc) {
   const size_t sm = sizeof(double) * 6 * (hp.tableN1 + 1);
   const int b = 128;
-  (void)blockSize;
-#define SPH_PAIR64(X, C, T) pairKernelFP64<X, C, T><<<gridFor(n, b), b, sm, s>>>(F, list, n, g, nl, t, hp, pacc)
-  if (hp.asph) {
-    if (hp.xsph) {
-      if (hp.compatible) SPH_PAIR64(true, true, true); else SPH_PAIR64(true, false, true);
-    } else {
-      if (hp.compatible) SPH_PAIR64(false, true, true); else SPH_PAIR64(false, false, true);
-    }
-  } else if (hp.xsph) {
-    if (hp.compatible) SPH_PAIR64(true, true, false); else SPH_PAIR64(true, false, false);
+#define SPH_PAIR64(X, C) pairKernelFP64<X, C><<<gridFor(n, b), b, sm, s>>>(F, list, n, g, nl, t, hp, pacc)
+  if (hp.xsph) {
+    if (hp.compatible) SPH_PAIR64(true, true); else SPH_PAIR64(true, false);
   } else {
-    if (hp.compatible) SPH_PAIR64(false, true, false); else SPH_PAIR64(false, false, false);
+    if (hp.compatible) SPH_PAIR64(false, true); else SPH_PAIR64(false, false);
   }
 #undef SPH_PAIR64
   lc->add(1);
@@ -1573,16 +1908,6 @@ void launchDt(Fields F, const int* list, long n, Grid g, NeighborLists nl, Hydro
   dtKernel<<<nb, 128, 0, s>>>(F, list, n, g, nl, hp, maxNperh, dScratch);
   dtFinalKernel<<<1, 256, 0, s>>>(dScratch, nb, dOut);
   lc->add(2);
-}
-void launchCompatibleEnergy(Fields F, long n, Grid g, NeighborLists nl, const double* pacc, const float* pacc32,
-                            double dt, cudaStream_t s, LaunchCounter* lc) {
-  if (pacc32) energyKernel<true><<<gridFor(n, 128), 128, 0, s>>>(F, n, g, nl, pacc, pacc32, dt);
-  else energyKernel<false><<<gridFor(n, 128), 128, 0, s>>>(F, n, g, nl, pacc, pacc32, dt);
-  lc->add(1);
-}
-void launchRestoreState0(Fields F, long n, bool tensor, bool crk, cudaStream_t s, LaunchCounter* lc) {
-  restoreState0Kernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, tensor ? 1 : 0, crk ? 1 : 0);
-  lc->add(1);
 }
 void launchRadius0(Fields F, long n, cudaStream_t s, LaunchCounter* lc) {
   radius0Kernel<<<gridFor(n, 256), 256, 0, s>>>(F, n);
@@ -1616,8 +1941,10 @@ void launchEOS(Fields F, const int* list, long n, const NodeListParams* lists, c
   eosKernel<<<gridFor(n, 256), 256, 0, s>>>(F, list, n, lists);
   lc->add(1);
 }
-void launchEnforce(Fields F, long n, Grid g, bool tensor, cudaStream_t s, LaunchCounter* lc) {
-  enforceKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, tensor ? 1 : 0);
+void launchEndStep(Fields F, long n, Grid g, bool tensor, StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
+  // at most 8 blocks per SM, each thread over several nodes: ten reductions and
+  // atomics per block, not per node
+  endStepKernel<<<std::min(gridFor(n, 256), 1216u), 256, 0, s>>>(F, n, g, tensor ? 1 : 0, sc);
   lc->add(1);
 }
 void launchConservation(Fields F, long n, bool gravity, double* dScratch, int nScratch, double* dOut, cudaStream_t s,
@@ -1628,11 +1955,6 @@ void launchConservation(Fields F, long n, bool gravity, double* dScratch, int nS
   conservationFinalKernel<<<1, 256, 0, s>>>(dScratch, nb, dOut);
   lc->add(2);
 }
-void launchCheckState(Fields F, long n, int* dFlag, cudaStream_t s, LaunchCounter* lc) {
-  checkStateKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, dFlag);
-  lc->add(1);
-}
-
 void launchExchangeGet(Fields F, const int* inv, const int* idx, long count, ExchangeFields ef, double* out,
                        cudaStream_t s, LaunchCounter* lc) {
   if (count <= 0) return;
@@ -1679,37 +2001,34 @@ void launchCountsOut(const int* counts, const int* orig, double* stage, long n, 
   lc->add(1);
 }
 
-void launchItemFlags(const uint32_t* keys, long n, int shift, const int* cellStart, int width, int* flag,
-                     cudaStream_t s, LaunchCounter* lc) {
-  itemFlagKernel<<<gridFor(n, 256), 256, 0, s>>>(keys, n, shift, cellStart, width, flag);
-  lc->add(1);
-}
-void launchItemFill(const int* flag, const long long* pos, long n, int* items, cudaStream_t s, LaunchCounter* lc) {
-  itemFillKernel<<<gridFor(n, 256), 256, 0, s>>>(flag, pos, n, items);
-  lc->add(1);
-}
-void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, int nItems, const long long* dItems,
-                         int width, Grid g, const int* cellStart, const int* cellEnd, int* counts, int* maxCount,
-                         uint32_t* nbr, int cap, double ext2, bool tensor, const float4* box, const int* chunkOf,
+void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, int nItems, StepScratch* sc,
+                         int width, Grid g, const int* cellStart, const int* cellEnd, int* counts, uint32_t* nbr, int cap, double ext2, bool tensor, const float4* box, const int* chunkOf,
                          cudaStream_t s, LaunchCounter* lc) {
   float lo, hi;
   neighborBand(g, ext2, lo, hi);
+  if (!tensor) {
+    // four warps per item while the items alone would leave SMs idle (below
+    // ~16 items per SM): 3,375 nodes 60 -> see DESIGN table; one warp above
+    const bool wide = nItems < kWideItems;
+    const unsigned gb = wide ? (unsigned)nItems : (unsigned)((nItems + 3) / 4);
+#define SPH_NBM(WR, CW)                                                                                          \
+  neighborMaskKernel<WR, CW><<<gb, 128, 0, s>>>(F, P, items, nItems, width, g, cellStart, cellEnd, counts,     \
+                                                WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, sc, box, chunkOf)
+    if (nbr) { if (wide) SPH_NBM(true, 4); else SPH_NBM(true, 1); }
+    else { if (wide) SPH_NBM(false, 4); else SPH_NBM(false, 1); }
+#undef SPH_NBM
+    lc->add(1);
+    return;
+  }
   const long threads = (long)nItems * width;
   const unsigned gb = (unsigned)((threads + 127) / 128);
-#define SPH_NBR(WR, WD, TE)                                                                                        \
-  neighborWarpKernel<WR, WD, TE><<<gb, 128, 0, s>>>(F, P, n, items, nItems, g, cellStart, cellEnd, counts,        \
-                                                    WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, maxCount, dItems, \
-                                                    box, chunkOf)
-  if (tensor) {
-    if (nbr) {
-      if (width == 8) SPH_NBR(true, 8, true); else if (width == 16) SPH_NBR(true, 16, true); else SPH_NBR(true, 32, true);
-    } else {
-      if (width == 8) SPH_NBR(false, 8, true); else if (width == 16) SPH_NBR(false, 16, true); else SPH_NBR(false, 32, true);
-    }
-  } else if (nbr) {
-    if (width == 8) SPH_NBR(true, 8, false); else if (width == 16) SPH_NBR(true, 16, false); else SPH_NBR(true, 32, false);
+#define SPH_NBR(WR, WD)                                                                                            \
+  neighborWarpKernel<WR, WD, true><<<gb, 128, 0, s>>>(F, P, n, items, nItems, g, cellStart, cellEnd, counts,      \
+                                                      WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, sc, box, chunkOf)
+  if (nbr) {
+    if (width == 8) SPH_NBR(true, 8); else if (width == 16) SPH_NBR(true, 16); else SPH_NBR(true, 32);
   } else {
-    if (width == 8) SPH_NBR(false, 8, false); else if (width == 16) SPH_NBR(false, 16, false); else SPH_NBR(false, 32, false);
+    if (width == 8) SPH_NBR(false, 8); else if (width == 16) SPH_NBR(false, 16); else SPH_NBR(false, 32);
   }
 #undef SPH_NBR
   lc->add(1);

@@ -23,25 +23,7 @@ using namespace dev;
 
 __global__ void prepareKernel(Fields F, Fields32 P, long n, Grid g) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  // the same mirror values as the update kernel writes, by the same
-  // integer-pipe conversions (the FP64 pipe bounds this kernel otherwise)
-  int c[3];
-  unpackCell(P.cell[i], c);
-  const double ox = g.lo[0] + smallIntToDouble(c[0]) * g.cell[0];
-  const double oy = g.lo[1] + smallIntToDouble(c[1]) * g.cell[1];
-  const double oz = g.lo[2] + smallIntToDouble(c[2]) * g.cell[2];
-  P.posh[i] = make_float4(toFloatRN(F.f[F_X][i] - ox), toFloatRN(F.f[F_Y][i] - oy), toFloatRN(F.f[F_Z][i] - oz),
-                          toFloatRN(F.f[F_HINV][i]));
-  P.velm[i] = make_float4(toFloatRN(F.f[F_VX][i]), toFloatRN(F.f[F_VY][i]), toFloatRN(F.f[F_VZ][i]),
-                          toFloatRN(F.f[F_MASS][i]));
-  // omega / (omega^2 + 1e-30) in FP32: an FP64 division here would cost
-  // more on the narrow FP64 pipe than the rest of the kernel
-  const float om = toFloatRN(F.f[F_OMEGA][i]);
-  P.thermo[i] = make_float4(toFloatRN(F.f[F_RHO][i]), toFloatRN(F.f[F_P][i]), toFloatRN(F.f[F_CS][i]),
-                            om / (om * om + 1.0e-30f));
-  if (P.hten) writeTensorMirror(F, P, i);
-  if (P.vol) P.vol[i] = toFloatRN(F.f[F_VOL][i]);
+  if (i < n) writeMirrors(F, i, P, i, P.cell[i], g, true);
 }
 
 //------------------------------------------------------------------------------
@@ -65,6 +47,16 @@ __device__ __forceinline__ void lookupPacked(const float4* __restrict__ ta, cons
   }
 }
 
+// The packed table in shared memory with a zero interval behind it: an eta at
+// or beyond the extent reads zeros, no branch.
+constexpr int kTab32 = kMaxTable / 3 + 1;
+__device__ __forceinline__ void loadTable32(float4* ta, float2* tb, const TableDev& t, int N1) {
+  for (int k = threadIdx.x; k <= N1 + 1; k += blockDim.x) {
+    ta[k] = k <= N1 ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tb) tb[k] = k <= N1 ? t.p32b[k] : make_float2(0.f, 0.f);
+  }
+}
+
 // TENSOR (ASPH): H_i, H_j from the FP32 tensor mirror (eta = H r,
 // grad W = gW H eta^, both in a fixed order so the pair force stays bitwise
 // antisymmetric), the second moment of ASPHClassicSmoothingScale and its
@@ -84,10 +76,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
                                                       float* __restrict__ pacc) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
   const int nint = hp.tableN1 + 1;
   for (int k = threadIdx.x; k < nint; k += blockDim.x) { ta[k] = t.p32a[k]; tb[k] = t.p32b[k]; }
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
   __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -133,7 +123,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
                   long long k) {
     const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
     float rx, ry, rz;
-    relSepTab(pi, pj, dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
+    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
     float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
     mirrorVel((uint32_t)dcode & mm, vxj, vyj, vzj);
     const float aj = pj.w, mj = vj4.w, rhoj = thj.x, Pj = thj.y, csj = thj.z, sOj = thj.w;
@@ -256,9 +246,10 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     sumAdd(sdy, cdy, pay, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
     sumAdd(sdz, cdz, paz, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
     if (COMPAT) {
-      pacc[3 * k] = pax;
-      pacc[3 * k + 1] = pay;
-      pacc[3 * k + 2] = paz;
+      float* out = pacc + paccSlot(k);
+      out[0] = pax;
+      out[32] = pay;
+      out[64] = paz;
     }
     const float vg = vx * gwix + vy * gwiy + vz * gwiz;
     sumAdd(se, ce, mj * (Prhoi + qai) * vg, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
@@ -379,283 +370,755 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
 }
 
 //------------------------------------------------------------------------------
-// Density sum, FP32 (computeSPHSumMassDensity.cc:15-87, gathered).
+// SPH pair loop for isotropic H (src/SPH/SPH.cc:294-470) + SPHSmoothingScale
+// moments, FP32.  With H = a I both kernel gradients lie along the separation,
+// grad W = a^4 W'(a |r|) r / |r|, so the pair reduces to scalars times r:
+//
+//   u     = m_j W'_i / |r|              (velocity gradient, M, grad rho)
+//   mu    = a min(v . r, 0) / (a^2 r^2 + eps2),  e = mu (Cq mu - Cl c)
+//   C     = Prho + e / (2 rho)          (both sides)
+//   g     = -m_j (C_i a_i^4 W'_i + C_j a_j^4 W'_j) / |r|,  a_ij = g r.
+//
+// The scalar in brackets is formed from commutative operations on values both
+// sides of the pair compute alike, and r is bitwise antisymmetric, so for
+// equal masses slot (j, i) holds the bitwise negation of slot (i, j).
+//
+// The limited Q's velocity correction enters only through v . r:
+// v_q . r = v . r - 2 phi (q_i + q_j), q = h^T DvDx h, h = r/2, so the Q's
+// DvDx is read as its symmetric part, and the van Leer factor of the ratios
+// q_i/q_j and q_j/q_i is 4 q_i q_j / (q_i + q_j)^2 for q_i q_j > 0, else 0.
+//
+// L lanes per node, U slots per iteration (their gathers issued together, the
+// next iteration's entries loaded ahead).  KERN 1: cubic B-spline in
+// registers, its normalisation A carried by Prho and 1 / (2 rho) (pairInputs32)
+// and applied to the other sums per node; 0: packed table.  LEAN: compensated sums, no tensile correction
+// and the standard Q expansion fixed at compile time; otherwise read from hp.
 //------------------------------------------------------------------------------
-template <bool TENSOR>
-__global__ void __launch_bounds__(128) sumDensityKernel32(Fields F, Fields32 P, const int* __restrict__ list, long n,
-                                                          Grid g, NeighborLists nl, TableDev t, HydroParams hp) {
-  __shared__ float tw[kMaxTable];
-  const int ntab = 3 * (hp.tableN1 + 1);
-  for (int k = threadIdx.x; k < ntab; k += blockDim.x) tw[k] = t.w32[k];
-  __syncthreads();
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int ci[3];
-  unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i];
-  const float mi = P.velm[i].w;
-  const bool multi = hp.numLists > 1;
-  const int li = multi ? list[i] : 0;
-  const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
-  const int N1 = hp.tableN1;
-  float s = 0.f, c = 0.f;
-  const int cnt = nl.count[i];
-  for (int q = 0; q < cnt; ++q) {
-    const long long k = nbSlot(i, q, nl.cap);
-    const uint32_t ent = nl.nbr[k];
-    const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-    const float4 pj = P.posh[j];
-    float rx, ry, rz;
-    relSep(pi, pj, dcode, mm, cx, cy, cz, rx, ry, rz);
-    float eta, Hdj;
-    if (TENSOR) {   // |H_j r| with H_j through the mirrors
-      float4 h0, h1;
-      loadTensor32(P, j, (uint32_t)dcode & mm, h0, h1);
-      eta = sqrtf(eta2Sym32(h0, h1, rx, ry, rz));
-      Hdj = h1.z;
+template <int KERN>
+struct Kernel32 {
+  const float4* ta;
+  const float2* tb;
+  int N1;
+  float invStep;
+  __device__ __forceinline__ int index(float eta) const { return min(N1 + 1, (int)(eta * invStep)); }
+  __device__ __forceinline__ float value(float eta) const {
+    if (KERN) return bsplineW(eta);
+    const float4 A = ta[index(eta)];
+    return __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
+  }
+  __device__ __forceinline__ void both(float eta, float& w, float& g) const {
+    if (KERN) {
+      w = bsplineW(eta);
+      g = bsplineGrad(eta);
     } else {
-      const float aj = pj.w;
-      eta = aj * sqrtf(rx * rx + ry * ry + rz * rz);
-      Hdj = aj * aj * aj;
-    }
-    if (eta < extent) {
-      const int i0 = 3 * min(N1, (int)(eta * invStep));
-      const float w = Hdj * (tw[i0] + (tw[i0 + 1] + tw[i0 + 2] * eta) * eta);
-      sumAdd(s, c, ((multi ? list[j] == li : true) ? P.velm[j].w : mi) * w, hp.plainSums);
+      const int k = index(eta);
+      const float4 A = ta[k];
+      const float2 B = tb[k];
+      w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
+      g = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
     }
   }
-  const double a = F.f[F_HINV][i];
-  const double Hdeti = TENSOR ? symDet(loadSym(F, F_HT_XX, i)) : (a * a) * a;
-  const double self = F.f[F_MASS][i] * (Hdeti * hp.W0);
-  const double rho = self + kahanValue(s, c);
-  F.f[F_RHO][i] = rho;
-  P.thermo[i].x = (float)rho;
+  __device__ __forceinline__ float grad(float eta) const {
+    if (KERN) return bsplineGrad(eta);
+    const int k = index(eta);
+    const float2 B = tb[k];
+    return __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, ta[k].w);
+  }
+};
+
+template <bool XSPH, bool COMPAT, bool MULTI, bool LIMQ, bool LEAN, bool MIR, int KERN, int L, int U, int MINB>
+__global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 P, const int* __restrict__ list, long n,
+                                                             Grid g, NeighborLists nl, TableDev t, HydroParams hp,
+                                                             float* __restrict__ pacc) {
+  constexpr int NT = KERN ? 1 : kTab32;
+  __shared__ float4 ta[NT];
+  __shared__ float2 tb[NT];
+  if (!KERN) loadTable32(ta, tb, t, hp.tableN1);
+  __syncthreads();
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  if (L == 1 && !live) return;
+  const long i = live ? node : n - 1;   // whole groups run to the shuffles
+  const Kernel32<KERN> K{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};
+  int ci[3];
+  unpackCell(P.cell[i], ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
+  const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i];
+  const int li = MULTI ? list[i] : 0;
+  const float ai = pi.w, mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w;
+  const float ai2 = ai * ai, A4i = __fmul_rn(ai2, ai2);
+  const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
+  const float epsT = (float)hp.epsTensile, iWnPerh = 1.0f / (float)hp.WnPerh;
+  const float etaCrit = (float)hp.etaCrit, iFold = 1.0f / (float)hp.etaFold;
+  float4 qa = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 qb = make_float2(0.f, 0.f);
+  if (LIMQ) {
+    qa = P.dvq[2 * i];
+    const float4 q1 = P.dvq[2 * i + 1];
+    qb = make_float2(q1.x, q1.y);
+  }
+  PairSums32 a;
+  a.w = a.mw = a.ve = a.g0 = a.m1x = a.m1y = a.m1z = a.gx = a.gy = a.gz = a.maxE = 0.f;
+  a.xw = a.xdx = a.xdy = a.xdz = 0.f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) a.D[k] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) a.M[k] = 0.f;
+  float sdx = 0.f, cdx = 0.f, sdy = 0.f, cdy = 0.f, sdz = 0.f, cdz = 0.f, se = 0.f, ce = 0.f;
+  const int plain = LEAN ? 0 : hp.plainSums;
+
+  auto slot = [&](uint32_t ent, const float4& pj, const float4& vj4, const float4& kj, const float4& q0,
+                  const float4& q1, float* out) {
+    const uint32_t dcode = ent >> kIndexBits;
+    float rx, ry, rz;
+    relSepEntry<MIR>(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
+    float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
+    if (MIR) mirrorVel(dcode & mm, vxj, vyj, vzj);
+    const float aj = pj.w, mj = vj4.w, rhoj = kj.x, Prhoj = kj.y, mClcj = kj.z, hirj = kj.w;
+    const bool same = MULTI ? (list[ent & kIndexMask] == li) : true;
+    const float r2 = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
+    const float ir = rsqrtf(fmaxf(r2, 1.0e-36f));
+    const float rm = __fmul_rn(r2, ir);
+    const float etai = __fmul_rn(ai, rm), etaj = __fmul_rn(aj, rm);
+    float w, gi;
+    K.both(etai, w, gi);
+    float wj = 0.f, gj;
+    if (XSPH) K.both(etaj, wj, gj);
+    else gj = K.grad(etaj);
+    const float aj2 = __fmul_rn(aj, aj);
+    const float Gi = __fmul_rn(A4i, gi), Gj = __fmul_rn(__fmul_rn(aj2, aj2), gj);
+    const float vx = vi.x - vxj, vy = vi.y - vyj, vz = vi.z - vzj;
+    const float vr = __fmaf_rn(vz, rz, __fmaf_rn(vy, ry, __fmul_rn(vx, rx)));
+    float vq = vr;
+    if (LIMQ) {
+      float jxy = q0.w, jxz = q1.x, jyz = q1.y;
+      const uint32_t mq = dcode & mm;
+      if (MIR && mq) {
+        const float sx = (mq & 3u) ? -1.f : 1.f, sy = (mq & 12u) ? -1.f : 1.f, sz = (mq & 48u) ? -1.f : 1.f;
+        jxy *= sx * sy; jxz *= sx * sz; jyz *= sy * sz;
+      }
+      const float xx = __fmul_rn(rx, rx), yy = __fmul_rn(ry, ry), zz = __fmul_rn(rz, rz);
+      const float xy = __fmul_rn(rx, ry), xz = __fmul_rn(rx, rz), yz = __fmul_rn(ry, rz);
+      const float gri = __fmaf_rn(qb.y, yz, __fmaf_rn(qb.x, xz, __fmaf_rn(qa.w, xy,
+                        __fmaf_rn(qa.z, zz, __fmaf_rn(qa.y, yy, __fmul_rn(qa.x, xx))))));
+      const float grj = __fmaf_rn(jyz, yz, __fmaf_rn(jxz, xz, __fmaf_rn(jxy, xy,
+                        __fmaf_rn(q0.z, zz, __fmaf_rn(q0.y, yy, __fmul_rn(q0.x, xx))))));
+      // phi = 4 x (1 - x) with x = q_i / (q_i + q_j), as a symmetric product
+      const float sum = __fadd_rn(gri, grj);
+      const float inv = __frcp_rn(sum);
+      float phi = __fmul_rn(4.0f, __fmul_rn(__fmul_rn(gri, inv), __fmul_rn(grj, inv)));
+      if (!(phi > 0.f) || fabsf(sum) < 2.0e-30f) phi = 0.f;
+      const float etaij = fminf(etai, etaj);
+      if (etaij < etaCrit) {
+        const float z = __fmul_rn(etaij - etaCrit, iFold);
+        phi *= expf(-(z * z));
+      }
+      vq = __fmaf_rn(-2.0f * phi, sum, vr);
+    }
+    const float di = __fmaf_rn(etai, etai, eps2), dj = __fmaf_rn(etaj, etaj, eps2);
+    float ei, ej;
+    if (LEAN) {
+      const float vn = fminf(vq, 0.f);
+      const float mni = __fdividef(__fmul_rn(ai, vn), di), mnj = __fdividef(__fmul_rn(aj, vn), dj);
+      ei = __fmul_rn(mni, __fmaf_rn(Cq, mni, mClci));
+      ej = __fmul_rn(mnj, __fmaf_rn(Cq, mnj, mClcj));
+    } else {
+      const float mui = __fdividef(__fmul_rn(ai, vq), di), muj = __fdividef(__fmul_rn(aj, vq), dj);
+      const float mni = fminf(0.f, mui), mnj = fminf(0.f, muj);
+      const float li_ = hp.linearInExpansion ? mui : mni, lj_ = hp.linearInExpansion ? muj : mnj;
+      const float qi_ = hp.quadraticInExpansion ? -(mui < 0.f ? -1.f : 1.f) * mui * mui : mni * mni;
+      const float qj_ = hp.quadraticInExpansion ? -(muj < 0.f ? -1.f : 1.f) * muj * muj : mnj * mnj;
+      ei = __fmaf_rn(Cq, qi_, __fmul_rn(mClci, li_));
+      ej = __fmaf_rn(Cq, qj_, __fmul_rn(mClcj, lj_));
+    }
+    float pri = Prhoi, prj = Prhoj;
+    if (!LEAN && epsT != 0.f) {   // P_eff = P (1 - epsT (W / W(1/nPerh))^4) in tension
+      float wjt = wj;
+      if (!XSPH) { float gt; K.both(etaj, wjt, gt); }
+      const float ti = w * iWnPerh, tj = wjt * iWnPerh;
+      if (pri < 0.f) pri = __fmul_rn(pri, 1.0f - epsT * ((ti * ti) * (ti * ti)));
+      if (prj < 0.f) prj = __fmul_rn(prj, 1.0f - epsT * ((tj * tj) * (tj * tj)));
+    }
+    const float Ci = __fmaf_rn(ei, hiri, pri), Cj = __fmaf_rn(ej, hirj, prj);
+    const float S = __fmul_rn(__fadd_rn(__fmul_rn(Ci, Gi), __fmul_rn(Cj, Gj)), ir);
+    const float gf = __fmul_rn(-mj, S);
+    const float pax = __fmul_rn(gf, rx), pay = __fmul_rn(gf, ry), paz = __fmul_rn(gf, rz);
+    if (COMPAT) { out[0] = pax; out[32] = pay; out[64] = paz; }
+    sumAdd(sdx, cdx, pax, plain);
+    sumAdd(sdy, cdy, pay, plain);
+    sumAdd(sdz, cdz, paz, plain);
+    const float u = mj * (gi * ir);
+    sumAdd(se, ce, __fmul_rn(Ci, __fmul_rn(u, vr)), plain);
+    const float ux = u * rx, uy = u * ry, uz = u * rz;
+    a.D[0] += vx * ux; a.D[1] += vx * uy; a.D[2] += vx * uz;
+    a.D[3] += vy * ux; a.D[4] += vy * uy; a.D[5] += vy * uz;
+    a.D[6] += vz * ux; a.D[7] += vz * uy; a.D[8] += vz * uz;
+    a.M[0] += rx * ux; a.M[1] += rx * uy; a.M[2] += rx * uz;
+    a.M[3] += ry * uy; a.M[4] += ry * uz; a.M[5] += rz * uz;
+    const float dr = rhoj - rhoi;
+    a.gx += dr * ux; a.gy += dr * uy; a.gz += dr * uz;
+    if (same) {
+      a.w += w;
+      a.mw += mj * w;
+    }
+    a.ve += (mj * hirj) * (ei * w);
+    a.maxE = fmaxf(a.maxE, ei);
+    if (XSPH) {
+      const float wx = 0.5f * (2.0f * mi * hiri * (ai2 * ai) * w + 2.0f * mj * hirj * (aj2 * aj) * wj);
+      a.xw += wx;
+      a.xdx -= wx * vx; a.xdy -= wx * vy; a.xdz -= wx * vz;
+    }
+    float wg = fabsf(gi);
+    if (MULTI && !same) wg *= mj * rhoi / (mi * rhoj);
+    a.g0 += wg;
+    a.m1x += wg * rx; a.m1y += wg * ry; a.m1z += wg * rz;
+  };
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int cnt = live ? nl.count[i] : 0;
+  const int mine = (cnt - sub + L - 1) / L;   // slots of this lane
+  const long long s0 = nbSlot(i, 0, nl.cap) + 32 * sub;
+  const uint32_t* __restrict__ nb = nl.nbr + s0;
+  float* out = COMPAT ? pacc + paccSlot(s0) : nullptr;
+  constexpr int ST = 32 * L;
+  uint32_t nx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) nx[u] = u < mine ? nb[u * ST] : 0u;
+  int q = 0;
+  for (; q + U <= mine; q += U) {
+    uint32_t e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = nx[u];
+    float4 pp[U], vv[U], kk[U], q0[U], q1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t j = e[u] & kIndexMask;
+      pp[u] = P.posh[j]; vv[u] = P.velm[j]; kk[u] = P.pk[j];
+      q0[u] = LIMQ ? P.dvq[2 * j] : zero4;
+      q1[u] = LIMQ ? P.dvq[2 * j + 1] : zero4;
+    }
+    nb += U * ST;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (q + U + u < mine) nx[u] = nb[u * ST];
+#pragma unroll
+    for (int u = 0; u < U; ++u) slot(e[u], pp[u], vv[u], kk[u], q0[u], q1[u], out + 3 * u * ST);
+    if (COMPAT) out += 3 * U * ST;
+  }
+  if (U > 1) {
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u) {
+      if (q + u < mine) {
+        const uint32_t j = nx[u] & kIndexMask;
+        slot(nx[u], P.posh[j], P.velm[j], P.pk[j], LIMQ ? P.dvq[2 * j] : zero4, LIMQ ? P.dvq[2 * j + 1] : zero4,
+             out + 3 * u * ST);
+      }
+    }
+  }
+  if (L > 1) {
+    a.w = laneSum<L>(a.w); a.mw = laneSum<L>(a.mw); a.ve = laneSum<L>(a.ve); a.g0 = laneSum<L>(a.g0);
+    a.m1x = laneSum<L>(a.m1x); a.m1y = laneSum<L>(a.m1y); a.m1z = laneSum<L>(a.m1z);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) a.D[k] = laneSum<L>(a.D[k]);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) a.M[k] = laneSum<L>(a.M[k]);
+    a.gx = laneSum<L>(a.gx); a.gy = laneSum<L>(a.gy); a.gz = laneSum<L>(a.gz);
+    a.maxE = laneMax<L>(a.maxE);
+    if (XSPH) {
+      a.xw = laneSum<L>(a.xw); a.xdx = laneSum<L>(a.xdx); a.xdy = laneSum<L>(a.xdy); a.xdz = laneSum<L>(a.xdz);
+    }
+    laneSumKahan<L>(sdx, cdx); laneSumKahan<L>(sdy, cdy); laneSumKahan<L>(sdz, cdz); laneSumKahan<L>(se, ce);
+    if (sub != 0 || !live) return;
+  }
+  a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
+  a.deps = kahanValue(se, ce);
+  finalizePair32<KERN == 1>(F, i, MULTI ? li : list[i], a, ai, mi, rhoi, cnt, hp, t.herm);
 }
 
 //------------------------------------------------------------------------------
-// Fused start-of-step sweep of the mixed mode: the density sum
-// (computeSPHSumMassDensity.cc:15-87) and the time-step vote
-// (GenericHydro.cc:113-381, pairwise velocity limit on the same neighbour
-// data, node limits with the new density) in one pass over the lists.
+// The same pair loop in the arithmetic of the earlier releases: W and W' from
+// the table at |a r| of each side, grad W_i and grad W_j as vectors, the pair
+// force added componentwise, one lane per node.  A node whose energy rate
+// cancels to rounding takes its share of a pair's work by the sign of that
+// rounding (SpecificThermalEnergyPolicy's weights), a 1e-3 change of its
+// energy; some node of a large run is always that close, so large runs keep
+// these roundings (kExactNodes) and small ones take the cheaper form above.
+// Per-node values (rho, Prho, -Cl c, 1/rho) come from the record, mirror
+// tests and table branches are gone and the accelerations go out in planes:
+// 2.69 -> see launchPairFP32 for the measured times.
 //------------------------------------------------------------------------------
-template <bool TENSOR, bool LEAN>
-__global__ void __launch_bounds__(128) densityDtKernel32(Fields F, Fields32 P, const int* __restrict__ list, long n,
-                                                         Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                                                         double maxNperh, double* __restrict__ part) {
-  __shared__ float tw[kMaxTable];
-  __shared__ double sv[128];
-  __shared__ int sr[128];
-  const int ntab = 3 * (hp.tableN1 + 1);
-  for (int k = threadIdx.x; k < ntab; k += blockDim.x) tw[k] = t.w32[k];
+template <bool LIMQ, bool MIR, bool SPLINE, int U, int MINB>
+__global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32 P, const int* __restrict__ list,
+                                                              long n, Grid g, NeighborLists nl, TableDev t,
+                                                              HydroParams hp, float* __restrict__ pacc) {
+  __shared__ float4 tg[kTab32];   // (g0, g1, g2, w0)
+  __shared__ float2 tw[SPLINE ? 1 : kTab32];
+  for (int k = threadIdx.x; k <= hp.tableN1 + 1; k += blockDim.x) {
+    const bool in = k <= hp.tableN1;
+    const float4 A = in ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 B = in ? t.p32b[k] : make_float2(0.f, 0.f);
+    tg[k] = make_float4(A.w, B.x, B.y, A.x);
+    if (!SPLINE) tw[k] = make_float2(A.y, A.z);
+  }
   __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  double best = DBL_MAX;
-  int reason = -1;
-  if (i < n) {
-    int ci[3];
-    unpackCell(P.cell[i], ci);
-    const uint32_t mm = mirrorMask(g, ci);
-    const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-    const float4 pi = P.posh[i], vi = P.velm[i];
-    const float mi = vi.w;
-    const bool multi = !LEAN && hp.numLists > 1;
-    const int li = multi ? list[i] : 0;
-    const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
-    const int N1 = hp.tableN1;
-    float s = 0.f, c = 0.f, worstPair = 0.0f;
-    // the node scale of GenericHydro::dt: 1/h, the largest eigenvalue of H
-    const float lmaxi = TENSOR ? P.hten[2 * i + 1].w : pi.w;
-    const int cnt = nl.count[i];
-    // software pipeline: entry two slots ahead, node data one slot ahead
-    uint32_t entA = 0u, entB = 0u;
-    float4 pjA = make_float4(0.f, 0.f, 0.f, 0.f), vjA = pjA, hA0 = pjA, hA1 = pjA;
-    if (cnt > 0) {
-      entA = nl.nbr[nbSlot(i, 0, nl.cap)];
-      const int j0 = (int)(entA & kIndexMask);
-      pjA = P.posh[j0]; vjA = P.velm[j0];
-      if (TENSOR) { hA0 = P.hten[2 * j0]; hA1 = P.hten[2 * j0 + 1]; }
-    }
-    if (cnt > 1) entB = nl.nbr[nbSlot(i, 1, nl.cap)];
-    for (int q = 0; q < cnt; ++q) {
-      const uint32_t ent = entA;
-      const float4 pj = pjA, vj = vjA;
-      float4 h0 = hA0, h1 = hA1;
-      if (q + 1 < cnt) {
-        const int jn = (int)(entB & kIndexMask);
-        pjA = P.posh[jn]; vjA = P.velm[jn];
-        if (TENSOR) { hA0 = P.hten[2 * jn]; hA1 = P.hten[2 * jn + 1]; }
-        entA = entB;
-      }
-      if (q + 2 < cnt) entB = nl.nbr[nbSlot(i, q + 2, nl.cap)];
-      const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-      float rx, ry, rz;
-      relSep(pi, pj, dcode, mm, cx, cy, cz, rx, ry, rz);
-      float eta, Hdj, lmaxj;
-      if (TENSOR) {   // |H_j r| with H_j through the mirrors
-        const uint32_t mq = (uint32_t)dcode & mm;
-        if (mq) {
-          const float sx = (mq & 3u) ? -1.f : 1.f, sy = (mq & 12u) ? -1.f : 1.f, sz = (mq & 48u) ? -1.f : 1.f;
-          h0.y *= sx * sy;
-          h0.z *= sx * sz;
-          h1.x *= sy * sz;
+  if (i >= n) return;
+  const int N1 = hp.tableN1;
+  const float invStep = (float)(1.0 / hp.tableXstep);
+  int ci[3];
+  unpackCell(P.cell[i], ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
+  const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i];
+  const float ai = pi.w, mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w;
+  const float Hdeti = ai * ai * ai;
+  const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
+  const float etaCrit = (float)hp.etaCrit, etaFold = (float)hp.etaFold;
+  float DQi[9];   // the limited Q's DvDx of node i
+  if (LIMQ) {
+    const float4 d0 = P.dvq[3 * i], d1 = P.dvq[3 * i + 1], d2 = P.dvq[3 * i + 2];
+    DQi[0] = d0.x; DQi[1] = d0.y; DQi[2] = d0.z; DQi[3] = d0.w;
+    DQi[4] = d1.x; DQi[5] = d1.y; DQi[6] = d1.z; DQi[7] = d1.w; DQi[8] = d2.x;
+  }
+  float sw = 0.f, smw = 0.f, sve = 0.f, maxE = 0.f;
+  float sdx = 0.f, cdx = 0.f, sdy = 0.f, cdy = 0.f, sdz = 0.f, cdz = 0.f, se = 0.f, ce = 0.f;
+  float gx = 0.f, gy = 0.f, gz = 0.f, m0 = 0.f, m1x = 0.f, m1y = 0.f, m1z = 0.f;
+  float D[9], M[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { D[k] = 0.f; M[k] = 0.f; }
+  const int cnt = nl.count[i];
+  float* out = pacc + paccSlot(nbSlot(i, 0, nl.cap));
+  struct Rec {
+    float4 p, v, k, d0, d1, d2;
+  };
+  laneSlots<1, U, Rec>(
+      nl, i, 0, cnt,
+      [&](uint32_t j, Rec& r) {
+        r.p = P.posh[j];
+        r.v = P.velm[j];
+        r.k = P.pk[j];
+        if (LIMQ) { r.d0 = P.dvq[3 * j]; r.d1 = P.dvq[3 * j + 1]; r.d2 = P.dvq[3 * j + 2]; }
+      },
+      [&](uint32_t ent, const Rec& q) {
+        const uint32_t dcode = ent >> kIndexBits;
+        float rx, ry, rz;
+        relSepEntry<MIR>(pi, q.p, ent, mm, cx, cy, cz, rx, ry, rz);
+        float vxj = q.v.x, vyj = q.v.y, vzj = q.v.z;
+        if (MIR) mirrorVel(dcode & mm, vxj, vyj, vzj);
+        const float aj = q.p.w, mj = q.v.w, rhoj = q.k.x, Prhoj = q.k.y, mClcj = q.k.z, hirj = q.k.w;
+        const float Hdetj = aj * aj * aj;
+        const float eix = ai * rx, eiy = ai * ry, eiz = ai * rz;
+        const float ejx = aj * rx, ejy = aj * ry, ejz = aj * rz;
+        const float e2i = __fmaf_rn(eiz, eiz, __fmaf_rn(eiy, eiy, __fmul_rn(eix, eix)));
+        const float e2j = __fmaf_rn(ejz, ejz, __fmaf_rn(ejy, ejy, __fmul_rn(ejx, ejx)));
+        const float ri = rsqrtf(fmaxf(e2i, 1.0e-30f)), rj = rsqrtf(fmaxf(e2j, 1.0e-30f));
+        const float etai = __fmul_rn(e2i, ri), etaj = __fmul_rn(e2j, rj);
+        const int ti = min(N1 + 1, (int)(etai * invStep));
+        const float4 Gi = tg[ti], Gj = tg[min(N1 + 1, (int)(etaj * invStep))];
+        const float gi = __fmaf_rn(__fmaf_rn(Gi.z, etai, Gi.y), etai, Gi.x);
+        const float gj = __fmaf_rn(__fmaf_rn(Gj.z, etaj, Gj.y), etaj, Gj.x);
+        // W feeds only massDensitySum, normalization and effViscousPressure
+        float w;
+        if (SPLINE) w = bsplineW(etai);
+        else w = __fmaf_rn(__fmaf_rn(tw[ti].y, etai, tw[ti].x), etai, Gi.w);
+        const float fi = __fmul_rn(__fmul_rn(__fmul_rn(Hdeti, gi), ai), ri);
+        const float fj = __fmul_rn(__fmul_rn(__fmul_rn(Hdetj, gj), aj), rj);
+        const float gwix = fi * eix, gwiy = fi * eiy, gwiz = fi * eiz;
+        const float gwjx = fj * ejx, gwjy = fj * ejy, gwjz = fj * ejz;
+        const float vx = vi.x - vxj, vy = vi.y - vyj, vz = vi.z - vzj;
+        float vqx = vx, vqy = vy, vqz = vz;
+        if (LIMQ) {
+          // LimitedMonaghanGingoldViscosity.cc:171-200 in a form symmetric in
+          // (i, j): v_q = v_ij - phi (DvDx_i + DvDx_j) x_ij with x_ij = r/2
+          float Dj[9] = {q.d0.x, q.d0.y, q.d0.z, q.d0.w, q.d1.x, q.d1.y, q.d1.z, q.d1.w, q.d2.x};
+          const uint32_t mq = dcode & mm;
+          if (MIR && mq) {
+            const float sg[3] = {(mq & 3u) ? -1.f : 1.f, (mq & 12u) ? -1.f : 1.f, (mq & 48u) ? -1.f : 1.f};
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+              for (int cc = 0; cc < 3; ++cc) Dj[3 * r + cc] *= sg[r] * sg[cc];
+          }
+          const float hx = 0.5f * rx, hy = 0.5f * ry, hz = 0.5f * rz;
+          const float aix = __fmaf_rn(DQi[2], hz, __fmaf_rn(DQi[1], hy, __fmul_rn(DQi[0], hx)));
+          const float aiy = __fmaf_rn(DQi[5], hz, __fmaf_rn(DQi[4], hy, __fmul_rn(DQi[3], hx)));
+          const float aiz = __fmaf_rn(DQi[8], hz, __fmaf_rn(DQi[7], hy, __fmul_rn(DQi[6], hx)));
+          const float ajx = __fmaf_rn(Dj[2], hz, __fmaf_rn(Dj[1], hy, __fmul_rn(Dj[0], hx)));
+          const float ajy = __fmaf_rn(Dj[5], hz, __fmaf_rn(Dj[4], hy, __fmul_rn(Dj[3], hx)));
+          const float ajz = __fmaf_rn(Dj[8], hz, __fmaf_rn(Dj[7], hy, __fmul_rn(Dj[6], hx)));
+          const float gri = __fmaf_rn(aiz, hz, __fmaf_rn(aiy, hy, __fmul_rn(aix, hx)));
+          const float grj = __fmaf_rn(ajz, hz, __fmaf_rn(ajy, hy, __fmul_rn(ajx, hx)));
+          const float rri = __fdiv_rn(gri, (grj < 0.f ? -1.f : 1.f) * fmaxf(1.0e-30f, fabsf(grj)));
+          const float rrj = __fdiv_rn(grj, (gri < 0.f ? -1.f : 1.f) * fmaxf(1.0e-30f, fabsf(gri)));
+          const float xl = fminf(rri, rrj);
+          float phi = xl > 0.f ? __fdiv_rn(4.0f * xl, __fmul_rn(1.0f + xl, 1.0f + xl)) : 0.f;   // van Leer
+          const float etaij = fminf(etai, etaj);
+          if (etaij < etaCrit) {
+            const float z = __fdiv_rn(etaij - etaCrit, etaFold);
+            phi *= expf(-(z * z));
+          }
+          vqx = __fsub_rn(vx, __fmul_rn(phi, __fadd_rn(aix, ajx)));
+          vqy = __fsub_rn(vy, __fmul_rn(phi, __fadd_rn(aiy, ajy)));
+          vqz = __fsub_rn(vz, __fmul_rn(phi, __fadd_rn(aiz, ajz)));
         }
-        eta = etaFromSq(eta2Sym32(h0, h1, rx, ry, rz));
-        Hdj = h1.z;
-        lmaxj = h1.w;
-      } else {
-        const float aj = pj.w;
-        eta = aj * etaFromSq(rx * rx + ry * ry + rz * rz);
-        Hdj = aj * aj * aj;
-        lmaxj = aj;
-      }
-      if (eta < extent) {
-        const int i0 = 3 * min(N1, (int)(eta * invStep));
-        const float w = Hdj * (tw[i0] + (tw[i0 + 1] + tw[i0 + 2] * eta) * eta);
-        sumAdd(s, c, ((multi ? list[j] == li : true) ? vj.w : mi) * w, LEAN ? 0 : hp.plainSums);
-      }
-      float vxj = vj.x, vyj = vj.y, vzj = vj.z;
-      mirrorVel((uint32_t)dcode & mm, vxj, vyj, vzj);
-      const float dx = vi.x - vxj, dy = vi.y - vyj, dz = vi.z - vzj;
-      // min over pairs of min(h_i, h_j)/|v_ij| = 1/sqrt(max over pairs of
-      // (max(a_i, a_j) |v_ij|)^2): no division or root per pair
-      const float am = fmaxf(lmaxi, lmaxj);
-      worstPair = fmaxf(worstPair, (am * am) * (dx * dx + dy * dy + dz * dz));
+        const float mui = __fdividef(__fmaf_rn(vqz, eiz, __fmaf_rn(vqy, eiy, __fmul_rn(vqx, eix))), __fadd_rn(e2i, eps2));
+        const float muj = __fdividef(__fmaf_rn(vqz, ejz, __fmaf_rn(vqy, ejy, __fmul_rn(vqx, ejx))), __fadd_rn(e2j, eps2));
+        const float mni = fminf(0.f, mui), mnj = fminf(0.f, muj);
+        const float ei = __fmaf_rn(Cq, __fmul_rn(mni, mni), __fmul_rn(mClci, mni));
+        const float ej = __fmaf_rn(Cq, __fmul_rn(mnj, mnj), __fmul_rn(mClcj, mnj));
+        // (Prho_i + Q_i/2) gradW_i + (Prho_j + Q_j/2) gradW_j: commutative
+        // operations only, so slot (j, i) holds the bitwise negation
+        const float ci_ = __fadd_rn(Prhoi, __fmul_rn(ei, hiri)), cj_ = __fadd_rn(Prhoj, __fmul_rn(ej, hirj));
+        const float ddx = __fadd_rn(__fmul_rn(ci_, gwix), __fmul_rn(cj_, gwjx));
+        const float ddy = __fadd_rn(__fmul_rn(ci_, gwiy), __fmul_rn(cj_, gwjy));
+        const float ddz = __fadd_rn(__fmul_rn(ci_, gwiz), __fmul_rn(cj_, gwjz));
+        const float pax = __fmul_rn(-mj, ddx), pay = __fmul_rn(-mj, ddy), paz = __fmul_rn(-mj, ddz);
+        out[0] = pax; out[32] = pay; out[64] = paz;
+        out += 96;
+        kahanAdd(sdx, cdx, pax);
+        kahanAdd(sdy, cdy, pay);
+        kahanAdd(sdz, cdz, paz);
+        const float vg = vx * gwix + vy * gwiy + vz * gwiz;
+        kahanAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg));
+        const float mvx = mj * vx, mvy = mj * vy, mvz = mj * vz;
+        D[0] -= mvx * gwix; D[1] -= mvx * gwiy; D[2] -= mvx * gwiz;
+        D[3] -= mvy * gwix; D[4] -= mvy * gwiy; D[5] -= mvy * gwiz;
+        D[6] -= mvz * gwix; D[7] -= mvz * gwiy; D[8] -= mvz * gwiz;
+        const float mrx = mj * rx, mry = mj * ry, mrz = mj * rz;
+        M[0] -= mrx * gwix; M[1] -= mrx * gwiy; M[2] -= mrx * gwiz;
+        M[3] -= mry * gwix; M[4] -= mry * gwiy; M[5] -= mry * gwiz;
+        M[6] -= mrz * gwix; M[7] -= mrz * gwiy; M[8] -= mrz * gwiz;
+        const float gr = mj * (rhoj - rhoi);
+        gx += gr * gwix; gy += gr * gwiy; gz += gr * gwiz;
+        sw += w;
+        smw += mj * w;
+        sve += (mj * hirj) * (ei * w);
+        maxE = fmaxf(maxE, ei);
+        const float wg = fabsf(gi);
+        m0 += wg;
+        m1x -= wg * eix; m1y -= wg * eiy; m1z -= wg * eiz;
+      });
+  if (SPLINE) { sw = timesSplineA(sw); smw = timesSplineA(smw); sve = timesSplineA(sve); }
+  NodeAcc32 a;
+  a.rhoSum = Hdeti * smw; a.norm = mi * (2.0f * hiri) * Hdeti * sw;
+  a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
+  a.deps = kahanValue(se, ce);
+  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * Hdeti * sve;
+  a.xw = a.xdx = a.xdy = a.xdz = 0.f;
+  a.m0 = m0; a.m1x = m1x; a.m1y = m1y; a.m1z = m1z;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { a.D[k] = D[k]; a.M[k] = M[k]; }
+  finalizeNode32<false>(F, i, list[i], a, cnt, hp, t.herm);
+}
+
+// Per-node inputs of the isotropic pair loop: (rho, Omega^-1 P / rho^2,
+// -Cl c, 1 / (2 rho)), once per node instead of once per pair; with the
+// limited Q also the symmetric part of the Q's DvDx for h = r/2
+// (xx yy zz xy | xz yz, off-diagonal pairs summed), or for the exact form
+// (full) all nine components.  spline: times the cubic B-spline's A.
+__global__ void pairInputs32(Fields F, Fields32 P, long n, float Cl, int limitedQ, int spline, int full) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 th = P.thermo[i];
+  const float ir = __frcp_rn(th.x);
+  float pr = __fmul_rn(__fmul_rn(__fmul_rn(th.w, th.y), ir), ir), hir = 0.5f * ir;
+  if (spline) { pr = timesSplineA(pr); hir = timesSplineA(hir); }
+  P.pk[i] = make_float4(th.x, pr, __fmul_rn(-Cl, th.z), hir);
+  if (limitedQ) {
+    float v[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = toFloatRN(F.f[F_DVDXQ_XX + k][i]);
+    if (full) {
+      P.dvq[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
+      P.dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
+      P.dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
+      return;
     }
-    const float bestPair = worstPair > 0.0f ? rsqrtf(worstPair) : 3.0e38f;
-    const double a = F.f[F_HINV][i];
-    const double Hdeti = TENSOR ? symDet(loadSym(F, F_HT_XX, i)) : (a * a) * a;
-    const double rho = F.f[F_MASS][i] * (Hdeti * hp.W0) + kahanValue(s, c);
-    F.f[F_RHO][i] = rho;
-    P.thermo[i].x = (float)rho;
-    // Node limits of GenericHydro::dt in FP32 (the vote only picks the
-    // minimum; GB300's FP64 divide and square root sequences would dominate
-    // the sweep otherwise).
-    const float tiny = (float)DBL_EPSILON;
-    const NodeListParams L = hp.lists[multi ? li : list[i]];
-    const float nodeScalei = 1.0f / (lmaxi * (float)L.nPerh);
-    float bestf = 3.0e38f;
-    const float csDt = nodeScalei / (P.thermo[i].z + tiny);
-    if (csDt < bestf) { bestf = csDt; reason = 0; }
-    const float csqDt = nodeScalei / (sqrtf((float)F.f[F_MAXQ][i] / (float)rho) + tiny);
-    if (csqDt < bestf) { bestf = csqDt; reason = 1; }
-    const float divv = (float)(F.f[F_DVDX_XX][i] + F.f[F_DVDX_YY][i] + F.f[F_DVDX_ZZ][i]);
-    const float divvDt = 1.0f / (fabsf(divv) + tiny);
-    if (divvDt < bestf) { bestf = divvDt; reason = 2; }
-    const float vmag = sqrtf(vi.x * vi.x + vi.y * vi.y + vi.z * vi.z);
-    const float ax = (float)F.f[F_DVDT_X][i], ay = (float)F.f[F_DVDT_Y][i], az = (float)F.f[F_DVDT_Z][i];
-    const float dtAcc = 0.1f * fmaxf(nodeScalei / (vmag + tiny), vmag / (sqrtf(ax * ax + ay * ay + az * az) + tiny));
-    if (dtAcc < bestf) { bestf = dtAcc; reason = 3; }
-    if (hp.useVelMagDt) {
-      const float velDt = nodeScalei / (vmag + 1.0e-10f);
-      if (velDt < bestf) { bestf = velDt; reason = 4; }
-    }
-    const float pairDt = bestPair / (float)maxNperh;
-    if (pairDt < bestf) { bestf = pairDt; reason = 5; }
-    best = isGhost(hp, i) ? DBL_MAX : (double)bestf;   // halo copies do not vote
-    if (isGhost(hp, i)) reason = -1;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] *= 0.25f;
+    P.dvq[2 * i] = make_float4(v[0], v[4], v[8], v[1] + v[3]);
+    P.dvq[2 * i + 1] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
   }
-  sv[threadIdx.x] = best;
-  sr[threadIdx.x] = reason;
+}
+
+// Block size of the light sweeps.  With one lane per node a block of 512
+// consecutive nodes shares most of its neighbours, so more of its gathers hit
+// L1 than those of four separate blocks of 128 (2.1 M nodes: density/dt 1162 ->
+// 1029 us, energy 892 -> 860); small problems need the finer blocks to spread.
+__host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 512 : 128; }
+
+//------------------------------------------------------------------------------
+// Time-step vote.  The smallest limit travels as one 64-bit word, the bits of
+// a positive double order as integers: the mixed step's FP32 limits carry the
+// reason code in the low mantissa bits that a widened float leaves zero.
+//------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long warpMin64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w < v ? w : v;
+  }
+  return v;
+}
+__device__ __forceinline__ unsigned long long dtKey(double v, int reason) {
+  return ((unsigned long long)__double_as_longlong(v) & ~7ULL) | (unsigned)reason;
+}
+
+// FP32 node limits of GenericHydro::dt (GenericHydro.cc:113-381): the smallest
+// of them and of the pair limit, with its reason.  Every term is positive.
+__device__ __forceinline__ float nodeDt32(float ns, float cs, float maxQ, float rho, float divv, float vmag,
+                                          float amag, bool velDt, float pairDt, int& reason) {
+  const float tiny = (float)DBL_EPSILON;
+  float best = 3.0e38f;
+  reason = -1;
+  auto vote = [&](float v, int r) {
+    if (v < best) { best = v; reason = r; }
+  };
+  vote(ns / (cs + tiny), 0);
+  vote(ns / (sqrtf(maxQ / rho) + tiny), 1);
+  vote(1.0f / (fabsf(divv) + tiny), 2);
+  vote(0.1f * fmaxf(ns / (vmag + tiny), vmag / (amag + tiny)), 3);
+  if (velDt) vote(ns / (vmag + 1.0e-10f), 4);
+  vote(pairDt, 5);
+  return best;
+}
+
+// H_j through the mirrors of an entry (FP32 tensor mirror): the off-diagonal
+// components flip once per mirrored index.
+__device__ __forceinline__ void mirrorTensor32(uint32_t mq, float4& h0, float4& h1) {
+  if (mq) {
+    const float sx = (mq & 3u) ? -1.f : 1.f, sy = (mq & 12u) ? -1.f : 1.f, sz = (mq & 48u) ? -1.f : 1.f;
+    h0.y *= sx * sy;
+    h0.z *= sx * sz;
+    h1.x *= sy * sz;
+  }
+}
+
+struct SweepRec {   // a neighbour's record in the density / dt / grad-h sweeps
+  float4 p, v, h0, h1;
+};
+
+//------------------------------------------------------------------------------
+// Density sum (computeSPHSumMassDensity.cc:15-87, gathered) and, with DT, the
+// time-step vote of the same step (GenericHydro.cc:113-381: pairwise velocity
+// limit on the same neighbour data, node limits with the new density), in one
+// pass over the lists.  KERN 1: cubic B-spline in registers, else the table.
+// LEAN: one NodeList and compensated sums fixed at compile time.  L lanes per
+// node, U slots per iteration.  dtOut receives the smallest dtKey.
+//------------------------------------------------------------------------------
+template <bool TENSOR, bool DT, bool LEAN, bool MIR, int KERN, int L, int U>
+__global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Fields32 P, const int* __restrict__ list, long n,
+                                                       Grid g, NeighborLists nl, TableDev t, HydroParams hp,
+                                                       float maxNperh, unsigned long long* __restrict__ dtOut) {
+  constexpr int NT = KERN ? 1 : kTab32;
+  __shared__ float4 ta[NT];
+  __shared__ unsigned long long sv[sweepBlock(L) / 32];
+  if (!KERN) loadTable32(ta, nullptr, t, hp.tableN1);
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o && sv[threadIdx.x + o] < sv[threadIdx.x]) {
-      sv[threadIdx.x] = sv[threadIdx.x + o];
-      sr[threadIdx.x] = sr[threadIdx.x + o];
-    }
-    __syncthreads();
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  const long i = live ? node : n - 1;   // whole warps run to the shuffles
+  int ci[3];
+  unpackCell(P.cell[i], ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
+  const float4 pi = P.posh[i], vi = P.velm[i];
+  const bool multi = !LEAN && hp.numLists > 1;
+  const int li = multi ? list[i] : 0;
+  const Kernel32<KERN> K{ta, nullptr, hp.tableN1, (float)(1.0 / hp.tableXstep)};
+  float s = 0.f, c = 0.f, worst = 0.0f;
+  // the node scale of GenericHydro::dt: 1/h, the largest eigenvalue of H
+  const float lmaxi = TENSOR ? P.hten[2 * i + 1].w : pi.w;
+  const int cnt = live ? nl.count[i] : 0;
+  laneSlots<L, U, SweepRec>(
+      nl, i, sub, cnt,
+      [&](uint32_t j, SweepRec& r) {
+        r.p = P.posh[j];
+        r.v = P.velm[j];
+        if (TENSOR) { r.h0 = P.hten[2 * j]; r.h1 = P.hten[2 * j + 1]; }
+      },
+      [&](uint32_t ent, SweepRec& r) {
+        const uint32_t dcode = ent >> kIndexBits;
+        float rx, ry, rz;
+        relSepEntry<MIR>(pi, r.p, ent, mm, cx, cy, cz, rx, ry, rz);
+        float eta, Hdj, lmaxj;
+        if (TENSOR) {   // |H_j r|
+          if (MIR) mirrorTensor32(dcode & mm, r.h0, r.h1);
+          eta = etaFromSq(eta2Sym32(r.h0, r.h1, rx, ry, rz));
+          Hdj = r.h1.z;
+          lmaxj = r.h1.w;
+        } else {
+          const float aj = r.p.w;
+          eta = aj * etaFromSq(rx * rx + ry * ry + rz * rz);
+          Hdj = aj * aj * aj;
+          lmaxj = aj;
+        }
+        const float w = K.value(eta);
+        const bool same = multi ? list[ent & kIndexMask] == li : true;
+        sumAdd(s, c, (same ? r.v.w : vi.w) * (Hdj * w), LEAN ? 0 : hp.plainSums);
+        if (DT) {
+          float vxj = r.v.x, vyj = r.v.y, vzj = r.v.z;
+          if (MIR) mirrorVel(dcode & mm, vxj, vyj, vzj);
+          const float dx = vi.x - vxj, dy = vi.y - vyj, dz = vi.z - vzj;
+          // min over pairs of min(h_i, h_j)/|v_ij| = 1/sqrt(max over pairs of
+          // (max(a_i, a_j) |v_ij|)^2): no division or root per pair
+          const float am = fmaxf(lmaxi, lmaxj);
+          worst = fmaxf(worst, (am * am) * (dx * dx + dy * dy + dz * dz));
+        }
+      });
+  if (L > 1) {
+    laneSumKahan<L>(s, c);
+    if (DT) worst = laneMax<L>(worst);
   }
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = sv[0]; part[2 * blockIdx.x + 1] = (double)sr[0]; }
+  unsigned long long key = ~0ULL;
+  if (live && sub == 0) {
+    const double Hdeti = TENSOR ? symDet(loadSym(F, F_HT_XX, i)) : (F.f[F_HINV][i] * F.f[F_HINV][i]) * F.f[F_HINV][i];
+    const double rho = F.f[F_MASS][i] * (Hdeti * hp.W0) + (KERN ? kSplineA * kahanValue(s, c) : kahanValue(s, c));
+    F.f[F_RHO][i] = rho;
+    const float rhof = toFloatRN(rho);
+    P.thermo[i].x = rhof;
+    if (DT && !isGhost(hp, i)) {   // halo copies do not vote
+      // FP32 node limits (the vote only picks the minimum; FP64 divide and
+      // square root sequences would dominate the sweep otherwise)
+      const NodeListParams Li = hp.lists[multi ? li : list[i]];
+      const float ax = toFloatRN(F.f[F_DVDT_X][i]), ay = toFloatRN(F.f[F_DVDT_Y][i]), az = toFloatRN(F.f[F_DVDT_Z][i]);
+      const float divv = toFloatRN(F.f[F_DVDX_XX][i] + F.f[F_DVDX_YY][i] + F.f[F_DVDX_ZZ][i]);
+      int reason;
+      const float best = nodeDt32(1.0f / (lmaxi * (float)Li.nPerh), P.thermo[i].z, toFloatRN(F.f[F_MAXQ][i]), rhof,
+                                  divv, sqrtf(vi.x * vi.x + vi.y * vi.y + vi.z * vi.z),
+                                  sqrtf(ax * ax + ay * ay + az * az), hp.useVelMagDt != 0,
+                                  (worst > 0.0f ? rsqrtf(worst) : 3.0e38f) / maxNperh, reason);
+      if (reason >= 0) key = dtKey(toDouble(best), reason);
+    }
+  }
+  if (DT) {
+    key = warpMin64(key);
+    if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = key;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < sweepBlock(L) / 32; ++w) key = sv[w] < key ? sv[w] : key;
+      if (key != ~0ULL) atomicMin(dtOut, key);
+    }
+  }
 }
 
 //------------------------------------------------------------------------------
 // Grad-h correction, FP32 sums (computeSPHOmegaGradhCorrection.cc:15-116).
 //------------------------------------------------------------------------------
 // LEAN: compensated sums fixed at compile time.
-template <bool TENSOR, bool LEAN>
-__global__ void __launch_bounds__(128) gradhKernel32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
+template <bool TENSOR, bool LEAN, bool MIR, int KERN, int L, int U>
+__global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
                                                      TableDev t, HydroParams hp) {
-  __shared__ float4 ta[kMaxTable / 3];
-  __shared__ float2 tb[kMaxTable / 3];
-  __shared__ float4 sOff[64];
-  const int nint = hp.tableN1 + 1;
-  for (int k = threadIdx.x; k < nint; k += blockDim.x) { ta[k] = t.p32a[k]; tb[k] = t.p32b[k]; }
-  fillCellOffsets(sOff, g.cellf[0], g.cellf[1], g.cellf[2]);
+  constexpr int NT = KERN ? 1 : kTab32;
+  __shared__ float4 ta[NT];
+  __shared__ float2 tb[NT];
+  if (!KERN) loadTable32(ta, tb, t, hp.tableN1);
   __syncthreads();
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  if (L == 1 && !live) return;
+  const long i = live ? node : n - 1;
+  const Kernel32<KERN> K{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};
   int ci[3];
   unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
   const float4 pi = P.posh[i];
   const float ai = pi.w;
   float4 hi0 = make_float4(0.f, 0.f, 0.f, 0.f), hi1 = hi0;
   if (TENSOR) { hi0 = P.hten[2 * i]; hi1 = P.hten[2 * i + 1]; }
-  const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
-  const int N1 = hp.tableN1;
   float ws = 0.f, wc = 0.f, gs = 0.f, gc = 0.f;
-  const int cnt = nl.count[i];
-  // software pipeline: entry two slots ahead, node position one slot ahead
-  uint32_t entA = 0u, entB = 0u;
-  float4 pjA = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (cnt > 0) {
-    entA = nl.nbr[nbSlot(i, 0, nl.cap)];
-    pjA = P.posh[(int)(entA & kIndexMask)];
-  }
-  if (cnt > 1) entB = nl.nbr[nbSlot(i, 1, nl.cap)];
-  for (int q = 0; q < cnt; ++q) {
-    const uint32_t ent = entA;
-    const float4 pj = pjA;
-    if (q + 1 < cnt) {
-      pjA = P.posh[(int)(entB & kIndexMask)];
-      entA = entB;
-    }
-    if (q + 2 < cnt) entB = nl.nbr[nbSlot(i, q + 2, nl.cap)];
-    const int dcode = (int)(ent >> kIndexBits);
-    float rx, ry, rz;
-    relSepTab(pi, pj, dcode, mm, cx, cy, cz, sOff, rx, ry, rz);
-    float eta;
-    if (TENSOR) {
-      eta = etaFromSq(eta2Sym32(hi0, hi1, rx, ry, rz));
-    } else {
-      const float ex = ai * rx, ey = ai * ry, ez = ai * rz;
-      eta = etaFromSq(__fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex))));
-    }
-    float w, gr;
-    lookupPacked(ta, tb, N1, invStep, eta, extent, w, gr);
-    sumAdd(ws, wc, w, LEAN ? 0 : hp.plainSums);
-    sumAdd(gs, gc, eta * gr, LEAN ? 0 : hp.plainSums);
+  const int cnt = live ? nl.count[i] : 0;
+  laneSlots<L, U, float4>(
+      nl, i, sub, cnt, [&](uint32_t j, float4& p) { p = P.posh[j]; },
+      [&](uint32_t ent, const float4& p) {
+        float rx, ry, rz;
+        relSepEntry<MIR>(pi, p, ent, mm, cx, cy, cz, rx, ry, rz);
+        float eta;
+        if (TENSOR) eta = etaFromSq(eta2Sym32(hi0, hi1, rx, ry, rz));
+        else if (KERN) eta = ai * etaFromSq(__fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx))));
+        else {
+          const float ex = ai * rx, ey = ai * ry, ez = ai * rz;
+          eta = etaFromSq(__fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex))));
+        }
+        float w, gr;
+        K.both(eta, w, gr);
+        sumAdd(ws, wc, w, LEAN ? 0 : hp.plainSums);
+        sumAdd(gs, gc, __fmul_rn(eta, gr), LEAN ? 0 : hp.plainSums);
+      });
+  if (L > 1) {
+    laneSumKahan<L>(ws, wc);
+    laneSumKahan<L>(gs, gc);
+    if (sub != 0 || !live) return;
   }
   // Omega = -sum eta dW/deta / (3 (sum W + W0)) (Hdet cancels), in FP32 from
   // the compensated sums
   float omega = 1.0f;
-  if (cnt > 0) omega = fmaxf(1.0e-30f, -(gs - gc) / (3.0f * ((ws - wc) + (float)hp.W0)));
-  F.f[F_OMEGA][i] = (double)omega;
+  if (cnt > 0) omega = fmaxf(1.0e-30f, -(gs - gc) / (3.0f * ((ws - wc) + (KERN ? 1.0f : (float)hp.W0))));
+  F.f[F_OMEGA][i] = toDouble(omega);
   P.thermo[i].w = omega / (omega * omega + 1.0e-30f);
 }
 
 //------------------------------------------------------------------------------
-// GenericHydro::dt with the pairwise velocity limit in FP32.
+// GenericHydro::dt with the pairwise velocity limit in FP32 and the node
+// limits in FP64.  Each node first forms all its limits in FP32; only a node
+// whose FP32 limit is within 1e-4 of the smallest seen so far (estOut, which
+// only falls) can hold the minimum and repeats its node limits in FP64.
 //------------------------------------------------------------------------------
-template <bool TENSOR>
+template <bool TENSOR, bool MIR, int L, int U>
 __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const int* __restrict__ list, long n, Grid g,
                                                   NeighborLists nl, HydroParams hp, double maxNperh,
-                                                  double* __restrict__ part) {
-  __shared__ double sv[128];
-  __shared__ int sr[128];
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const double tiny = DBL_EPSILON;
-  double best = DBL_MAX;
-  int reason = -1;
-  if (i < n && !isGhost(hp, i)) {
-    int ci[3];
-    unpackCell(P.cell[i], ci);
-    const uint32_t mm = mirrorMask(g, ci);
-    const NodeListParams L = hp.lists[list[i]];
+                                                  unsigned* __restrict__ estOut,
+                                                  unsigned long long* __restrict__ dtOut) {
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  const long i = live ? node : n - 1;
+  int ci[3];
+  unpackCell(P.cell[i], ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
+  const float4 vi = P.velm[i];
+  const float lmaxi = TENSOR ? P.hten[2 * i + 1].w : P.posh[i].w;
+  float worst = 0.0f;
+  laneSlots<L, U, float4>(
+      nl, i, sub, live ? nl.count[i] : 0,
+      [&](uint32_t j, float4& v) {
+        v = P.velm[j];
+        v.w = TENSOR ? P.hten[2 * j + 1].w : P.posh[j].w;
+      },
+      [&](uint32_t ent, const float4& v) {
+        float vxj = v.x, vyj = v.y, vzj = v.z;
+        if (MIR) mirrorVel((ent >> kIndexBits) & mm, vxj, vyj, vzj);
+        const float dx = vi.x - vxj, dy = vi.y - vyj, dz = vi.z - vzj;
+        const float am = fmaxf(lmaxi, v.w);
+        worst = fmaxf(worst, (am * am) * (dx * dx + dy * dy + dz * dz));
+      });
+  if (L > 1) worst = laneMax<L>(worst);
+  const float bestPair = worst > 0.0f ? rsqrtf(worst) : 3.0e38f;
+  const bool votes = live && sub == 0 && !isGhost(hp, i);
+  float est = 3.0e38f;
+  const NodeListParams Li = hp.lists[list[i]];
+  if (votes) {
+    const float ax = toFloatRN(F.f[F_DVDT_X][i]), ay = toFloatRN(F.f[F_DVDT_Y][i]), az = toFloatRN(F.f[F_DVDT_Z][i]);
+    const float divv = toFloatRN(F.f[F_DVDX_XX][i] + F.f[F_DVDX_YY][i] + F.f[F_DVDX_ZZ][i]);
+    int reason;
+    est = nodeDt32(1.0f / (lmaxi * (float)Li.nPerh), toFloatRN(F.f[F_CS][i]), toFloatRN(F.f[F_MAXQ][i]),
+                   toFloatRN(F.f[F_RHO][i]), divv, sqrtf(vi.x * vi.x + vi.y * vi.y + vi.z * vi.z),
+                   sqrtf(ax * ax + ay * ay + az * az), hp.useVelMagDt != 0, bestPair / (float)maxNperh, reason);
+  }
+  const float wmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(est)));
+  if ((threadIdx.x & 31) == 0 && wmin < 3.0e38f) atomicMin(estOut, __float_as_uint(wmin));
+  const float seen = __uint_as_float(*(volatile unsigned*)estOut);
+  // NaN compares false: a node with a NaN limit takes the FP64 limits too
+  if (votes && !(est > fminf(seen, wmin) * 1.0001f)) {
+    const double tiny = DBL_EPSILON;
+    double best = DBL_MAX;
+    int reason = -1;
     const double ai = F.f[TENSOR ? F_HLMAX : F_HINV][i];   // largest eigenvalue of H
-    const double nodeScalei = 1.0 / ai / L.nPerh;
+    const double nodeScalei = 1.0 / ai / Li.nPerh;
     const double vxi = F.f[F_VX][i], vyi = F.f[F_VY][i], vzi = F.f[F_VZ][i];
     const double rhoi = F.f[F_RHO][i];
     const double csDt = nodeScalei / (F.f[F_CS][i] + tiny);
@@ -672,59 +1135,21 @@ __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const in
       const double velDt = nodeScalei / (vmag + 1.0e-10);
       if (velDt < best) { best = velDt; reason = 4; }
     }
-    const float4 vi = P.velm[i];
-    const float hi = 1.0f / (TENSOR ? P.hten[2 * i + 1].w : P.posh[i].w);
-    float bestPair = 3.0e38f;
-    const int cnt = nl.count[i];
-    for (int q = 0; q < cnt; ++q) {
-      const long long k = nbSlot(i, q, nl.cap);
-      const uint32_t ent = nl.nbr[k];
-      const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-      const float4 vj = P.velm[j];
-      float vxj = vj.x, vyj = vj.y, vzj = vj.z;
-      mirrorVel((uint32_t)dcode & mm, vxj, vyj, vzj);
-      const float dx = vi.x - vxj, dy = vi.y - vyj, dz = vi.z - vzj;
-      const float hmin = fminf(hi, 1.0f / (TENSOR ? P.hten[2 * j + 1].w : P.posh[j].w));
-      const float dtv = hmin / fmaxf(1.0e-30f, sqrtf(dx * dx + dy * dy + dz * dz));
-      bestPair = fminf(bestPair, dtv);
-    }
     const double pairDt = (double)bestPair / maxNperh;
     if (pairDt < best) { best = pairDt; reason = 5; }
+    if (reason >= 0) atomicMin(dtOut, dtKey(best, reason));
   }
-  sv[threadIdx.x] = best;
-  sr[threadIdx.x] = reason;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o && sv[threadIdx.x + o] < sv[threadIdx.x]) {
-      sv[threadIdx.x] = sv[threadIdx.x + o];
-      sr[threadIdx.x] = sr[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = sv[0]; part[2 * blockIdx.x + 1] = (double)sr[0]; }
 }
-__global__ void dtFinalKernel32(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  __shared__ double sv[256];
-  __shared__ double sr[256];
-  double best = DBL_MAX, reason = -1.0;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    if (part[2 * b] < best) { best = part[2 * b]; reason = part[2 * b + 1]; }
-  sv[threadIdx.x] = best;
-  sr[threadIdx.x] = reason;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o && sv[threadIdx.x + o] < sv[threadIdx.x]) {
-      sv[threadIdx.x] = sv[threadIdx.x + o];
-      sr[threadIdx.x] = sr[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { out[0] = sv[0]; out[1] = sr[0]; }
+
+__global__ void dtInitKernel(StepScratch* __restrict__ sc) {
+  sc->voteKey = ~0ULL;
+  sc->voteEst = 0x7f7fffffu;   // FLT_MAX
 }
 
 //------------------------------------------------------------------------------
 // Compatible-energy sweep of the mixed mode (SpecificThermalEnergyPolicy.cc:110-173).
-// v12 = v + a dt/2 is formed once per node in FP64; the per-pair work
+// v12 = v0 + a dt/2 is formed once per node in FP64 from the beginning-of-step
+// velocity; the per-pair work
 // du_ij = (v12_j - v12_i) . pacc_ij uses the FP64 velocity difference rounded
 // to FP32 and the FP32 pair acceleration; the weighted shares are summed and
 // applied to the specific energy in FP64.
@@ -734,9 +1159,9 @@ __global__ void halfStepVelocityKernel(Fields F, long n, double hdt, float4* __r
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   // v12 = v + a dt/2 in FP64, stored as an unevaluated float pair hi + lo
-  const double x = F.f[F_VX][i] + F.f[F_DVDT_X][i] * hdt;
-  const double y = F.f[F_VY][i] + F.f[F_DVDT_Y][i] * hdt;
-  const double z = F.f[F_VZ][i] + F.f[F_DVDT_Z][i] * hdt;
+  const double x = F.f[F_VX0][i] + F.f[F_DVDT_X][i] * hdt;
+  const double y = F.f[F_VY0][i] + F.f[F_DVDT_Y][i] * hdt;
+  const double z = F.f[F_VZ0][i] + F.f[F_DVDT_Z][i] * hdt;
   const float hx = (float)x, hy = (float)y, hz = (float)z;
   vhi[i] = make_float4(hx, hy, hz, (float)F.f[F_DEPSDT][i]);
   vlo[i] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.0f);
@@ -744,27 +1169,30 @@ __global__ void halfStepVelocityKernel(Fields F, long n, double hdt, float4* __r
 
 // B: slots per batch (the gathers and pair-acceleration reads in flight per
 // thread); every B adds in the same slot order, so the result is the same.
-template <int B>
-__global__ void __launch_bounds__(128) energyKernel32(Fields F, long n, Grid g, NeighborLists nl,
+// L lanes per node.
+template <bool MIR, int B, int L>
+__global__ void __launch_bounds__(sweepBlock(L)) energyKernel32(Fields F, long n, Grid g, NeighborLists nl,
                                                       const float4* __restrict__ vhi, const float4* __restrict__ vlo,
                                                       const float* __restrict__ pacc, double dt) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  if (L == 1 && !live) return;
+  const long i = live ? node : n - 1;
   int ci[3];
   unpackCell(nl.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
   const float4 hi = vhi[i], lo = vlo[i];
   const float d0i = hi.w;
   const float feps = (float)DBL_EPSILON;
   float s = 0.0f, c = 0.0f;
-  const int cnt = nl.count[i];
-  // One slot: du = (v_j - v_i) . pacc_ij with the half-step velocities as
+  // One slot: du = (v_j - v_i) . a_ij with the half-step velocities as
   // hi + lo float pairs, split by the DepsDt0 weights.
   auto slot = [&](uint32_t ent, float4 hj, float4 lj, float p0, float p1, float p2) {
-    const int dcode = (int)(ent >> kIndexBits);
+    const uint32_t dcode = ent >> kIndexBits;
     float hx = hj.x, hy = hj.y, hz = hj.z, lx = lj.x, ly = lj.y, lz = lj.z;
-    const uint32_t mir = (uint32_t)dcode & mm;
-    if (mir) {
+    const uint32_t mir = dcode & mm;
+    if (MIR && mir) {
       if (mir & 3u) { hx = -hx; lx = -lx; }
       if (mir & 12u) { hy = -hy; ly = -ly; }
       if (mir & 48u) { hz = -hz; lz = -lz; }
@@ -774,54 +1202,62 @@ __global__ void __launch_bounds__(128) energyKernel32(Fields F, long n, Grid g, 
     const float wy = __fadd_rn(__fsub_rn(hy, hi.y), __fsub_rn(ly, lo.y));
     const float wz = __fadd_rn(__fsub_rn(hz, hi.z), __fsub_rn(lz, lo.z));
     const float du = __fmaf_rn(wz, p2, __fmaf_rn(wy, p1, __fmul_rn(wx, p0)));
-    const float sg = du < 0.0f ? -1.0f : 1.0f;
-    const float weighti = fmaxf(feps, d0i * sg);
-    const float weightj = fmaxf(feps, hj.w * sg);
+    const float weighti = fmaxf(feps, du < 0.0f ? -d0i : d0i);
+    const float weightj = fmaxf(feps, du < 0.0f ? -hj.w : hj.w);
     // The split of du between i and j: both sides divide by the same sum with
     // IEEE rounding, so the two shares add up to du with unbiased rounding
-    // errors.  (An approximate reciprocal here leaves a one-signed error on
-    // every pair, which accumulates into a steady energy drift.)
+    // errors.  (An approximate reciprocal here, even after a Newton step,
+    // leaves a one-signed error on every pair, which accumulates into a
+    // steady energy drift.)
     kahanAdd(s, c, __fmul_rn(__fdiv_rn(weighti, __fadd_rn(weighti, weightj)), du));
   };
   // Batches of B slots: all their loads are issued before any is used, so B
   // gathers and pair-acceleration reads are in flight together.  The entries
   // of the next batch are loaded while this batch's gathers are in flight.
-  int q = 0;
+  const int cnt = live ? nl.count[i] : 0;
+  const int mine = (cnt - sub + L - 1) / L;   // slots of this lane
+  const long long s0 = nbSlot(i, 0, nl.cap) + 32 * sub;
+  const uint32_t* __restrict__ nb = nl.nbr + s0;
+  const float* __restrict__ pa = pacc + paccSlot(s0);
+  constexpr int ST = 32 * L;
   uint32_t en[B];
-  if (B <= cnt) {
 #pragma unroll
-    for (int u = 0; u < B; ++u) en[u] = nl.nbr[nbSlot(i, u, nl.cap)];
-  }
-  for (; q + B <= cnt; q += B) {
+  for (int u = 0; u < B; ++u) en[u] = u < mine ? nb[u * ST] : 0u;
+  int q = 0;
+  for (; q + B <= mine; q += B) {
     uint32_t e[B];
-    float4 H[B], L[B];
+    float4 H[B], Lo[B];
     float p[B][3];
 #pragma unroll
     for (int u = 0; u < B; ++u) e[u] = en[u];
-    if (q + 2 * B <= cnt) {
-#pragma unroll
-      for (int u = 0; u < B; ++u) en[u] = nl.nbr[nbSlot(i, q + B + u, nl.cap)];
-    }
 #pragma unroll
     for (int u = 0; u < B; ++u) {
-      const long long k = nbSlot(i, q + u, nl.cap);
-      const int j = (int)(e[u] & kIndexMask);
+      const uint32_t j = e[u] & kIndexMask;
       H[u] = vhi[j];
-      L[u] = vlo[j];
-      p[u][0] = pacc[3 * k]; p[u][1] = pacc[3 * k + 1]; p[u][2] = pacc[3 * k + 2];
-    }
+      Lo[u] = vlo[j];
 #pragma unroll
-    for (int u = 0; u < B; ++u) slot(e[u], H[u], L[u], p[u][0], p[u][1], p[u][2]);
+      for (int k = 0; k < 3; ++k) p[u][k] = pa[3 * u * ST + 32 * k];
+    }
+    nb += B * ST;
+    pa += 3 * B * ST;
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (q + B + u < mine) en[u] = nb[u * ST];
+#pragma unroll
+    for (int u = 0; u < B; ++u) slot(e[u], H[u], Lo[u], p[u][0], p[u][1], p[u][2]);
   }
-  for (; q < cnt; ++q) {
-    const long long k = nbSlot(i, q, nl.cap);
-    const uint32_t ent = nl.nbr[k];
-    const int j = (int)(ent & kIndexMask);
-    slot(ent, vhi[j], vlo[j], pacc[3 * k], pacc[3 * k + 1], pacc[3 * k + 2]);
+  for (; q < mine; ++q, nb += ST, pa += 3 * ST) {
+    const uint32_t ent = nb[0];
+    const uint32_t j = ent & kIndexMask;
+    slot(ent, vhi[j], vlo[j], pa[0], pa[32], pa[64]);
+  }
+  if (L > 1) {
+    laneSumKahan<L>(s, c);
+    if (sub != 0 || !live) return;
   }
   const double sum = kahanValue(s, c);
   F.f[F_DEPS_COMPAT][i] = sum;
-  F.f[F_EPS][i] += sum * dt;
+  F.f[F_EPS][i] = F.f[F_EPS0][i] + sum * dt;
 }
 
 inline unsigned gridFor(long n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -833,36 +1269,40 @@ void launchPrepareFP32(Fields F, Fields32 F32, long n, Grid g, cudaStream_t s, L
   lc->add(1);
 }
 
-// variant (compatible energy, no XSPH, one NodeList): 0 the software-
-// pipelined loop at 4 blocks per SM (<= 128 registers), 1 the same at 5
-// (<= 102 registers), 2 two slots per iteration at 4, 3 four slots per
-// iteration at 3 (<= 168 registers); with the limited Q, 0-1 the pipelined
-// loop and 2-3 two slots per iteration.  Lean forms where the configuration
-// allows.  Chosen at run time by the autotuner (kPairVariants); every
-// variant gives the same bits.
+constexpr int kDensU = 2, kGradhU = 4;   // slots per iteration of the density and grad-h sweeps
+// Lanes per node.  One lane per node leaves the GPU idle below ~300,000 nodes
+// (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
+// shuffles and the partly filled last slots; the sweeps with light pair bodies
+// gain from two lanes at any size (two list rows per warp access).  Lines set
+// where the measured times cross.
+constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
+int lanesPair(long n) { return n >= 80000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
+int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
+int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16))); }
+
+// variant (isotropic, lean path, one lane per node, standard Q): two slots per
+// iteration at 4 blocks per SM (even, <= 128 registers) or 5 (odd, <= 102).
+// At 2.1 M nodes 1741 / 1620 us, the limited Q spills at 102 (180 / 242 us at
+// 104,000 nodes); one slot per iteration ran 1800, four slots at 3 blocks 1890.
 void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                     HydroParams hp, float* pacc, int variant, cudaStream_t s,
                     LaunchCounter* lc) {
   const int b = 128;
-  const unsigned gb = gridFor(n, b);
   const bool multi = hp.numLists > 1;
-  // lean forms (no run-time flag in the loop) when the configuration allows:
-  // 1 with compensated sums, 2 with plain ones
-  const int lean = (hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion) ? (hp.plainSums ? 2 : 1) : 0;
-#define SPH_PAIR32(X, C, M, MB, PF, LQ) \
-  pairKernelFP32<X, C, M, MB, PF, LQ, false><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc)
+  // lean forms (no run-time flag in the loop) when the configuration allows
+  const bool lean = hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.plainSums;
+  if (hp.asph) {
+    const unsigned gb = gridFor(n, b);
 #define SPH_PAIR32T(X, C, LQ)                                                                     \
   do {                                                                                            \
     if (variant & 1) pairKernelFP32<X, C, true, 4, true, LQ, true><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
     else pairKernelFP32<X, C, true, 3, true, LQ, true><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);             \
   } while (0)
-  // ASPH (tensor H): NodeList test at run time; odd variants cap the
-  // registers at 128 (4 blocks per SM), even ones at 168 (3); variants 0-1
-  // the pipelined loop, 2-3 (compatible energy, no XSPH, standard Q) two
-  // slots per iteration
-  if (hp.asph) {
+    // tensor H: NodeList test at run time; odd variants cap the registers at
+    // 128 (4 blocks per SM), even ones at 168 (3); variants 0-1 the pipelined
+    // loop, 2-3 (compatible energy, no XSPH, standard Q) two slots per iteration
     if (!hp.xsph && hp.compatible && !hp.limitedQ && variant >= 2) {
-      if (lean == 1) {
+      if (lean) {
         if (variant & 1) pairKernelFP32<false, true, true, 4, 2, false, true, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
         else pairKernelFP32<false, true, true, 3, 2, false, true, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
       } else {
@@ -876,103 +1316,174 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
       if (hp.compatible) { if (hp.limitedQ) SPH_PAIR32T(false, true, true); else SPH_PAIR32T(false, true, false); }
       else { if (hp.limitedQ) SPH_PAIR32T(false, false, true); else SPH_PAIR32T(false, false, false); }
     }
-  } else if (hp.limitedQ) {   // LimitedMonaghanGingoldViscosity
-    if (!hp.xsph && hp.compatible && !multi) {
-      if (lean == 1) {
-        if (variant >= 2) pairKernelFP32<false, true, false, 4, 2, true, false, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-        else pairKernelFP32<false, true, false, 4, 1, true, false, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      } else {
-        if (variant >= 2) pairKernelFP32<false, true, false, 4, 2, true, false, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-        else pairKernelFP32<false, true, false, 4, 1, true, false, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      }
-    } else if (hp.xsph) {
-      if (hp.compatible) SPH_PAIR32(true, true, true, 4, false, true);
-      else SPH_PAIR32(true, false, true, 4, false, true);
-    } else {
-      if (hp.compatible) SPH_PAIR32(false, true, true, 4, false, true);
-      else SPH_PAIR32(false, false, true, 4, false, true);
-    }
-  } else if (!hp.xsph && hp.compatible && !multi) {
-#define SPH_PAIR32V(MB, PF) \
-  do {                                                                                                            \
-    if (lean == 1) pairKernelFP32<false, true, false, MB, PF, false, false, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else if (lean == 2) pairKernelFP32<false, true, false, MB, PF, false, false, 2><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else pairKernelFP32<false, true, false, MB, PF, false, false, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-  } while (0)
-    switch (variant) {
-      case 1: SPH_PAIR32V(5, 1); break;
-      case 2: SPH_PAIR32V(4, 2); break;
-      case 3: SPH_PAIR32V(3, 4); break;
-      default: SPH_PAIR32V(4, 1); break;
-    }
-#undef SPH_PAIR32V
-  } else if (hp.xsph) {
-    if (hp.compatible) {
-      if (multi) SPH_PAIR32(true, true, true, 5, false, false); else SPH_PAIR32(true, true, false, 5, false, false);
-    } else {
-      if (multi) SPH_PAIR32(true, false, true, 5, false, false); else SPH_PAIR32(true, false, false, 5, false, false);
-    }
-  } else {
-    if (hp.compatible) SPH_PAIR32(false, true, true, 5, false, false);
-    else { if (multi) SPH_PAIR32(false, false, true, 5, false, false); else SPH_PAIR32(false, false, false, 5, false, false); }
-  }
-#undef SPH_PAIR32
 #undef SPH_PAIR32T
-  lc->add(1);
+    lc->add(1);
+    return;
+  }
+  const bool plainPath = lean && !hp.xsph && hp.compatible && !multi;
+  const bool exact = plainPath && n >= kExactNodes, fast = plainPath && !exact && hp.cubicSpline;
+  pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, (float)hp.Cl, hp.limitedQ, fast ? 1 : 0, exact ? 1 : 0);
+  const int L = lanesPair(n);
+#define SPH_ISO(X, C, M, Q, LE, MI, K, LA, U, MB) \
+  pairKernelIso32<X, C, M, Q, LE, MI, K, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc)
+  if (exact) {
+#define SPH_LEAN(Q, MI)                                                                                              \
+  do {                                                                                                               \
+    if (!hp.cubicSpline) pairKernelLean32<Q, MI, false, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
+    else if (Q) pairKernelLean32<Q, MI, true, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
+    else if (variant & 1) pairKernelLean32<Q, MI, true, 3, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
+    else pairKernelLean32<Q, MI, true, 4, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);       \
+  } while (0)
+    if (hasMirrors(g)) { if (hp.limitedQ) SPH_LEAN(true, true); else SPH_LEAN(false, true); }
+    else { if (hp.limitedQ) SPH_LEAN(true, false); else SPH_LEAN(false, false); }
+#undef SPH_LEAN
+  } else if (fast) {
+#define SPH_ISOL(Q, MI)                                                                   \
+  switch (L) {                                                                            \
+    case 2: SPH_ISO(false, true, false, Q, true, MI, 1, 2, 2, 4); break;                  \
+    case 4: SPH_ISO(false, true, false, Q, true, MI, 1, 4, 2, 4); break;                  \
+    case 8: SPH_ISO(false, true, false, Q, true, MI, 1, 8, 2, 4); break;                  \
+    default: SPH_ISO(false, true, false, Q, true, MI, 1, 16, 2, 4); break;                \
+  }
+    if (hasMirrors(g)) {
+      if (hp.limitedQ) { SPH_ISOL(true, true) } else { SPH_ISOL(false, true) }
+    } else {
+      if (hp.limitedQ) { SPH_ISOL(true, false) } else { SPH_ISOL(false, false) }
+    }
+#undef SPH_ISOL
+  } else {
+#define SPH_ISOG(X, C)                                                      \
+  do {                                                                      \
+    if (hp.limitedQ) SPH_ISO(X, C, true, true, false, true, 0, 4, 1, 3);          \
+    else SPH_ISO(X, C, true, false, false, true, 0, 4, 1, 3);                     \
+  } while (0)
+    if (hp.xsph) { if (hp.compatible) SPH_ISOG(true, true); else SPH_ISOG(true, false); }
+    else { if (hp.compatible) SPH_ISOG(false, true); else SPH_ISOG(false, false); }
+#undef SPH_ISOG
+  }
+#undef SPH_ISO
+  lc->add(2);
+}
+
+// Slots per iteration of the density and grad-h sweeps: see densityKernel32.
+#define SPH_BY_LANES(L, CALL)      \
+  switch (L) {                     \
+    case 1: CALL(1); break;        \
+    case 2: CALL(2); break;        \
+    case 4: CALL(4); break;        \
+    case 8: CALL(8); break;        \
+    default: CALL(16); break;      \
+  }
+
+static void launchDensity32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
+                            const HydroParams& hp, bool dt, double maxNperh, unsigned long long* key, cudaStream_t s) {
+  const int L = lanesSweep(n);
+#define SPH_DENS(T, D, LE, MI, K, LA, U) \
+  densityKernel32<T, D, LE, MI, K, LA, U><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, F32, list, n, g, nl, t, hp, (float)maxNperh, key)
+  // lean: one NodeList and compensated sums fixed at compile time
+  const bool lean = hp.numLists == 1 && !hp.plainSums;
+  if (dt && lean && (n >= kExactNodes || hp.asph)) {
+#define SPH_DX(LA)                                                          \
+  do {                                                                      \
+    if (hp.asph) SPH_DENS(true, true, true, true, 0, LA, 2);                \
+    else if (hasMirrors(g)) SPH_DENS(false, true, true, true, 0, LA, kDensU); \
+    else SPH_DENS(false, true, true, false, 0, LA, kDensU);                 \
+  } while (0)
+    SPH_BY_LANES(L, SPH_DX)
+#undef SPH_DX
+  } else if (dt && lean && hp.cubicSpline) {
+#define SPH_DL(LA)                                                          \
+  do {                                                                      \
+    if (hasMirrors(g)) SPH_DENS(false, true, true, true, 1, LA, kDensU);    \
+    else SPH_DENS(false, true, true, false, 1, LA, kDensU);                 \
+  } while (0)
+    SPH_BY_LANES(L, SPH_DL)
+#undef SPH_DL
+  } else if (dt) {
+    if (hp.asph) SPH_DENS(true, true, false, true, 0, 4, 1); else SPH_DENS(false, true, false, true, 0, 4, 2);
+  } else {
+    if (hp.asph) SPH_DENS(true, false, false, true, 0, 4, 1); else SPH_DENS(false, false, false, true, 0, 4, 2);
+  }
+#undef SPH_DENS
 }
 
 void launchSumDensityFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                           HydroParams hp, cudaStream_t s, LaunchCounter* lc) {
-  if (hp.asph) sumDensityKernel32<true><<<gridFor(n, 128), 128, 0, s>>>(F, F32, list, n, g, nl, t, hp);
-  else sumDensityKernel32<false><<<gridFor(n, 128), 128, 0, s>>>(F, F32, list, n, g, nl, t, hp);
+  launchDensity32(F, F32, list, n, g, nl, t, hp, false, 1.0, nullptr, s);
   lc->add(1);
 }
 
 void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                      cudaStream_t s, LaunchCounter* lc) {
-  if (hp.asph) {
-    if (hp.plainSums) gradhKernel32<true, false><<<gridFor(n, 128), 128, 0, s>>>(F, F32, n, g, nl, t, hp);
-    else gradhKernel32<true, true><<<gridFor(n, 128), 128, 0, s>>>(F, F32, n, g, nl, t, hp);
+  const int L = lanesSweep(n);
+#define SPH_GH(T, LE, MI, K, LA, U) gradhKernel32<T, LE, MI, K, LA, U><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, F32, n, g, nl, t, hp)
+  if (!hp.plainSums && (n >= kExactNodes || hp.asph)) {
+#define SPH_GX(LA)                                                    \
+  do {                                                                \
+    if (hp.asph) SPH_GH(true, true, true, 0, LA, 2);                  \
+    else if (hasMirrors(g)) SPH_GH(false, true, true, 0, LA, kGradhU); \
+    else SPH_GH(false, true, false, 0, LA, kGradhU);                  \
+  } while (0)
+    SPH_BY_LANES(L, SPH_GX)
+#undef SPH_GX
+  } else if (!hp.plainSums && hp.cubicSpline) {
+#define SPH_GL(LA)                                                    \
+  do {                                                                \
+    if (hasMirrors(g)) SPH_GH(false, true, true, 1, LA, kGradhU);     \
+    else SPH_GH(false, true, false, 1, LA, kGradhU);                  \
+  } while (0)
+    SPH_BY_LANES(L, SPH_GL)
+#undef SPH_GL
+  } else if (hp.asph) {
+    SPH_GH(true, false, true, 0, 4, 2);
   } else {
-    if (hp.plainSums) gradhKernel32<false, false><<<gridFor(n, 128), 128, 0, s>>>(F, F32, n, g, nl, t, hp);
-    else gradhKernel32<false, true><<<gridFor(n, 128), 128, 0, s>>>(F, F32, n, g, nl, t, hp);
+    SPH_GH(false, false, true, 0, 4, 2);
   }
+#undef SPH_GH
   lc->add(1);
 }
 
 void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
-                  double maxNperh, double* dScratch, int nScratch, double* dOut,
-                  cudaStream_t s, LaunchCounter* lc) {
-  (void)nScratch;
-  const int nb = (int)gridFor(n, 128);
-  if (hp.asph) dtKernel32<true><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, dScratch);
-  else dtKernel32<false><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, dScratch);
-  dtFinalKernel32<<<1, 256, 0, s>>>(dScratch, nb, dOut);
+                  double maxNperh, StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
+  dtInitKernel<<<1, 1, 0, s>>>(sc);
+  const int L = lanesSweep(n);
+#define SPH_DT(LA)                                                                                                     \
+  do {                                                                                                                 \
+    if (hp.asph) dtKernel32<true, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, &sc->voteEst, &sc->voteKey); \
+    else dtKernel32<false, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, &sc->voteEst, &sc->voteKey);        \
+  } while (0)
+  SPH_BY_LANES(L, SPH_DT)
+#undef SPH_DT
   lc->add(2);
 }
 
 void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
                                 float4* vlo, double dt, int variant, cudaStream_t s, LaunchCounter* lc) {
   halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, 0.5 * dt, vhi, vlo);
-  if (variant == 1) energyKernel32<8><<<gridFor(n, 128), 128, 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt);
-  else if (variant == 2) energyKernel32<2><<<gridFor(n, 128), 128, 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt);
-  else energyKernel32<4><<<gridFor(n, 128), 128, 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt);
+  const int L = lanesEnergy(n);
+#define SPH_EN(B, LA)                                                                                                    \
+  if (hasMirrors(g)) energyKernel32<true, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt); \
+  else energyKernel32<false, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt)
+#define SPH_ENL(B)                 \
+  switch (L) {                     \
+    case 1: SPH_EN(B, 1); break;   \
+    case 2: SPH_EN(B, 2); break;   \
+    case 4: SPH_EN(B, 4); break;   \
+    case 8: SPH_EN(B, 8); break;   \
+    default: SPH_EN(B, 16); break; \
+  }
+  if (variant == 1) { SPH_ENL(8) } else if (variant == 2) { SPH_ENL(2) } else { SPH_ENL(4) }
+#undef SPH_ENL
+#undef SPH_EN
   lc->add(2);
 }
 
 void launchDensityDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                         HydroParams hp, double maxNperh, double* dScratch,
-                         double* dOut, cudaStream_t s, LaunchCounter* lc) {
-  const int nb = (int)gridFor(n, 128);
-  // lean: one NodeList and compensated sums fixed at compile time
-  const bool lean = hp.numLists == 1 && !hp.plainSums;
-  if (hp.asph) {
-    if (lean) densityDtKernel32<true, true><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, t, hp, maxNperh, dScratch);
-    else densityDtKernel32<true, false><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, t, hp, maxNperh, dScratch);
-  } else if (lean) densityDtKernel32<false, true><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, t, hp, maxNperh, dScratch);
-  else densityDtKernel32<false, false><<<nb, 128, 0, s>>>(F, F32, list, n, g, nl, t, hp, maxNperh, dScratch);
-  dtFinalKernel32<<<1, 256, 0, s>>>(dScratch, nb, dOut);
-  lc->add(2);
+                         HydroParams hp, double maxNperh, StepScratch* sc, bool reset, cudaStream_t s,
+                         LaunchCounter* lc) {
+  if (reset) dtInitKernel<<<1, 1, 0, s>>>(sc);
+  launchDensity32(F, F32, list, n, g, nl, t, hp, true, maxNperh, &sc->voteKey, s);
+  lc->add(reset ? 2 : 1);
 }
 
 }  // namespace sph

@@ -23,6 +23,20 @@ struct NeighborLists {
   const uint32_t* cell;     // home cell of every node (packed, 10 bits per axis)
 };
 
+constexpr int kEntrySums = 32;
+// Values the kernels of a step leave for the host, one per handle.  Reset by
+// the first kernel of a neighbour build.
+struct StepScratch {
+  long long bounds[10];        // end of step: order keys of min h^-1, min xyz, max xyz, tensor half-widths
+  int bad;                     // non-finite or non-positive state
+  int sortTimeout;             // a bounded wait of the sort ran out
+  int maxCount;                // largest neighbour count of the search
+  int items;                   // work chunks of the search
+  unsigned long long entries[kEntrySums];   // neighbour entries (partial sums)
+  unsigned long long voteKey;  // smallest dtKey of the mixed sweep
+  unsigned voteEst, pad;       // running FP32 estimate of the dt query
+};
+
 // Reductions ------------------------------------------------------------------
 // out[0] = min hinv, out[1..3] = min x,y,z, out[4..6] = max x,y,z,
 // out[7..9] = (tensor H) max over nodes of sqrt((H^-2)_aa) per axis, else 0
@@ -31,34 +45,31 @@ void launchBounds(const Fields& F, long n, bool tensor, double* dScratch, int nS
                   LaunchCounter* lc);
 
 // Neighbour build -------------------------------------------------------------
-void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, cudaStream_t s,
-                    LaunchCounter* lc);
+void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
+                    cudaStream_t s, LaunchCounter* lc);   // resets *sc
 // carriedOnly: move only the state and the derivatives the next step reads
 // before recomputing them (the step rewrites every other field before it
-// returns); otherwise every permuted field.
+// returns); otherwise every permuted field.  The same pass writes the cells'
+// node ranges (cellStart, cellEnd; cleared before) and the FP32 mirrors
+// (mirrors false: only what the search reads).
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
-                   bool carriedOnly, bool tensor, bool crk, cudaStream_t s, LaunchCounter* lc);
+                   bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
+                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, cudaStream_t s,
+                   LaunchCounter* lc);
 // The limited Q's DvDx <- the hydro DvDx; and its FP32 mirror (3 float4 per node).
 void launchCopyQGradient(Fields F, long n, cudaStream_t s, LaunchCounter* lc);
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc);
-// shift: sub-cell key bits below the cell key (Grid::subShift).
-void launchCellRanges(const uint32_t* sortedKeys, long n, int shift, int* cellStart, int* cellEnd, cudaStream_t s,
-                      LaunchCounter* lc);
-// Bounding boxes of the work chunks (for the batch culling of the search).
-void launchItemBoxes(const int* items, const long long* dItems, int nItemsBound, long n, int width, Fields32 P,
-                     float4* box, int* chunkOf, cudaStream_t s, LaunchCounter* lc);
-// Group-cooperative neighbour search over items (first node of each chunk of
-// up to `width` nodes of a cell).
-// width: nodes per work item of the group-cooperative search (8, 16 or 32).
-void launchItemFlags(const uint32_t* keys, long n, int shift, const int* cellStart, int width, int* flag,
-                     cudaStream_t s, LaunchCounter* lc);
-void launchItemFill(const int* flag, const long long* pos, long n, int* items, cudaStream_t s, LaunchCounter* lc);
-// nItems: an upper bound on the item count (sizes the grid); *dItems (device)
-// holds the count itself.
-void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, int nItems, const long long* dItems,
-                         int width, Grid g, const int* cellStart, const int* cellEnd, int* counts, int* maxCount,
-                         uint32_t* nbr, int cap, double ext2, bool tensor, const float4* box, const int* chunkOf,
+// Work items of the group-cooperative search: the chunks of up to `width` (8,
+// 16 or 32) consecutive nodes of a cell, their first nodes, each cell's first
+// chunk and the chunks' bounding boxes; the count goes to sc->items.
+void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
+                 int nItemsBound, Fields32 P, int* items, int* chunkOf, float4* box, StepScratch* sc, cudaStream_t s,
+                 LaunchCounter* lc);
+// nItems: an upper bound on the item count (sizes the grid); sc->items holds
+// the count itself.  The largest count and the sum of all go to *sc.
+void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, int nItems, StepScratch* sc,
+                         int width, Grid g, const int* cellStart, const int* cellEnd, int* counts, uint32_t* nbr, int cap, double ext2, bool tensor, const float4* box, const int* chunkOf,
                          cudaStream_t s, LaunchCounter* lc);
 
 // Sweeps ---------------------------------------------------------------------
@@ -67,8 +78,23 @@ void launchSumDensity(Fields F, const int* list, long n, Grid g, NeighborLists n
 void launchGradh(Fields F, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp, cudaStream_t s,
                  LaunchCounter* lc);
 void launchPairFP64(Fields F, const int* list, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                    double* pacc, int blockSize, cudaStream_t s, LaunchCounter* lc);
-constexpr int kPairVariants = 4;   // autotuned variants of launchPairFP32 (common path)
+                    double* pacc, cudaStream_t s, LaunchCounter* lc);   // tensor H, as launchSumDensity, launchGradh
+// FP64 sweeps with isotropic H (hydro64.cu).  rec: n node records of
+// nodeRecordBytes64() bytes; launchDensityDt64 takes the density sum, the dt
+// vote (dOut as launchDt; dScratch 2 doubles per block) or both in one pass;
+// launchEnergy64 serves every FP64 mode (vel: 4 doubles per node).
+size_t nodeRecordBytes64();
+void launchDensityDt64(Fields F, void* rec, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
+                       HydroParams hp, bool density, bool dt, double maxNperh, double* dScratch, double* dOut,
+                       cudaStream_t s, LaunchCounter* lc);
+void launchGradh64(Fields F, void* rec, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp, cudaStream_t s,
+                   LaunchCounter* lc);
+void launchPair64(Fields F, void* rec, const int* list, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
+                  double* pacc, cudaStream_t s, LaunchCounter* lc);
+void launchEnergy64(Fields F, void* vel, long n, Grid g, NeighborLists nl, const double* pacc, double dt,
+                    cudaStream_t s, LaunchCounter* lc);
+constexpr int kPairVariants = 2;   // autotuned variants of launchPairFP32 (isotropic H)
+constexpr int kPairVariantsMax = 4;   // values sphgpu_set_pair_variant takes (any path)
 constexpr int kRetuneAfter = 2;    // uses between an autotuner's first timing and its one retiming
 constexpr int kPairVariantsTensor = 4;   // of its tensor-H (ASPH) path
 constexpr int kPairVariantsCRK = 2;      // of the mixed CRKSPH pair kernel
@@ -81,26 +107,21 @@ void launchSumDensityFP32(Fields F, Fields32 F32, const int* list, long n, Grid 
 void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                      cudaStream_t s, LaunchCounter* lc);
 void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
-                  double maxNperh, double* dScratch, int nScratch, double* dOut,
-                  cudaStream_t s, LaunchCounter* lc);
-// Mixed mode: density sum and dt vote fused in one sweep (dOut as launchDt).
+                  double maxNperh, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
+// Mixed mode: density sum and dt vote fused in one sweep; the vote goes to
+// sc->voteKey (reset: clear it first; the neighbour build has done so).
 void launchDensityDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                         HydroParams hp, double maxNperh, double* dScratch,
-                         double* dOut, cudaStream_t s, LaunchCounter* lc);
+                         HydroParams hp, double maxNperh, StepScratch* sc, bool reset, cudaStream_t s,
+                         LaunchCounter* lc);
 // dt: writes per-block (value, reason) pairs then a final min into dOut[0], dOut[1] (reason as double)
 void launchDt(Fields F, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
               double maxNperh, double* dScratch, int nScratch, double* dOut,
               cudaStream_t s, LaunchCounter* lc);
-void launchCompatibleEnergy(Fields F, long n, Grid g, NeighborLists nl, const double* pacc, const float* pacc32,
-                            double dt, cudaStream_t s, LaunchCounter* lc);
 // variant: slots per batch of the sweep, 0 -> 4, 1 -> 8, 2 -> 2 (the same
 // result for every variant; picked by the autotuner).
 constexpr int kEnergyVariants = 3;
 void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
                                 float4* vlo, double dt, int variant, cudaStream_t s, LaunchCounter* lc);
-// state0 -> state (the copy is taken by the half-step update); tensor: also
-// the tensor H (ASPH)
-void launchRestoreState0(Fields F, long n, bool tensor, bool crk, cudaStream_t s, LaunchCounter* lc);
 // CRKSPH (crk.cu): the RK volumes (RKCorrections::preStepInitialize), the CRK
 // mass density sum (CRKSPHBase::preStepInitialize), the LinearOrder
 // corrections (RKCorrections::initialize) and the CRKSPH pair loop with the
@@ -141,7 +162,8 @@ void launchASPHEnd(Fields F, Fields32 P, const int* list, long n, Grid g, Neighb
                    HydroParams hp, cudaStream_t s, LaunchCounter* lc);
 // lists: device table of NodeListParams (HydroParams::lists).
 void launchEOS(Fields F, const int* list, long n, const NodeListParams* lists, cudaStream_t s, LaunchCounter* lc);
-void launchEnforce(Fields F, long n, Grid g, bool tensor, cudaStream_t s, LaunchCounter* lc);
+// Walls, end-of-step check and the next build's bounds (sc->bad, sc->bounds).
+void launchEndStep(Fields F, long n, Grid g, bool tensor, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 // out[0..7] conservation totals
 void launchConservation(Fields F, long n, bool gravity, double* dScratch, int nScratch, double* dOut, cudaStream_t s,
                         LaunchCounter* lc);
@@ -169,8 +191,6 @@ void launchScatterInHost(Fields F, const int* inv, const double* src, int first,
 void launchGatherOutHost(Fields F, const int* inv, double* dst, int first, int ncomp, int stride, bool isoH, long n,
                          cudaStream_t s, LaunchCounter* lc);
 void launchCountsOut(const int* counts, const int* orig, double* stage, long n, cudaStream_t s, LaunchCounter* lc);
-// check finite / positive state: writes a flag
-void launchCheckState(Fields F, long n, int* dFlag, cudaStream_t s, LaunchCounter* lc);
 
 // Gravity (gravity.cu) ---------------------------------------------------------
 struct GravityWork;

@@ -4,6 +4,8 @@
 // order -- and with it every summation order downstream -- is reproducible.
 #include "sort.cuh"
 
+#include <algorithm>
+
 namespace sph {
 
 namespace {
@@ -117,100 +119,178 @@ template void scanExclusive<long long>(const long long*, long long*, long, void*
                                        LaunchCounter*);
 
 //------------------------------------------------------------------------------
-// Stable LSD radix sort, 8-bit digits.
+// Stable LSD radix sort, 8-bit digits, one kernel per digit.
+//
+// One pass over the keys counts the digits of every place; each digit's kernel
+// then ranks its tile, obtains the number of equal digits in the tiles before
+// it from their published counts (decoupled look-back) and scatters.  Tiles
+// take their numbers from a counter, so every tile a block waits for has
+// already started; the wait is bounded all the same and reports through
+// `timeout` (the scatter is then skipped, so the output keeps what it held).
+// A sort is 2 + digits launches (a clear, the count, one per digit) where the
+// count / scan / scatter form took 5 per digit, which bound the neighbour
+// build of small problems (radix sort at 3,375 nodes, 2 digits: 52 us).
 //------------------------------------------------------------------------------
 namespace {
 constexpr int kSortThreads = 256;
 constexpr int kSortRounds = 8;
 constexpr int kSortTile = kSortThreads * kSortRounds;
 constexpr int kWarps = kSortThreads / 32;
+constexpr int kMaxDigits = 8;
+constexpr unsigned kAggregate = 1u << 30, kInclusive = 2u << 30, kCountMask = (1u << 30) - 1u;
+constexpr int kLookbackLimit = 1 << 24;   // polls before a wait gives up
 
-__global__ void radixHistKernel(const uint32_t* __restrict__ keys, long n, int shift, int numBlocks,
-                                unsigned* __restrict__ blockHist) {
-  __shared__ unsigned hist[256];
-  hist[threadIdx.x] = 0;
-  __syncthreads();
-  const long base = (long)blockIdx.x * kSortTile;
-#pragma unroll
-  for (int r = 0; r < kSortRounds; ++r) {
-    const long idx = base + (long)r * kSortThreads + threadIdx.x;
-    if (idx < n) atomicAdd(&hist[(keys[idx] >> shift) & 0xffu], 1u);
-  }
-  __syncthreads();
-  blockHist[(long)threadIdx.x * numBlocks + blockIdx.x] = hist[threadIdx.x];
+// Workspace: digit counts [kMaxDigits][256] | tile counters [kMaxDigits] | tile status [digits][tiles][256]
+struct SortWs {
+  unsigned *hist, *ticket, *status;
+};
+SortWs sortWs(void* ws) {
+  unsigned* u = static_cast<unsigned*>(ws);
+  return SortWs{u, u + kMaxDigits * 256, u + kMaxDigits * 256 + 64};
 }
 
-__global__ void radixScatterKernel(const uint32_t* __restrict__ keysIn, const int* __restrict__ valsIn, long n,
-                                   int shift, int numBlocks, const long long* __restrict__ offsets,
-                                   uint32_t* __restrict__ keysOut, int* __restrict__ valsOut) {
-  __shared__ unsigned warpCnt[kWarps][256];
-  __shared__ unsigned running[256];
-  __shared__ unsigned roundTot[256];
-  __shared__ long long blockOff[256];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  running[t] = 0;
-  blockOff[t] = offsets[(long)t * numBlocks + blockIdx.x];
-  const long base = (long)blockIdx.x * kSortTile;
-  const unsigned lanemaskLt = (1u << lane) - 1u;
-  for (int r = 0; r < kSortRounds; ++r) {
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) warpCnt[w][t] = 0;
-    __syncthreads();
-    const long idx = base + (long)r * kSortThreads + t;
-    const bool valid = idx < n;
-    uint32_t key = 0;
-    int val = 0;
-    unsigned digit = 256u + (unsigned)lane;   // unique dummy digit for idle lanes
-    if (valid) { key = keysIn[idx]; val = valsIn[idx]; digit = (key >> shift) & 0xffu; }
-    const unsigned peers = __match_any_sync(0xffffffffu, digit);
-    const unsigned rankInWarp = __popc(peers & lanemaskLt);
-    const int leader = __ffs(peers) - 1;
-    if (valid && lane == leader) warpCnt[warp][digit] = __popc(peers);
-    __syncthreads();
-    unsigned tot = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) tot += warpCnt[w][t];
-    roundTot[t] = tot;
-    if (valid) {
-      unsigned before = 0;
-      for (int w = 0; w < warp; ++w) before += warpCnt[w][digit];
-      const long long pos = blockOff[digit] + running[digit] + before + rankInWarp;
-      keysOut[pos] = key;
-      valsOut[pos] = val;
+template <typename K>
+__global__ void __launch_bounds__(kSortThreads) radixCountKernel(const K* __restrict__ keys, long n, int digits,
+                                                                 unsigned* __restrict__ hist) {
+  __shared__ unsigned h[kMaxDigits][256];
+  for (int d = 0; d < digits; ++d) h[d][threadIdx.x] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (long b = blockIdx.x * (long)blockDim.x + threadIdx.x - lane; b < n; b += (long)gridDim.x * blockDim.x) {
+    const bool valid = b + lane < n;
+    const K k = valid ? keys[b + lane] : 0;
+    for (int d = 0; d < digits; ++d) {
+      const unsigned digit = valid ? (unsigned)(k >> (8 * d)) & 0xffu : 256u;
+      int all;   // nearly sorted input: the high digits of a warp are mostly equal
+      __match_all_sync(0xffffffffu, digit, &all);
+      if (all) {
+        if (lane == 0) atomicAdd(&h[d][digit], 32u);
+      } else if (valid) {
+        atomicAdd(&h[d][digit], 1u);
+      }
     }
-    __syncthreads();
-    running[t] += roundTot[t];
-    __syncthreads();
   }
+  __syncthreads();
+  for (int d = 0; d < digits; ++d)
+    if (const unsigned c = h[d][threadIdx.x]) atomicAdd(&hist[d * 256 + threadIdx.x], c);
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kSortThreads) radixPassKernel(const K* __restrict__ keysIn,
+                                                                const int* __restrict__ valsIn, long n, int shift,
+                                                                const unsigned* __restrict__ hist,
+                                                                unsigned* __restrict__ ticket,
+                                                                unsigned* __restrict__ status, K* __restrict__ keysOut,
+                                                                int* __restrict__ valsOut, int* __restrict__ timeout) {
+  __shared__ unsigned warpHist[kWarps][256];
+  __shared__ unsigned base[256];
+  __shared__ unsigned scanWs[32];
+  __shared__ unsigned sTile;
+  __shared__ int sFail;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (t == 0) { sTile = atomicAdd(ticket, 1u); sFail = 0; }
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) warpHist[w][t] = 0;
+  __syncthreads();
+  const unsigned tile = sTile;
+  // each warp takes a contiguous segment, so (warp, round, lane) is input order
+  const long first = (long)tile * kSortTile + warp * (32 * kSortRounds) + lane;
+  K key[kSortRounds];
+  int val[kSortRounds];
+  unsigned rank[kSortRounds];
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    const long idx = first + 32 * r;
+    key[r] = 0;
+    val[r] = 0;
+    if (idx < n) { key[r] = keysIn[idx]; val[r] = valsIn[idx]; }
+  }
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    const bool valid = first + 32 * r < n;
+    const unsigned digit = valid ? (unsigned)(key[r] >> shift) & 0xffu : 256u + lane;   // idle lanes stand alone
+    const unsigned peers = __match_any_sync(0xffffffffu, digit);
+    unsigned old = 0;
+    if (valid && lane == __ffs(peers) - 1) {
+      old = warpHist[warp][digit];
+      warpHist[warp][digit] = old + __popc(peers);
+    }
+    old = __shfl_sync(0xffffffffu, old, __ffs(peers) - 1);
+    rank[r] = old + __popc(peers & below);
+    __syncwarp();
+  }
+  __syncthreads();
+  // digit t: counts before each warp, the tile's count
+  unsigned count = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    const unsigned c = warpHist[w][t];
+    warpHist[w][t] = count;
+    count += c;
+  }
+  volatile unsigned* st = status;
+  st[(size_t)tile * 256 + t] = (tile == 0 ? kInclusive : kAggregate) | count;
+  const unsigned digitStart = blockExclusiveScan<unsigned>(hist[t], scanWs, nullptr);
+  unsigned before = 0;
+  if (tile > 0) {
+    long p = (long)tile - 1;
+    int polls = 0;
+    while (true) {
+      const unsigned v = st[(size_t)p * 256 + t];
+      if (v & (kAggregate | kInclusive)) {
+        before += v & kCountMask;
+        if (v & kInclusive) break;
+        --p;
+      } else if (++polls > kLookbackLimit) {
+        sFail = 1;
+        break;
+      }
+    }
+    st[(size_t)tile * 256 + t] = kInclusive | (before + count);
+  }
+  base[t] = digitStart + before;
+  __syncthreads();
+  if (sFail) {
+    if (t == 0) atomicExch(timeout, 1);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r)
+    if (first + 32 * r < n) {
+      const unsigned digit = (unsigned)(key[r] >> shift) & 0xffu;
+      const unsigned pos = base[digit] + warpHist[warp][digit] + rank[r];
+      keysOut[pos] = key[r];
+      valsOut[pos] = val[r];
+    }
 }
 }  // namespace
 
 size_t radixSortWorkspaceBytes(long n) {
   const long nb = (n + kSortTile - 1) / kSortTile;
-  const long nh = nb * 256;
-  return (size_t)nh * sizeof(unsigned) + (size_t)nh * sizeof(long long) + scanWorkspaceBytes(nh) + 64;
+  return ((size_t)kMaxDigits * 256 + 64 + (size_t)kMaxDigits * nb * 256) * sizeof(unsigned);
 }
 
-void radixSortPairs(uint32_t*& keys, int*& vals, uint32_t*& keysAlt, int*& valsAlt, long n, int bits,
-                    void* workspace, cudaStream_t s, LaunchCounter* lc) {
+template <typename K>
+void radixSortPairs(K*& keys, int*& vals, K*& keysAlt, int*& valsAlt, long n, int bits, void* workspace, int* timeout,
+                    cudaStream_t s, LaunchCounter* lc) {
   if (n <= 1) return;
   const long nb = (n + kSortTile - 1) / kSortTile;
-  const long nh = nb * 256;
-  char* ws = static_cast<char*>(workspace);
-  unsigned* hist = reinterpret_cast<unsigned*>(ws);
-  long long* offs = reinterpret_cast<long long*>(ws + ((nh * sizeof(unsigned) + 15) / 16) * 16);
-  void* scanWs = reinterpret_cast<char*>(offs) + nh * sizeof(long long);
-  long long* dTot = reinterpret_cast<long long*>(static_cast<char*>(scanWs) + scanWorkspaceBytes(nh) - 16);
-  for (int shift = 0; shift < bits; shift += 8) {
-    radixHistKernel<<<(unsigned)nb, kSortThreads, 0, s>>>(keys, n, shift, (int)nb, hist);
-    scanExclusive<unsigned>(hist, offs, nh, scanWs, dTot, s, lc);
-    radixScatterKernel<<<(unsigned)nb, kSortThreads, 0, s>>>(keys, vals, n, shift, (int)nb, offs, keysAlt, valsAlt);
-    if (lc) lc->add(2);
+  const int digits = (bits + 7) / 8;
+  const SortWs w = sortWs(workspace);
+  cudaMemsetAsync(workspace, 0, ((size_t)kMaxDigits * 256 + 64 + (size_t)digits * nb * 256) * sizeof(unsigned), s);
+  radixCountKernel<K><<<(unsigned)std::min<long>(nb, 1216), kSortThreads, 0, s>>>(keys, n, digits, w.hist);
+  for (int d = 0; d < digits; ++d) {
+    radixPassKernel<K><<<(unsigned)nb, kSortThreads, 0, s>>>(keys, vals, n, 8 * d, w.hist + 256 * d, w.ticket + d,
+                                                             w.status + (size_t)d * nb * 256, keysAlt, valsAlt, timeout);
     std::swap(keys, keysAlt);
     std::swap(vals, valsAlt);
   }
+  if (lc) lc->add(1 + digits);
 }
-template void scanExclusive<unsigned>(const unsigned*, long long*, long, void*, long long*, cudaStream_t,
-                                      LaunchCounter*);
+template void radixSortPairs<uint32_t>(uint32_t*&, int*&, uint32_t*&, int*&, long, int, void*, int*, cudaStream_t,
+                                       LaunchCounter*);
+template void radixSortPairs<uint64_t>(uint64_t*&, int*&, uint64_t*&, int*&, long, int, void*, int*, cudaStream_t,
+                                       LaunchCounter*);
 
 }  // namespace sph

@@ -19,9 +19,12 @@ void scanExclusive(const Tin* in, long long* out, long n, void* workspace, long 
                    LaunchCounter* lc);
 
 size_t radixSortWorkspaceBytes(long n);
-// Stable sort of (keys, vals) by the low `bits` bits of keys.  The pointers are
-// ping-ponged: on return keys/vals point at the sorted data.
-void radixSortPairs(uint32_t*& keys, int*& vals, uint32_t*& keysAlt, int*& valsAlt, long n, int bits,
-                    void* workspace, cudaStream_t s, LaunchCounter* lc);
+// Stable sort of (keys, vals) by the low `bits` bits of keys (uint32_t or
+// uint64_t, at most 2^30 pairs).  The pointers are ping-ponged: on return
+// keys/vals point at the sorted data.  *timeout (device) is set when a bounded
+// wait inside the sort ran out; the output is then not sorted.
+template <typename K>
+void radixSortPairs(K*& keys, int*& vals, K*& keysAlt, int*& valsAlt, long n, int bits, void* workspace, int* timeout,
+                    cudaStream_t s, LaunchCounter* lc);
 
 }  // namespace sph

@@ -385,10 +385,10 @@ __device__ __forceinline__ Sym incrementASPHHtensor(const Sym& H, const Sym& D, 
 
 // FP32 mirror of tensor H for the FP32 sweeps and the neighbour pre-filter:
 // (xx xy xz yy) (yz zz det(H) lambda_max).
-__device__ __forceinline__ void writeTensorMirror(const Fields& F, const Fields32& P, long i) {
+__device__ __forceinline__ void writeTensorMirror(const Fields& F, long i, const Fields32& P, long k) {
   const Sym h = loadSym(F, F_HT_XX, i);
-  P.hten[2 * i] = make_float4((float)h.xx, (float)h.xy, (float)h.xz, (float)h.yy);
-  P.hten[2 * i + 1] = make_float4((float)h.yz, (float)h.zz, (float)symDet(h), (float)F.f[F_HLMAX][i]);
+  P.hten[2 * k] = make_float4(toFloatRN(h.xx), toFloatRN(h.xy), toFloatRN(h.xz), toFloatRN(h.yy));
+  P.hten[2 * k + 1] = make_float4(toFloatRN(h.yz), toFloatRN(h.zz), toFloatRN(symDet(h)), toFloatRN(F.f[F_HLMAX][i]));
 }
 // H_j of a neighbour entry from the mirror, seen through the mirror-axis bits
 // mir (dcode layout) of the entry.
