@@ -24,35 +24,6 @@ using namespace dev;
 inline unsigned gridFor(long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 
-// Packed table lookup: W and dW/deta at eta (zero beyond the extent).
-__device__ __forceinline__ void lookup(const float4* __restrict__ ta, const float2* __restrict__ tb, int N1,
-                                       float invStep, float eta, float extent, float& w, float& gr) {
-  if (eta < extent) {
-    const int k = min(N1, (int)(eta * invStep));
-    const float4 A = ta[k];
-    const float2 B = tb[k];
-    w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
-    gr = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
-  } else {
-    w = 0.0f;
-    gr = 0.0f;
-  }
-}
-
-struct Tab32 {
-  const float4* ta;
-  const float2* tb;
-  int N1;
-  float invStep, extent;
-};
-
-__device__ __forceinline__ Tab32 loadTab32(float4* ta, float2* tb, const TableDev& t, const HydroParams& hp) {
-  const int nint = hp.tableN1 + 1;
-  for (int k = threadIdx.x; k < nint; k += blockDim.x) { ta[k] = t.p32a[k]; tb[k] = t.p32b[k]; }
-  __syncthreads();
-  return Tab32{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep), (float)hp.extent};
-}
-
 // |eta| from eta (MUFU reciprocal square root, deterministic).
 __device__ __forceinline__ float etaMag(float ex, float ey, float ez, float& e2, float& re) {
   e2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
@@ -62,10 +33,10 @@ __device__ __forceinline__ float etaMag(float ex, float ey, float ez, float& e2,
 
 // Base kernel of H = a I at eta = a x: w = a^3 W(|eta|), dW = a^3 W'(|eta|) a eta^.
 // G returns the bare W'(|eta|) (the SPH moment weight is |G|).
-__device__ __forceinline__ void base32(const Tab32& T, float a, float ex, float ey, float ez, float em, float re,
+__device__ __forceinline__ void base32(const Kernel32<0>& T, float a, float ex, float ey, float ez, float em, float re,
                                        float& w, float& dwx, float& dwy, float& dwz, float& G) {
   float W;
-  lookup(T.ta, T.tb, T.N1, T.invStep, em, T.extent, W, G);
+  T.both(em, W, G);
   const float Hdet = __fmul_rn(__fmul_rn(a, a), a);
   w = __fmul_rn(Hdet, W);
   const float f = __fmul_rn(__fmul_rn(__fmul_rn(Hdet, G), a), re);
@@ -113,34 +84,45 @@ __device__ __forceinline__ void loadRKC(const float4* __restrict__ rkc, long j, 
   C[12] = d.x; C[13] = d.y; C[14] = d.z; C[15] = d.w;
 }
 
+// The sweeps below take L lanes per node and U slots per iteration (their
+// gathers issued together); MIR false: no wall reflects.
+#define SPH_CRK_SETUP()                                                       \
+  __shared__ float4 ta[kTab32];                                               \
+  __shared__ float2 tb[kTab32];                                               \
+  loadTable32(ta, tb, t, hp.tableN1);                                         \
+  __syncthreads();                                                            \
+  const Kernel32<0> T{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};      \
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;        \
+  const int sub = threadIdx.x % L;                                            \
+  const bool live = node < n;                                                 \
+  if (L == 1 && !live) return;                                                \
+  const long i = live ? node : n - 1;                                         \
+  int ci[3];                                                                  \
+  unpackCell(P.cell[i], ci);                                                  \
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;                           \
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];              \
+  const float4 pi = P.posh[i];                                                \
+  const int cnt = live ? nl.count[i] : 0
+
 //------------------------------------------------------------------------------
 // RKSumVolume: V_i = min(etaVolMax / Hdet_i, 1 / (sum_j W(|H_i r_ij|) + Hdet_i W0)).
 //------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) rkSumVolume32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
-                                                     TableDev t, HydroParams hp) {
-  __shared__ float4 ta[kMaxTable / 3];
-  __shared__ float2 tb[kMaxTable / 3];
-  const Tab32 T = loadTab32(ta, tb, t, hp);
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int ci[3];
-  unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i];
+template <bool MIR, int L, int U>
+__global__ void __launch_bounds__(sweepBlock(L)) rkSumVolume32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
+                                                               TableDev t, HydroParams hp) {
+  SPH_CRK_SETUP();
   const float ai = pi.w;
   float s = 0.f, c = 0.f;
-  const int cnt = nl.count[i];
-  for (int q = 0; q < cnt; ++q) {
-    const uint32_t ent = nl.nbr[nbSlot(i, q, nl.cap)];
-    const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-    float rx, ry, rz;
-    relSepEntry(pi, P.posh[j], ent, mm, cx, cy, cz, rx, ry, rz);
-    float e2, re;
-    const float em = etaMag(ai * rx, ai * ry, ai * rz, e2, re);
-    float W, G;
-    lookup(T.ta, T.tb, T.N1, T.invStep, em, T.extent, W, G);
-    kahanAdd(s, c, W);
+  laneSlots<L, U, float4>(
+      nl, i, sub, cnt, [&](uint32_t j, float4& p) { p = P.posh[j]; },
+      [&](uint32_t ent, const float4& p) {
+        float rx, ry, rz, e2, re;
+        relSepEntry<MIR>(pi, p, ent, mm, cx, cy, cz, rx, ry, rz);
+        kahanAdd(s, c, T.value(etaMag(ai * rx, ai * ry, ai * rz, e2, re)));
+      });
+  if (L > 1) {
+    laneSumKahan<L>(s, c);
+    if (sub != 0 || !live) return;
   }
   const double a = F.f[F_HINV][i];
   const double Hdet = (a * a) * a;
@@ -154,48 +136,48 @@ __global__ void __launch_bounds__(128) rkSumVolume32(Fields F, Fields32 P, long 
 //------------------------------------------------------------------------------
 // CRK mass density, FP32 sums over the same-NodeList neighbours.
 //------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) crkDensity32(Fields F, Fields32 P, const int* __restrict__ list, long n,
-                                                    Grid g, NeighborLists nl, TableDev t, HydroParams hp) {
-  __shared__ float4 ta[kMaxTable / 3];
-  __shared__ float2 tb[kMaxTable / 3];
-  const Tab32 T = loadTab32(ta, tb, t, hp);
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int ci[3];
-  unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i];
+struct DensityRec32 {
+  float4 p;
+  float v, m;
+};
+template <bool MIR, int L, int U>
+__global__ void __launch_bounds__(sweepBlock(L)) crkDensity32(Fields F, Fields32 P, const int* __restrict__ list,
+                                                              long n, Grid g, NeighborLists nl, TableDev t,
+                                                              HydroParams hp) {
+  SPH_CRK_SETUP();
   const bool multi = hp.numLists > 1;
   const int li = list[i];
   float sw = 0.f, cw = 0.f, sr = 0.f, cr = 0.f, sv = 0.f, cv = 0.f;
-  const int cnt = nl.count[i];
-  for (int q = 0; q < cnt; ++q) {
-    const uint32_t ent = nl.nbr[nbSlot(i, q, nl.cap)];
-    const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-    if (multi && list[j] != li) continue;
-    const float4 pj = P.posh[j];
-    float rx, ry, rz;
-    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
-    const float aj = pj.w;
-    float e2, re;
-    const float em = etaMag(aj * rx, aj * ry, aj * rz, e2, re);
-    float W, G;
-    lookup(T.ta, T.tb, T.N1, T.invStep, em, T.extent, W, G);
-    const float Wj = __fmul_rn(__fmul_rn(__fmul_rn(aj, aj), aj), W);
-    const float Vj = P.vol[j];
-    const float VW = __fmul_rn(Vj, Wj);
-    kahanAdd(sw, cw, VW);
-    kahanAdd(sr, cr, __fmul_rn(P.velm[j].w, VW));
-    kahanAdd(sv, cv, __fmul_rn(Vj, VW));
+  laneSlots<L, U, DensityRec32>(
+      nl, i, sub, cnt,
+      [&](uint32_t j, DensityRec32& r) {
+        r.p = P.posh[j];
+        r.v = P.vol[j];
+        r.m = P.velm[j].w;
+      },
+      [&](uint32_t ent, const DensityRec32& r) {
+        if (multi && list[ent & kIndexMask] != li) return;
+        float rx, ry, rz, e2, re;
+        relSepEntry<MIR>(pi, r.p, ent, mm, cx, cy, cz, rx, ry, rz);
+        const float aj = r.p.w;
+        const float W = T.value(etaMag(aj * rx, aj * ry, aj * rz, e2, re));
+        const float Wj = __fmul_rn(__fmul_rn(__fmul_rn(aj, aj), aj), W);
+        const float VW = __fmul_rn(r.v, Wj);
+        kahanAdd(sw, cw, VW);
+        kahanAdd(sr, cr, __fmul_rn(r.m, VW));
+        kahanAdd(sv, cv, __fmul_rn(r.v, VW));
+      });
+  if (L > 1) {
+    laneSumKahan<L>(sw, cw); laneSumKahan<L>(sr, cr); laneSumKahan<L>(sv, cv);
+    if (sub != 0 || !live) return;
   }
-  const NodeListParams L = hp.lists[li];
+  const NodeListParams Li = hp.lists[li];
   const double ai = F.f[F_HINV][i], mi = F.f[F_MASS][i], Vi = F.f[F_VOL][i];
   const double Hdeti = (ai * ai) * ai;
   const double wsum = kahanValue(sw, cw) + Vi * Hdeti * hp.W0;
   const double vol1 = (kahanValue(sv, cv) + Vi * Vi * Hdeti * hp.W0) / wsum;
-  const double rho = fmax(fmax(L.rhoMin, 0.1 * mi * Hdeti),
-                          fmin(L.rhoMax, (kahanValue(sr, cr) + mi * Vi * Hdeti * hp.W0) / (wsum * vol1)));
+  const double rho = fmax(fmax(Li.rhoMin, 0.1 * mi * Hdeti),
+                          fmin(Li.rhoMax, (kahanValue(sr, cr) + mi * Vi * Hdeti * hp.W0) / (wsum * vol1)));
   F.f[F_RHO][i] = rho;
   P.thermo[i].x = (float)rho;
 }
@@ -208,18 +190,14 @@ __device__ __forceinline__ int symIdx(int k, int l) {
   return k <= l ? (k * 4 - (k * (k - 1)) / 2 + (l - k)) : (l * 4 - (l * (l - 1)) / 2 + (k - l));
 }
 
+struct CorrectionRec32 {
+  float4 p;
+  float v;
+};
+template <bool MIR, int L, int U>
 __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
                                                        TableDev t, HydroParams hp) {
-  __shared__ float4 ta[kMaxTable / 3];
-  __shared__ float2 tb[kMaxTable / 3];
-  const Tab32 T = loadTab32(ta, tb, t, hp);
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int ci[3];
-  unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i];
+  SPH_CRK_SETUP();
   const float ai = pi.w, iai = 1.0f / ai;
   float Ms[10], Mc[10], dM[3][10];
 #pragma unroll
@@ -244,29 +222,40 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
         }
       }
   };
-  const int cnt = nl.count[i];
-  for (int q = 0; q < cnt; ++q) {
-    const uint32_t ent = nl.nbr[nbSlot(i, q, nl.cap)];
-    const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-    const float4 pj = P.posh[j];
-    float rx, ry, rz;
-    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
-    const float aj = pj.w;
-    const float ex = aj * rx, ey = aj * ry, ez = aj * rz;
-    float e2, re;
-    const float em = etaMag(ex, ey, ez, e2, re);
-    float w, dwx, dwy, dwz, G;
-    base32(T, aj, ex, ey, ez, em, re, w, dwx, dwy, dwz, G);
-    add(P.vol[j], rx, ry, rz, w, dwx, dwy, dwz);
+  laneSlots<L, U, CorrectionRec32>(
+      nl, i, sub, cnt,
+      [&](uint32_t j, CorrectionRec32& r) {
+        r.p = P.posh[j];
+        r.v = P.vol[j];
+      },
+      [&](uint32_t ent, const CorrectionRec32& r) {
+        float rx, ry, rz, e2, re;
+        relSepEntry<MIR>(pi, r.p, ent, mm, cx, cy, cz, rx, ry, rz);
+        const float aj = r.p.w;
+        const float ex = aj * rx, ey = aj * ry, ez = aj * rz;
+        const float em = etaMag(ex, ey, ez, e2, re);
+        float w, dwx, dwy, dwz, G;
+        base32(T, aj, ex, ey, ez, em, re, w, dwx, dwy, dwz, G);
+        add(r.v, rx, ry, rz, w, dwx, dwy, dwz);
+      });
+  if (L > 1) {
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+      laneSumKahan<L>(Ms[k], Mc[k]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) dM[d][k] = laneSum<L>(dM[d][k]);
+    }
+    if (sub != 0 || !live) return;
   }
   {   // self: x = 0, the gradient along the unit vector (1, 0, 0) of a zero eta
     float W, G;
-    lookup(T.ta, T.tb, T.N1, T.invStep, 0.0f, T.extent, W, G);
+    T.both(0.0f, W, G);
     const float Hdet = ai * ai * ai;
     add(P.vol[i], 0.f, 0.f, 0.f, Hdet * W, Hdet * G * ai, 0.f, 0.f);
   }
   // FP64 solve of M~ C~ = e_0, dC~_d = -M~^-1 (dM^_d C~) (LU, partial pivoting)
-  double A[4][4];
+  // one reciprocal per pivot (the FP64 unit is narrow: 16 divisions less)
+  double A[4][4], ip[4];
   int piv[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -285,10 +274,10 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
       for (int c2 = 0; c2 < 4; ++c2) { const double tmp = A[k][c2]; A[k][c2] = A[p][c2]; A[p][c2] = tmp; }
       const int tp = piv[k]; piv[k] = piv[p]; piv[p] = tp;
     }
-    const double inv = 1.0 / A[k][k];
+    ip[k] = 1.0 / A[k][k];
 #pragma unroll
     for (int r = k + 1; r < 4; ++r) {
-      const double f = A[r][k] * inv;
+      const double f = A[r][k] * ip[k];
       A[r][k] = f;
 #pragma unroll
       for (int c2 = k + 1; c2 < 4; ++c2) A[r][c2] -= f * A[k][c2];
@@ -308,7 +297,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
       double v = yv[r];
 #pragma unroll
       for (int c2 = r + 1; c2 < 4; ++c2) v -= A[r][c2] * x[c2];
-      x[r] = v / A[r][r];
+      x[r] = v * ip[r];
     }
   };
   const double a = (double)ai;
@@ -342,26 +331,19 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
 //------------------------------------------------------------------------------
 // CRKSPH pair loop, FP32.
 //------------------------------------------------------------------------------
-// U: neighbour slots per loop iteration (1, or 2 with both slots' gathers
-// issued together); the slots are evaluated in list order either way, so
-// both give the same bits.
-template <bool XSPH, bool COMPAT, bool LIMQ, int U = 1>
-__global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, const int* __restrict__ list, long n,
-                                                       Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                                                       float* __restrict__ pacc) {
-  __shared__ float4 ta[kMaxTable / 3];
-  __shared__ float2 tb[kMaxTable / 3];
-  const Tab32 T = loadTab32(ta, tb, t, hp);
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int ci[3];
-  unpackCell(P.cell[i], ci);
-  const uint32_t mm = mirrorMask(g, ci);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i], vi = P.velm[i], thi = P.thermo[i];
+// The record's fourth thermodynamic value is the RK volume (crkInputs32).
+struct PairRec32 {
+  float4 p, v, t, c0, c1, c2, c3;
+};
+template <bool XSPH, bool COMPAT, bool LIMQ, bool MIR, int L, int U, int MINB>
+__global__ void __launch_bounds__(128, MINB) pairKernelCRK32(Fields F, Fields32 P, const int* __restrict__ list, long n,
+                                                             Grid g, NeighborLists nl, TableDev t, HydroParams hp,
+                                                             float* __restrict__ pacc) {
+  SPH_CRK_SETUP();
+  const float4 vi = P.velm[i], thi = P.pk[i];
   const bool multi = hp.numLists > 1;
   const int li = list[i];
-  const float ai = pi.w, mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, Vi = P.vol[i];
+  const float ai = pi.w, mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, Vi = thi.w;
   const float invMi = __frcp_rn(mi);
   float Ci[16];
   loadRKC(P.rkc, i, Ci);
@@ -380,20 +362,20 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
 #pragma unroll
   for (int k = 0; k < 9; ++k) D[k] = 0.f;
 
-  const int cnt = nl.count[i];
-  // One neighbour slot (list slot `slot`, entry `ent`, node j's mirrors and
-  // corrections already gathered): its contributions to node i's sums.
-  auto pairSlot = [&](long long slot, uint32_t ent, const float4& pj, const float4& vj4, const float4& thj,
-                      float Vj, float* Cj) {
+  float* out = COMPAT ? pacc + paccSlot(nbSlot(i, 0, nl.cap) + 32 * sub) : nullptr;
+  // One neighbour slot: its contributions to node i's sums.
+  auto pairSlot = [&](uint32_t ent, const PairRec32& q) {
     const int j = (int)(ent & kIndexMask), dcode = (int)(ent >> kIndexBits);
-    const uint32_t mq = (uint32_t)dcode & mm;
+    const uint32_t mq = MIR ? (uint32_t)dcode & mm : 0u;
     float rx, ry, rz;
-    relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
-    float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
-    mirrorVel(mq, vxj, vyj, vzj);
-    const float aj = pj.w, mj = vj4.w, rhoj = thj.x, Pj = thj.y, csj = thj.z;
+    relSepEntry<MIR>(pi, q.p, ent, mm, cx, cy, cz, rx, ry, rz);
+    float vxj = q.v.x, vyj = q.v.y, vzj = q.v.z;
+    if (MIR) mirrorVel(mq, vxj, vyj, vzj);
+    const float aj = q.p.w, mj = q.v.w, rhoj = q.t.x, Pj = q.t.y, csj = q.t.z, Vj = q.t.w;
     const bool same = multi ? (list[j] == li) : true;
-    mirrorRKC(mq, Cj);
+    float Cj[16] = {q.c0.x, q.c0.y, q.c0.z, q.c0.w, q.c1.x, q.c1.y, q.c1.z, q.c1.w,
+                    q.c2.x, q.c2.y, q.c2.z, q.c2.w, q.c3.x, q.c3.y, q.c3.z, q.c3.w};
+    if (MIR) mirrorRKC(mq, Cj);
 
     const float eix = ai * rx, eiy = ai * ry, eiz = ai * rz;
     const float ejx = aj * rx, ejy = aj * ry, ejz = aj * rz;
@@ -414,7 +396,7 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
     if (LIMQ) {
       const float4 d0 = P.dvq[3 * (long)j], d1 = P.dvq[3 * (long)j + 1], d2 = P.dvq[3 * (long)j + 2];
       float Dj[9] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w, d2.x};
-      if (mq) {
+      if (MIR && mq) {
         const float sg[3] = {(mq & 3u) ? -1.f : 1.f, (mq & 12u) ? -1.f : 1.f, (mq & 48u) ? -1.f : 1.f};
 #pragma unroll
         for (int r = 0; r < 3; ++r)
@@ -465,10 +447,10 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
     kahanAdd(sdy, cdy, -ay);
     kahanAdd(sdz, cdz, -az);
     if (COMPAT) {
-      float* out = pacc + paccSlot(slot);
       out[0] = -ax;
       out[32] = -ay;
       out[64] = -az;
+      out += 96 * L;
     }
     // DepsDt_i += V_i V_j / 2 (P_j + rho_j e_j) v_ij . (gradW_j - gradW_i) / m_i
     const float vdg = __fmaf_rn(vz, dgz, __fmaf_rn(vy, dgy, __fmul_rn(vx, dgx)));
@@ -487,38 +469,34 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
     m0 += fwW;
     m1x -= fwW * eix; m1y -= fwW * eiy; m1z -= fwW * eiz;
   };
-  int q = 0;
-  if (U == 2) {
-    for (; q + 1 < cnt; q += 2) {
-      const long long s0 = nbSlot(i, q, nl.cap), s1 = s0 + 32;
-      const uint32_t e0 = nl.nbr[s0], e1 = nl.nbr[s1];
-      const int j0 = (int)(e0 & kIndexMask), j1 = (int)(e1 & kIndexMask);
-      const float4 p0 = P.posh[j0], v0 = P.velm[j0], t0 = P.thermo[j0];
-      const float4 p1 = P.posh[j1], v1 = P.velm[j1], t1 = P.thermo[j1];
-      const float V0 = P.vol[j0], V1 = P.vol[j1];
-      float C0[16], C1[16];
-      loadRKC(P.rkc, j0, C0);
-      loadRKC(P.rkc, j1, C1);
-      pairSlot(s0, e0, p0, v0, t0, V0, C0);
-      pairSlot(s1, e1, p1, v1, t1, V1, C1);
-    }
-  }
-  for (; q < cnt; ++q) {
-    const long long slot = nbSlot(i, q, nl.cap);
-    const uint32_t ent = nl.nbr[slot];
-    const int j = (int)(ent & kIndexMask);
-    float Cj[16];
-    loadRKC(P.rkc, j, Cj);
-    pairSlot(slot, ent, P.posh[j], P.velm[j], P.thermo[j], P.vol[j], Cj);
+  laneSlots<L, U, PairRec32>(
+      nl, i, sub, cnt,
+      [&](uint32_t j, PairRec32& r) {
+        r.p = P.posh[j];
+        r.v = P.velm[j];
+        r.t = P.pk[j];
+        const float4* c = P.rkc + 4 * (size_t)j;
+        r.c0 = c[0]; r.c1 = c[1]; r.c2 = c[2]; r.c3 = c[3];
+      },
+      pairSlot);
+  if (L > 1) {
+    laneSumKahan<L>(sdx, cdx); laneSumKahan<L>(sdy, cdy); laneSumKahan<L>(sdz, cdz); laneSumKahan<L>(se, ce);
+    maxQ = laneMax<L>(maxQ);
+    effQ = laneSum<L>(effQ);
+    xdx = laneSum<L>(xdx); xdy = laneSum<L>(xdy); xdz = laneSum<L>(xdz);
+    m0 = laneSum<L>(m0); m1x = laneSum<L>(m1x); m1y = laneSum<L>(m1y); m1z = laneSum<L>(m1z);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) D[k] = laneSum<L>(D[k]);
+    if (sub != 0 || !live) return;
   }
   // node finalize: the sums leave as FP64 values, the per-node arithmetic is
   // FP32 (GB300's FP64 rate would make it visible next to the pair loop)
   const float trace = D[0] + D[4] + D[8];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) { F.f[F_DVDX_XX + k][i] = D[k]; F.f[F_M_XX + k][i] = 0.0; }
+  for (int k = 0; k < 9; ++k) { F.f[F_DVDX_XX + k][i] = toDouble(D[k]); F.f[F_M_XX + k][i] = 0.0; }
   const double dvx = kahanValue(sdx, cdx), dvy = kahanValue(sdy, cdy), dvz = kahanValue(sdz, cdz);
   const double deps = kahanValue(se, ce);
-  F.f[F_DRHODT][i] = (double)(-rhoi * trace);
+  F.f[F_DRHODT][i] = toDouble(-rhoi * trace);
   F.f[F_DVDT_X][i] = dvx;
   F.f[F_DVDT_Y][i] = dvy;
   F.f[F_DVDT_Z][i] = dvz;
@@ -528,15 +506,15 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
   } else {
     F.f[F_DEPSDT][i] = deps;
   }
-  F.f[F_MAXQ][i] = maxQ;
-  F.f[F_EFFQ][i] = effQ;
+  F.f[F_MAXQ][i] = toDouble(maxQ);
+  F.f[F_EFFQ][i] = toDouble(effQ);
   F.f[F_RHOSUM][i] = 0.0;
   F.f[F_NORM][i] = 0.0;
   F.f[F_GRADRHO_X][i] = 0.0; F.f[F_GRADRHO_Y][i] = 0.0; F.f[F_GRADRHO_Z][i] = 0.0;
   F.f[F_XSPHW][i] = 0.0;
-  F.f[F_XSPHDV_X][i] = xdx;
-  F.f[F_XSPHDV_Y][i] = xdy;
-  F.f[F_XSPHDV_Z][i] = xdz;
+  F.f[F_XSPHDV_X][i] = toDouble(xdx);
+  F.f[F_XSPHDV_Y][i] = toDouble(xdy);
+  F.f[F_XSPHDV_Z][i] = toDouble(xdz);
   if (XSPH) {
     F.f[F_DXDT_X][i] = F.f[F_VX][i] + xdx;
     F.f[F_DXDT_Y][i] = F.f[F_VY][i] + xdy;
@@ -548,19 +526,27 @@ __global__ void __launch_bounds__(128) pairKernelCRK32(Fields F, Fields32 P, con
   }
   // SPHSmoothingScale finalize in FP32: DHDt = -(H/3) tr(DvDx), Hideal =
   // clamp(H / f, 1/hmax, 1/hmin)
-  const NodeListParams L = hp.lists[li];
+  const NodeListParams Ln = hp.lists[li];
   const float m0r = cbrtf(fmaxf(0.0f, m0));
-  F.f[F_M0][i] = m0r;
-  F.f[F_M1_X][i] = m1x;
-  F.f[F_M1_Y][i] = m1y;
-  F.f[F_M1_Z][i] = m1z;
+  F.f[F_M0][i] = toDouble(m0r);
+  F.f[F_M1_X][i] = toDouble(m1x);
+  F.f[F_M1_Y][i] = toDouble(m1y);
+  F.f[F_M1_Z][i] = toDouble(m1z);
   F.f[F_DHDT][i] = (double)(-(ai * (1.0f / 3.0f)) * trace);
-  const float nPerh = (float)L.nPerh;
+  const float nPerh = (float)Ln.nPerh;
   const bool isolated = fabsf(m0r) <= 1.0e-15f * fmaxf(1.0f, fabsf(m0r));
   const float cur = isolated ? 0.5f * nPerh : fmaxf(0.0f, hermiteLookup32(t.herm, hp, m0r));
   const float sr = fminf(4.0f, fmaxf(0.25f, nPerh / (cur + 1.0e-30f)));
   const float aa = sr < 1.0f ? 0.4f * (1.0f + sr * sr) : 0.4f * (1.0f + 1.0f / (sr * sr * sr));
-  F.f[F_HIDEAL][i] = fmin(L.hminInv, fmax(L.hmaxInv, (double)(ai / (1.0f - aa + aa * sr))));
+  F.f[F_HIDEAL][i] = fmin(Ln.hminInv, fmax(Ln.hmaxInv, (double)(ai / (1.0f - aa + aa * sr))));
+}
+
+// Per-node inputs of the CRKSPH pair loop: (rho, P, c, V).
+__global__ void crkInputs32(Fields32 P, long n) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 th = P.thermo[i];
+  P.pk[i] = make_float4(th.x, th.y, th.z, P.vol[i]);
 }
 
 __global__ void volumeMirrorKernel(Fields F, Fields32 P, long n) {
@@ -570,10 +556,23 @@ __global__ void volumeMirrorKernel(Fields F, Fields32 P, long n) {
 
 }  // namespace
 
+#define SPH_CRK_SWEEP(KERNEL, U, ...)                                                                              \
+  do {                                                                                                             \
+    const int L = lanesSweep(n);                                                                                   \
+    if (hasMirrors(g)) { SPH_CRK_LANES(KERNEL, true, U, __VA_ARGS__) } else { SPH_CRK_LANES(KERNEL, false, U, __VA_ARGS__) } \
+  } while (0)
+#define SPH_CRK_LANES(KERNEL, MI, U, ...)                                                                          \
+  switch (L) {                                                                                                     \
+    case 1: KERNEL<MI, 1, U><<<gridFor(n, sweepBlock(1)), sweepBlock(1), 0, s>>>(__VA_ARGS__); break;              \
+    case 4: KERNEL<MI, 4, U><<<gridFor(4 * n, 128), 128, 0, s>>>(__VA_ARGS__); break;                              \
+    case 8: KERNEL<MI, 8, U><<<gridFor(8 * n, 128), 128, 0, s>>>(__VA_ARGS__); break;                              \
+    default: KERNEL<MI, 16, U><<<gridFor(16 * n, 128), 128, 0, s>>>(__VA_ARGS__); break;                           \
+  }
+
 void launchRKVolumesFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                          cudaStream_t s, LaunchCounter* lc) {
   if (hp.rkVolume == 1) {
-    rkSumVolume32<<<gridFor(n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp);
+    SPH_CRK_SWEEP(rkSumVolume32, 4, F, P, n, g, nl, t, hp);
     lc->add(1);
   } else {   // the per-node volume types in FP64, then the mirror
     launchRKVolumes(F, n, g, nl, t, hp, s, lc);
@@ -581,40 +580,50 @@ void launchRKVolumesFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
     lc->add(1);
   }
 }
-void launchVolumeMirror(Fields F, Fields32 P, long n, cudaStream_t s, LaunchCounter* lc) {
-  volumeMirrorKernel<<<gridFor(n, 256), 256, 0, s>>>(F, P, n);
-  lc->add(1);
-}
 void launchCRKDensityFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                           HydroParams hp, cudaStream_t s, LaunchCounter* lc) {
-  crkDensity32<<<gridFor(n, 128), 128, 0, s>>>(F, P, list, n, g, nl, t, hp);
+  SPH_CRK_SWEEP(crkDensity32, 2, F, P, list, n, g, nl, t, hp);
   lc->add(1);
 }
 void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                              cudaStream_t s, LaunchCounter* lc) {
-  rkCorrections32<<<gridFor(n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp);
+  // several lanes repeat the FP64 solve's issue for fewer nodes per warp: only
+  // where one lane per node leaves SMs idle
+  const bool mir = hasMirrors(g);
+#define SPH_RKC(MI, LA) rkCorrections32<MI, LA, 2><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp)
+  if (n >= 40000) { if (mir) SPH_RKC(true, 1); else SPH_RKC(false, 1); }
+  else if (n >= 15000) { if (mir) SPH_RKC(true, 2); else SPH_RKC(false, 2); }
+  else { if (mir) SPH_RKC(true, 4); else SPH_RKC(false, 4); }
+#undef SPH_RKC
   lc->add(1);
 }
+// variant 0: one slot per iteration, 1: two (compatible energy, no XSPH).
 void launchPairCRKFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                        HydroParams hp, float* pacc, int variant, cudaStream_t s, LaunchCounter* lc) {
-  const unsigned gb = gridFor(n, 128);
-#define SPH_CRK32(X, C, Q) pairKernelCRK32<X, C, Q><<<gb, 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc)
-  // variant 1: two slots per iteration (compatible energy, no XSPH)
-  if (variant == 1 && !hp.xsph && hp.compatible) {
-    if (hp.limitedQ) pairKernelCRK32<false, true, true, 2><<<gb, 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc);
-    else pairKernelCRK32<false, true, false, 2><<<gb, 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc);
-    lc->add(1);
-    return;
-  }
-  if (hp.limitedQ) {
-    if (hp.xsph) { if (hp.compatible) SPH_CRK32(true, true, true); else SPH_CRK32(true, false, true); }
-    else { if (hp.compatible) SPH_CRK32(false, true, true); else SPH_CRK32(false, false, true); }
+  crkInputs32<<<gridFor(n, 256), 256, 0, s>>>(P, n);
+  const int L = n >= 100000 ? 1 : (n >= 20000 ? 2 : 4);
+  const bool mir = hasMirrors(g);
+#define SPH_CRK32(X, C, Q, MI, LA, U, MB) \
+  pairKernelCRK32<X, C, Q, MI, LA, U, MB><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc)
+#define SPH_CRK32L(Q, MI)                                                                                  \
+  do {                                                                                                     \
+    if (L == 1) { if (variant & 1) SPH_CRK32(false, true, Q, MI, 1, 2, 2); else SPH_CRK32(false, true, Q, MI, 1, 1, 4); } \
+    else if (L == 2) SPH_CRK32(false, true, Q, MI, 2, 1, 4);                                               \
+    else SPH_CRK32(false, true, Q, MI, 4, 1, 4);                                                           \
+  } while (0)
+  if (!hp.xsph && hp.compatible) {
+    if (mir) { if (hp.limitedQ) SPH_CRK32L(true, true); else SPH_CRK32L(false, true); }
+    else { if (hp.limitedQ) SPH_CRK32L(true, false); else SPH_CRK32L(false, false); }
+  } else if (hp.limitedQ) {
+    if (hp.xsph) { if (hp.compatible) SPH_CRK32(true, true, true, true, 1, 1, 3); else SPH_CRK32(true, false, true, true, 1, 1, 3); }
+    else SPH_CRK32(false, false, true, true, 1, 1, 3);
   } else {
-    if (hp.xsph) { if (hp.compatible) SPH_CRK32(true, true, false); else SPH_CRK32(true, false, false); }
-    else { if (hp.compatible) SPH_CRK32(false, true, false); else SPH_CRK32(false, false, false); }
+    if (hp.xsph) { if (hp.compatible) SPH_CRK32(true, true, false, true, 1, 1, 3); else SPH_CRK32(true, false, false, true, 1, 1, 3); }
+    else SPH_CRK32(false, false, false, true, 1, 1, 3);
   }
+#undef SPH_CRK32L
 #undef SPH_CRK32
-  lc->add(1);
+  lc->add(2);
 }
 
 }  // namespace sph

@@ -99,6 +99,89 @@ __device__ __forceinline__ void resetScratch(StepScratch* sc) {
   sc->voteEst = 0x7f7fffffu;   // FLT_MAX
 }
 
+__device__ __forceinline__ void lookupPacked(const float4* __restrict__ ta, const float2* __restrict__ tb, int N1,
+                                             float invStep, float eta, float extent, float& w, float& gr) {
+  if (eta < extent) {
+    const int k = min(N1, (int)(eta * invStep));
+    const float4 A = ta[k];
+    const float2 B = tb[k];
+    w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
+    gr = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
+  } else {
+    w = 0.0f;
+    gr = 0.0f;
+  }
+}
+
+// The packed table in shared memory with a zero interval behind it: an eta at
+// or beyond the extent reads zeros, no branch.
+constexpr int kTab32 = kMaxTable / 3 + 1;
+__device__ __forceinline__ void loadTable32(float4* ta, float2* tb, const TableDev& t, int N1) {
+  for (int k = threadIdx.x; k <= N1 + 1; k += blockDim.x) {
+    ta[k] = k <= N1 ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tb) tb[k] = k <= N1 ? t.p32b[k] : make_float2(0.f, 0.f);
+  }
+}
+
+// W and W' of the sweeps: KERN 1 the cubic B-spline over A in registers, 0
+// the packed table.
+template <int KERN>
+struct Kernel32 {
+  const float4* ta;
+  const float2* tb;
+  int N1;
+  float invStep;
+  __device__ __forceinline__ int index(float eta) const { return min(N1 + 1, (int)(eta * invStep)); }
+  __device__ __forceinline__ float value(float eta) const {
+    if (KERN) return bsplineW(eta);
+    const float4 A = ta[index(eta)];
+    return __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
+  }
+  __device__ __forceinline__ void both(float eta, float& w, float& g) const {
+    if (KERN) {
+      w = bsplineW(eta);
+      g = bsplineGrad(eta);
+    } else {
+      const int k = index(eta);
+      const float4 A = ta[k];
+      const float2 B = tb[k];
+      w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
+      g = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
+    }
+  }
+  __device__ __forceinline__ float grad(float eta) const {
+    if (KERN) return bsplineGrad(eta);
+    const int k = index(eta);
+    const float2 B = tb[k];
+    return __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, ta[k].w);
+  }
+};
+
+// Block size of the light sweeps.  With one lane per node a block of 512
+// consecutive nodes shares most of its neighbours, so more of its gathers hit
+// L1 than those of four separate blocks of 128 (2.1 M nodes: density/dt 1162 ->
+// 1029 us, energy 892 -> 860); small problems need the finer blocks to spread.
+__host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 512 : 128; }
+
+// Lanes per node.  One lane per node leaves the GPU idle below ~300,000 nodes
+// (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
+// shuffles and the partly filled last slots; the sweeps with light pair bodies
+// gain from two lanes at any size (two list rows per warp access).  Lines set
+// where the measured times cross.
+constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
+inline int lanesPair(long n) { return n >= 80000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
+inline int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
+inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16))); }
+
+#define SPH_BY_LANES(L, CALL)      \
+  switch (L) {                     \
+    case 1: CALL(1); break;        \
+    case 2: CALL(2); break;        \
+    case 4: CALL(4); break;        \
+    case 8: CALL(8); break;        \
+    default: CALL(16); break;      \
+  }
+
 // Velocity of a mirror image: the components along the mirrored axes flip
 // (mir: per-axis bits of the entry's cell-offset code that cross a wall).
 __device__ __forceinline__ void mirrorVel(uint32_t mir, float& vx, float& vy, float& vz) {

@@ -33,30 +33,6 @@ __global__ void prepareKernel(Fields F, Fields32 P, long n, Grid g) {
 // MUFU reciprocal square root and fast division), so slot (j, i) holds the
 // bitwise negation of slot (i, j).
 //------------------------------------------------------------------------------
-__device__ __forceinline__ void lookupPacked(const float4* __restrict__ ta, const float2* __restrict__ tb, int N1,
-                                             float invStep, float eta, float extent, float& w, float& gr) {
-  if (eta < extent) {
-    const int k = min(N1, (int)(eta * invStep));
-    const float4 A = ta[k];
-    const float2 B = tb[k];
-    w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
-    gr = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
-  } else {
-    w = 0.0f;
-    gr = 0.0f;
-  }
-}
-
-// The packed table in shared memory with a zero interval behind it: an eta at
-// or beyond the extent reads zeros, no branch.
-constexpr int kTab32 = kMaxTable / 3 + 1;
-__device__ __forceinline__ void loadTable32(float4* ta, float2* tb, const TableDev& t, int N1) {
-  for (int k = threadIdx.x; k <= N1 + 1; k += blockDim.x) {
-    ta[k] = k <= N1 ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tb) tb[k] = k <= N1 ? t.p32b[k] : make_float2(0.f, 0.f);
-  }
-}
-
 // TENSOR (ASPH): H_i, H_j from the FP32 tensor mirror (eta = H r,
 // grad W = gW H eta^, both in a fixed order so the pair force stays bitwise
 // antisymmetric), the second moment of ASPHClassicSmoothingScale and its
@@ -394,38 +370,6 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
 // and applied to the other sums per node; 0: packed table.  LEAN: compensated sums, no tensile correction
 // and the standard Q expansion fixed at compile time; otherwise read from hp.
 //------------------------------------------------------------------------------
-template <int KERN>
-struct Kernel32 {
-  const float4* ta;
-  const float2* tb;
-  int N1;
-  float invStep;
-  __device__ __forceinline__ int index(float eta) const { return min(N1 + 1, (int)(eta * invStep)); }
-  __device__ __forceinline__ float value(float eta) const {
-    if (KERN) return bsplineW(eta);
-    const float4 A = ta[index(eta)];
-    return __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
-  }
-  __device__ __forceinline__ void both(float eta, float& w, float& g) const {
-    if (KERN) {
-      w = bsplineW(eta);
-      g = bsplineGrad(eta);
-    } else {
-      const int k = index(eta);
-      const float4 A = ta[k];
-      const float2 B = tb[k];
-      w = __fmaf_rn(__fmaf_rn(A.z, eta, A.y), eta, A.x);
-      g = __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, A.w);
-    }
-  }
-  __device__ __forceinline__ float grad(float eta) const {
-    if (KERN) return bsplineGrad(eta);
-    const int k = index(eta);
-    const float2 B = tb[k];
-    return __fmaf_rn(__fmaf_rn(B.y, eta, B.x), eta, ta[k].w);
-  }
-};
-
 template <bool XSPH, bool COMPAT, bool MULTI, bool LIMQ, bool LEAN, bool MIR, int KERN, int L, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 P, const int* __restrict__ list, long n,
                                                              Grid g, NeighborLists nl, TableDev t, HydroParams hp,
@@ -841,12 +785,6 @@ __global__ void pairInputs32(Fields F, Fields32 P, long n, float Cl, int limited
     P.dvq[2 * i + 1] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
   }
 }
-
-// Block size of the light sweeps.  With one lane per node a block of 512
-// consecutive nodes shares most of its neighbours, so more of its gathers hit
-// L1 than those of four separate blocks of 128 (2.1 M nodes: density/dt 1162 ->
-// 1029 us, energy 892 -> 860); small problems need the finer blocks to spread.
-__host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 512 : 128; }
 
 //------------------------------------------------------------------------------
 // Time-step vote.  The smallest limit travels as one 64-bit word, the bits of
@@ -1270,16 +1208,6 @@ void launchPrepareFP32(Fields F, Fields32 F32, long n, Grid g, cudaStream_t s, L
 }
 
 constexpr int kDensU = 2, kGradhU = 4;   // slots per iteration of the density and grad-h sweeps
-// Lanes per node.  One lane per node leaves the GPU idle below ~300,000 nodes
-// (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
-// shuffles and the partly filled last slots; the sweeps with light pair bodies
-// gain from two lanes at any size (two list rows per warp access).  Lines set
-// where the measured times cross.
-constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
-int lanesPair(long n) { return n >= 80000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
-int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
-int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16))); }
-
 // variant (isotropic, lean path, one lane per node, standard Q): two slots per
 // iteration at 4 blocks per SM (even, <= 128 registers) or 5 (odd, <= 102).
 // At 2.1 M nodes 1741 / 1620 us, the limited Q spills at 102 (180 / 242 us at
@@ -1366,15 +1294,6 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
 }
 
 // Slots per iteration of the density and grad-h sweeps: see densityKernel32.
-#define SPH_BY_LANES(L, CALL)      \
-  switch (L) {                     \
-    case 1: CALL(1); break;        \
-    case 2: CALL(2); break;        \
-    case 4: CALL(4); break;        \
-    case 8: CALL(8); break;        \
-    default: CALL(16); break;      \
-  }
-
 static void launchDensity32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                             const HydroParams& hp, bool dt, double maxNperh, unsigned long long* key, cudaStream_t s) {
   const int L = lanesSweep(n);
