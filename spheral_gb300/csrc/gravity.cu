@@ -44,6 +44,7 @@
 // it is retaken in FP64 with the reference's expression, so the set of far
 // cells and opened leaves is the FP64 walk's.
 #include "kernels.cuh"
+#include "recip64.cuh"
 #include "sort.cuh"
 #include "../../include/sphgpu.h"
 
@@ -345,23 +346,51 @@ __global__ void momentKernel(TreeCell* __restrict__ cells, long long numCells, i
 //------------------------------------------------------------------------------
 // Walk (TreeGravity::applyTreeForces, TreeGravity.cc:819-932).
 //------------------------------------------------------------------------------
-__device__ __forceinline__ void addMonopole(double M, double dx, double dy, double dz, double r2, double soft2,
-                                            double& ax, double& ay, double& az, double& phi) {
+__device__ __forceinline__ void addMonopole(double M, double dx, double dy, double dz, double soft2, double& ax,
+                                            double& ay, double& az, double& phi) {
   // nhat = unitVector(xji); rji2 += soft2; a += M/rji2 nhat; phi -= M/sqrt(rji2)
-  double nx = 1.0, ny = 0.0, nz = 0.0;
-  const double r = sqrt(r2);
-  if (r > 1.0e-50) {
-    const double ir = 1.0 / r;
-    nx = dx * ir; ny = dy * ir; nz = dz * ir;
+  const double r2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+  const double irs = dev::rsqrt64(r2 + soft2);
+  const double m = M * irs;
+  if (__double2hiint(r2) > 0x2b000000) {   // r > ~1e-50
+    const double f = (m * irs) * dev::rsqrt64(r2);
+    ax = __fma_rn(f, dx, ax); ay = __fma_rn(f, dy, ay); az = __fma_rn(f, dz, az);
+  } else {
+    ax = __fma_rn(m, irs, ax);   // the unit vector of a zero separation is (1, 0, 0)
   }
-  const double r2s = r2 + soft2;
-  const double irs = rsqrt(r2s);
-  const double f = M * (irs * irs);
-  ax += f * nx; ay += f * ny; az += f * nz;
-  phi -= M * irs;
+  phi -= m;
 }
 
-__global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell* __restrict__ cells, long long numCells,
+// The walk's opening decision for one lane: FP32 on double-float separations,
+// repeated in FP64 with the reference's expression inside a guard band of
+// +-4e-6 (far above the FP32 error) and where FP32 would leave its normal
+// range.  Every lane decides as the FP64 walk does.
+struct WalkCell {
+  float4 a, b;   // xh yh zh M | xl yl zl open2
+};
+__device__ __forceinline__ bool farCell(const WalkCell& q, float xh, float yh, float zh, float xl, float yl, float zl,
+                                        float& dx, float& dy, float& dz, float& r2, bool& unsure) {
+  dx = __fadd_rn(__fsub_rn(q.a.x, xh), __fsub_rn(q.b.x, xl));
+  dy = __fadd_rn(__fsub_rn(q.a.y, yh), __fsub_rn(q.b.y, yl));
+  dz = __fadd_rn(__fsub_rn(q.a.z, zh), __fsub_rn(q.b.z, zl));
+  r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+  constexpr float kBand = 4.0e-6f;
+  const float o2 = q.b.w;
+  const bool far = r2 > o2 * (1.0f + kBand), near = r2 < o2 * (1.0f - kBand);
+  unsure = !(far | near) | !(fmaxf(r2, o2) > 1.0e-30f);
+  return far;
+}
+__device__ __forceinline__ bool farCell64(const TreeCell& cd, double x, double y, double z, double thr) {
+  const double ex = __dsub_rn(cd.x, x), ey = __dsub_rn(cd.y, y), ez = __dsub_rn(cd.z, z);
+  const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
+  return q2 > __dadd_rn(thr, cd.r2cc);
+}
+
+// FP64 walk.  The decisions take FP32 (farCell), so the FP64 unit, two
+// operations per SM and clock, only sees the interactions: ~24 instructions
+// each instead of ~60 per visited cell.
+__global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restrict__ c32,
+                                                     const TreeCell* __restrict__ cells, long long numCells,
                                                      const TreeNode* __restrict__ tpos, const int* __restrict__ vals,
                                                      long n, const double* __restrict__ thrLevel, double soft2,
                                                      double softening, double G, Fields F,
@@ -379,6 +408,10 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell* __restrict
     const TreeNode p = tpos[k];
     xi = p.x; yi = p.y; zi = p.z; mi = p.m;
   }
+  float xh, yh, zh, xl, yl, zl;
+  splitDF(xi, xh, xl);
+  splitDF(yi, yh, yl);
+  splitDF(zi, zh, zl);
   double ax = 0, ay = 0, az = 0, phi = 0;
   // until: this lane ignores cells below this pre-order index
   unsigned until = valid ? 0u : 0xFFFFFFFFu;
@@ -386,25 +419,32 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell* __restrict
   const unsigned nc = (unsigned)numCells;
   if (__all_sync(0xffffffffu, !valid)) c = nc;
   while (c < nc) {
-    const double2* cp = reinterpret_cast<const double2*>(cells + c);
-    const double2 qa = __ldg(cp), qb = __ldg(cp + 1), qc = __ldg(cp + 2);
-    const int4 qi = __ldg(reinterpret_cast<const int4*>(cp + 3));
-    const double cxm = qa.x, cym = qa.y, czm = qb.x, cM = qb.y, r2cc = qc.x;
+    const float4* cp = reinterpret_cast<const float4*>(c32 + c);
+    const WalkCell q{__ldg(cp), __ldg(cp + 1)};
+    const int4 qi = __ldg(reinterpret_cast<const int4*>(cp + 2));
     const unsigned skip = (unsigned)qi.x;
     const int start = qi.y, count = qi.z, level = qi.w & 255, leaf = qi.w >> 8;
     bool descend = false;
     if (c >= until) {
-      const double dx = __dsub_rn(cxm, xi), dy = __dsub_rn(cym, yi), dz = __dsub_rn(czm, zi);
-      const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-      if (r2 > __dadd_rn(thr[level], r2cc)) {
-        addMonopole(cM, dx, dy, dz, r2, soft2, ax, ay, az, phi);
+      float dx, dy, dz, r2;
+      bool unsure;
+      bool far = farCell(q, xh, yh, zh, xl, yl, zl, dx, dy, dz, r2, unsure);
+      if (unsure) far = farCell64(cells[c], xi, yi, zi, thr[level]);
+      if (far) {
+        const double2* dp = reinterpret_cast<const double2*>(cells + c);
+        const double2 qa = __ldg(dp), qb = __ldg(dp + 1);
+        addMonopole(qb.y, qa.x - xi, qa.y - yi, qb.x - zi, soft2, ax, ay, az, phi);
         until = skip;
       } else if (leaf) {
         for (int j = start; j < start + count; ++j) {
           const TreeNode p = loadNode(tpos + j);
           const double ex = __dsub_rn(p.x, xi), ey = __dsub_rn(p.y, yi), ez = __dsub_rn(p.z, zi);
+          // s2 / soft2 > 1e-10, the division only near the limit
           const double s2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-          if (__ddiv_rn(s2, soft2) > 1.0e-10) addMonopole(p.m, ex, ey, ez, s2, soft2, ax, ay, az, phi);
+          const double lim = 1.0e-10 * soft2;
+          bool use = s2 > lim * 1.001;
+          if (!use && s2 >= lim * 0.999) use = __ddiv_rn(s2, soft2) > 1.0e-10;
+          if (use) addMonopole(p.m, ex, ey, ez, soft2, ax, ay, az, phi);
         }
         until = skip;
       } else {
@@ -476,14 +516,14 @@ struct Acc32 {
 
 __device__ __forceinline__ void addMonopole32(float M, float dx, float dy, float dz, float r2, float soft2,
                                               Acc32& a) {
-  const float ir = r2 > 1.0e-30f ? rsqrtf(r2) : 0.0f;
-  const float nx = r2 > 1.0e-30f ? dx * ir : 1.0f, ny = dy * ir, nz = dz * ir;
   const float irs = rsqrtf(r2 + soft2);
-  const float f = M * (irs * irs);
-  kahan(a.sx, a.cx, f * nx);
-  kahan(a.sy, a.cy, f * ny);
-  kahan(a.sz, a.cz, f * nz);
-  kahan(a.sp, a.cp, -M * irs);
+  const float m = M * irs, f0 = m * irs;
+  const bool apart = r2 > 1.0e-30f;
+  const float f = apart ? f0 * rsqrtf(r2) : f0;
+  kahan(a.sx, a.cx, f * (apart ? dx : 1.0f));   // the unit vector of a zero separation is (1, 0, 0)
+  kahan(a.sy, a.cy, f * dy);
+  kahan(a.sz, a.cz, f * dz);
+  kahan(a.sp, a.cp, -m);
 }
 
 __global__ void __launch_bounds__(128) treeWalkMixedKernel(
@@ -506,7 +546,6 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
     xd = p.x; yd = p.y; zd = p.z; mi = p.m;
   }
   const float soft2 = (float)soft2d;
-  constexpr float kBand = 4.0e-6f;
   Acc32 acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   unsigned until = valid ? 0u : 0xFFFFFFFFu;
   unsigned c = 1;
@@ -514,28 +553,18 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
   if (__all_sync(0xffffffffu, !valid)) c = nc;
   while (c < nc) {
     const float4* cp = reinterpret_cast<const float4*>(c32 + c);
-    const float4 qa = __ldg(cp), qb = __ldg(cp + 1);
+    const WalkCell q{__ldg(cp), __ldg(cp + 1)};
     const int4 qi = __ldg(reinterpret_cast<const int4*>(cp + 2));
     const unsigned skip = (unsigned)qi.x;
     const int start = qi.y, count = qi.z, level = qi.w & 255, leaf = qi.w >> 8;
     bool descend = false;
     if (c >= until) {
-      const float dx = __fadd_rn(__fsub_rn(qa.x, me.xh), __fsub_rn(qb.x, me.xl));
-      const float dy = __fadd_rn(__fsub_rn(qa.y, me.yh), __fsub_rn(qb.y, me.yl));
-      const float dz = __fadd_rn(__fsub_rn(qa.z, me.zh), __fsub_rn(qb.z, me.zl));
-      const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-      const float o2 = qb.w;
-      bool far;
-      if (r2 > o2 * (1.0f + kBand)) far = true;
-      else if (r2 < o2 * (1.0f - kBand)) far = false;
-      else {   // guard band: the reference's FP64 test
-        const TreeCell& cd = cells[c];
-        const double ex = __dsub_rn(cd.x, xd), ey = __dsub_rn(cd.y, yd), ez = __dsub_rn(cd.z, zd);
-        const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-        far = q2 > __dadd_rn(thr[level], cd.r2cc);
-      }
+      float dx, dy, dz, r2;
+      bool unsure;
+      bool far = farCell(q, me.xh, me.yh, me.zh, me.xl, me.yl, me.zl, dx, dy, dz, r2, unsure);
+      if (unsure) far = farCell64(cells[c], xd, yd, zd, thr[level]);
       if (far) {
-        addMonopole32(qa.w, dx, dy, dz, r2, soft2, acc);
+        addMonopole32(q.a.w, dx, dy, dz, r2, soft2, acc);
         until = skip;
       } else if (leaf) {
         for (int j = start; j < start + count; ++j) {
@@ -731,19 +760,18 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
                                               w->box.as<double>(), w->mx.as<double>());
   }
   lc->add(kMaxLevel + 1);
-  if (mixed) {
-    GCHK(w->cells32.ensure(numCells * sizeof(TreeCell32)));
-    cells32Kernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->thr.as<double>(), w->cells32.as<TreeCell32>());
+  GCHK(w->cells32.ensure(numCells * sizeof(TreeCell32)));
+  cells32Kernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->thr.as<double>(), w->cells32.as<TreeCell32>());
+  if (mixed)
     treeWalkMixedKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells,
                                                w->tpos32.as<TreeNode32>(), w->tpos.as<TreeNode>(), vals, n,
                                                w->thr.as<double>(), softening * softening, softening, G, F,
                                                w->dtBits.as<unsigned long long>(), w->energy.as<double>());
-    lc->add(1);
-  } else {
-    treeWalkKernel<<<nbWalk, 128, 0, s>>>(cells, numCells, w->tpos.as<TreeNode>(), vals, n, w->thr.as<double>(),
-                                          softening * softening, softening, G, F,
+  else
+    treeWalkKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells, w->tpos.as<TreeNode>(), vals,
+                                          n, w->thr.as<double>(), softening * softening, softening, G, F,
                                           w->dtBits.as<unsigned long long>(), w->energy.as<double>());
-  }
+  lc->add(1);
   walkFinalKernel<<<1, 256, 0, s>>>(w->energy.as<double>(), nbWalk, w->dtBits.as<unsigned long long>(), G, dOut);
   lc->add(2);
   GCHK(cudaGetLastError());

@@ -17,6 +17,7 @@
 //    third-order Householder step;
 //  * comparisons of positive values and index arithmetic use the integer pipe.
 #include "device.cuh"
+#include "recip64.cuh"
 
 namespace sph {
 namespace {
@@ -24,22 +25,6 @@ using namespace dev;
 
 inline unsigned gridFor(long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// 1/sqrt(x), x normal and positive: y the hardware seed, e = 1 - x y^2,
-// y (1 + e/2 + 3 e^2/8) (Householder's method of third order; the
-// remainder is below 2^-56).
-__device__ __forceinline__ double rsqrt64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
-  return __fma_rn(__dmul_rn(e, y), __fma_rn(e, 0.375, 0.5), y);
-}
-// 1/x, x normal: r (1 + e + e^2) with e = 1 - x r (third order).
-__device__ __forceinline__ double rcp64(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = __fma_rn(-x, r, 1.0);
-  return __fma_rn(r, __fma_rn(e, e, e), r);
-}
 __device__ __forceinline__ long long bits(double x) { return __double_as_longlong(x); }
 // max of two non-negative values
 __device__ __forceinline__ double maxPos(double a, double b) { return bits(a) > bits(b) ? a : b; }
