@@ -30,9 +30,11 @@
 // of a warp (neighbours in Morton order) walk the pre-order cell array
 // together: a lane that applies a cell (far or leaf) skips that cell's
 // subtree; the warp descends into a cell while any lane still needs it open.
-// Forces, potentials and the decision are evaluated in FP64 with the
-// reference's expressions (no fused multiply-add in the opening test);
-// summation order is pre-order instead of level order.
+// (In the FP64 walk a warp walks for 8 nodes and queues the interactions.)
+// Forces and potentials are evaluated in FP64; so is the decision wherever FP32
+// could take it differently, with the reference's expression (no fused
+// multiply-add).  Summation order is pre-order, split over the lanes of a node,
+// instead of level order.
 //
 // Mixed precision (the mixed-mode package).  GB300's FP64 pipe is thin, so
 // the mixed walk evaluates each interaction in FP32 on double-float
@@ -44,6 +46,7 @@
 // it is retaken in FP64 with the reference's expression, so the set of far
 // cells and opened leaves is the FP64 walk's.
 #include "kernels.cuh"
+#include "packed32.cuh"
 #include "recip64.cuh"
 #include "sort.cuh"
 #include "../../include/sphgpu.h"
@@ -74,6 +77,10 @@ struct __align__(32) TreeCell {
 };
 static_assert(sizeof(TreeCell) == 64, "TreeCell layout");
 
+struct __align__(32) Sums4 {
+  double x, y, z, w;   // sums of m x, m y, m z and m
+};
+
 // Node in tree order: position and mass.
 struct __align__(32) TreeNode {
   double x, y, z, m;
@@ -85,12 +92,17 @@ __device__ __forceinline__ TreeNode loadNode(const TreeNode* __restrict__ p) {
   return TreeNode{a.x, a.y, b.x, b.y};
 }
 
-// Mixed-walk copies: double-float centre of mass, FP32 mass, FP32 opening
-// threshold thr[level] + rcm2cc2; same skip/start/count/lvl.
+// What a walk reads of a cell it visits: the double-float centre of mass in
+// pairs for the packed operations, the mass, and the decision thresholds.  With
+// r2 the FP32 squared separation, r2 > hi: the cell's monopole applies (a far
+// cell, or a one-node leaf, whose monopole is its node); r2 < lo: it does not
+// (an internal cell is opened, a one-node leaf is the node itself); between
+// them FP64 decides.
 struct __align__(16) TreeCell32 {
-  float xh, yh, zh, M;
-  float xl, yl, zl, open2;
-  int skip, start, count, lvl;
+  float xh, yh, xl, yl;
+  float zh, zl, hi, lo;
+  float M;
+  int skip, start, cnt;   // cnt: nodes of a leaf, 0 for an internal cell
 };
 static_assert(sizeof(TreeCell32) == 48, "TreeCell32 layout");
 
@@ -185,10 +197,13 @@ __global__ void boxFinalKernel(const double* __restrict__ part, int nb, double o
                                double* __restrict__ thr, unsigned long long* __restrict__ dtBits) {
   __shared__ double v[6];
   __shared__ double sL2;
-  if (threadIdx.x < 6) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;   // a warp per component
+  if (warp < 6) {
     double r = DBL_MAX;
-    for (int b = 0; b < nb; ++b) r = fmin(r, part[b * 6 + threadIdx.x]);
-    v[threadIdx.x] = r;
+    for (int b = lane; b < nb; b += 32) r = fmin(r, part[b * 6 + warp]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r = fmin(r, __shfl_xor_sync(0xffffffffu, r, o));
+    if (lane == 0) v[warp] = r;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -299,48 +314,120 @@ __global__ void cellBuildKernel(const uint64_t* __restrict__ skey, long n, const
   }
 }
 
-// Monopoles of the cells of one level (children are one level deeper and
-// already done).  Leaves sum their nodes; a one-node leaf keeps the node's
-// position exactly, as the reference's single-node cell does.
-__global__ void momentKernel(TreeCell* __restrict__ cells, long long numCells, int level,
-                             const TreeNode* __restrict__ tpos, const uint64_t* __restrict__ skey,
-                             const double* __restrict__ box, double* __restrict__ mx) {
+// Parent and number of daughters of every cell.
+__global__ void linkKernel(const TreeCell* __restrict__ cells, long long numCells, int* __restrict__ parent,
+                           int* __restrict__ pending) {
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (c >= numCells) return;
+  if (c == 0) parent[0] = -1;
+  if (cells[c].lvl >> 8) return;
+  const int end = cells[c].skip;
+  int m = 0;
+  for (int ch = (int)c + 1; ch < end; ch = cells[ch].skip) { parent[ch] = (int)c; ++m; }
+  pending[c] = m;
+}
+
+// The walks' thresholds (TreeCell32) from the squared opening distance and,
+// for a one-node leaf, the separation limit 1e-10 eps^2 below which the node
+// does not act.  The guard bands (4e-6, and 1e-3 for the limit) are far above
+// the FP32 error of r2; values near underflow are left to FP64.
+__device__ __forceinline__ void setThresholds(TreeCell32& o, double open2, double soft2) {
+  constexpr float kBand = 4.0e-6f, kTiny = 1.0e-30f;
+  const float o2 = (float)open2;
+  float hi = o2 * (1.0f + kBand), lo = o2 * (1.0f - kBand);
+  if (o.cnt == 1) {
+    const float lim = 1.0e-10f * (float)soft2;
+    hi = fminf(hi, lim * 1.001f);
+    lo = fminf(lo, lim * 0.999f);
+  }
+  o.hi = fmaxf(hi, kTiny);
+  o.lo = lo > kTiny ? lo : -1.0f;
+}
+
+__device__ __forceinline__ void cell32(const TreeCell& cl, double thr, double soft2, TreeCell32* __restrict__ out) {
+  TreeCell32 o;
+  splitDF(cl.x, o.xh, o.xl);
+  splitDF(cl.y, o.yh, o.yl);
+  splitDF(cl.z, o.zh, o.zl);
+  o.M = (float)cl.M;
+  o.skip = cl.skip;
+  o.start = cl.start;
+  o.cnt = (cl.lvl >> 8) ? cl.count : 0;
+  setThresholds(o, __dadd_rn(thr, cl.r2cc), soft2);
+  *out = o;
+}
+
+// Sums of m and m x of every cell, bottom-up in one launch: a thread per leaf
+// sums its nodes and climbs; the last daughter to arrive at a cell sums its
+// daughters in pre-order (so the sums do not depend on who arrives last).  Few
+// lanes of a warp climb far, so only the additions are done here: with the
+// divisions and opening distances it took 232 us at 222,119 cells, without them
+// 67 us and cellFinalKernel 27 us.
+__global__ void momentKernel(const TreeCell* __restrict__ cells, long long numCells,
+                             const TreeNode* __restrict__ tpos, const int* __restrict__ parent,
+                             int* __restrict__ pending, Sums4* __restrict__ sums) {
+  const long long c0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (c0 >= numCells) return;
+  {
+    const TreeCell& cl = cells[c0];
+    if (!(cl.lvl >> 8)) return;
+    double M = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+    for (int j = cl.start; j < cl.start + cl.count; ++j) {
+      const TreeNode p = tpos[j];
+      M += p.m; sx += p.m * p.x; sy += p.m * p.y; sz += p.m * p.z;
+    }
+    sums[c0] = Sums4{sx, sy, sz, M};
+  }
+  for (int c = parent[c0]; c >= 0; c = parent[c]) {
+    __threadfence();
+    if (atomicSub(&pending[c], 1) != 1) return;
+    __threadfence();
+    // the daughters' sums come from other threads: volatile reads pass L1
+    const int end = cells[c].skip;
+    double M = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+    for (int ch = c + 1; ch < end; ch = cells[ch].skip) {
+      const volatile double* m = reinterpret_cast<const volatile double*>(sums + ch);
+      sx += m[0]; sy += m[1]; sz += m[2]; M += m[3];
+    }
+    sums[c] = Sums4{sx, sy, sz, M};
+  }
+}
+
+// Centres of mass, opening distances and the walks' copy.  A one-node leaf
+// keeps the node's position exactly, as the reference's single-node cell does.
+__global__ void cellFinalKernel(TreeCell* __restrict__ cells, long long numCells, const TreeNode* __restrict__ tpos,
+                                const uint64_t* __restrict__ skey, const double* __restrict__ box,
+                                const double* __restrict__ thrLevel, double soft2, const Sums4* __restrict__ sums,
+                                TreeCell32* __restrict__ c32) {
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= numCells) return;
   TreeCell cl = cells[c];
-  if ((cl.lvl & 255) != level) return;
-  double M = 0.0, sx = 0.0, sy = 0.0, sz = 0.0, x, y, z;
-  if (cl.lvl >> 8) {
-    if (cl.count == 1) {
-      const TreeNode p = tpos[cl.start];
-      M = p.m; x = p.x; y = p.y; z = p.z;
-      sx = p.m * p.x; sy = p.m * p.y; sz = p.m * p.z;
-    } else {
-      for (int j = cl.start; j < cl.start + cl.count; ++j) {
-        const TreeNode p = tpos[j];
-        M += p.m; sx += p.m * p.x; sy += p.m * p.y; sz += p.m * p.z;
-      }
-      x = sx / M; y = sy / M; z = sz / M;
-    }
+  const int level = cl.lvl & 255;
+  const Sums4 sm = sums[c];
+  if ((cl.lvl >> 8) && cl.count == 1) {
+    const TreeNode p = tpos[cl.start];
+    cl.x = p.x; cl.y = p.y; cl.z = p.z; cl.M = p.m;
   } else {
-    for (long long ch = c + 1; ch < cl.skip; ch = cells[ch].skip) {
-      M += cells[ch].M;
-      sx += mx[3 * ch]; sy += mx[3 * ch + 1]; sz += mx[3 * ch + 2];
-    }
-    x = sx / M; y = sy / M; z = sz / M;
+    // one reciprocal, each quotient with its residual: a division's rounding but
+    // for rare last-bit cases, at a third of its FP64 operations
+    const double r = fabs(sm.w) > 1.0e-290 ? dev::rcp64(sm.w) : 1.0 / sm.w;
+    auto quotient = [&](double a) {
+      const double q = a * r;
+      return __fma_rn(__fma_rn(-q, sm.w, a), r, q);
+    };
+    cl.x = quotient(sm.x); cl.y = quotient(sm.y); cl.z = quotient(sm.z); cl.M = sm.w;
   }
-  mx[3 * c] = sx; mx[3 * c + 1] = sy; mx[3 * c + 2] = sz;
   // Geometric centre: xmin + (ix + 0.5) * cellsize, cellsize = boxLength / 2^level.
   const uint64_t key = skey[cl.start];
   const int sh = kMaxLevel - level;
-  const double cs = __ddiv_rn(box[3], (double)(1u << level));
+  const double cs = __dmul_rn(box[3], __hiloint2double((1023 - level) << 20, 0));
   const double cx = __dadd_rn(box[0], __dmul_rn((double)(compact3(key) >> sh) + 0.5, cs));
   const double cy = __dadd_rn(box[1], __dmul_rn((double)(compact3(key >> 1) >> sh) + 0.5, cs));
   const double cz = __dadd_rn(box[2], __dmul_rn((double)(compact3(key >> 2) >> sh) + 0.5, cs));
-  const double dx = __dsub_rn(x, cx), dy = __dsub_rn(y, cy), dz = __dsub_rn(z, cz);
-  cl.x = x; cl.y = y; cl.z = z; cl.M = M;
+  const double dx = __dsub_rn(cl.x, cx), dy = __dsub_rn(cl.y, cy), dz = __dsub_rn(cl.z, cz);
   cl.r2cc = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   cells[c] = cl;
+  cell32(cl, thrLevel[level], soft2, c32 + c);
 }
 
 //------------------------------------------------------------------------------
@@ -361,34 +448,58 @@ __device__ __forceinline__ void addMonopole(double M, double dx, double dy, doub
   phi -= m;
 }
 
-// The walk's opening decision for one lane: FP32 on double-float separations,
-// repeated in FP64 with the reference's expression inside a guard band of
-// +-4e-6 (far above the FP32 error) and where FP32 would leave its normal
-// range.  Every lane decides as the FP64 walk does.
-struct WalkCell {
-  float4 a, b;   // xh yh zh M | xl yl zl open2
+// A node in the walks' double-float form, negated so that separations are sums.
+struct WalkNode {
+  dev::f32x2 nxyh, nxyl, nz;
 };
-__device__ __forceinline__ bool farCell(const WalkCell& q, float xh, float yh, float zh, float xl, float yl, float zl,
-                                        float& dx, float& dy, float& dz, float& r2, bool& unsure) {
-  dx = __fadd_rn(__fsub_rn(q.a.x, xh), __fsub_rn(q.b.x, xl));
-  dy = __fadd_rn(__fsub_rn(q.a.y, yh), __fsub_rn(q.b.y, yl));
-  dz = __fadd_rn(__fsub_rn(q.a.z, zh), __fsub_rn(q.b.z, zl));
-  r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-  constexpr float kBand = 4.0e-6f;
-  const float o2 = q.b.w;
-  const bool far = r2 > o2 * (1.0f + kBand), near = r2 < o2 * (1.0f - kBand);
-  unsure = !(far | near) | !(fmaxf(r2, o2) > 1.0e-30f);
-  return far;
-}
-__device__ __forceinline__ bool farCell64(const TreeCell& cd, double x, double y, double z, double thr) {
-  const double ex = __dsub_rn(cd.x, x), ey = __dsub_rn(cd.y, y), ez = __dsub_rn(cd.z, z);
-  const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-  return q2 > __dadd_rn(thr, cd.r2cc);
+__device__ __forceinline__ WalkNode walkNode(double x, double y, double z) {
+  float xh, yh, zh, xl, yl, zl;
+  splitDF(x, xh, xl);
+  splitDF(y, yh, yl);
+  splitDF(z, zh, zl);
+  return WalkNode{dev::pack2(-xh, -yh), dev::pack2(-xl, -yl), dev::pack2(-zh, -zl)};
 }
 
-// FP64 walk.  The decisions take FP32 (farCell), so the FP64 unit, two
-// operations per SM and clock, only sees the interactions: ~24 instructions
-// each instead of ~60 per visited cell.
+struct WalkCell {
+  ulonglong2 xy;   // (xh yh) (xl yl)
+  ulonglong2 zt;   // (zh zl) (hi lo)
+  int4 q;          // M skip start cnt
+};
+__device__ __forceinline__ WalkCell loadCell(const TreeCell32* __restrict__ c32, unsigned c) {
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(c32 + c);
+  return WalkCell{__ldg(p), __ldg(p + 1), __ldg(reinterpret_cast<const int4*>(p + 2))};
+}
+
+// Separation (hi_c - hi_i) + (lo_c - lo_i) and its square.
+__device__ __forceinline__ float separation(const WalkCell& q, const WalkNode& me, dev::f32x2& dxy, float& dz) {
+  dxy = dev::add2(dev::add2(q.xy.x, me.nxyh), dev::add2(q.xy.y, me.nxyl));
+  float zh, zl, dx, dy;
+  dev::unpack2(dev::add2(q.zt.x, me.nz), zh, zl);
+  dz = __fadd_rn(zh, zl);
+  dev::unpack2(dxy, dx, dy);
+  return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+// The FP64 decision, the reference's expressions: does the cell's monopole
+// apply (far, or a one-node leaf beyond the separation limit)?
+__device__ __noinline__ bool applies64(const TreeCell* __restrict__ cells, unsigned c, double x, double y, double z,
+                                       const double* thr, double soft2) {
+  const TreeCell& cd = cells[c];
+  const double ex = __dsub_rn(cd.x, x), ey = __dsub_rn(cd.y, y), ez = __dsub_rn(cd.z, z);
+  const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
+  if (q2 > __dadd_rn(thr[cd.lvl & 255], cd.r2cc)) return true;
+  return (cd.lvl >> 8) && cd.count == 1 && __ddiv_rn(q2, soft2) > 1.0e-10;
+}
+
+// FP64 walk.  GB300's FP64 unit takes a warp instruction every 16 cycles per
+// SM, so what counts is the number of warp interactions of ~22 FP64 operations:
+// the decisions take FP32 (TreeCell32), and a warp walks for 8 nodes, which
+// queue the cells that apply in shared memory; all 32 lanes (4 per node) then
+// work through the queues.  Of 32 nodes that walk in step only 12 apply a cell
+// at a time; the queues bring that to 28.  They drain to half their length, so
+// that short ones need not keep up.  30,011 nodes of the Evrard sphere: gravity
+// 4764 -> 1881 us per step.
+constexpr int kWalkLanes = 4, kWalkNodes = 32 / kWalkLanes, kQueue = 128;
 __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restrict__ c32,
                                                      const TreeCell* __restrict__ cells, long long numCells,
                                                      const TreeNode* __restrict__ tpos, const int* __restrict__ vals,
@@ -399,64 +510,83 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restri
   __shared__ double thr[kMaxLevel + 1];
   __shared__ double esum[4];
   __shared__ double dmin[4];
+  __shared__ unsigned queues[4][kWalkNodes][kQueue + kWalkLanes];   // the odd 4 spread the banks
   if (threadIdx.x <= kMaxLevel) thr[threadIdx.x] = thrLevel[threadIdx.x];
   __syncthreads();
-  const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long k = (blockIdx.x * (long)blockDim.x + threadIdx.x) / kWalkLanes;
+  const int sub = threadIdx.x % kWalkLanes;
   const bool valid = k < n;
   double xi = 0, yi = 0, zi = 0, mi = 0;
   if (valid) {
     const TreeNode p = tpos[k];
     xi = p.x; yi = p.y; zi = p.z; mi = p.m;
   }
-  float xh, yh, zh, xl, yl, zl;
-  splitDF(xi, xh, xl);
-  splitDF(yi, yh, yl);
-  splitDF(zi, zh, zl);
+  const WalkNode me = walkNode(xi, yi, zi);
   double ax = 0, ay = 0, az = 0, phi = 0;
+  unsigned* queue = queues[threadIdx.x >> 5][(threadIdx.x & 31) / kWalkLanes];
+  unsigned head = 0, tail = 0;
+  auto drain = [&](unsigned keep) {
+    __syncwarp();
+    while (__any_sync(0xffffffffu, tail - head > keep)) {
+      const unsigned e = head + sub;
+      if (e < tail) {
+        const double2* dp = reinterpret_cast<const double2*>(cells + queue[e % kQueue]);
+        const double2 qa = __ldg(dp), qb = __ldg(dp + 1);
+        addMonopole(qb.y, qa.x - xi, qa.y - yi, qb.x - zi, soft2, ax, ay, az, phi);
+      }
+      head = min(head + kWalkLanes, tail);
+    }
+    __syncwarp();
+  };
   // until: this lane ignores cells below this pre-order index
   unsigned until = valid ? 0u : 0xFFFFFFFFu;
   unsigned c = 1;   // the walk starts at the root's daughters
   const unsigned nc = (unsigned)numCells;
   if (__all_sync(0xffffffffu, !valid)) c = nc;
   while (c < nc) {
-    const float4* cp = reinterpret_cast<const float4*>(c32 + c);
-    const WalkCell q{__ldg(cp), __ldg(cp + 1)};
-    const int4 qi = __ldg(reinterpret_cast<const int4*>(cp + 2));
-    const unsigned skip = (unsigned)qi.x;
-    const int start = qi.y, count = qi.z, level = qi.w & 255, leaf = qi.w >> 8;
+    const WalkCell q = loadCell(c32, c);
+    const unsigned skip = (unsigned)q.q.y;
     bool descend = false;
     if (c >= until) {
-      float dx, dy, dz, r2;
-      bool unsure;
-      bool far = farCell(q, xh, yh, zh, xl, yl, zl, dx, dy, dz, r2, unsure);
-      if (unsure) far = farCell64(cells[c], xi, yi, zi, thr[level]);
-      if (far) {
-        const double2* dp = reinterpret_cast<const double2*>(cells + c);
-        const double2 qa = __ldg(dp), qb = __ldg(dp + 1);
-        addMonopole(qb.y, qa.x - xi, qa.y - yi, qb.x - zi, soft2, ax, ay, az, phi);
-        until = skip;
-      } else if (leaf) {
-        for (int j = start; j < start + count; ++j) {
+      dev::f32x2 dxy;
+      float dz, hi, lo;
+      const float r2 = separation(q, me, dxy, dz);
+      dev::unpack2(q.zt.y, hi, lo);
+      bool apply = r2 > hi;
+      if (!apply && !(r2 < lo)) apply = applies64(cells, c, xi, yi, zi, thr, soft2);
+      descend = !apply && q.q.w == 0;
+      if (!descend) until = skip;
+      if (apply) {
+        if (sub == 0) queue[tail % kQueue] = c;
+        ++tail;
+      } else if (q.q.w > 1) {   // nodes that share a deepest cell
+        const double lim = 1.0e-10 * soft2;
+        for (int j = q.q.z + sub; j < q.q.z + q.q.w; j += kWalkLanes) {
           const TreeNode p = loadNode(tpos + j);
           const double ex = __dsub_rn(p.x, xi), ey = __dsub_rn(p.y, yi), ez = __dsub_rn(p.z, zi);
           // s2 / soft2 > 1e-10, the division only near the limit
           const double s2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-          const double lim = 1.0e-10 * soft2;
           bool use = s2 > lim * 1.001;
           if (!use && s2 >= lim * 0.999) use = __ddiv_rn(s2, soft2) > 1.0e-10;
           if (use) addMonopole(p.m, ex, ey, ez, soft2, ax, ay, az, phi);
         }
-        until = skip;
-      } else {
-        descend = true;
       }
     }
-    if (__any_sync(0xffffffffu, descend)) ++c;
-    else c = __reduce_min_sync(0xffffffffu, until);
+    if (__any_sync(0xffffffffu, tail - head == kQueue)) drain(kQueue / 2);
+    // the lanes that passed over c left it by its skip, the others lie beyond
+    c = __any_sync(0xffffffffu, descend) ? c + 1 : skip;
+  }
+  drain(0);
+#pragma unroll
+  for (int o = kWalkLanes / 2; o > 0; o >>= 1) {
+    ax += __shfl_xor_sync(0xffffffffu, ax, o);
+    ay += __shfl_xor_sync(0xffffffffu, ay, o);
+    az += __shfl_xor_sync(0xffffffffu, az, o);
+    phi += __shfl_xor_sync(0xffffffffu, phi, o);
   }
   // Outputs: a, phi times G; dt vote sqrt(softening / |a|) before G.
   double vote = DBL_MAX, e = 0.0;
-  if (valid) {
+  if (valid && sub == 0) {
     const int i = vals[k];
     F.f[F_GRAV_X][i] = G * ax;
     F.f[F_GRAV_Y][i] = G * ay;
@@ -483,49 +613,49 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restri
   }
 }
 
-__global__ void cells32Kernel(const TreeCell* __restrict__ cells, long long numCells,
-                              const double* __restrict__ thrLevel, TreeCell32* __restrict__ c32) {
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= numCells) return;
-  const TreeCell cl = cells[c];
-  TreeCell32 o;
-  splitDF(cl.x, o.xh, o.xl);
-  splitDF(cl.y, o.yh, o.yl);
-  splitDF(cl.z, o.zh, o.zl);
-  o.M = (float)cl.M;
-  o.open2 = (float)__dadd_rn(thrLevel[cl.lvl & 255], cl.r2cc);
-  o.skip = cl.skip;
-  o.start = cl.start;
-  o.count = cl.count;
-  o.lvl = cl.lvl;
-  c32[c] = o;
-}
-
-__device__ __forceinline__ void kahan(float& s, float& c, float x) {
-  const float y = __fsub_rn(x, c);
-  const float t = __fadd_rn(s, y);
-  c = __fsub_rn(__fsub_rn(t, s), y);
+// Compensated (Kahan) FP32 sums of (a_x, a_y) and (a_z, phi): the sum and the
+// negated compensation, y = x + nc, t = s + y, nc = y - (t - s).
+struct Acc32 {
+  dev::f32x2 xy, zp, nxy, nzp;
+};
+__device__ __forceinline__ void kahan2(dev::f32x2& s, dev::f32x2& nc, dev::f32x2 x) {
+  const dev::f32x2 kMinus = 0xBF800000BF800000ull;   // (-1, -1)
+  const dev::f32x2 y = dev::add2(x, nc), t = dev::add2(s, y);
+  nc = dev::add2(y, dev::fma2(t, kMinus, s));
   s = t;
 }
-
-// FP32 monopole term on a double-float separation: a += M/(r^2+eps^2) rhat,
-// phi -= M/sqrt(r^2+eps^2), compensated sums.
-struct Acc32 {
-  float sx, sy, sz, sp, cx, cy, cz, cp;
-};
-
-__device__ __forceinline__ void addMonopole32(float M, float dx, float dy, float dz, float r2, float soft2,
-                                              Acc32& a) {
+// 1 / sqrt of a normal number.
+__device__ __forceinline__ float rsqrtNormal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// Monopole term: a += M/(r^2+eps^2) rhat, phi -= M/sqrt(r^2+eps^2); r2 > 1e-30.
+__device__ __forceinline__ void addMonopole32(float M, dev::f32x2 dxy, float dz, float r2, float soft2, Acc32& a) {
+  const float irs = rsqrtNormal(r2 + soft2);
+  const float m = M * irs;
+  const float f = (m * irs) * rsqrtNormal(r2);
+  kahan2(a.xy, a.nxy, dev::mul2(dxy, dev::pack2(f, f)));
+  kahan2(a.zp, a.nzp, dev::pack2(f * dz, -m));
+}
+// The same for any r2: the unit vector of a zero separation is (1, 0, 0).
+__device__ __forceinline__ void addMonopole32Any(float M, dev::f32x2 dxy, float dz, float r2, float soft2, Acc32& a) {
+  float dx, dy;
+  dev::unpack2(dxy, dx, dy);
   const float irs = rsqrtf(r2 + soft2);
   const float m = M * irs, f0 = m * irs;
   const bool apart = r2 > 1.0e-30f;
   const float f = apart ? f0 * rsqrtf(r2) : f0;
-  kahan(a.sx, a.cx, f * (apart ? dx : 1.0f));   // the unit vector of a zero separation is (1, 0, 0)
-  kahan(a.sy, a.cy, f * dy);
-  kahan(a.sz, a.cz, f * dz);
-  kahan(a.sp, a.cp, -m);
+  kahan2(a.xy, a.nxy, dev::pack2(f * (apart ? dx : 1.0f), f * dy));
+  kahan2(a.zp, a.nzp, dev::pack2(f * dz, -m));
 }
 
+// Mixed walk: 32 nodes in step.  Bound by issue slots (~1900 visits per warp at
+// 150,001 nodes) and the latency of the next cell: the thresholds, the one-node
+// leaves and the next cell's index come with the cell, the separations and
+// compensated sums are packed pairs; ~50 instructions per visit.  150,001 nodes:
+// 893 us.  Loading both cells that may come next ahead of the decision took 89
+// registers and 1173 us.
 __global__ void __launch_bounds__(128) treeWalkMixedKernel(
     const TreeCell32* __restrict__ c32, const TreeCell* __restrict__ cells, long long numCells,
     const TreeNode32* __restrict__ t32, const TreeNode* __restrict__ tpos, const int* __restrict__ vals, long n,
@@ -538,65 +668,73 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
   __syncthreads();
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const bool valid = k < n;
-  TreeNode32 me{0, 0, 0, 0, 0, 0, 0, 0};
   double xd = 0, yd = 0, zd = 0, mi = 0;
   if (valid) {
-    me = t32[k];
     const TreeNode p = tpos[k];
     xd = p.x; yd = p.y; zd = p.z; mi = p.m;
   }
+  const WalkNode me = walkNode(xd, yd, zd);
   const float soft2 = (float)soft2d;
-  Acc32 acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  Acc32 acc{0ull, 0ull, 0ull, 0ull};
   unsigned until = valid ? 0u : 0xFFFFFFFFu;
   unsigned c = 1;
   const unsigned nc = (unsigned)numCells;
   if (__all_sync(0xffffffffu, !valid)) c = nc;
   while (c < nc) {
-    const float4* cp = reinterpret_cast<const float4*>(c32 + c);
-    const WalkCell q{__ldg(cp), __ldg(cp + 1)};
-    const int4 qi = __ldg(reinterpret_cast<const int4*>(cp + 2));
-    const unsigned skip = (unsigned)qi.x;
-    const int start = qi.y, count = qi.z, level = qi.w & 255, leaf = qi.w >> 8;
+    const WalkCell q = loadCell(c32, c);
+    const unsigned skip = (unsigned)q.q.y;
     bool descend = false;
     if (c >= until) {
-      float dx, dy, dz, r2;
-      bool unsure;
-      bool far = farCell(q, me.xh, me.yh, me.zh, me.xl, me.yl, me.zl, dx, dy, dz, r2, unsure);
-      if (unsure) far = farCell64(cells[c], xd, yd, zd, thr[level]);
-      if (far) {
-        addMonopole32(q.a.w, dx, dy, dz, r2, soft2, acc);
+      const float M = __int_as_float(q.q.x);
+      dev::f32x2 dxy;
+      float dz, hi, lo;
+      const float r2 = separation(q, me, dxy, dz);
+      dev::unpack2(q.zt.y, hi, lo);
+      if (r2 > hi) {
+        addMonopole32(M, dxy, dz, r2, soft2, acc);
         until = skip;
-      } else if (leaf) {
-        for (int j = start; j < start + count; ++j) {
-          const TreeNode32 p = t32[j];
-          const float ex = __fadd_rn(__fsub_rn(p.xh, me.xh), __fsub_rn(p.xl, me.xl));
-          const float ey = __fadd_rn(__fsub_rn(p.yh, me.yh), __fsub_rn(p.yl, me.yl));
-          const float ez = __fadd_rn(__fsub_rn(p.zh, me.zh), __fsub_rn(p.zl, me.zl));
-          const float q2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
-          const float lim = 1.0e-10f * soft2;
-          bool use;
-          if (q2 > lim * 1.001f) use = true;
-          else if (q2 < lim * 0.999f) use = false;
-          else {   // the reference's r2 / soft2 > 1e-10 in FP64
-            const TreeNode pd = tpos[j];
-            const double fx = __dsub_rn(pd.x, xd), fy = __dsub_rn(pd.y, yd), fz = __dsub_rn(pd.z, zd);
-            const double w2 = __dadd_rn(__dadd_rn(__dmul_rn(fx, fx), __dmul_rn(fy, fy)), __dmul_rn(fz, fz));
-            use = __ddiv_rn(w2, soft2d) > 1.0e-10;
-          }
-          if (use) addMonopole32(p.m, ex, ey, ez, q2, soft2, acc);
-        }
+      } else if (!(r2 < lo) && applies64(cells, c, xd, yd, zd, thr, soft2d)) {
+        addMonopole32Any(M, dxy, dz, r2, soft2, acc);
         until = skip;
       } else {
-        descend = true;
+        descend = q.q.w == 0;
+        if (!descend) until = skip;
+        if (q.q.w > 1) {   // nodes that share a deepest cell
+          const float lim = 1.0e-10f * soft2;
+          for (int j = q.q.z; j < q.q.z + q.q.w; ++j) {
+            const TreeNode32 p = t32[j];
+            WalkCell w;
+            w.xy = make_ulonglong2(dev::pack2(p.xh, p.yh), dev::pack2(p.xl, p.yl));
+            w.zt.x = dev::pack2(p.zh, p.zl);
+            dev::f32x2 exy;
+            float ez;
+            const float q2 = separation(w, me, exy, ez);
+            bool use;
+            if (q2 > lim * 1.001f) use = true;
+            else if (q2 < lim * 0.999f) use = false;
+            else {   // the reference's r2 / soft2 > 1e-10 in FP64
+              const TreeNode pd = tpos[j];
+              const double fx = __dsub_rn(pd.x, xd), fy = __dsub_rn(pd.y, yd), fz = __dsub_rn(pd.z, zd);
+              const double w2 = __dadd_rn(__dadd_rn(__dmul_rn(fx, fx), __dmul_rn(fy, fy)), __dmul_rn(fz, fz));
+              use = __ddiv_rn(w2, soft2d) > 1.0e-10;
+            }
+            if (use) addMonopole32Any(p.m, exy, ez, q2, soft2, acc);
+          }
+        }
       }
     }
-    if (__any_sync(0xffffffffu, descend)) ++c;
-    else c = __reduce_min_sync(0xffffffffu, until);
+    // the lanes that passed over c left it by its skip, the others lie beyond
+    c = __any_sync(0xffffffffu, descend) ? c + 1 : skip;
   }
   double vote = DBL_MAX, e = 0.0;
   if (valid) {
-    const double ax = (double)acc.sx - (double)acc.cx, ay = (double)acc.sy - (double)acc.cy;
-    const double az = (double)acc.sz - (double)acc.cz, phi = (double)acc.sp - (double)acc.cp;
+    float sx, sy, sz, sp, cx, cy, cz, cp;
+    dev::unpack2(acc.xy, sx, sy);
+    dev::unpack2(acc.zp, sz, sp);
+    dev::unpack2(acc.nxy, cx, cy);
+    dev::unpack2(acc.nzp, cz, cp);
+    const double ax = (double)sx + (double)cx, ay = (double)sy + (double)cy;
+    const double az = (double)sz + (double)cz, phi = (double)sp + (double)cp;
     const int i = vals[k];
     F.f[F_GRAV_X][i] = G * ax;
     F.f[F_GRAV_Y][i] = G * ay;
@@ -653,7 +791,7 @@ __global__ void zeroGravityKernel(Fields F, long n, double G, double* __restrict
 
 struct GravityWork {
   GBuf part, box, thr, dtBits, key64, timeout, vals, vals2, sortWs, skey, tpos, nc, off, scanWs, total, cells, mx,
-      energy, tpos32, cells32;
+      energy, tpos32, cells32, parent, pending;
   long long* hTotal = nullptr;
   long long lastCells = 0;
 };
@@ -668,7 +806,7 @@ void gravityDestroy(GravityWork* w) {
   if (!w) return;
   GBuf* all[] = {&w->part, &w->box, &w->thr, &w->dtBits, &w->key64, &w->timeout, &w->vals, &w->vals2,
                  &w->sortWs, &w->skey, &w->tpos, &w->nc, &w->off, &w->scanWs, &w->total, &w->cells, &w->mx,
-                 &w->energy, &w->tpos32, &w->cells32};
+                 &w->energy, &w->tpos32, &w->cells32, &w->parent, &w->pending};
   for (GBuf* b : all) b->release();
   if (w->hTotal) cudaFreeHost(w->hTotal);
   delete w;
@@ -715,11 +853,11 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   GCHK(w->off.ensure((n + 1) * sizeof(long long)));
   GCHK(w->scanWs.ensure(scanWorkspaceBytes(n)));
   GCHK(w->total.ensure(sizeof(long long)));
-  const int nbWalk = blocksFor(n, 128);
+  const int nbWalk = blocksFor(mixed ? n : kWalkLanes * n, 128);
   GCHK(w->energy.ensure(nbWalk * sizeof(double)));
 
   boxPartialKernel<<<nbBox, kThreads, 0, s>>>(F, n, w->part.as<double>());
-  boxFinalKernel<<<1, 32, 0, s>>>(w->part.as<double>(), nbBox, opening, w->box.as<double>(), w->thr.as<double>(),
+  boxFinalKernel<<<1, 192, 0, s>>>(w->part.as<double>(), nbBox, opening, w->box.as<double>(), w->thr.as<double>(),
                                  w->dtBits.as<unsigned long long>());
   treeKeyKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, n, w->box.as<double>(), w->key64.as<uint64_t>(),
                                                            w->vals.as<int>());
@@ -749,19 +887,22 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   }
   w->lastCells = numCells;
   GCHK(w->cells.ensure(numCells * sizeof(TreeCell)));
-  GCHK(w->mx.ensure(numCells * 3 * sizeof(double)));
+  GCHK(w->mx.ensure(numCells * sizeof(Sums4)));
   TreeCell* cells = w->cells.as<TreeCell>();
   cellBuildKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(skey, n, w->off.as<long long>(),
                                                              numCells, cells);
   lc->add(1);
   const int nbCells = (int)((numCells + kThreads - 1) / kThreads);
-  for (int l = kMaxLevel; l >= 0; --l) {
-    momentKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, l, w->tpos.as<TreeNode>(), skey,
-                                              w->box.as<double>(), w->mx.as<double>());
-  }
-  lc->add(kMaxLevel + 1);
   GCHK(w->cells32.ensure(numCells * sizeof(TreeCell32)));
-  cells32Kernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->thr.as<double>(), w->cells32.as<TreeCell32>());
+  GCHK(w->parent.ensure(numCells * sizeof(int)));
+  GCHK(w->pending.ensure(numCells * sizeof(int)));
+  linkKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->parent.as<int>(), w->pending.as<int>());
+  momentKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->tpos.as<TreeNode>(), w->parent.as<int>(),
+                                            w->pending.as<int>(), w->mx.as<Sums4>());
+  cellFinalKernel<<<nbCells, kThreads, 0, s>>>(cells, numCells, w->tpos.as<TreeNode>(), skey, w->box.as<double>(),
+                                               w->thr.as<double>(), softening * softening, w->mx.as<Sums4>(),
+                                               w->cells32.as<TreeCell32>());
+  lc->add(3);
   if (mixed)
     treeWalkMixedKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells,
                                                w->tpos32.as<TreeNode32>(), w->tpos.as<TreeNode>(), vals, n,
@@ -771,7 +912,6 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
     treeWalkKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells, w->tpos.as<TreeNode>(), vals,
                                           n, w->thr.as<double>(), softening * softening, softening, G, F,
                                           w->dtBits.as<unsigned long long>(), w->energy.as<double>());
-  lc->add(1);
   walkFinalKernel<<<1, 256, 0, s>>>(w->energy.as<double>(), nbWalk, w->dtBits.as<unsigned long long>(), G, dOut);
   lc->add(2);
   GCHK(cudaGetLastError());

@@ -12,6 +12,7 @@
 // entry carries a 6-bit image code and the neighbour's coordinates are mapped
 // with the reference's own plane formula (imageCoord).
 #include "device.cuh"
+#include "packed32.cuh"
 #include <algorithm>
 #include <climits>
 
@@ -534,31 +535,6 @@ __global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, 
 // ~9 for the test and ~3 for the writing.
 //------------------------------------------------------------------------------
 constexpr int kTile = 32;   // batches listed at a time
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // min(a, |b|, |c|) for a >= 0
 __device__ __forceinline__ float minAbs3(float a, float b, float c) {
   float r;

@@ -117,3 +117,24 @@ def test_elongated_grids(native_lib, oracle_mod, shape):
     orc.evaluate_derivatives()
     bad = compare_fields(eng, orc, ["DvDt", "DepsDt", "DvDx"], 1e-12)
     assert not bad, bad
+
+
+@pytest.mark.parametrize("n", [2, 3, 7, 8, 9, 31, 33, 127, 1025])
+@pytest.mark.parametrize("softening", [1e-15, 0.01, 30.0])
+def test_gravity_forms(native_lib, oracle_mod, n, softening):
+    """Eight nodes per warp (FP64) and 32 (mixed); softenings whose separation
+    limit, 1e-5 of them, excludes no node, none but the node itself, and many.
+    The bounds are the FP64 and mixed walks' of the gravity parity tests."""
+    from spheral_gb300.engine import Engine
+    p = problems.evrard(n=n, seed=n, softening=softening)
+    p.pos[n // 2] = p.pos[0] + 1e-5   # close to and, at 30, inside the limit
+    orc = oracle_mod.Oracle(p)
+    orc.initialize()
+    orc.evaluate_derivatives()
+    orc.gravity()
+    for precision, tol in (("fp64", 1e-12), ("fp32", 2e-6)):
+        eng = Engine.from_problem(p, precision=precision)
+        eng.initialize()
+        eng.evaluate_derivatives()
+        bad = compare_fields(eng, orc, ["DvDtGravity", "potential"], tol)
+        assert not bad, (precision, bad)
