@@ -180,16 +180,12 @@ struct sphgpu_ctx {
   long energyTunedN = 0;
   bool energyPinned = false; // batch depth set by the caller
   DBuf itemBox, chunkOf;     // bounding boxes of the search's work chunks, chunk of each chunk's first node
-  int tunedWidth = 0;        // autotuned group width (0: not tuned yet)
-  int pinnedWidth = 0;       // group width set by the caller (0: autotuned)
+  int pinnedWidth = 0;       // items' width set by the caller (0: 32)
   // The autotuners time their options at the first use for a problem size
   // and once more kRetuneAfter uses later, when the state has moved away
-  // from its initial conditions (ASPH H fields, for one, relax in the first
-  // steps and change which search width is fastest).
-  long listBuilds = 0, widthRetuneAt = -1;
+  // from its initial conditions.
   long pairEvals = 0, pairRetuneAt = -1;
   long energyEvals = 0, energyRetuneAt = -1;
-  long widthTunedN = 0;      // node count it was tuned at
   bool capCheckPending = false;
   double cachedBounds[kBoundsVals] = {};   // min h^-1, min x y z, max x y z, tensor extents of the current state
   bool boundsValid = false;      // cachedBounds describe the current state
@@ -590,32 +586,22 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   c->check();
   c->counts.ensure(n * sizeof(int));
   // work items: first node of every chunk of up to `width` nodes of a cell.
-  // The first guess of the group width follows the mean occupancy of the
-  // cells so that few lanes of a group idle; the autotuner below then times
-  // the widths once per problem size.
-  const double cellsTotal = (double)g.nc[0] * g.nc[1] * g.nc[2];
-  const double occupancy = (double)n / cellsTotal;
-  // The isotropic search runs 32 lanes per item at any width, so 32 it is.
-  const int guess = (!c->hp.asph || occupancy >= 24.0) ? 32 : (occupancy >= 12.0 ? 16 : 8);
-  ++c->listBuilds;
-  const bool retuneWidth = c->widthRetuneAt >= 0 && c->listBuilds >= c->widthRetuneAt;
-  if (!c->hp.asph) c->tunedWidth = guess, c->widthTunedN = n;
-  const bool tuned = c->pinnedWidth > 0 || !c->hp.asph ||
-                     (!retuneWidth && c->tunedWidth > 0 && std::labs(n - c->widthTunedN) <= c->widthTunedN / 8);
+  // The search runs 32 lanes per item at any width, so 32 unless the caller
+  // has set another.
   c->items.ensure(n * sizeof(int));
-  c->itemBox.ensure(2 * (size_t)n * sizeof(float4));
+  c->itemBox.ensure((c->hp.asph ? 3 : 2) * (size_t)n * sizeof(float4));
   c->chunkOf.ensure(n * sizeof(int));
-  auto makeItems = [&](int width, bool fresh) {
-    c->itemWidth = width;
-    // every non-empty cell adds at most one partial chunk
-    c->itemBound = (int)std::min<double>((double)n, (double)(n / width) + cellsTotal);
-    if (!fresh) CUDA_OK(cudaMemsetAsync(&c->step()->items, 0, sizeof(int), c->stream));
+  c->itemWidth = c->pinnedWidth > 0 ? c->pinnedWidth : 32;
+  // every non-empty cell adds at most one partial chunk
+  const double cellsTotal = (double)g.nc[0] * g.nc[1] * g.nc[2];
+  c->itemBound = (int)std::min<double>((double)n, (double)(n / c->itemWidth) + cellsTotal);
+  {
     Scope sc(c->prof, "neighbor_items");
-    launchItems(k, n, g.subShift, (uint32_t)space, c->cellEnd(), width, c->itemBound, c->f32(), c->items.as<int>(),
-                c->chunkOf.as<int>(), c->itemBox.as<float4>(), c->step(), c->stream, &c->lc);
+    launchItems(k, n, g.subShift, (uint32_t)space, c->cellEnd(), c->itemWidth, c->itemBound, g, c->hp.asph != 0,
+                c->f32(), c->items.as<int>(), c->chunkOf.as<int>(), c->itemBox.as<float4>(), c->step(), c->stream,
+                &c->lc);
     c->check();
-  };
-  makeItems(c->pinnedWidth > 0 ? c->pinnedWidth : (tuned ? c->tunedWidth : guess), true);
+  }
   if (c->nbCapNext > 0) {   // adopt a smaller capacity decided at the previous build
     c->nbCap = c->nbCapNext;
     c->nbCapNext = 0;
@@ -625,36 +611,6 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
     Scope sc(c->prof, "neighbor_count");
     searchLists(c, false);
     c->nbCap = capFor(readMaxCount(c));
-    fresh = false;
-  }
-  if (!tuned) {
-    // Autotuner: the lists do not depend on the group width (the candidate
-    // order is the cell order in every width), so each width writes them
-    // once, timed, and the fastest is kept for this problem size.
-    cudaEvent_t e0, e1;
-    CUDA_OK(cudaEventCreate(&e0));
-    CUDA_OK(cudaEventCreate(&e1));
-    // two rounds, best time per width: the first launches after a new
-    // build run on cold caches
-    float best = 1e30f;
-    int bestW = guess;
-    for (int round = 0; round < 2; ++round)
-      for (const int w : {8, 16, 32}) {
-        if (w != c->itemWidth) makeItems(w, false);
-        CUDA_OK(cudaEventRecord(e0, c->stream));
-        writeLists(c, false);
-        CUDA_OK(cudaEventRecord(e1, c->stream));
-        CUDA_OK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CUDA_OK(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) { best = ms; bestW = w; }
-      }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    c->tunedWidth = bestW;
-    c->widthTunedN = n;
-    c->widthRetuneAt = retuneWidth ? -1 : c->listBuilds + kRetuneAfter;
-    if (bestW != c->itemWidth) makeItems(bestW, false);
     fresh = false;
   }
   writeLists(c, fresh);
@@ -1678,7 +1634,6 @@ int sphgpu_set_neighbor_width(sphgpu_handle c, int width) {
   API_BEGIN(c)
   if (width != 0 && width != 8 && width != 16 && width != 32) throw Error(SPHGPU_E_ARG, "group width not 0, 8, 16 or 32");
   c->pinnedWidth = width;
-  if (width == 0) c->tunedWidth = 0;   // time the widths again at the next build
   API_END(c)
 }
 

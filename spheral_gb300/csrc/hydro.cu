@@ -129,16 +129,11 @@ __global__ void permuteKernel(Fields Fin, Fields Fout, const int* __restrict__ p
 // threshold; candidates inside the band get the exact FP64 test with the
 // reference's operation order, so the neighbour sets are exact.
 //
-// The search is group-cooperative.  A group of W lanes (W = 8, 16 or 32,
-// chosen from the mean cell occupancy so few lanes idle) owns a chunk of up
-// to W consecutive nodes of one cell (an "item"), so the 27 candidate cells,
-// their offset codes and mirror flags are uniform across the group.  Each
-// candidate cell is read in coalesced batches of W nodes staged in shared
-// memory; every lane tests its own node against the batch.  Candidate cells
-// are visited in a fixed order (dz, dy, dx from -1 to 1) and nodes within a
-// cell in sorted order, so every list has a reproducible order.
+// Candidate cells are visited in a fixed order (dz, dy, dx from -1 to 1) and
+// nodes within a cell in sorted order, so every list has a reproducible order.
 // WRITE false: count only; true: count and write the warp-interleaved lists
 // (slots beyond cap are counted, not written).
+
 // Relative half-width of the FP32 band around |H r|^2 = ext^2 for a node with
 // eigenvalues in [lmin, lmax].  Each FP32 separation component carries at
 // most ~10 u C of rounding (C the largest cell edge, u = 2^-24), and the
@@ -162,377 +157,42 @@ __device__ __noinline__ bool exactTensorCriterion(const Fields& F, const Grid& g
   return eta2ExactSym(loadSym(F, F_HT_XX, i), qx, qy, qz) <= ext2 || eta2ExactSym(Hj, qx, qy, qz) <= ext2;
 }
 
-// TENSOR (ASPH): h^-1 in the FP32 mirror is the smallest eigenvalue of H, so
-// the scalar pre-filter bounds |H r| from below and rejects the far
-// candidates; the rest take |H_i r|^2 and |H_j r|^2 in FP32 from the tensor
-// mirror with a per-node band (tensorBand), and only those inside a band
-// take the exact FP64 tensor test.
-//
-// Batch culling: every chunk of up to W consecutive nodes of a cell has a
-// bounding box (itemBoxKernel); a candidate batch whose box is farther from
-// the group's own box than the largest FP32 band edge of the group allows,
-// at the smaller of the two boxes' smallest h^-1, holds no neighbour of any
-// of the group's nodes and is skipped whole (a group-uniform decision).
-// With the sub-cell key order the chunks are compact, so the boxes are
-// small and the far batches of the 27 cells drop out.
-template <bool WRITE, int W, bool TENSOR>
-__global__ void __launch_bounds__(128) neighborWarpKernel(Fields F, Fields32 P, long n, const int* __restrict__ items,
-                                                          int nItems, Grid g, const int* __restrict__ cellStart,
-                                                          const int* __restrict__ cellEnd, int* __restrict__ counts,
-                                                          uint32_t* __restrict__ nbr, double ext2, float bandA,
-                                                          float bandB, int cap, StepScratch* __restrict__ sc,
-                                                          const float4* __restrict__ box,
-                                                          const int* __restrict__ chunkOf) {
-  constexpr int G = 128 / W;             // groups per 128-thread block
-  __shared__ float4 stage[G][W];         // one candidate batch per group
-  constexpr int HW = TENSOR ? 2 * W : 1;
-  __shared__ float4 stageH[G][HW];       // TENSOR: the batch's H (xx xy xz yy | yz zz band .)
-  __shared__ int4 cinfo[G][27];          // the 27 candidate cells: node range, first work chunk, cell-offset code
-  __shared__ float4 coff[G][27];         // the cell offset (ox, oy, oz) of each
-  // Isotropic H: each batch's culling box is loaded a batch ahead (in lanes
-  // 0 and 1) and passed through shared memory; the tensor path, heavier in
-  // registers already, loads it when its batch comes up.
-  constexpr bool BOXAHEAD = !TENSOR;
-  __shared__ float4 sbox[G][2];          // the current batch's box (lo, hi)
-  const int item = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) / W);
-  const int lane = threadIdx.x % W, wib = threadIdx.x / W;
-  // lanes of this group within the warp
-  const unsigned gmask = (W == 32) ? 0xffffffffu : (((1u << W) - 1u) << ((threadIdx.x & 31) / W * W));
-  // the grid is sized for an upper bound; the item count itself is on the device
-  if (item >= min(nItems, sc->items)) return;   // group-uniform
-  const int k0 = items[item];
-  const uint32_t cc = P.cell[k0];
-  int hc[3];
-  unpackCell(cc, hc);
-  // The 27 cell ranges are independent loads: fetch them lane-parallel so
-  // their latencies overlap, with each cell's first work chunk (its batches'
-  // boxes follow consecutively) and its offset code and offset.  Cell t is
-  // (dx, dy, dz) = (t%3, t/3%3, t/9) - 1.
-  for (int t = lane; t < 27; t += W) {
-    const int d[3] = {t % 3 - 1, (t / 3) % 3 - 1, t / 9 - 1};
-    int cell[3];
-    bool ok = true;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      int nn = hc[a] + d[a];
-      if (nn < 0) {
-        if (g.kindLo[a] == AXIS_PERIODIC) nn = g.nc[a] - 1;
-        else if (g.kindLo[a] == AXIS_REFLECT) nn = 0;
-        else ok = false;
-      } else if (nn >= g.nc[a]) {
-        if (g.kindHi[a] == AXIS_PERIODIC) nn = 0;
-        else if (g.kindHi[a] == AXIS_REFLECT) nn = g.nc[a] - 1;
-        else ok = false;
-      }
-      cell[a] = nn;
-    }
-    const int d0 = t % 3, d1 = (t / 3) % 3, d2 = t / 9;   // 0, 1, 2 for -1, 0, +1
-    const int dcode = (d0 == 0 ? 1 : (d0 == 2 ? 2 : 0)) | ((d1 == 0 ? 1 : (d1 == 2 ? 2 : 0)) << 2) |
-                      ((d2 == 0 ? 1 : (d2 == 2 ? 2 : 0)) << 4);
-    int4 r = make_int4(0, 0, 0, dcode);
-    if (ok) {
-      const uint32_t key = cellKey(g, (uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2], 0);
-      r.x = cellStart[key];
-      r.y = cellEnd[key];
-      if (r.x < r.y) r.z = chunkOf[r.x];
-    }
-    cinfo[wib][t] = r;
-    coff[wib][t] = make_float4(d0 == 0 ? g.cellf[0] : (d0 == 2 ? -g.cellf[0] : 0.0f),
-                               d1 == 0 ? g.cellf[1] : (d1 == 2 ? -g.cellf[1] : 0.0f),
-                               d2 == 0 ? g.cellf[2] : (d2 == 2 ? -g.cellf[2] : 0.0f), 0.0f);
-  }
-  __syncwarp(gmask);
-  const int k1 = min(k0 + W, cinfo[wib][13].y);   // cell 13 is the home cell
-  const long i = k0 + lane;
-  const bool active = i < k1;
-  const float4 pi = active ? P.posh[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float ai2 = pi.w * pi.w;
-  const float del = __fmaf_rn(bandA, pi.w, bandB);   // per-node band half-width (relative)
-  const float e2t = g.ext2f;
-  const float bandLo = del < 0.5f ? e2t * (1.0f - del) : -1.0f;
-  const float bandHi = del < 0.5f ? e2t * (1.0f + del) : FLT_MAX;
-  const uint32_t mm = mirrorMask(g, hc);
-  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  float4 hi0 = make_float4(0.f, 0.f, 0.f, 0.f), hi1 = hi0;
-  float tLo = 0.f, tHi = 0.f;
-  if (TENSOR && active) {
-    hi0 = P.hten[2 * i];
-    hi1 = P.hten[2 * i + 1];
-    const float dI = tensorBand(hi1.w, pi.w, g);
-    tLo = dI < 0.5f ? e2t * (1.0f - dI) : -1.0f;
-    tHi = dI < 0.5f ? e2t * (1.0f + dI) : FLT_MAX;
-  }
-  int cnt = 0;
-  // the group's box and the culling threshold on gap^2 min(a)^2: the largest
-  // band edge of the group's nodes, widened against FP32 rounding; no
-  // culling where a band is wide open
-  const float4 gLo = box[2 * item], gHi = box[2 * item + 1];
-  const float delMax = __fmaf_rn(bandA, gHi.w, bandB);
-  const bool cull = delMax < 0.5f;
-  const float cullThr = e2t * (1.0f + delMax) * 1.0001f;
-  // slot 0 of node i in the warp-interleaved lists; slot q is 32 entries further per q
-  uint32_t* out = WRITE ? nbr + nbSlot(i, 0, cap) : nullptr;
-  // first batch of the first non-empty cell (and its box), loaded ahead of use
-  int tn = 0;
-  while (tn < 27 && cinfo[wib][tn].x >= cinfo[wib][tn].y) ++tn;
-  float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 hn0 = qn, hn1 = qn, nbox = qn;
-  if (tn < 27) {
-    const int4 c0 = cinfo[wib][tn];
-    if (c0.x + lane < c0.y) {
-      qn = P.posh[c0.x + lane];
-      if (TENSOR) { hn0 = P.hten[2 * (c0.x + lane)]; hn1 = P.hten[2 * (c0.x + lane) + 1]; }
-    }
-    if (BOXAHEAD && cull && lane < 2) nbox = box[2 * c0.z + lane];
-  }
-  while (tn < 27) {
-    const int t = tn;
-    const int4 ct = cinfo[wib][t];
-    const int s = ct.x, e = ct.y, dcode = ct.w;
-    const float4 off = coff[wib][t];
-    const uint32_t mir = (uint32_t)dcode & mm;
-    const float ox = off.x, oy = off.y, oz = off.z;
-    // next non-empty cell
-    ++tn;
-    while (tn < 27 && cinfo[wib][tn].x >= cinfo[wib][tn].y) ++tn;
-    for (int base = s, cb = ct.z; base < e; base += W, ++cb) {
-      float4 q = qn;
-      float4 qh0 = hn0, qh1 = hn1;
-      if (BOXAHEAD && cull) {
-        if (lane < 2) sbox[wib][lane] = nbox;
-        __syncwarp(gmask);
-      }
-      // prefetch the next batch's candidates (and box: that of chunk cb + 1,
-      // or of the next cell's first chunk)
-      if (base + W < e) {            // another batch of this cell follows
-        const bool ok = base + W + lane < e;
-        qn = ok ? P.posh[base + W + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (TENSOR && ok) { hn0 = P.hten[2 * (base + W + lane)]; hn1 = P.hten[2 * (base + W + lane) + 1]; }
-        if (BOXAHEAD && cull && lane < 2) nbox = box[2 * (cb + 1) + lane];
-      } else if (tn < 27) {          // last batch: prefetch the next cell's first batch
-        const int4 cn = cinfo[wib][tn];
-        const bool ok = cn.x + lane < cn.y;
-        qn = ok ? P.posh[cn.x + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (TENSOR && ok) { hn0 = P.hten[2 * (cn.x + lane)]; hn1 = P.hten[2 * (cn.x + lane) + 1]; }
-        if (BOXAHEAD && cull && lane < 2) nbox = box[2 * cn.z + lane];
-      }
-      if (cull) {
-        float4 bLo, bHi;
-        if (BOXAHEAD) { bLo = sbox[wib][0]; bHi = sbox[wib][1]; }
-        else { bLo = box[2 * cb]; bHi = box[2 * cb + 1]; }
-        // the batch's box in the frame of the group's cell: a candidate at q
-        // (mirrored where the entry crosses a wall) sits at q - o there
-        float lx = bLo.x, hx = bHi.x, ly = bLo.y, hy = bHi.y, lz = bLo.z, hz = bHi.z;
-        if (mir & 3u) { lx = cx - bHi.x; hx = cx - bLo.x; }
-        if (mir & 12u) { ly = cy - bHi.y; hy = cy - bLo.y; }
-        if (mir & 48u) { lz = cz - bHi.z; hz = cz - bLo.z; }
-        const float gx = fmaxf(0.0f, fmaxf((lx - ox) - gHi.x, gLo.x - (hx - ox)));
-        const float gy = fmaxf(0.0f, fmaxf((ly - oy) - gHi.y, gLo.y - (hy - oy)));
-        const float gz = fmaxf(0.0f, fmaxf((lz - oz) - gHi.z, gLo.z - (hz - oz)));
-        const float am = fminf(gLo.w, bLo.w);
-        if ((am * am) * (gx * gx + gy * gy + gz * gz) > cullThr) continue;   // group-uniform
-      }
-      if (TENSOR) {   // band of node j, then H_j seen through the mirrors
-        qh1.z = tensorBand(qh1.w, q.w, g);
-        const float sx = (mir & 3u) ? -1.f : 1.f, sy = (mir & 12u) ? -1.f : 1.f, sz = (mir & 48u) ? -1.f : 1.f;
-        qh0.y *= sx * sy;   // xy
-        qh0.z *= sx * sz;   // xz
-        qh1.x *= sy * sz;   // yz
-        stageH[wib][2 * lane] = qh0;
-        stageH[wib][2 * lane + 1] = qh1;
-      }
-      if (mir) {
-        if (mir & 3u) q.x = cx - q.x;
-        if (mir & 12u) q.y = cy - q.y;
-        if (mir & 48u) q.z = cz - q.z;
-      }
-      q.w = q.w * q.w;   // (h_j^-1)^2
-      // Stage the batch in shared memory: each lane then reads every
-      // candidate with one broadcast load.
-      stage[wib][lane] = q;
-      __syncwarp(gmask);
-      const int nval = min(W, e - base);
-      // the home cell's own batch contains node i itself
-      const int self = (dcode == 0 && i >= base && i < base + nval) ? (int)(i - base) : -1;
-      if (!TENSOR && active) {
-        // Isotropic H.  The common path takes no branch per candidate: every
-        // candidate up to the top of the band is stored, and the largest
-        // stored e2 tells whether one of them sits inside the band; the
-        // (rare) batches that hold one are written again in candidate order
-        // with the exact FP64 criterion for the band candidates, so a list
-        // is the same for every group width (and so is the rounding of its
-        // sums).  The capacity is
-        // checked once per batch unless the batch could overflow it, and
-        // the self test runs only in the group's own batch of the home cell.
-        const uint32_t ebase = (uint32_t)base | ((uint32_t)dcode << kIndexBits);
-        const float px = __fadd_rn(pi.x, ox), py = __fadd_rn(pi.y, oy), pz = __fadd_rn(pi.z, oz);
-        const bool own = dcode == 0 && base == k0;   // group-uniform: here candidate `lane` is node i
-        const int cnt0 = cnt;
-        bool amb = false;
-        if (!WRITE || cnt + nval <= cap) {
-          uint32_t* o = WRITE ? out + (size_t)cnt * 32 : nullptr;
-          int c = 0;
-          float mx = -1.0f;   // largest e2 stored
-          if (!own) {
-#pragma unroll 4
-            for (int u = 0; u < nval; ++u) {
-              const float4 cq = stage[wib][u];
-              const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-              const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-              if (e2 <= bandHi) {
-                if (WRITE) o[(size_t)c * 32] = ebase + (uint32_t)u;
-                ++c;
-                mx = fmaxf(mx, e2);
-              }
-            }
-          } else {
-#pragma unroll 4
-            for (int u = 0; u < nval; ++u) {
-              const float4 cq = stage[wib][u];
-              const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-              const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-              if ((e2 <= bandHi) & (u != lane)) {
-                if (WRITE) o[(size_t)c * 32] = ebase + (uint32_t)u;
-                ++c;
-                mx = fmaxf(mx, e2);
-              }
-            }
-          }
-          amb = mx >= bandLo;
-          cnt += c;
-        } else {   // this batch may reach the capacity: count past it, store below it
-          for (int u = 0; u < nval; ++u) {
-            const float4 cq = stage[wib][u];
-            const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-            const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-            amb |= (e2 >= bandLo) & (e2 <= bandHi);
-            if ((e2 < bandLo) & (u != self)) {
-              if (WRITE && cnt < cap) out[(size_t)cnt * 32] = ebase + (uint32_t)u;
-              ++cnt;
-            }
-          }
-        }
-        if (amb) {   // guard band: the batch again, band candidates by the exact FP64 criterion
-          cnt = cnt0;
-          for (int u = 0; u < nval; ++u) {
-            const float4 cq = stage[wib][u];
-            const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-            const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-            if (e2 > bandHi || u == self) continue;
-            bool in = e2 < bandLo;
-            if (!in) {
-              const int j = base + u;
-              double xjd = F.f[F_X][j], yjd = F.f[F_Y][j], zjd = F.f[F_Z][j];
-              imagePos(g, imageCode(g, hc, dcode), xjd, yjd, zjd);
-              const double qx = __dsub_rn(F.f[F_X][i], xjd), qy = __dsub_rn(F.f[F_Y][i], yjd),
-                           qz = __dsub_rn(F.f[F_Z][i], zjd);
-              in = eta2Exact(F.f[F_HINV][i], qx, qy, qz) <= ext2 || eta2Exact(F.f[F_HINV][j], qx, qy, qz) <= ext2;
-            }
-            if (in) {
-              if (WRITE && cnt < cap) out[(size_t)cnt * 32] = ebase + (uint32_t)u;
-              ++cnt;
-            }
-          }
-        }
-      }
-      if (TENSOR && active) {
-        // Tensor H: the scalar pre-filter (h^-1 the smallest eigenvalue)
-        // rejects the far candidates, the rest take the FP32 tensor test on
-        // each side with its own band; candidates inside a band only raise a
-        // flag, and flagged batches are written again in candidate order with
-        // the exact FP64 tensor criterion for the flagged candidates.
-        const uint32_t ebase = (uint32_t)base | ((uint32_t)dcode << kIndexBits);
-        // this node shifted by the cell offset: r = (x_i + o) - x_j
-        const float px = __fadd_rn(pi.x, ox), py = __fadd_rn(pi.y, oy), pz = __fadd_rn(pi.z, oz);
-        const int cnt0 = cnt;
-        bool amb = false;
-#pragma unroll 4
-        for (int u = 0; u < nval; ++u) {
-          const float4 cq = stage[wib][u];
-          const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-          const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-          if (e2 <= bandHi) {
-            const float4 h0 = stageH[wib][2 * u], h1 = stageH[wib][2 * u + 1];
-            const float e2i = eta2Sym32(hi0, hi1, rx, ry, rz);
-            const float e2j = eta2Sym32(h0, h1, rx, ry, rz);
-            const float jLo = h1.z < 0.5f ? e2t * (1.0f - h1.z) : -1.0f;
-            const float jHi = h1.z < 0.5f ? e2t * (1.0f + h1.z) : FLT_MAX;
-            const bool in = (e2i <= tLo) | (e2j <= jLo);
-            amb |= !in & !((e2i >= tHi) & (e2j >= jHi));
-            if (in & (u != self)) {
-              if (WRITE && cnt < cap) out[(size_t)cnt * 32] = ebase + (uint32_t)u;
-              ++cnt;
-            }
-          }
-        }
-        if (amb) {   // guard band: the batch again, flagged candidates by the exact FP64 tensor criterion
-          const int code = imageCode(g, hc, dcode);
-          cnt = cnt0;
-          for (int u = 0; u < nval; ++u) {
-            const float4 cq = stage[wib][u];
-            const float rx = __fsub_rn(px, cq.x), ry = __fsub_rn(py, cq.y), rz = __fsub_rn(pz, cq.z);
-            const float e2 = fminf(ai2, cq.w) * (rx * rx + ry * ry + rz * rz);
-            if (e2 > bandHi || u == self) continue;
-            const float4 h0 = stageH[wib][2 * u], h1 = stageH[wib][2 * u + 1];
-            const float e2i = eta2Sym32(hi0, hi1, rx, ry, rz);
-            const float e2j = eta2Sym32(h0, h1, rx, ry, rz);
-            const float jLo = h1.z < 0.5f ? e2t * (1.0f - h1.z) : -1.0f;
-            const float jHi = h1.z < 0.5f ? e2t * (1.0f + h1.z) : FLT_MAX;
-            bool in = (e2i <= tLo) | (e2j <= jLo);
-            if (!in && !((e2i >= tHi) & (e2j >= jHi))) {
-              const int j = base + u;
-              double xjd = F.f[F_X][j], yjd = F.f[F_Y][j], zjd = F.f[F_Z][j];
-              imagePos(g, code, xjd, yjd, zjd);
-              const double qx = __dsub_rn(F.f[F_X][i], xjd), qy = __dsub_rn(F.f[F_Y][i], yjd),
-                           qz = __dsub_rn(F.f[F_Z][i], zjd);
-              in = exactTensorCriterion(F, g, i, j, code, qx, qy, qz, ext2);
-            }
-            if (in) {
-              if (WRITE && cnt < cap) out[(size_t)cnt * 32] = ebase + (uint32_t)u;
-              ++cnt;
-            }
-          }
-        }
-      }
-      __syncwarp(gmask);
-    }
-  }
-  // The stored count never exceeds the capacity: sweeps that run before an
-  // overflow is noticed read only written slots.  The true maximum goes to
-  // maxCount (the overflow signal).
-  if (active) counts[i] = WRITE ? min(cnt, cap) : cnt;
-  // one atomic per group: a per-node atomic on a single address serialises
-  const int gmax = __reduce_max_sync(gmask, active ? cnt : 0);
-  const int gsum = __reduce_add_sync(gmask, active ? cnt : 0);
-  if (lane == 0) {
-    if (gmax > *(volatile int*)&sc->maxCount) atomicMax(&sc->maxCount, gmax);
-    atomicAdd(&sc->entries[blockIdx.x & (kEntrySums - 1)], (unsigned long long)gsum);
-  }
-}
-
 //------------------------------------------------------------------------------
-// Isotropic search.  A warp (CW = 1) or the block's four warps (CW = 4) own one
-// work item: up to 32 consecutive nodes of a cell, one per lane.
+// The search.  A warp (CW = 1) or the block's four warps (CW = 4) own one work
+// item: up to 32 consecutive nodes of a cell, one per lane, so the 27 candidate
+// cells, their offset codes and mirror flags are uniform across it.
 //
 //  1. The chunks of the 27 candidate cells (in cell order, up to kTile at a
 //     time) are listed and culled lane-parallel: a chunk whose bounding box is
 //     farther from the item's box than the item's largest FP32 band edge
 //     allows holds no neighbour of any lane.
-//  2. Each surviving chunk (a batch of up to 32 candidates) is staged and
-//     tested two candidates per packed FP32 operation; the lane's hits up to
-//     the top of its guard band form a 32-bit mask.  A lane whose largest hit
-//     lies inside the band forms the mask of that batch again with the exact
-//     FP64 criterion.  (CW = 4: the warps take the batches in turn.)
-//  3. The masks are written out as list entries, the q-th hit of every lane in
+//  2. The candidates of the surviving chunks, one per lane, are culled against
+//     the item's box in the same way, and the rest are staged densely in the
+//     item's frame (a candidate at q in its cell sits at q - o there).
+//  3. Every 32 staged candidates (a batch) are tested two per packed FP32
+//     operation; the lane's hits up to the top of its guard band form a 32-bit
+//     mask.  A lane whose largest hit lies inside the band forms the mask of
+//     that batch again with the exact FP64 criterion.
+//  4. The masks are written out as list entries, the q-th hit of every lane in
 //     the same iteration, so a row of the warp-interleaved list is one 128-byte
-//     store.  (CW = 4: the warps take a quarter of the batches each.)
+//     store.
+// CW = 4: the warps take a quarter of a tile's chunks each, in order.
 //
 // Every list is in candidate order, whatever the item width and CW.
 //
+// TENSOR (ASPH): h^-1 of the FP32 mirror is the smallest eigenvalue of H, which
+// bounds |H r| from below for the culling, as does a diagonal bound of H^2
+// (itemBoxKernel); the test takes |H_i r|^2 and |H_j r|^2 from the tensor
+// mirror, each with its node's band (tensorBand), and a batch that may hold a
+// candidate inside a band repeats its mask with the exact FP64 tensor criterion
+// for those.
+//
 // What bounds it: instruction issue.  Testing and storing candidate by
-// candidate took ~36 warp instructions per candidate of a group (predicated
-// store, list pointer, counter and band flag per candidate); the masks take
-// ~9 for the test and ~3 for the writing.
+// candidate took ~36 warp instructions per candidate of a group; the masks take
+// ~9 (TENSOR ~20, the FMA pipe, which a packed operation fills for two) for the
+// test and ~3 for the writing, and the culling of single candidates ~1.  With
+// the last, 2.1 M nodes of a Kelvin-Helmholtz slab (cells sized by the light
+// layer's h): 1704 -> 1345 us; 303,912 ASPH nodes: 820 -> 600 us.
 //------------------------------------------------------------------------------
 constexpr int kTile = 32;   // batches listed at a time
 // min(a, |b|, |c|) for a >= 0
@@ -583,21 +243,28 @@ __device__ __forceinline__ CandidateCell candidateCell(int t, const int* hc, con
   return r;
 }
 
-template <bool WRITE, int CW>
-__global__ void __launch_bounds__(128, 6) neighborMaskKernel(Fields F, Fields32 P, const int* __restrict__ items,
+template <bool WRITE, int CW, bool TENSOR>
+__global__ void __launch_bounds__(128, TENSOR ? 4 : 6) neighborMaskKernel(Fields F, Fields32 P, const int* __restrict__ items,
                                                           int nItems, int width, Grid g,
                                                           const int* __restrict__ cellStart,
                                                           const int* __restrict__ cellEnd, int* __restrict__ counts,
                                                           uint32_t* __restrict__ nbr, double ext2, float bandA,
                                                           float bandB, int cap, StepScratch* __restrict__ sc,
                                                           const float4* __restrict__ box,
+                                                          const float4* __restrict__ tbox,
                                                           const int* __restrict__ chunkOf) {
-  constexpr int G = 4 / CW;                          // items per block
-  __shared__ __align__(16) float stage[4][4][32];    // per warp: -x, -y, -z, (h^-1)^2 of a batch
-  __shared__ int2 desc[G][kTile];                    // kept batches: entry of the first node, size
-  __shared__ float4 offs[G][kTile];                  // and the cell offset
-  __shared__ uint32_t masks[G][kTile][32];
-  __shared__ int part[CW == 4 ? 4 : 1][32];          // CW = 4: hits per lane of each warp's batches
+  constexpr int G = 4 / CW;                  // items per block
+  constexpr int UNROLL = TENSOR ? 1 : 8;     // 35 loads per iteration with TENSOR
+  constexpr int NB = CW == 4 ? 8 : 16;       // ring of batches whose masks wait for the writing
+  // per warp, 64 slots: the staged candidates' -x, -y, -z and (h^-1)^2; TENSOR:
+  // H (xx xy xz yy yz zz) as seen through the mirrors, minus the band's top and
+  // its bottom
+  __shared__ __align__(16) float stage[4][TENSOR ? 11 : 4][64];
+  __shared__ uint32_t masks[4][NB][32], ids[4][NB][32];   // hits of each lane; list entries of the slots
+  __shared__ int2 desc[G][kTile];            // kept chunks: entry of the first node, size
+  __shared__ float4 offs[G][kTile];          // and the cell offset
+  __shared__ float4 diag[TENSOR ? G : 1][TENSOR ? kTile : 1];   // and the diagonal bound with the item's
+  __shared__ int part[CW == 4 ? 4 : 1][32];  // CW = 4: hits per lane of each warp's chunks
   __shared__ int keptCount[G];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = CW == 4 ? 0 : warp, sub = CW == 4 ? warp : 0;
@@ -616,21 +283,35 @@ __global__ void __launch_bounds__(128, 6) neighborMaskKernel(Fields F, Fields32 
   const bool active = i < k1;
   const float4 pi = active ? P.posh[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float ai2 = pi.w * pi.w;
-  const float del = __fmaf_rn(bandA, pi.w, bandB);   // per-node band half-width (relative)
   const float e2t = g.ext2f;
-  const float bandLo = del < 0.5f ? e2t * (1.0f - del) : -1.0f;
-  const float bandHi = del < 0.5f ? e2t * (1.0f + del) : FLT_MAX;
-  // a candidate whose e2 is farther than this from bandHi is outside the band
-  // on one side or the other (with room for the rounding of the difference)
-  const float bandGap = del < 0.5f ? 1.01f * (bandHi - bandLo) + 4.0e-7f * bandHi : FLT_MAX;
+  // a band's bottom and top; a candidate whose e2 is farther than the returned
+  // gap from the top is outside the band on one side or the other (with room
+  // for the rounding of the difference)
+  auto bandOf = [&](float d, float& lo, float& hi) {
+    lo = d < 0.5f ? e2t * (1.0f - d) : -1.0f;
+    hi = d < 0.5f ? e2t * (1.0f + d) : FLT_MAX;
+    return d < 0.5f ? 1.01f * (hi - lo) + 4.0e-7f * hi : FLT_MAX;
+  };
+  float bandLo = 0.f, bandHi = 0.f, bandGap = 0.f;
+  f32x2 hxx = 0, hxy = 0, hxz = 0, hyy = 0, hyz = 0, hzz = 0;
+  if (!TENSOR) {
+    bandGap = bandOf(__fmaf_rn(bandA, pi.w, bandB), bandLo, bandHi);
+  } else if (active) {
+    const float4 h0 = P.hten[2 * i], h1 = P.hten[2 * i + 1];
+    bandGap = bandOf(tensorBand(h1.w, pi.w, g), bandLo, bandHi);
+    hxx = pack2(h0.x, h0.x); hxy = pack2(h0.y, h0.y); hxz = pack2(h0.z, h0.z);
+    hyy = pack2(h0.w, h0.w); hyz = pack2(h1.x, h1.x); hzz = pack2(h1.y, h1.y);
+  }
   const f32x2 nhi2 = pack2(-bandHi, -bandHi);
+  const f32x2 px2 = pack2(pi.x, pi.x), py2 = pack2(pi.y, pi.y), pz2 = pack2(pi.z, pi.z);
   const uint32_t mm = mirrorMask(g, hc);
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
   const float4 gLo = box[2 * item], gHi = box[2 * item + 1];
   const float delMax = __fmaf_rn(bandA, gHi.w, bandB);
   const bool cull = delMax < 0.5f;
   const float cullThr = e2t * (1.0f + delMax) * 1.0001f;
-  // batches of each candidate cell, and how many come before them
+  const float4 gT = TENSOR ? tbox[item] : make_float4(0.f, 0.f, 0.f, 0.f);
+  // chunks of each candidate cell, and how many come before them
   const int nb = (cc.end - cc.start + width - 1) / width;
   int before = nb;
 #pragma unroll
@@ -638,71 +319,209 @@ __global__ void __launch_bounds__(128, 6) neighborMaskKernel(Fields F, Fields32 
     const int y = __shfl_up_sync(0xffffffffu, before, o);
     if (lane >= o) before += y;
   }
-  const int batches = __shfl_sync(0xffffffffu, before, 31);
+  const int chunks = __shfl_sync(0xffffffffu, before, 31);
   before -= nb;
 
-  int cnt = 0;   // this lane's hits so far
-  for (int tile = 0; tile < batches; tile += kTile) {
-    const int inTile = min(kTile, batches - tile);
-    if (sub == 0) {
-      // list and cull the tile's batches, one per lane
-      {
-        const int b = tile + lane;
-        // the cell of batch b: the last one that starts at or before it
-        int t = 0;
+  int staged = 0, tested = 0;   // candidates staged, batches tested by this warp
+  int window = 0;               // first batch whose masks are not written yet
+  int selfPos = -1;             // where node i itself was staged
+  uint32_t nonempty = 0u;       // batches from `window` that hold hits of this lane
+  int hits = 0;                 // and their number
+  int cnt = 0;                  // this lane's hits so far
+
+  // Tests the next batch, of nval candidates.
+  auto test = [&](int nval) {
+    __syncwarp();
+    const int half = (tested & 1) * 32, ring = tested % NB;
+    float gap = bandGap;   // the widest band of the batch and this lane
+    if (TENSOR) {
+      const float jHi = -stage[warp][9][half + lane], jLo = stage[warp][10][half + lane];
+      const float jGap = jHi < FLT_MAX ? 1.01f * (jHi - jLo) + 4.0e-7f * jHi : FLT_MAX;
+      // positive floats order as integers
+      gap = fmaxf(gap, __uint_as_float(__reduce_max_sync(0xffffffffu, lane < nval ? __float_as_uint(jGap) : 0u)));
+    }
+    // e2 - top of the band: its sign bits, shifted in one by one, are the mask
+    // (bit order reversed), and its smallest magnitude tells whether a candidate
+    // may lie inside the band
+    uint32_t mask = 0u;
+    float near = FLT_MAX;
+#pragma unroll UNROLL
+    for (int u = 0; u < 32; u += 4) {
+      if (u >= nval) { mask <<= 32 - u; break; }   // uniform
+      auto at = [&](int c) { return *reinterpret_cast<const ulonglong2*>(&stage[warp][c][half + u]); };
+      const ulonglong2 X = at(0), Y = at(1), Z = at(2);
+      const f32x2 rx0 = add2(px2, X.x), ry0 = add2(py2, Y.x), rz0 = add2(pz2, Z.x);
+      const f32x2 rx1 = add2(px2, X.y), ry1 = add2(py2, Y.y), rz1 = add2(pz2, Z.y);
+      float e[4];
+      if (TENSOR) {
+        const ulonglong2 XX = at(3), XY = at(4), XZ = at(5), YY = at(6), YZ = at(7), ZZ = at(8), NH = at(9);
+        auto top = [](f32x2 xx, f32x2 xy, f32x2 xz, f32x2 yy, f32x2 yz, f32x2 zz, f32x2 x, f32x2 y, f32x2 z,
+                      f32x2 nh) {   // |H r|^2 - top
+          const f32x2 ex = fma2(xz, z, fma2(xy, y, mul2(xx, x)));
+          const f32x2 ey = fma2(yz, z, fma2(yy, y, mul2(xy, x)));
+          const f32x2 ez = fma2(zz, z, fma2(yz, y, mul2(xz, x)));
+          return fma2(ez, ez, fma2(ey, ey, fma2(ex, ex, nh)));
+        };
+        float d[4];
+        unpack2(top(hxx, hxy, hxz, hyy, hyz, hzz, rx0, ry0, rz0, nhi2), e[0], e[1]);
+        unpack2(top(XX.x, XY.x, XZ.x, YY.x, YZ.x, ZZ.x, rx0, ry0, rz0, NH.x), d[0], d[1]);
+        unpack2(top(hxx, hxy, hxz, hyy, hyz, hzz, rx1, ry1, rz1, nhi2), e[2], e[3]);
+        unpack2(top(XX.y, XY.y, XZ.y, YY.y, YZ.y, ZZ.y, rx1, ry1, rz1, NH.y), d[2], d[3]);
 #pragma unroll
-        for (int st = 16; st > 0; st >>= 1) {
-          const int c = __shfl_sync(0xffffffffu, before, min(t + st, 26));
-          if (t + st <= 26 && c <= b) t += st;
+        for (int v = 0; v < 4; ++v) {
+          mask = __funnelshift_l(__float_as_uint(e[v]) | __float_as_uint(d[v]), mask, 1);
+          near = minAbs3(near, e[v], d[v]);
         }
-        const int cs = __shfl_sync(0xffffffffu, cc.start, t), ce = __shfl_sync(0xffffffffu, cc.end, t);
-        const int cb = b - __shfl_sync(0xffffffffu, before, t);
-        const int chunk = __shfl_sync(0xffffffffu, cc.chunk, t) + cb;
-        const int dcode = __shfl_sync(0xffffffffu, cc.dcode, t);
-        const float ox = __shfl_sync(0xffffffffu, cc.ox, t), oy = __shfl_sync(0xffffffffu, cc.oy, t);
-        const float oz = __shfl_sync(0xffffffffu, cc.oz, t);
-        bool keep = lane < inTile;
-        if (keep && cull) {
-          // the batch's box in the frame of the item's cell: a candidate at q
-          // (mirrored where the entry crosses a wall) sits at q - o there
-          const float4 bLo = box[2 * chunk], bHi = box[2 * chunk + 1];
-          const uint32_t mir = (uint32_t)dcode & mm;
-          float lx = bLo.x, hx = bHi.x, ly = bLo.y, hy = bHi.y, lz = bLo.z, hz = bHi.z;
-          if (mir & 3u) { lx = cx - bHi.x; hx = cx - bLo.x; }
-          if (mir & 12u) { ly = cy - bHi.y; hy = cy - bLo.y; }
-          if (mir & 48u) { lz = cz - bHi.z; hz = cz - bLo.z; }
-          const float gx = fmaxf(0.0f, fmaxf((lx - ox) - gHi.x, gLo.x - (hx - ox)));
-          const float gy = fmaxf(0.0f, fmaxf((ly - oy) - gHi.y, gLo.y - (hy - oy)));
-          const float gz = fmaxf(0.0f, fmaxf((lz - oz) - gHi.z, gLo.z - (hz - oz)));
-          const float am = fminf(gLo.w, bLo.w);
-          keep = !((am * am) * (gx * gx + gy * gy + gz * gz) > cullThr);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-          const int first = cs + cb * width;
-          const int at = __popc(m & ((1u << lane) - 1u));
-          desc[grp][at] = make_int2(first | (int)((uint32_t)dcode << kIndexBits), min(width, ce - first));
-          offs[grp][at] = make_float4(ox, oy, oz, 0.0f);
-        }
-        if (lane == 0) keptCount[grp] = __popc(m);
+      } else {
+        const float4 A = *reinterpret_cast<const float4*>(&stage[warp][3][half + u]);
+        const f32x2 s0 = fma2(fma2(rz0, rz0, fma2(ry0, ry0, mul2(rx0, rx0))), pack2(fminf(ai2, A.x), fminf(ai2, A.y)), nhi2);
+        const f32x2 s1 = fma2(fma2(rz1, rz1, fma2(ry1, ry1, mul2(rx1, rx1))), pack2(fminf(ai2, A.z), fminf(ai2, A.w)), nhi2);
+        unpack2(s0, e[0], e[1]);
+        unpack2(s1, e[2], e[3]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) mask = __funnelshift_l(__float_as_uint(e[v]), mask, 1);
+        near = minAbs3(minAbs3(near, e[0], e[1]), e[2], e[3]);
       }
+    }
+    mask = __brev(mask);
+    if (nval < 32) mask &= (1u << nval) - 1u;
+    if (active && near <= gap) {   // guard band: this lane's mask again, band candidates by the exact FP64 criterion
+      mask = 0u;
+      for (int u = 0; u < nval; ++u) {
+        const float* st = &stage[warp][0][half + u];
+        const float rx = __fadd_rn(pi.x, st[0]), ry = __fadd_rn(pi.y, st[64]), rz = __fadd_rn(pi.z, st[128]);
+        bool in;
+        if (TENSOR) {
+          auto lo = [](f32x2 v) { return __uint_as_float((unsigned)v); };
+          const float e2i = eta2Sym32(make_float4(lo(hxx), lo(hxy), lo(hxz), lo(hyy)),
+                                      make_float4(lo(hyz), lo(hzz), 0.f, 0.f), rx, ry, rz);
+          const float e2j = eta2Sym32(make_float4(st[192], st[256], st[320], st[384]),
+                                      make_float4(st[448], st[512], 0.f, 0.f), rx, ry, rz);
+          in = (e2i <= bandLo) | (e2j <= st[640]);
+          if (!in && (e2i >= bandHi) & (e2j >= -st[576])) continue;
+        } else {
+          const float e2 = fminf(ai2, st[192]) * (rx * rx + ry * ry + rz * rz);
+          if (e2 > bandHi) continue;
+          in = e2 < bandLo;
+        }
+        if (!in) {
+          const uint32_t ent = ids[warp][ring][u];
+          const int j = (int)(ent & kIndexMask), code = imageCode(g, hc, (int)(ent >> kIndexBits));
+          double xjd = F.f[F_X][j], yjd = F.f[F_Y][j], zjd = F.f[F_Z][j];
+          imagePos(g, code, xjd, yjd, zjd);
+          const double qx = __dsub_rn(F.f[F_X][i], xjd), qy = __dsub_rn(F.f[F_Y][i], yjd),
+                       qz = __dsub_rn(F.f[F_Z][i], zjd);
+          in = TENSOR ? exactTensorCriterion(F, g, i, j, code, qx, qy, qz, ext2)
+                      : eta2Exact(F.f[F_HINV][i], qx, qy, qz) <= ext2 || eta2Exact(F.f[F_HINV][j], qx, qy, qz) <= ext2;
+        }
+        if (in) mask |= 1u << u;
+      }
+    }
+    const int own = selfPos - 32 * tested;
+    if (own >= 0 && own < 32) mask &= ~(1u << own);
+    if (!active) mask = 0u;
+    masks[warp][ring][lane] = mask;
+    if (mask) nonempty |= 1u << (tested - window);
+    hits += __popc(mask);
+    ++tested;
+    __syncwarp();
+  };
+  // Writes the hits of the window's batches from slot `at` of the lane's list.
+  auto writeOut = [&](int at) {
+    if (WRITE) {
+      uint32_t* out = nbr + nbSlot(active ? i : k0, 0, cap) + (size_t)at * 32;
+      const int stored = min(hits, cap - at);
+      const int most = __reduce_max_sync(0xffffffffu, stored);
+      uint32_t m = 0u;
+      int ring = 0;
+      for (int h = 0; h < most; ++h, out += 32)
+        if (h < stored) {
+          if (m == 0u) {
+            const int b = __ffs(nonempty) - 1;
+            nonempty &= nonempty - 1u;
+            ring = (window + b) % NB;
+            m = masks[warp][ring][lane];
+          }
+          *out = ids[warp][ring][__ffs(m) - 1];
+          m &= m - 1u;
+        }
+      __syncwarp();
+    }
+    window = tested;
+    nonempty = 0u;
+    hits = 0;
+  };
+
+  for (int tile = 0; tile < chunks; tile += kTile) {
+    const int inTile = min(kTile, chunks - tile);
+    if (sub == 0) {
+      // list and cull the tile's chunks, one per lane
+      const int b = tile + lane;
+      // the cell of chunk b: the last one that starts at or before it
+      int t = 0;
+#pragma unroll
+      for (int st = 16; st > 0; st >>= 1) {
+        const int c = __shfl_sync(0xffffffffu, before, min(t + st, 26));
+        if (t + st <= 26 && c <= b) t += st;
+      }
+      const int cs = __shfl_sync(0xffffffffu, cc.start, t), ce = __shfl_sync(0xffffffffu, cc.end, t);
+      const int cb = b - __shfl_sync(0xffffffffu, before, t);
+      const int chunk = __shfl_sync(0xffffffffu, cc.chunk, t) + cb;
+      const int dcode = __shfl_sync(0xffffffffu, cc.dcode, t);
+      const float ox = __shfl_sync(0xffffffffu, cc.ox, t), oy = __shfl_sync(0xffffffffu, cc.oy, t);
+      const float oz = __shfl_sync(0xffffffffu, cc.oz, t);
+      bool keep = lane < inTile;
+      float4 bT = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (TENSOR && keep) {
+        // x, y, z: the bound for both; w: the squared extent it is held against
+        bT = tbox[chunk];
+        const float band = fmaxf(gT.w, bT.w);
+        bT = make_float4(fminf(gT.x, bT.x), fminf(gT.y, bT.y), fminf(gT.z, bT.z),
+                         band < 0.5f ? e2t * (1.0f + band) * 1.0001f : FLT_MAX);
+      }
+      if (keep && cull) {
+        // the chunk's box in the item's frame
+        const float4 bLo = box[2 * chunk], bHi = box[2 * chunk + 1];
+        const uint32_t mir = (uint32_t)dcode & mm;
+        float lx = bLo.x, hx = bHi.x, ly = bLo.y, hy = bHi.y, lz = bLo.z, hz = bHi.z;
+        if (mir & 3u) { lx = cx - bHi.x; hx = cx - bLo.x; }
+        if (mir & 12u) { ly = cy - bHi.y; hy = cy - bLo.y; }
+        if (mir & 48u) { lz = cz - bHi.z; hz = cz - bLo.z; }
+        const float gx = fmaxf(0.0f, fmaxf((lx - ox) - gHi.x, gLo.x - (hx - ox)));
+        const float gy = fmaxf(0.0f, fmaxf((ly - oy) - gHi.y, gLo.y - (hy - oy)));
+        const float gz = fmaxf(0.0f, fmaxf((lz - oz) - gHi.z, gLo.z - (hz - oz)));
+        const float am = fminf(gLo.w, bLo.w);
+        keep = !((am * am) * (gx * gx + gy * gy + gz * gz) > cullThr) &&
+               !(TENSOR && bT.x * (gx * gx) + bT.y * (gy * gy) + bT.z * (gz * gz) > bT.w);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int first = cs + cb * width;
+        const int at = __popc(m & ((1u << lane) - 1u));
+        desc[grp][at] = make_int2(first | (int)((uint32_t)dcode << kIndexBits), min(width, ce - first));
+        offs[grp][at] = make_float4(ox, oy, oz, 0.0f);
+        if (TENSOR) diag[grp][at] = bT;
+      }
+      if (lane == 0) keptCount[grp] = __popc(m);
     }
     groupSync();
     const int kept = keptCount[grp];
-    // masks of this warp's batches (candidates of the next one loaded ahead)
-    // nonempty: the kept batches that hold hits of this lane
-    uint32_t nonempty = 0u;
-    int hits = 0;
-    float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (sub < kept && lane < desc[grp][sub].y) qn = P.posh[(desc[grp][sub].x & kIndexMask) + lane];
-    for (int b = sub; b < kept; b += CW) {
+    const int b0 = CW == 4 ? sub * kept / 4 : 0, b1 = CW == 4 ? (sub + 1) * kept / 4 : kept;
+    float4 qn = make_float4(0.f, 0.f, 0.f, 0.f), hn0 = qn, hn1 = qn;
+    auto ahead = [&](int b) {   // candidate `lane` of chunk b
+      const int2 d = desc[grp][b];
+      if (lane >= d.y) return;
+      const int j = (d.x & kIndexMask) + lane;
+      qn = P.posh[j];
+      if (TENSOR) { hn0 = P.hten[2 * j]; hn1 = P.hten[2 * j + 1]; }
+    };
+    if (b0 < b1) ahead(b0);
+    for (int b = b0; b < b1; ++b) {
       const int2 ds = desc[grp][b];
-      const int base = ds.x & kIndexMask, nval = ds.y, dcode = (int)((uint32_t)ds.x >> kIndexBits);
+      const int first = ds.x & kIndexMask, nval = ds.y, dcode = (int)((uint32_t)ds.x >> kIndexBits);
       float4 q = qn;
-      if (b + CW < kept) {
-        const int2 dn = desc[grp][b + CW];
-        if (lane < dn.y) qn = P.posh[(dn.x & kIndexMask) + lane];
-      }
+      const float4 qh0 = hn0, qh1 = hn1;
+      if (b + 1 < b1) ahead(b + 1);
       const uint32_t mir = (uint32_t)dcode & mm;
       if (mir) {
         if (mir & 3u) q.x = cx - q.x;
@@ -710,108 +529,69 @@ __global__ void __launch_bounds__(128, 6) neighborMaskKernel(Fields F, Fields32 
         if (mir & 48u) q.z = cz - q.z;
       }
       const float4 o = offs[grp][b];
-      // empty slots of the batch hold NaN: every comparison with them is false
-      stage[warp][0][lane] = lane < nval ? -q.x : __int_as_float(0x7fffffff);
-      stage[warp][1][lane] = -q.y;
-      stage[warp][2][lane] = -q.z;
-      stage[warp][3][lane] = q.w * q.w;
-      __syncwarp();
-      const float px = __fadd_rn(pi.x, o.x), py = __fadd_rn(pi.y, o.y), pz = __fadd_rn(pi.z, o.z);
-      const f32x2 px2 = pack2(px, px), py2 = pack2(py, py), pz2 = pack2(pz, pz);
-      // e2 - bandHi: its sign bits, shifted in one by one, are the mask (bit
-      // order reversed), and its smallest magnitude tells whether a candidate
-      // may lie inside the band
-      uint32_t mask = 0u;
-      float near = FLT_MAX;
-#pragma unroll
-      for (int u = 0; u < 32; u += 4) {
-        if (u >= nval) { mask <<= 32 - u; break; }   // uniform
-        const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&stage[warp][0][u]);
-        const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&stage[warp][1][u]);
-        const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&stage[warp][2][u]);
-        const float4 A = *reinterpret_cast<const float4*>(&stage[warp][3][u]);
-        const f32x2 rx0 = add2(px2, X.x), ry0 = add2(py2, Y.x), rz0 = add2(pz2, Z.x);
-        const f32x2 rx1 = add2(px2, X.y), ry1 = add2(py2, Y.y), rz1 = add2(pz2, Z.y);
-        const f32x2 s0 = fma2(fma2(rz0, rz0, fma2(ry0, ry0, mul2(rx0, rx0))), pack2(fminf(ai2, A.x), fminf(ai2, A.y)), nhi2);
-        const f32x2 s1 = fma2(fma2(rz1, rz1, fma2(ry1, ry1, mul2(rx1, rx1))), pack2(fminf(ai2, A.z), fminf(ai2, A.w)), nhi2);
-        float e[4];
-        unpack2(s0, e[0], e[1]);
-        unpack2(s1, e[2], e[3]);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) mask = __funnelshift_l(__float_as_uint(e[v]), mask, 1);
-        near = minAbs3(minAbs3(near, e[0], e[1]), e[2], e[3]);
-      }
-      mask = __brev(mask);
-      if (nval < 32) mask &= (1u << nval) - 1u;
-      if (dcode == 0 && base == k0) mask &= ~(1u << lane);   // the item's own batch: candidate `lane` is node i
-      if (active && near <= bandGap) {   // guard band: this lane's mask again, band candidates by the exact FP64 criterion
-        mask = 0u;
-        for (int u = 0; u < nval; ++u) {
-          const float rx = __fadd_rn(px, stage[warp][0][u]), ry = __fadd_rn(py, stage[warp][1][u]),
-                      rz = __fadd_rn(pz, stage[warp][2][u]);
-          const float e2 = fminf(ai2, stage[warp][3][u]) * (rx * rx + ry * ry + rz * rz);
-          if (e2 > bandHi || (dcode == 0 && base + u == i)) continue;
-          bool in = e2 < bandLo;
-          if (!in) {
-            const int j = base + u;
-            double xjd = F.f[F_X][j], yjd = F.f[F_Y][j], zjd = F.f[F_Z][j];
-            imagePos(g, imageCode(g, hc, dcode), xjd, yjd, zjd);
-            const double qx = __dsub_rn(F.f[F_X][i], xjd), qy = __dsub_rn(F.f[F_Y][i], yjd),
-                         qz = __dsub_rn(F.f[F_Z][i], zjd);
-            in = eta2Exact(F.f[F_HINV][i], qx, qy, qz) <= ext2 || eta2Exact(F.f[F_HINV][j], qx, qy, qz) <= ext2;
-          }
-          if (in) mask |= 1u << u;
+      const float nx = __fsub_rn(o.x, q.x), ny = __fsub_rn(o.y, q.y), nz = __fsub_rn(o.z, q.z);
+      bool keep = lane < nval;
+      if (keep && cull) {
+        const float gx = fmaxf(0.0f, fmaxf(-nx - gHi.x, gLo.x + nx));
+        const float gy = fmaxf(0.0f, fmaxf(-ny - gHi.y, gLo.y + ny));
+        const float gz = fmaxf(0.0f, fmaxf(-nz - gHi.z, gLo.z + nz));
+        const float am = fminf(gLo.w, q.w);
+        keep = !((am * am) * (gx * gx + gy * gy + gz * gz) > cullThr);
+        if (TENSOR) {
+          const float4 bT = diag[grp][b];
+          keep &= !(bT.x * (gx * gx) + bT.y * (gy * gy) + bT.z * (gz * gz) > bT.w);
         }
       }
-      if (!active) mask = 0u;
-      masks[grp][b][lane] = mask;
-      if (CW == 1) {
-        if (mask) nonempty |= 1u << b;
-        hits += __popc(mask);
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (dcode == 0 && first == k0) selfPos = staged + lane;   // the item's own chunk, none of it culled
+      if (keep) {
+        const int pos = staged + __popc(m & ((1u << lane) - 1u));
+        float* st = &stage[warp][0][pos & 63];
+        st[0] = nx;
+        st[64] = ny;
+        st[128] = nz;
+        if (TENSOR) {
+          float jLo, jHi;
+          bandOf(tensorBand(qh1.w, q.w, g), jLo, jHi);
+          const float sx = (mir & 3u) ? -1.f : 1.f, sy = (mir & 12u) ? -1.f : 1.f, sz = (mir & 48u) ? -1.f : 1.f;
+          st[192] = qh0.x; st[256] = qh0.y * (sx * sy); st[320] = qh0.z * (sx * sz);
+          st[384] = qh0.w; st[448] = qh1.x * (sy * sz); st[512] = qh1.y;
+          st[576] = -jHi; st[640] = jLo;
+        } else {
+          st[192] = q.w * q.w;
+        }
+        ids[warp][(pos >> 5) % NB][pos & 31] = (uint32_t)(ds.x + lane);
       }
-      __syncwarp();
+      staged += __popc(m);
+      if (staged - 32 * tested >= 32) {
+        test(32);
+        if (CW == 1 && tested - window == NB - 1) {
+          const int h = hits;
+          writeOut(cnt);
+          cnt += h;
+        }
+      }
     }
-    groupSync();
-    // entries: the nonempty batches of this warp (CW = 4: of its quarter of the
-    // batches), from the lane's hit `at`
-    int at = cnt;
     if (CW == 4) {
-      for (int b = sub * kept / 4; b < (sub + 1) * kept / 4; ++b) {
-        const uint32_t m = masks[grp][b][lane];
-        if (m) nonempty |= 1u << b;
-        hits += __popc(m);
-      }
+      if (staged > 32 * tested) test(staged - 32 * tested);
+      staged = 32 * tested;
       part[sub][lane] = hits;
       __syncthreads();
-      int all = 0;
+      int at = cnt;
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         if (w < sub) at += part[w][lane];
-        all += part[w][lane];
+        cnt += part[w][lane];
       }
-      cnt += all;
-    } else {
-      cnt += hits;
+      writeOut(at);
     }
-    if (WRITE) {
-      uint32_t* out = nbr + nbSlot(active ? i : k0, 0, cap) + (size_t)at * 32;
-      const int stored = min(hits, cap - at);
-      const int most = __reduce_max_sync(0xffffffffu, stored);
-      uint32_t m = 0u;
-      int first = 0;
-      for (int h = 0; h < most; ++h, out += 32)
-        if (h < stored) {
-          if (m == 0u) {
-            const int b = __ffs(nonempty) - 1;
-            nonempty &= nonempty - 1u;
-            m = masks[grp][b][lane];
-            first = desc[grp][b].x;
-          }
-          *out = (uint32_t)(first + __ffs(m) - 1);
-          m &= m - 1u;
-        }
-    }
-    groupSync();   // the next tile overwrites desc, masks and part
+    groupSync();   // the next tile overwrites desc, offs and part
+  }
+  if (CW == 1) {
+    if (staged > 32 * tested) test(staged - 32 * tested);
+    const int h = hits;
+    writeOut(cnt);
+    cnt += h;
   }
   if (sub != 0) return;
   // The stored count never exceeds the capacity: sweeps that run before an
@@ -857,9 +637,14 @@ __global__ void itemsKernel(const uint32_t* __restrict__ keys, long n, int shift
 // Bounding box of every work chunk in its cell's FP32 coordinates, with the
 // smallest and largest h^-1, W lanes per chunk: box[2k] = (min x, min y,
 // min z, min a), box[2k+1] = (max x, max y, max z, max a).
-template <int W>
+// TENSOR adds what bounds |H r|^2 of all its nodes from below and the widest
+// tensor band: tbox[k] = (d_x, d_y, d_z, band) with H^2 - diag(d) positive
+// semidefinite for every node, d_a = (H^2)_aa - sum_b |(H^2)_ab| (Gershgorin;
+// less a margin for the FP32 products, and not below zero).
+template <int W, bool TENSOR>
 __global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ items, const StepScratch* __restrict__ sc,
-                                                     long n, Fields32 P, float4* __restrict__ box) {
+                                                     long n, Grid g, Fields32 P, float4* __restrict__ box,
+                                                     float4* __restrict__ tbox) {
   const int k = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) / W);
   const int lane = threadIdx.x % W;
   const bool live = k < sc->items;
@@ -867,17 +652,29 @@ __global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ ite
   const long j = (long)s + lane;
   const bool in = live && j < n && P.cell[j] == P.cell[s];
   const float4 q = P.posh[in ? j : s];
-  float lo[4] = {q.x, q.y, q.z, q.w}, hi[4] = {q.x, q.y, q.z, q.w};
+  constexpr int NC = TENSOR ? 8 : 4;
+  float lo[NC] = {q.x, q.y, q.z, q.w}, hi[4] = {q.x, q.y, q.z, q.w};
+  if (TENSOR) {
+    const float4 a = P.hten[2 * (in ? j : s)], b = P.hten[2 * (in ? j : s) + 1];
+    const float xy = fabsf(a.x * a.y + a.y * a.w + a.z * b.x), xz = fabsf(a.x * a.z + a.y * b.x + a.z * b.y);
+    const float yz = fabsf(a.y * a.z + a.w * b.x + b.x * b.y);
+    const float m = 1.0e-5f * (b.w * b.w);
+    lo[4 % NC] = fmaxf(0.0f, a.x * a.x + a.y * a.y + a.z * a.z - xy - xz - m);
+    lo[5 % NC] = fmaxf(0.0f, a.y * a.y + a.w * a.w + b.x * b.x - xy - yz - m);
+    lo[6 % NC] = fmaxf(0.0f, a.z * a.z + b.x * b.x + b.y * b.y - xz - yz - m);
+    lo[7 % NC] = -tensorBand(b.w, q.w, g);
+  }
 #pragma unroll
-  for (int o = W / 2; o > 0; o >>= 1)
+  for (int o = W / 2; o > 0; o >>= 1) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-    }
+    for (int c = 0; c < NC; ++c) lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+#pragma unroll
+    for (int c = 0; c < 4; ++c) hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+  }
   if (live && lane == 0) {
     box[2 * k] = make_float4(lo[0], lo[1], lo[2], lo[3]);
     box[2 * k + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    if (TENSOR) tbox[k] = make_float4(lo[4 % NC], lo[5 % NC], lo[6 % NC], -lo[7 % NC]);
   }
 }
 
@@ -1824,13 +1621,16 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
   lc->add(1);
 }
 void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
-                 int nItemsBound, Fields32 P, int* items, int* chunkOf, float4* box, StepScratch* sc, cudaStream_t s,
-                 LaunchCounter* lc) {
+                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, float4* box,
+                 StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
   itemsKernel<<<gridFor(n, 256), 256, 0, s>>>(sortedKeys, n, shift, space, cellEnd, width, items, chunkOf, sc);
   const unsigned gb = gridFor((long)nItemsBound * width, 128);
-  if (width == 8) itemBoxKernel<8><<<gb, 128, 0, s>>>(items, sc, n, P, box);
-  else if (width == 16) itemBoxKernel<16><<<gb, 128, 0, s>>>(items, sc, n, P, box);
-  else itemBoxKernel<32><<<gb, 128, 0, s>>>(items, sc, n, P, box);
+#define SPH_BOX(W, T) itemBoxKernel<W, T><<<gb, 128, 0, s>>>(items, sc, n, g, P, box, box + 2 * n)
+#define SPH_BOXW(T) do { if (width == 8) SPH_BOX(8, T); else if (width == 16) SPH_BOX(16, T); else SPH_BOX(32, T); } while (0)
+  if (tensor) SPH_BOXW(true);
+  else SPH_BOXW(false);
+#undef SPH_BOXW
+#undef SPH_BOX
   lc->add(2);
 }
 // Band of the FP32 pre-filter on e2 = min(a_i, a_j)^2 r^2 around ext^2
@@ -1982,31 +1782,18 @@ void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, 
                          cudaStream_t s, LaunchCounter* lc) {
   float lo, hi;
   neighborBand(g, ext2, lo, hi);
-  if (!tensor) {
-    // four warps per item while the items alone would leave SMs idle (below
-    // ~16 items per SM): 3,375 nodes 60 -> see DESIGN table; one warp above
-    const bool wide = nItems < kWideItems;
-    const unsigned gb = wide ? (unsigned)nItems : (unsigned)((nItems + 3) / 4);
-#define SPH_NBM(WR, CW)                                                                                          \
-  neighborMaskKernel<WR, CW><<<gb, 128, 0, s>>>(F, P, items, nItems, width, g, cellStart, cellEnd, counts,     \
-                                                WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, sc, box, chunkOf)
-    if (nbr) { if (wide) SPH_NBM(true, 4); else SPH_NBM(true, 1); }
-    else { if (wide) SPH_NBM(false, 4); else SPH_NBM(false, 1); }
+  // four warps per item while the items alone would leave SMs idle (below
+  // ~16 items per SM), one warp above
+  const bool wide = nItems < kWideItems;
+  const unsigned gb = wide ? (unsigned)nItems : (unsigned)((nItems + 3) / 4);
+#define SPH_NBM(WR, CW, TE)                                                                                      \
+  neighborMaskKernel<WR, CW, TE><<<gb, 128, 0, s>>>(F, P, items, nItems, width, g, cellStart, cellEnd, counts, \
+                                                    WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, sc, box, box + 2 * n, chunkOf)
+#define SPH_NBW(WR, TE) do { if (wide) SPH_NBM(WR, 4, TE); else SPH_NBM(WR, 1, TE); } while (0)
+  if (nbr) { if (tensor) SPH_NBW(true, true); else SPH_NBW(true, false); }
+  else { if (tensor) SPH_NBW(false, true); else SPH_NBW(false, false); }
+#undef SPH_NBW
 #undef SPH_NBM
-    lc->add(1);
-    return;
-  }
-  const long threads = (long)nItems * width;
-  const unsigned gb = (unsigned)((threads + 127) / 128);
-#define SPH_NBR(WR, WD)                                                                                            \
-  neighborWarpKernel<WR, WD, true><<<gb, 128, 0, s>>>(F, P, n, items, nItems, g, cellStart, cellEnd, counts,      \
-                                                      WR ? nbr : nullptr, ext2, lo, hi, WR ? cap : 0, sc, box, chunkOf)
-  if (nbr) {
-    if (width == 8) SPH_NBR(true, 8); else if (width == 16) SPH_NBR(true, 16); else SPH_NBR(true, 32);
-  } else {
-    if (width == 8) SPH_NBR(false, 8); else if (width == 16) SPH_NBR(false, 16); else SPH_NBR(false, 32);
-  }
-#undef SPH_NBR
   lc->add(1);
 }
 

@@ -64,8 +64,8 @@ void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCoun
 // 16 or 32) consecutive nodes of a cell, their first nodes, each cell's first
 // chunk and the chunks' bounding boxes; the count goes to sc->items.
 void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
-                 int nItemsBound, Fields32 P, int* items, int* chunkOf, float4* box, StepScratch* sc, cudaStream_t s,
-                 LaunchCounter* lc);
+                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, float4* box,
+                 StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 // nItems: an upper bound on the item count (sizes the grid); sc->items holds
 // the count itself.  The largest count and the sum of all go to *sc.
 void launchNeighborsWarp(const Fields& F, Fields32 P, long n, const int* items, int nItems, StepScratch* sc,
