@@ -119,6 +119,7 @@ struct sphgpu_ctx {
 
   // parameters
   NodeListParams lists[kMaxNodeLists]{};
+  NodeListParams sentLists[kMaxNodeLists];   // what dLists holds
   DBuf dLists;   // device copy of lists
   DBuf dvq;      // limited Q, mixed mode: FP32 copy of the Q's DvDx (3 float4 per node)
   int numLists = 0;
@@ -372,14 +373,34 @@ void refreshParams(sphgpu_ctx* c) {
     L.gm1 = L.gamma - 1.0;
     L.ggm1 = L.gamma * L.gm1;
   }
-  c->dLists.ensure(sizeof(c->lists));
-  CUDA_OK(cudaMemcpyAsync(c->dLists.p, c->lists, sizeof(c->lists), cudaMemcpyHostToDevice, c->stream));
+  if (!c->dLists.p || std::memcmp(c->sentLists, c->lists, sizeof(c->lists)) != 0) {
+    c->dLists.ensure(sizeof(c->lists));
+    CUDA_OK(cudaMemcpyAsync(c->dLists.p, c->lists, sizeof(c->lists), cudaMemcpyHostToDevice, c->stream));
+    std::memcpy(c->sentLists, c->lists, sizeof(c->lists));
+  }
   hp.lists = c->dLists.as<NodeListParams>();
 }
 
 void requireState(sphgpu_ctx* c) {
   if (!c->haveTable) throw Error(SPHGPU_E_STATE, "no kernel table installed");
   if (c->n <= 0) throw Error(SPHGPU_E_STATE, "no particles");
+}
+
+// The kernels' scratch values, read back in stream order (valid after the
+// next synchronisation).
+void fetchScratch(sphgpu_ctx* c) {
+  CUDA_OK(cudaMemcpyAsync(c->hstep, c->step(), sizeof(StepScratch), cudaMemcpyDeviceToHost, c->stream));
+}
+// The bounds of hstep: order keys back to doubles, squared half-widths to
+// half-widths.
+void readBounds(sphgpu_ctx* c) {
+  for (int k = 0; k < kBoundsVals; ++k) {
+    long long b = c->hstep->bounds[k];
+    if (b < 0) b ^= 0x7fffffffffffffffLL;
+    double& v = c->cachedBounds[k];
+    std::memcpy(&v, &b, sizeof v);
+    if (k >= 7) v = std::sqrt(v);
+  }
 }
 
 //------------------------------------------------------------------------------
@@ -391,13 +412,11 @@ void requireState(sphgpu_ctx* c) {
 void buildGrid(sphgpu_ctx* c) {
   Scope sc(c->prof, "bounds");
   if (!c->boundsValid) {   // the bounds of the last step's check describe a changed state
-    double* d = c->small.as<double>() + 20;
-    c->scratch.ensure(kBoundsVals * sizeof(double) * 4096);
-    launchBounds(c->F, c->n, c->hp.asph != 0, c->scratch.as<double>(), kBoundsVals * 4096, d, c->stream, &c->lc);
+    launchBounds(c->F, c->n, c->hp.asph != 0, c->step(), c->stream, &c->lc);
     c->check();
-    CUDA_OK(cudaMemcpyAsync(c->hsmall + 20, d, kBoundsVals * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    fetchScratch(c);
     CUDA_OK(cudaStreamSynchronize(c->stream));
-    std::memcpy(c->cachedBounds, c->hsmall + 20, sizeof(c->cachedBounds));
+    readBounds(c);
   }
   c->boundsValid = false;   // consumed: the step moves the nodes
   const double* bnd = c->cachedBounds;
@@ -484,11 +503,6 @@ void buildGrid(sphgpu_ctx* c) {
 }
 
 int capFor(int m) { return std::max(32, ((m + m / 8 + 16 + 31) / 32) * 32); }
-// The kernels' scratch values, read back in stream order (valid after the
-// next synchronisation).
-void fetchScratch(sphgpu_ctx* c) {
-  CUDA_OK(cudaMemcpyAsync(c->hstep, c->step(), sizeof(StepScratch), cudaMemcpyDeviceToHost, c->stream));
-}
 int readMaxCount(sphgpu_ctx* c) {
   fetchScratch(c);
   CUDA_OK(cudaStreamSynchronize(c->stream));
@@ -549,9 +563,19 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   c->vals.ensure(n * sizeof(int));
   c->valsAlt.ensure(n * sizeof(int));
   c->sortWs.ensure(radixSortWorkspaceBytes(n));
+  const size_t space = (size_t)1 << keyBits;
+  if (space > c->cellSpace) {
+    c->cellRange.release();
+    c->cellRange.ensure(2 * space * sizeof(int));
+    c->cellSpace = space;
+  }
+  // empty cell ranges and the sort's counters, zeroed by the key kernel
+  const ClearedWords clear{{c->sortWs.as<unsigned>(), reinterpret_cast<unsigned*>(c->cellStart())},
+                           {(long long)radixSortClearedWords(n, sortBits), (long long)(c->cellSpace + space)}};
   {
     Scope sc(c->prof, "cell_keys");
-    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->step(), c->stream, &c->lc);
+    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->step(), clear, c->stream,
+                   &c->lc);
   }
   uint32_t* k = c->keys.as<uint32_t>();
   int* v = c->vals.as<int>();
@@ -559,16 +583,9 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   int* va = c->valsAlt.as<int>();
   {
     Scope sc(c->prof, "radix_sort");
-    radixSortPairs(k, v, ka, va, n, sortBits, c->sortWs.p, &c->step()->sortTimeout, c->stream, &c->lc);
+    radixSortPairs(k, v, ka, va, n, sortBits, c->sortWs.p, &c->step()->sortTimeout, true, c->stream, &c->lc);
   }
   c->check();
-  const size_t space = (size_t)1 << keyBits;
-  if (space > c->cellSpace) {
-    c->cellRange.release();
-    c->cellRange.ensure(2 * space * sizeof(int));
-    c->cellSpace = space;
-  }
-  CUDA_OK(cudaMemsetAsync(c->cellStart(), 0, (c->cellSpace + space) * sizeof(int), c->stream));
   {
     Scope sc(c->prof, "permute");
     const int nx = 1 - c->cur;
@@ -649,15 +666,6 @@ void ensurePacc(sphgpu_ctx* c) {
   c->pacc.ensure(std::max<size_t>(1, c->nbSlots()) * 3 * per);
 }
 
-// LimitedMonaghanGingoldViscosity reads the Q's own copy of DvDx, refreshed
-// from the hydro's at every postStateUpdate (ArtificialViscosityHandle.cc:167-183).
-void copyQGradient(sphgpu_ctx* c) {
-  if (!c->hp.limitedQ) return;
-  Scope sc(c->prof, "update");
-  launchCopyQGradient(c->F, c->n, c->stream, &c->lc);
-  c->check();
-}
-
 void prepare32(sphgpu_ctx* c) {
   if (!c->fp32()) return;
   Scope sc(c->prof, "prepare_fp32");
@@ -679,10 +687,11 @@ void sumDensity(sphgpu_ctx* c) {
     launchSumDensity(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   c->check();
 }
-void gradh(sphgpu_ctx* c) {
+// pf.on: the pair sweep's inputs follow.
+void gradh(sphgpu_ctx* c, const PairForm& pf = {}) {
   Scope sc(c->prof, "gradh");
   if (c->fp32())
-    launchGradhFP32(c->F, c->f32(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
+    launchGradhFP32(c->F, c->f32(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, pf, c->stream, &c->lc);
   else if (c->iso64())
     launchGradh64(c->F, c->rec64.p, c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   else
@@ -695,10 +704,15 @@ void settleOmega(sphgpu_ctx* c) {
   c->omegaStale = false;
 }
 
-void evalDerivs(sphgpu_ctx* c) {
+void ensureQMirror(sphgpu_ctx* c) {
+  if (c->fp32() && c->hp.limitedQ) c->dvq.ensure((size_t)c->n * 3 * sizeof(float4));
+}
+// inputs: the isotropic mixed pair sweep's per-node inputs are already those of
+// this state; half: the energy sweep's half-step velocities, wanted from it.
+void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}) {
   ensurePacc(c);
+  ensureQMirror(c);
   if (c->fp32() && c->hp.limitedQ) {   // FP32 mirror of the Q's DvDx in the current node order
-    c->dvq.ensure((size_t)c->n * 3 * sizeof(float4));
     if (c->hp.asph || c->hp.crk) {   // the isotropic SPH sweep writes its own form
       launchQGradient32(c->F, c->dvq.as<float4>(), c->n, c->stream, &c->lc);
       c->check();
@@ -750,7 +764,7 @@ void evalDerivs(sphgpu_ctx* c) {
   } else if (c->fp32()) {
     auto pair = [&](int v) {
       launchPairFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp,
-                     c->pacc.as<float>(), v, c->stream, &c->lc);
+                     c->pacc.as<float>(), v, inputs, half, c->stream, &c->lc);
     };
     tunePair(c->hp.asph ? kPairVariantsTensor : kPairVariants, pair);
     Scope sc(c->prof, "pair_fp32");
@@ -852,10 +866,11 @@ double selectDt(sphgpu_ctx* c, double dtMin, double dtMax, bool fusedDone = fals
   return dt;
 }
 
-// The end of the step in one pass: walls, the state check and the bounds the
-// next neighbour build needs, read back in one synchronisation.
-void endStep(sphgpu_ctx* c) {
-  {
+// The end of the step in one pass (launched: the update took it along): walls,
+// the state check and the bounds the next neighbour build needs, read back in
+// one synchronisation.
+void endStep(sphgpu_ctx* c, bool launched) {
+  if (!launched) {
     Scope sc(c->prof, "enforce");
     launchEndStep(c->F, c->n, c->grid, c->hp.asph != 0, c->step(), c->stream, &c->lc);
   }
@@ -863,11 +878,7 @@ void endStep(sphgpu_ctx* c) {
   fetchScratch(c);
   CUDA_OK(cudaStreamSynchronize(c->stream));
   if (c->hstep->bad) throw Error(SPHGPU_E_NAN, "non-finite or non-positive state after the step");
-  for (int k = 0; k < kBoundsVals; ++k) {   // order keys back to doubles
-    long long b = c->hstep->bounds[k];
-    if (b < 0) b ^= 0x7fffffffffffffffLL;
-    std::memcpy(&c->cachedBounds[k], &b, sizeof b);
-  }
+  readBounds(c);
   c->boundsValid = true;
 }
 
@@ -931,24 +942,38 @@ double step(sphgpu_ctx* c, double maxTime) {
     if (!(dt > 0.0) || !std::isfinite(dt)) throw Error(SPHGPU_E_STATE, "the domain exchange returned a bad dt");
   }
   const double hdt = 0.5 * dt;
+  // The update takes along the limited Q's copy of DvDx (the
+  // ArtificialViscosity's postStateUpdate, ArtificialViscosityHandle.cc:167-183)
+  // and the pair sweep's per-node inputs; an exchange between them and the pair
+  // sweep changes the halo's, so they are then formed at the sweep.
+  const Fields32 m32 = c->f32();
+  const bool isoPair = c->fp32() && !c->hp.asph && !c->hp.crk && !c->xfn;
+  UpdateExtras ex;
+  ex.copyQ = c->hp.limitedQ;
+  if (isoPair) ex.pair = pairForm32(c->n, c->hp);
+  ensureQMirror(c);
   {
     Scope sc(c->prof, "update");   // the half-step update also saves state0
-    const Fields32 m32 = c->f32();
-    launchUpdate(c->F, c->listp(), c->n, c->hp, hdt, true, c->cfg.gravity != 0, c->fp32() ? &m32 : nullptr, c->grid,
+    Fields32 m = m32;
+    m.dvq = c->dvq.as<float4>();
+    launchUpdate(c->F, c->listp(), c->n, c->hp, hdt, true, c->cfg.gravity != 0, c->fp32() ? &m : nullptr, c->grid, ex,
                  c->stream, &c->lc);
   }
   c->check();
   c->time = t + hdt;
-  copyQGradient(c);                                  // postStateUpdate (mid): the Q's DvDx
-  if (c->cfg.gradh_correction) gradh(c);             // postStateUpdate (mid)
+  if (c->cfg.gradh_correction) gradh(c, ex.pair);    // postStateUpdate (mid)
   c->omegaStale = false;
   if (c->cfg.gradh_correction) exchangePoint(c, SPHGPU_EXCHANGE_OMEGA);
-  evalDerivs(c);                                     // derivs.Zero(); evaluateDerivatives(t + dt/2)
+  HalfStep half;
+  if (c->fp32() && c->cfg.compatible_energy) {
+    c->v12.ensure(c->n * 2 * sizeof(float4));
+    if (!c->hp.crk && !c->xfn) half = HalfStep{c->v12.as<float4>(), c->v12.as<float4>() + c->n, hdt};
+  }
+  evalDerivs(c, isoPair, half);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
   exchangePoint(c, SPHGPU_EXCHANGE_DERIVS);          // the halo's accelerations and energy rates
   if (c->cfg.compatible_energy) {
     Scope sc(c->prof, "energy");
     if (c->fp32()) {
-      c->v12.ensure(c->n * 2 * sizeof(float4));
       ++c->energyEvals;
       const bool retune = c->energyRetuneAt >= 0 && c->energyEvals >= c->energyRetuneAt;
       if (!c->energyPinned &&
@@ -965,7 +990,7 @@ double step(sphgpu_ctx* c, double maxTime) {
           const int v = t % kEnergyVariants;
           CUDA_OK(cudaEventRecord(e0, c->stream));
           launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(),
-                                     c->v12.as<float4>() + c->n, 0.0, v, c->stream, &c->lc);
+                                     c->v12.as<float4>() + c->n, 0.0, v, !half.hi, c->stream, &c->lc);
           CUDA_OK(cudaEventRecord(e1, c->stream));
           CUDA_OK(cudaEventSynchronize(e1));
           c->check();
@@ -980,22 +1005,26 @@ double step(sphgpu_ctx* c, double maxTime) {
         c->energyRetuneAt = retune ? -1 : c->energyEvals + kRetuneAfter;
       }
       launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(),
-                                 c->v12.as<float4>() + c->n, dt, c->energyVariant, c->stream, &c->lc);
+                                 c->v12.as<float4>() + c->n, dt, c->energyVariant, !half.hi, c->stream, &c->lc);
     }
     else {
       c->v12.ensure(c->n * 4 * sizeof(double));
       launchEnergy64(c->F, c->v12.p, c->n, c->grid, c->nl(), c->pacc.as<double>(), dt, c->stream, &c->lc);
     }
   }
+  // the end of the step rides on the update unless a sweep of this state comes
+  // between them
+  const bool owed = (c->fp32() || c->bcs.empty()) && !c->hp.asphEnd;   // see below
+  const bool endHere = !c->hp.asphEnd && (!c->cfg.gradh_correction || owed);
+  ex.pair.on = 0;
+  ex.end = endHere ? c->step() : nullptr;
   {
     Scope sc(c->prof, "update");
-    const Fields32 m32 = c->f32();
     launchUpdate(c->F, c->listp(), c->n, c->hp, dt, false, c->cfg.gravity != 0, c->fp32() ? &m32 : nullptr, c->grid,
-                 c->stream, &c->lc);
+                 ex, c->stream, &c->lc);
   }
   c->check();
   c->time = t + dt;
-  copyQGradient(c);                                  // postStateUpdate (end): the Q's DvDx
   // postStateUpdate (end): the grad-h correction of the new state.  Nothing
   // of the next step reads it before the half-step postStateUpdate computes
   // it again (the density sum, the dt vote and the half-step update do not
@@ -1009,7 +1038,7 @@ double step(sphgpu_ctx* c, double maxTime) {
   if (c->cfg.gradh_correction) {
     // ASPHSmoothingScale changes H after this point: its Omega is the one of
     // the H before that change, so it is computed now
-    if ((c->fp32() || c->bcs.empty()) && !c->hp.asphEnd) c->omegaStale = true;
+    if (owed) c->omegaStale = true;
     else gradh(c);
   }
   if (c->hp.asphEnd) {   // postStepFinalize: ASPHSmoothingScale::finalize
@@ -1018,7 +1047,7 @@ double step(sphgpu_ctx* c, double maxTime) {
                   c->stream, &c->lc);
     c->check();
   }
-  endStep(c);
+  endStep(c, endHere);
   c->cycle += 1;
   c->lastDt = dt;
   return dt;

@@ -724,6 +724,40 @@ __device__ __forceinline__ void finalizeNode32(Fields& F, long i, int li, const 
   F.f[F_HIDEAL][i] = fmin(L.hminInv, fmax(L.hmaxInv, hid));
 }
 
+// v12 = v0 + a dt/2 of the compatible-energy sweep, formed in FP64 and stored
+// as an unevaluated float pair hi + lo.
+__device__ __forceinline__ void halfStepVelocity(const Fields& F, long i, double ax, double ay, double az, double deps,
+                                                 const HalfStep& half) {
+  const double x = F.f[F_VX0][i] + ax * half.hdt;
+  const double y = F.f[F_VY0][i] + ay * half.hdt;
+  const double z = F.f[F_VZ0][i] + az * half.hdt;
+  const float hx = (float)x, hy = (float)y, hz = (float)z;
+  half.hi[i] = make_float4(hx, hy, hz, (float)deps);
+  half.lo[i] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.0f);
+}
+// Per-node inputs of the isotropic pair sweep: (rho, Omega^-1 P / rho^2, -Cl c,
+// 1 / (2 rho)), once per node instead of once per pair.
+__device__ __forceinline__ float4 pairRecord(const float4& th, const PairForm& pf) {
+  const float ir = __frcp_rn(th.x);
+  float pr = __fmul_rn(__fmul_rn(__fmul_rn(th.w, th.y), ir), ir), hir = 0.5f * ir;
+  if (pf.spline) { pr = timesSplineA(pr); hir = timesSplineA(hir); }
+  return make_float4(th.x, pr, __fmul_rn(-pf.Cl, th.z), hir);
+}
+// The limited Q's DvDx for h = r/2: its symmetric part (xx yy zz xy | xz yz,
+// off-diagonal pairs summed), or for the exact form (full) all nine components.
+__device__ __forceinline__ void writeQGradient(const Fields32& P, long i, float* v, const PairForm& pf) {
+  if (pf.full) {
+    P.dvq[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
+    P.dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
+    P.dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) v[k] *= 0.25f;
+  P.dvq[2 * i] = make_float4(v[0], v[4], v[8], v[1] + v[3]);
+  P.dvq[2 * i + 1] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
+}
+
 // Node completion of the isotropic mixed pair loop: finalizeNode32 in terms
 // of the loop's reduced sums.  The FP32 results go into the FP64 fields by
 // integer conversions (the FP64 pipe is ~1/64 of the FP32 rate).
@@ -738,7 +772,7 @@ struct PairSums32 {
 template <bool SPLINE>
 __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSums32& a, float ai, float mi,
                                                float rhoi, int numNb, const HydroParams& hp,
-                                               const double* __restrict__ herm) {
+                                               const double* __restrict__ herm, const HalfStep& half) {
   auto put = [&](int f, float v) { F.f[f][i] = toDouble(v); };
   const float Hdeti = (ai * ai) * ai, W0 = (float)hp.W0;
   const float irho = 1.0f / rhoi;
@@ -790,6 +824,7 @@ __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSu
   const double deps = a.deps * toDouble(Hdeti * ai);
   F.f[F_DEPSDT][i] =
       hp.totalEnergy ? toDouble(mi) * ((vxi * a.dvx + vyi * a.dvy + vzi * a.dvz) + deps) : deps;
+  if (half.hi) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
   put(F_MAXQ, rhoi * a.maxE);
   put(F_EFFQ, 2.0f * rhoi * Hdeti * a.ve);
   float xw = a.xw;

@@ -867,7 +867,7 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   int* vals = w->vals.as<int>();
   int* valsAlt = w->vals2.as<int>();
   GCHK(cudaMemsetAsync(w->timeout.p, 0, sizeof(int), s));
-  radixSortPairs(skey, vals, skeyAlt, valsAlt, n, 3 * kMaxLevel, w->sortWs.p, w->timeout.as<int>(), s, lc);
+  radixSortPairs(skey, vals, skeyAlt, valsAlt, n, 3 * kMaxLevel, w->sortWs.p, w->timeout.as<int>(), false, s, lc);
   treeNodesKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, vals, n, w->tpos.as<TreeNode>(),
                                                              mixed ? w->tpos32.as<TreeNode32>() : nullptr);
   chainCountKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(skey, n, w->nc.as<int>());

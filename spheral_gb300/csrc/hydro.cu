@@ -25,48 +25,95 @@ using namespace dev;
 // largest half-width per axis of the unit ellipsoids {r : |H r| <= 1}, i.e.
 // sqrt((H^-2)_aa) = |row a of H^-1| (the cell edge per axis).
 //------------------------------------------------------------------------------
-__global__ void boundsKernel(Fields F, long n, int tensor, double* __restrict__ part) {
-  __shared__ double sm[32];
-  double ah = DBL_MAX, mnx = DBL_MAX, mny = DBL_MAX, mnz = DBL_MAX, mxx = -DBL_MAX, mxy = -DBL_MAX, mxz = -DBL_MAX;
-  double ex = 0.0, ey = 0.0, ez = 0.0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    ah = fmin(ah, F.f[F_HINV][i]);
-    const double x = F.f[F_X][i], y = F.f[F_Y][i], z = F.f[F_Z][i];
-    mnx = fmin(mnx, x); mny = fmin(mny, y); mnz = fmin(mnz, z);
-    mxx = fmax(mxx, x); mxy = fmax(mxy, y); mxz = fmax(mxz, z);
-    if (tensor) {
-      const Sym w = symInverse(loadSym(F, F_HT_XX, i));
-      ex = fmax(ex, sqrt(w.xx * w.xx + w.xy * w.xy + w.xz * w.xz));
-      ey = fmax(ey, sqrt(w.xy * w.xy + w.yy * w.yy + w.yz * w.yz));
-      ez = fmax(ez, sqrt(w.xz * w.xz + w.yz * w.yz + w.zz * w.zz));
+// A signed integer with the order of the double x (for non-NaN x; -0 sorts
+// just below +0, which only sends a node at a wall to the exact test).
+__device__ __forceinline__ long long orderKey(double x) {
+  const long long b = __double_as_longlong(x);
+  return b >= 0 ? b : (b ^ 0x7fffffffffffffffLL);
+}
+// Bit tests of the end-of-step check (integer pipe).
+__device__ __forceinline__ bool finiteBits(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+__device__ __forceinline__ bool positiveBits(double x) {   // x > 0 and finite
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b < 0x7ff0000000000000LL;
+}
+
+// Running bounds of a thread's nodes on order keys (the FP64 pipe, which
+// FP64 comparisons take, is narrow); NaN is passed over.
+struct NodeBounds {
+  long long mn[4] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MAX};
+  long long mx[6] = {LLONG_MIN, LLONG_MIN, LLONG_MIN, 0, 0, 0};
+  static __device__ bool isNaN(double x) {
+    return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ULL;
+  }
+  __device__ void add(double a, const double* p) {
+    if (!isNaN(a)) mn[0] = min(mn[0], orderKey(a));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (isNaN(p[k])) continue;
+      const long long o = orderKey(p[k]);
+      mn[1 + k] = min(mn[1 + k], o);
+      mx[k] = max(mx[k], o);
     }
   }
-  const double r[kBoundsVals] = {blockMin(ah, sm), blockMin(mnx, sm), blockMin(mny, sm), blockMin(mnz, sm),
-                                 blockMax(mxx, sm), blockMax(mxy, sm), blockMax(mxz, sm),
-                                 blockMax(ex, sm), blockMax(ey, sm), blockMax(ez, sm)};
-  if (threadIdx.x == 0)
-    for (int k = 0; k < kBoundsVals; ++k) part[blockIdx.x * kBoundsVals + k] = r[k];
-}
-__global__ void boundsFinalKernel(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  __shared__ double sm[32];
-  double v[kBoundsVals];
-  for (int k = 0; k < kBoundsVals; ++k) v[k] = k < 4 ? DBL_MAX : -DBL_MAX;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int k = 0; k < kBoundsVals; ++k)
-      v[k] = k < 4 ? fmin(v[k], part[b * kBoundsVals + k]) : fmax(v[k], part[b * kBoundsVals + k]);
-  for (int k = 0; k < kBoundsVals; ++k) {
-    const double r = k < 4 ? blockMin(v[k], sm) : blockMax(v[k], sm);
-    if (threadIdx.x == 0) out[k] = r;
+  __device__ void addTensor(const Sym& H) {   // squares: the host takes the roots of the largest
+    const Sym w = symInverse(H);
+    const double e[3] = {w.xx * w.xx + w.xy * w.xy + w.xz * w.xz, w.xy * w.xy + w.yy * w.yy + w.yz * w.yz,
+                         w.xz * w.xz + w.yz * w.yz + w.zz * w.zz};
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (!isNaN(e[k])) mx[3 + k] = max(mx[3 + k], orderKey(e[k]));
   }
+};
+// Block minima and maxima into sc->bounds.  Every thread of a 256-thread block
+// calls it; a bound is only written where it moves.
+__device__ __forceinline__ void mergeBounds(const NodeBounds& b, bool tensor, StepScratch* __restrict__ sc) {
+  __shared__ long long sm[8][10];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 10; ++k) {
+    if (k >= 7 && !tensor) break;
+    long long v = k < 4 ? b.mn[k] : b.mx[k - 4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long w = __shfl_xor_sync(0xffffffffu, v, o);
+      v = k < 4 ? min(v, w) : max(v, w);
+    }
+    if (lane == 0) sm[warp][k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < (tensor ? 10 : 7)) {
+    const int k = threadIdx.x;
+    long long v = sm[0][k];
+    for (int w = 1; w < 8; ++w) v = k < 4 ? min(v, sm[w][k]) : max(v, sm[w][k]);
+    const long long seen = *(volatile long long*)&sc->bounds[k];
+    if (k < 4) { if (v < seen) atomicMin(&sc->bounds[k], v); }
+    else { if (v > seen) atomicMax(&sc->bounds[k], v); }
+  }
+}
+__global__ void resetScratchKernel(StepScratch* __restrict__ sc) { resetScratch(sc); }
+__global__ void __launch_bounds__(256) boundsKernel(Fields F, long n, int tensor, StepScratch* __restrict__ sc) {
+  NodeBounds b;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const double p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
+    b.add(F.f[F_HINV][i], p);
+    if (tensor) b.addTensor(loadSym(F, F_HT_XX, i));
+  }
+  mergeBounds(b, tensor != 0, sc);
 }
 
 //------------------------------------------------------------------------------
 // Neighbour build.
 //------------------------------------------------------------------------------
 __global__ void cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ keys, int* __restrict__ vals,
-                              uint32_t* __restrict__ cellc, StepScratch* __restrict__ sc) {
+                              uint32_t* __restrict__ cellc, StepScratch* __restrict__ sc, ClearedWords clear) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i == 0) resetScratch(sc);
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    for (long long w = i; w < clear.n[k]; w += (long long)gridDim.x * blockDim.x) clear.p[k][w] = 0u;
   if (i >= n) return;
   const double p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
   uint32_t c[3], f[3];
@@ -107,9 +154,17 @@ __global__ void permuteKernel(Fields Fin, Fields Fout, const int* __restrict__ p
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int p = (int)min((unsigned)perm[k], (unsigned)(n - 1));
-  for (int r = 0; r < sel.n; ++r)
-#pragma unroll 4
-    for (int f = sel.first[r]; f < sel.last[r]; ++f) Fout.f[f][k] = Fin.f[f][p];
+  // gridDim.y > 1: the last row of blocks takes the rest, the others a share of
+  // the fields each
+  const int rows = gridDim.y > 1 ? gridDim.y - 1 : 1, row = blockIdx.y;
+  if (row < rows)
+    for (int r = 0; r < sel.n; ++r) {
+      const int len = sel.last[r] - sel.first[r];
+      const int f1 = sel.first[r] + len * (row + 1) / rows;
+#pragma unroll 8
+      for (int f = sel.first[r] + len * row / rows; f < f1; ++f) Fout.f[f][k] = Fin.f[f][p];
+    }
+  if (row != (int)gridDim.y - 1) return;
   origOut[k] = origIn[p];
   listOut[k] = listIn[p];
   const uint32_t cell = cellIn[p];
@@ -1178,6 +1233,87 @@ __global__ void tensorExtentKernel(Fields F, long n) {
   storeExtent(F, i, loadSym(F, F_HT_XX, i));
 }
 
+__global__ void eosKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  eosNode(F, i, lists[list[i]]);
+}
+
+// Boundary::setAllViolationNodes + enforceBoundary (PlanarBoundary.cc:153-190,
+// ReflectingBoundary.cc:465-473): nodes strictly outside a plane are mapped
+// back; reflecting walls also mirror the velocity.
+__device__ __forceinline__ bool fuzzyZero(double x) { return fabs(x) <= 1.0e-15 * fmax(1.0, fabs(x)); }
+// tensor: the H of a node mapped back through a reflecting wall is reflected
+// too (PlanarBoundary::updateViolationNodes -> enforceBoundary(Hfield),
+// (R H R).Symmetric()).
+// p: the node's position, in and out.
+__device__ __forceinline__ void enforceNode(Fields& F, long i, double* p_, const Grid& g, int tensor) {
+  auto reflectH = [&](int a) {
+    if (!tensor) return;
+    if (a == 0) { F.f[F_HT_XY][i] = -F.f[F_HT_XY][i]; F.f[F_HT_XZ][i] = -F.f[F_HT_XZ][i]; }
+    else if (a == 1) { F.f[F_HT_XY][i] = -F.f[F_HT_XY][i]; F.f[F_HT_YZ][i] = -F.f[F_HT_YZ][i]; }
+    else { F.f[F_HT_XZ][i] = -F.f[F_HT_XZ][i]; F.f[F_HT_YZ][i] = -F.f[F_HT_YZ][i]; }
+  };
+  double* P[3] = {F.f[F_X], F.f[F_Y], F.f[F_Z]};
+  double* V[3] = {F.f[F_VX], F.f[F_VY], F.f[F_VZ]};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double lo = g.wallLo[a], hi = g.wallHi[a];
+    double p = p_[a];
+    // Integer pre-test on order-preserving keys of the bit patterns: a node
+    // strictly inside (lo, hi) needs nothing, and the FP64 tests below (the
+    // FP64 pipe is narrow) run only for the few on or beyond a wall.
+    if (orderKey(p) > orderKey(lo) && orderKey(p) < orderKey(hi)) continue;
+    const double sdLo = p - lo, sdHi = hi - p;
+    if (g.kindLo[a] == AXIS_PERIODIC) {
+      if (sdLo < 0.0 && !fuzzyZero(sdLo)) p = imageCoord(p, 2, AXIS_PERIODIC, AXIS_PERIODIC, lo, hi);
+      else if (sdHi < 0.0 && !fuzzyZero(sdHi)) p = imageCoord(p, 1, AXIS_PERIODIC, AXIS_PERIODIC, lo, hi);
+      P[a][i] = p_[a] = p;
+    } else {
+      if (g.kindLo[a] == AXIS_REFLECT && sdLo < 0.0 && !fuzzyZero(sdLo)) {
+        p = imageCoord(p, 1, AXIS_REFLECT, g.kindHi[a], lo, hi);
+        P[a][i] = p_[a] = p;
+        V[a][i] = -V[a][i];
+        reflectH(a);
+      }
+      const double sdHi2 = hi - p;
+      if (g.kindHi[a] == AXIS_REFLECT && sdHi2 < 0.0 && !fuzzyZero(sdHi2)) {
+        p = imageCoord(p, 2, g.kindLo[a], AXIS_REFLECT, lo, hi);
+        P[a][i] = p_[a] = p;
+        V[a][i] = -V[a][i];
+        reflectH(a);
+      }
+    }
+  }
+}
+
+// End of a node's step: a node outside a wall is mapped back, the state is
+// checked (finite, positive) and the bounds the next neighbour build needs are
+// taken.  Returns whether the state is bad.
+__device__ __forceinline__ bool endNode(Fields& F, long i, double* p, double vx, double vy, double vz, double m,
+                                        double rho, double a, double eps, const Sym& H, bool tensor, const Grid& g,
+                                        NodeBounds& b) {
+  enforceNode(F, i, p, g, tensor);
+  b.add(a, p);
+  if (tensor) b.addTensor(H);   // the mirror of H through a wall has the same squares
+  return !positiveBits(m) | !positiveBits(rho) | !positiveBits(a) | !finiteBits(eps) | !finiteBits(p[0]) |
+         !finiteBits(p[1]) | !finiteBits(p[2]) | !finiteBits(vx) | !finiteBits(vy) | !finiteBits(vz);
+}
+// The same pass by itself, where something has to run between it and the update.
+__global__ void __launch_bounds__(256) endStepKernel(Fields F, long n, Grid g, int tensor, StepScratch* __restrict__ sc) {
+  NodeBounds b;
+  bool bad = false;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    double p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
+    Sym H{};
+    if (tensor) H = loadSym(F, F_HT_XX, i);
+    bad |= endNode(F, i, p, F.f[F_VX][i], F.f[F_VY][i], F.f[F_VZ][i], F.f[F_MASS][i], F.f[F_RHO][i], F.f[F_HINV][i],
+                   F.f[F_EPS][i], H, tensor != 0, g, b);
+  }
+  if (bad) atomicExch(&sc->bad, 1);
+  mergeBounds(b, tensor != 0, sc);
+}
+
 // The half-step update (mid) advances the current state and keeps its
 // beginning-of-step copy (state0); the full update advances state0 itself
 // (State::update after the reference's state.assign(state0)), eps already
@@ -1190,12 +1326,15 @@ __global__ void tensorExtentKernel(Fields F, long n) {
 // 1 IntegrateH (both updates increment H by DHDt), 2 FixedH (H never changes).
 // asphEnd (ASPHSmoothingScale): both updates integrate H with
 // IncrementASPHHtensor (fixShape / radialOnly forms) unless FixedH.
-template <bool TENSOR>
-__global__ void updateKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists,
+// ex: what the step wants done in the same pass (UpdateExtras); END: its end.
+template <bool TENSOR, bool END>
+__global__ void __launch_bounds__(256) updateKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists,
                              double mult, int mid, int gravity, int epsIncrement, int hUpdate, int totalEnergy,
-                             int crk, Fields32 P, Grid g, int asphEnd, int fixShape, int radialOnly) {
+                             int crk, Fields32 P, Grid g, int asphEnd, int fixShape, int radialOnly,
+                                                    UpdateExtras ex) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  NodeBounds bounds;
+  if (i < n) {
   const NodeListParams L = lists[list[i]];
   // state the update starts from
   const int bx = mid ? F_X : F_X0, bvx = mid ? F_VX : F_VX0;
@@ -1205,7 +1344,7 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
   const double vxOld = F.f[bvx][i], vyOld = F.f[bvx + 1][i], vzOld = F.f[bvx + 2][i];
   const double rhoOld = F.f[mid ? F_RHO : F_RHO0][i], hOld = F.f[mid ? F_HINV : F_HINV0][i];
   const double volOld = crk ? F.f[mid ? F_VOL : F_VOL0][i] : 0.0;
-  Sym HOld{};
+  Sym HOld{}, HNew{};
   if (TENSOR) HOld = loadSym(F, mid ? F_HT_XX : F_HT0_XX, i);
   double eps = F.f[mid || !epsIncrement ? F_EPS : F_EPS0][i];
   if (mid) {   // state0
@@ -1256,10 +1395,12 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
   const bool increment = mid || hUpdate == 1;
   if (hUpdate == 2) {   // FixedH: both copies hold the same H
     h = hOld;
+    HNew = HOld;
   } else if (TENSOR && asphEnd) {
     const Sym t = incrementASPHHtensor(HOld, loadSym(F, F_DHDTT_XX, i), mult, xOld, yOld, zOld, fixShape != 0,
                                        radialOnly != 0, hminInv, hmaxInv, L.hminratio);
     storeSym(F, F_HT_XX, i, t);
+    HNew = t;
     if (P.posh) storeExtent32(F, i, t);
     else storeExtent(F, i, t);
     h = F.f[F_HINV][i];
@@ -1274,6 +1415,7 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     }
     t = symBound(t, hmaxInv, hminInv);
     storeSym(F, F_HT_XX, i, t);
+    HNew = t;
     if (P.posh) storeExtent32(F, i, t);
     else storeExtent(F, i, t);
     h = F.f[F_HINV][i];
@@ -1311,132 +1453,32 @@ __global__ void updateKernel(Fields F, const int* __restrict__ list, long n, con
     P.posh[i] = make_float4(toFloatRN(x - ox), toFloatRN(y - oy), toFloatRN(z - oz), toFloatRN(h));
     P.velm[i] = make_float4(toFloatRN(vx), toFloatRN(vy), toFloatRN(vz), toFloatRN(F.f[F_MASS][i]));
     const float om = toFloatRN(F.f[F_OMEGA][i]);
-    P.thermo[i] = make_float4(toFloatRN(rho), toFloatRN(p), cs, om / (om * om + 1.0e-30f));
+    const float4 th = make_float4(toFloatRN(rho), toFloatRN(p), cs, om / (om * om + 1.0e-30f));
+    P.thermo[i] = th;
+    if (!TENSOR && ex.pair.on) P.pk[i] = pairRecord(th, ex.pair);
     if (TENSOR) writeTensorMirror(F, i, P, i);
     if (crk && P.vol) P.vol[i] = toFloatRN(F.f[F_VOL][i]);
   } else {
     eosNode(F, i, L);
   }
+  if (ex.copyQ) {   // ArtificialViscosityHandle::postStateUpdate
+    float v[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const double d = F.f[F_DVDX_XX + k][i];
+      F.f[F_DVDXQ_XX + k][i] = d;
+      v[k] = toFloatRN(d);
+    }
+    if (!TENSOR && ex.pair.on && ex.pair.limited) writeQGradient(P, i, v, ex.pair);
+  }
+  if (END) {
+    double p[3] = {x, y, z};
+    if (endNode(F, i, p, vx, vy, vz, F.f[F_MASS][i], rho, h, eps, HNew, TENSOR, g, bounds)) atomicExch(&ex.end->bad, 1);
+  }
+  }
+  if (END) mergeBounds(bounds, TENSOR, ex.end);
 }
 
-__global__ void eosKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  eosNode(F, i, lists[list[i]]);
-}
-
-// Boundary::setAllViolationNodes + enforceBoundary (PlanarBoundary.cc:153-190,
-// ReflectingBoundary.cc:465-473): nodes strictly outside a plane are mapped
-// back; reflecting walls also mirror the velocity.
-__device__ __forceinline__ bool fuzzyZero(double x) { return fabs(x) <= 1.0e-15 * fmax(1.0, fabs(x)); }
-// A signed integer with the order of the double x (for non-NaN x; -0 sorts
-// just below +0, which only sends a node at a wall to the exact test).
-__device__ __forceinline__ long long orderKey(double x) {
-  const long long b = __double_as_longlong(x);
-  return b >= 0 ? b : (b ^ 0x7fffffffffffffffLL);
-}
-// tensor: the H of a node mapped back through a reflecting wall is reflected
-// too (PlanarBoundary::updateViolationNodes -> enforceBoundary(Hfield),
-// (R H R).Symmetric()).
-__device__ __forceinline__ void enforceNode(Fields& F, long i, const Grid& g, int tensor) {
-  auto reflectH = [&](int a) {
-    if (!tensor) return;
-    if (a == 0) { F.f[F_HT_XY][i] = -F.f[F_HT_XY][i]; F.f[F_HT_XZ][i] = -F.f[F_HT_XZ][i]; }
-    else if (a == 1) { F.f[F_HT_XY][i] = -F.f[F_HT_XY][i]; F.f[F_HT_YZ][i] = -F.f[F_HT_YZ][i]; }
-    else { F.f[F_HT_XZ][i] = -F.f[F_HT_XZ][i]; F.f[F_HT_YZ][i] = -F.f[F_HT_YZ][i]; }
-  };
-  double* P[3] = {F.f[F_X], F.f[F_Y], F.f[F_Z]};
-  double* V[3] = {F.f[F_VX], F.f[F_VY], F.f[F_VZ]};
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const double lo = g.wallLo[a], hi = g.wallHi[a];
-    double p = P[a][i];
-    // Integer pre-test on order-preserving keys of the bit patterns: a node
-    // strictly inside (lo, hi) needs nothing, and the FP64 tests below (the
-    // FP64 pipe is narrow) run only for the few on or beyond a wall.
-    if (orderKey(p) > orderKey(lo) && orderKey(p) < orderKey(hi)) continue;
-    const double sdLo = p - lo, sdHi = hi - p;
-    if (g.kindLo[a] == AXIS_PERIODIC) {
-      if (sdLo < 0.0 && !fuzzyZero(sdLo)) p = imageCoord(p, 2, AXIS_PERIODIC, AXIS_PERIODIC, lo, hi);
-      else if (sdHi < 0.0 && !fuzzyZero(sdHi)) p = imageCoord(p, 1, AXIS_PERIODIC, AXIS_PERIODIC, lo, hi);
-      P[a][i] = p;
-    } else {
-      if (g.kindLo[a] == AXIS_REFLECT && sdLo < 0.0 && !fuzzyZero(sdLo)) {
-        p = imageCoord(p, 1, AXIS_REFLECT, g.kindHi[a], lo, hi);
-        P[a][i] = p;
-        V[a][i] = -V[a][i];
-        reflectH(a);
-      }
-      const double sdHi2 = hi - p;
-      if (g.kindHi[a] == AXIS_REFLECT && sdHi2 < 0.0 && !fuzzyZero(sdHi2)) {
-        p = imageCoord(p, 2, g.kindLo[a], AXIS_REFLECT, lo, hi);
-        P[a][i] = p;
-        V[a][i] = -V[a][i];
-        reflectH(a);
-      }
-    }
-  }
-}
-
-// Bit tests of the end-of-step check (integer pipe).
-__device__ __forceinline__ bool finiteBits(double x) {
-  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
-}
-__device__ __forceinline__ bool positiveBits(double x) {   // x > 0 and finite
-  const long long b = __double_as_longlong(x);
-  return b > 0 && b < 0x7ff0000000000000LL;
-}
-
-// End of the step in one pass: nodes outside a wall are mapped back, the state
-// is checked (finite, positive) and the bounds the next neighbour build needs
-// are taken (as boundsKernel; the comparisons on order keys).
-__global__ void __launch_bounds__(256) endStepKernel(Fields F, long n, Grid g, int tensor, StepScratch* __restrict__ sc) {
-  long long mn[4] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MAX};
-  long long mx[6] = {LLONG_MIN, LLONG_MIN, LLONG_MIN, 0, 0, 0};
-  bool bad = false;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    enforceNode(F, i, g, tensor);
-    const double a = F.f[F_HINV][i], p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
-    bad |= !positiveBits(F.f[F_MASS][i]) | !positiveBits(F.f[F_RHO][i]) | !positiveBits(a) | !finiteBits(F.f[F_EPS][i]) |
-           !finiteBits(p[0]) | !finiteBits(p[1]) | !finiteBits(p[2]) | !finiteBits(F.f[F_VX][i]) |
-           !finiteBits(F.f[F_VY][i]) | !finiteBits(F.f[F_VZ][i]);
-    mn[0] = min(mn[0], orderKey(a));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const long long o = orderKey(p[k]);
-      mn[1 + k] = min(mn[1 + k], o);
-      mx[k] = max(mx[k], o);
-    }
-    if (tensor) {
-      const Sym w = symInverse(loadSym(F, F_HT_XX, i));
-      mx[3] = max(mx[3], orderKey(sqrt(w.xx * w.xx + w.xy * w.xy + w.xz * w.xz)));
-      mx[4] = max(mx[4], orderKey(sqrt(w.xy * w.xy + w.yy * w.yy + w.yz * w.yz)));
-      mx[5] = max(mx[5], orderKey(sqrt(w.xz * w.xz + w.yz * w.yz + w.zz * w.zz)));
-    }
-  }
-  __shared__ long long sm[8][10];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 10; ++k) {
-    if (k >= 7 && !tensor) break;
-    long long v = k < 4 ? mn[k] : mx[k - 4];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long w = __shfl_xor_sync(0xffffffffu, v, o);
-      v = k < 4 ? min(v, w) : max(v, w);
-    }
-    if (lane == 0) sm[warp][k] = v;
-  }
-  if (bad) atomicExch(&sc->bad, 1);
-  __syncthreads();
-  if (threadIdx.x < (tensor ? 10 : 7)) {
-    const int k = threadIdx.x;
-    long long v = sm[0][k];
-    for (int w = 1; w < 8; ++w) v = k < 4 ? min(v, sm[w][k]) : max(v, sm[w][k]);
-    if (k < 4) atomicMin(&sc->bounds[k], v);
-    else atomicMax(&sc->bounds[k], v);
-  }
-}
 
 // SpheralConservation totals (SpheralConservation.py:54-150) in FP64:
 // mass, momentum, kinetic, thermal, gravitational (1/2 m phi).
@@ -1562,25 +1604,15 @@ inline unsigned gridFor(long n, int b) { return (unsigned)((n + b - 1) / b); }
 //==============================================================================
 // Launchers
 //==============================================================================
-void launchBounds(const Fields& F, long n, bool tensor, double* dScratch, int nScratch, double* dOut, cudaStream_t s,
-                  LaunchCounter* lc) {
-  int nb = (int)std::min<long>((n + 255) / 256, nScratch / kBoundsVals);
-  if (nb < 1) nb = 1;
-  boundsKernel<<<nb, 256, 0, s>>>(F, n, tensor ? 1 : 0, dScratch);
-  boundsFinalKernel<<<1, 256, 0, s>>>(dScratch, nb, dOut);
+void launchBounds(const Fields& F, long n, bool tensor, StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
+  resetScratchKernel<<<1, 1, 0, s>>>(sc);
+  boundsKernel<<<std::min(gridFor(n, 256), 1216u), 256, 0, s>>>(F, n, tensor ? 1 : 0, sc);
   lc->add(2);
 }
 void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
-                    cudaStream_t s, LaunchCounter* lc) {
-  cellKeyKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, keys, vals, cellc, sc);
+                    ClearedWords clear, cudaStream_t s, LaunchCounter* lc) {
+  cellKeyKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, keys, vals, cellc, sc, clear);
   lc->add(1);
-}
-// ArtificialViscosityHandle::postStateUpdate: the Q's DvDx = the hydro DvDx.
-__global__ void copyQGradientKernel(Fields F, long n) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) F.f[F_DVDXQ_XX + k][i] = F.f[F_DVDX_XX + k][i];
 }
 // FP32 mirror of the Q's DvDx for the mixed pair sweep.
 __global__ void qGradient32Kernel(Fields F, float4* __restrict__ dvq, long n) {
@@ -1593,14 +1625,11 @@ __global__ void qGradient32Kernel(Fields F, float4* __restrict__ dvq, long n) {
   dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
   dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
 }
-void launchCopyQGradient(Fields F, long n, cudaStream_t s, LaunchCounter* lc) {
-  copyQGradientKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n);
-  lc->add(1);
-}
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc) {
   qGradient32Kernel<<<gridFor(n, 256), 256, 0, s>>>(F, dvq, n);
   lc->add(1);
 }
+constexpr long kSplitPermute = 200000;
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
                    bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
@@ -1616,7 +1645,9 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
     add(F_NUM_CARRIED, tensor ? (int)F_VOL : (int)F_HIDEALT_XX);
     if (crk) add(F_VOL, F_NUM_PERMUTED);
   }
-  permuteKernel<<<gridFor(n, 256), 256, 0, s>>>(Fin, Fout, perm, origIn, origOut, listIn, listOut, cellIn, cellOut, n,
+  // a few blocks leave the SMs idle: spread the fields over more
+  const dim3 grid(gridFor(n, 256), n < kSplitPermute ? 9 : 1);
+  permuteKernel<<<grid, 256, 0, s>>>(Fin, Fout, perm, origIn, origOut, listIn, listOut, cellIn, cellOut, n,
                                                 sel, P, g, mirrors ? 1 : 0, sortedKeys, space, cellStart, cellEnd);
   lc->add(1);
 }
@@ -1693,18 +1724,22 @@ void launchTensorExtent(Fields F, long n, cudaStream_t s, LaunchCounter* lc) {
   tensorExtentKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n);
   lc->add(1);
 }
-void launchUpdate(Fields F, const int* list, long n, HydroParams hp, double mult,
-                  bool mid, bool gravity, const Fields32* mirror, const Grid& g, cudaStream_t s, LaunchCounter* lc) {
+void launchUpdate(Fields F, const int* list, long n, HydroParams hp, double mult, bool mid, bool gravity,
+                  const Fields32* mirror, const Grid& g, const UpdateExtras& ex, cudaStream_t s, LaunchCounter* lc) {
   const int epsInc = (mid || !hp.compatible) ? 1 : 0;
   Fields32 P{};
   if (mirror) P = *mirror;
-  if (hp.asph)
-    updateKernel<true><<<gridFor(n, 256), 256, 0, s>>>(F, list, n, hp.lists, mult, mid ? 1 : 0, gravity ? 1 : 0, epsInc,
-                                                       hp.hUpdate, hp.totalEnergy, 0, P, g, hp.asphEnd, hp.fixShape,
-                                                       hp.radialOnly);
-  else
-    updateKernel<false><<<gridFor(n, 256), 256, 0, s>>>(F, list, n, hp.lists, mult, mid ? 1 : 0, gravity ? 1 : 0,
-                                                        epsInc, hp.hUpdate, hp.totalEnergy, hp.crk, P, g, 0, 0, 0);
+#define SPH_UPD(T, E, CRK, AE, FS, RO)                                                                              \
+  updateKernel<T, E><<<gridFor(n, 256), 256, 0, s>>>(F, list, n, hp.lists, mult, mid ? 1 : 0, gravity ? 1 : 0,     \
+                                                     epsInc, hp.hUpdate, hp.totalEnergy, CRK, P, g, AE, FS, RO, ex)
+  if (hp.asph) {
+    if (ex.end) SPH_UPD(true, true, 0, hp.asphEnd, hp.fixShape, hp.radialOnly);
+    else SPH_UPD(true, false, 0, hp.asphEnd, hp.fixShape, hp.radialOnly);
+  } else {
+    if (ex.end) SPH_UPD(false, true, hp.crk, 0, 0, 0);
+    else SPH_UPD(false, false, hp.crk, 0, 0, 0);
+  }
+#undef SPH_UPD
   lc->add(1);
 }
 void launchASPHEnd(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,

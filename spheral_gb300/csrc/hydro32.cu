@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
 template <bool XSPH, bool COMPAT, bool MULTI, bool LIMQ, bool LEAN, bool MIR, int KERN, int L, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 P, const int* __restrict__ list, long n,
                                                              Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                                                             float* __restrict__ pacc) {
+                                                             float* __restrict__ pacc, HalfStep half) {
   constexpr int NT = KERN ? 1 : kTab32;
   __shared__ float4 ta[NT];
   __shared__ float2 tb[NT];
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   }
   a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
   a.deps = kahanValue(se, ce);
-  finalizePair32<KERN == 1>(F, i, MULTI ? li : list[i], a, ai, mi, rhoi, cnt, hp, t.herm);
+  finalizePair32<KERN == 1>(F, i, MULTI ? li : list[i], a, ai, mi, rhoi, cnt, hp, t.herm, half);
 }
 
 //------------------------------------------------------------------------------
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
 template <bool LIMQ, bool MIR, bool SPLINE, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32 P, const int* __restrict__ list,
                                                               long n, Grid g, NeighborLists nl, TableDev t,
-                                                              HydroParams hp, float* __restrict__ pacc) {
+                                                              HydroParams hp, float* __restrict__ pacc, HalfStep half) {
   __shared__ float4 tg[kTab32];   // (g0, g1, g2, w0)
   __shared__ float2 tw[SPLINE ? 1 : kTab32];
   for (int k = threadIdx.x; k <= hp.tableN1 + 1; k += blockDim.x) {
@@ -754,35 +754,18 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
 #pragma unroll
   for (int k = 0; k < 9; ++k) { a.D[k] = D[k]; a.M[k] = M[k]; }
   finalizeNode32<false>(F, i, list[i], a, cnt, hp, t.herm);
+  if (half.hi) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
 }
-
-// Per-node inputs of the isotropic pair loop: (rho, Omega^-1 P / rho^2,
-// -Cl c, 1 / (2 rho)), once per node instead of once per pair; with the
-// limited Q also the symmetric part of the Q's DvDx for h = r/2
-// (xx yy zz xy | xz yz, off-diagonal pairs summed), or for the exact form
-// (full) all nine components.  spline: times the cubic B-spline's A.
-__global__ void pairInputs32(Fields F, Fields32 P, long n, float Cl, int limitedQ, int spline, int full) {
+// The pair sweep's per-node inputs, where the update has not written them.
+__global__ void pairInputs32(Fields F, Fields32 P, long n, PairForm pf) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float4 th = P.thermo[i];
-  const float ir = __frcp_rn(th.x);
-  float pr = __fmul_rn(__fmul_rn(__fmul_rn(th.w, th.y), ir), ir), hir = 0.5f * ir;
-  if (spline) { pr = timesSplineA(pr); hir = timesSplineA(hir); }
-  P.pk[i] = make_float4(th.x, pr, __fmul_rn(-Cl, th.z), hir);
-  if (limitedQ) {
+  P.pk[i] = pairRecord(P.thermo[i], pf);
+  if (pf.limited) {
     float v[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) v[k] = toFloatRN(F.f[F_DVDXQ_XX + k][i]);
-    if (full) {
-      P.dvq[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
-      P.dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
-      P.dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
-      return;
-    }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) v[k] *= 0.25f;
-    P.dvq[2 * i] = make_float4(v[0], v[4], v[8], v[1] + v[3]);
-    P.dvq[2 * i + 1] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
+    writeQGradient(P, i, v, pf);
   }
 }
 
@@ -948,7 +931,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Field
 // LEAN: compensated sums fixed at compile time.
 template <bool TENSOR, bool LEAN, bool MIR, int KERN, int L, int U>
 __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
-                                                     TableDev t, HydroParams hp) {
+                                                     TableDev t, HydroParams hp, PairForm pf) {
   constexpr int NT = KERN ? 1 : kTab32;
   __shared__ float4 ta[NT];
   __shared__ float2 tb[NT];
@@ -997,7 +980,13 @@ __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields3
   float omega = 1.0f;
   if (cnt > 0) omega = fmaxf(1.0e-30f, -(gs - gc) / (3.0f * ((ws - wc) + (KERN ? 1.0f : (float)hp.W0))));
   F.f[F_OMEGA][i] = toDouble(omega);
-  P.thermo[i].w = omega / (omega * omega + 1.0e-30f);
+  const float iom = omega / (omega * omega + 1.0e-30f);
+  P.thermo[i].w = iom;
+  if (!TENSOR && pf.on) {
+    float4 th = P.thermo[i];
+    th.w = iom;
+    P.pk[i] = pairRecord(th, pf);
+  }
 }
 
 //------------------------------------------------------------------------------
@@ -1092,17 +1081,10 @@ __global__ void dtInitKernel(StepScratch* __restrict__ sc) {
 // to FP32 and the FP32 pair acceleration; the weighted shares are summed and
 // applied to the specific energy in FP64.
 //------------------------------------------------------------------------------
-__global__ void halfStepVelocityKernel(Fields F, long n, double hdt, float4* __restrict__ vhi,
-                                       float4* __restrict__ vlo) {
+__global__ void halfStepVelocityKernel(Fields F, long n, HalfStep half) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  // v12 = v + a dt/2 in FP64, stored as an unevaluated float pair hi + lo
-  const double x = F.f[F_VX0][i] + F.f[F_DVDT_X][i] * hdt;
-  const double y = F.f[F_VY0][i] + F.f[F_DVDT_Y][i] * hdt;
-  const double z = F.f[F_VZ0][i] + F.f[F_DVDT_Z][i] * hdt;
-  const float hx = (float)x, hy = (float)y, hz = (float)z;
-  vhi[i] = make_float4(hx, hy, hz, (float)F.f[F_DEPSDT][i]);
-  vlo[i] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.0f);
+  halfStepVelocity(F, i, F.f[F_DVDT_X][i], F.f[F_DVDT_Y][i], F.f[F_DVDT_Z][i], F.f[F_DEPSDT][i], half);
 }
 
 // B: slots per batch (the gathers and pair-acceleration reads in flight per
@@ -1208,12 +1190,30 @@ void launchPrepareFP32(Fields F, Fields32 F32, long n, Grid g, cudaStream_t s, L
 }
 
 constexpr int kDensU = 2, kGradhU = 4;   // slots per iteration of the density and grad-h sweeps
+// The lean path: one NodeList, compensated sums, the standard Q, no tensile
+// correction, compatible energy, no XSPH.  From kExactNodes on it keeps the
+// earlier arithmetic; below it the reduced one, with the spline in registers.
+static bool leanPair(const HydroParams& hp) {
+  return hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.plainSums && !hp.xsph && hp.compatible && hp.numLists == 1;
+}
+static bool exactPair(long n, const HydroParams& hp) { return leanPair(hp) && n >= kExactNodes; }
+static bool reducedPair(long n, const HydroParams& hp) { return leanPair(hp) && n < kExactNodes && hp.cubicSpline; }
+PairForm pairForm32(long n, const HydroParams& hp) {
+  PairForm f;
+  f.on = 1;
+  f.Cl = (float)hp.Cl;
+  f.spline = reducedPair(n, hp) ? 1 : 0;
+  f.limited = hp.limitedQ;
+  f.full = exactPair(n, hp) ? 1 : 0;
+  return f;
+}
+
 // variant (isotropic, lean path, one lane per node, standard Q): two slots per
 // iteration at 4 blocks per SM (even, <= 128 registers) or 5 (odd, <= 102).
 // At 2.1 M nodes 1741 / 1620 us, the limited Q spills at 102 (180 / 242 us at
 // 104,000 nodes); one slot per iteration ran 1800, four slots at 3 blocks 1890.
 void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                    HydroParams hp, float* pacc, int variant, cudaStream_t s,
+                    HydroParams hp, float* pacc, int variant, bool inputs, const HalfStep& half, cudaStream_t s,
                     LaunchCounter* lc) {
   const int b = 128;
   const bool multi = hp.numLists > 1;
@@ -1245,22 +1245,22 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
       else { if (hp.limitedQ) SPH_PAIR32T(false, false, true); else SPH_PAIR32T(false, false, false); }
     }
 #undef SPH_PAIR32T
-    lc->add(1);
+    if (half.hi) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, half);
+    lc->add(half.hi ? 2 : 1);
     return;
   }
-  const bool plainPath = lean && !hp.xsph && hp.compatible && !multi;
-  const bool exact = plainPath && n >= kExactNodes, fast = plainPath && !exact && hp.cubicSpline;
-  pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, (float)hp.Cl, hp.limitedQ, fast ? 1 : 0, exact ? 1 : 0);
+  const bool exact = exactPair(n, hp), fast = reducedPair(n, hp);
+  if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
   const int L = lanesPair(n);
 #define SPH_ISO(X, C, M, Q, LE, MI, K, LA, U, MB) \
-  pairKernelIso32<X, C, M, Q, LE, MI, K, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc)
+  pairKernelIso32<X, C, M, Q, LE, MI, K, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
   if (exact) {
 #define SPH_LEAN(Q, MI)                                                                                              \
   do {                                                                                                               \
-    if (!hp.cubicSpline) pairKernelLean32<Q, MI, false, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else if (Q) pairKernelLean32<Q, MI, true, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else if (variant & 1) pairKernelLean32<Q, MI, true, 3, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else pairKernelLean32<Q, MI, true, 4, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);       \
+    if (!hp.cubicSpline) pairKernelLean32<Q, MI, false, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
+    else if (Q) pairKernelLean32<Q, MI, true, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
+    else if (variant & 1) pairKernelLean32<Q, MI, true, 3, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
+    else pairKernelLean32<Q, MI, true, 4, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half);       \
   } while (0)
     if (hasMirrors(g)) { if (hp.limitedQ) SPH_LEAN(true, true); else SPH_LEAN(false, true); }
     else { if (hp.limitedQ) SPH_LEAN(true, false); else SPH_LEAN(false, false); }
@@ -1290,7 +1290,7 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
 #undef SPH_ISOG
   }
 #undef SPH_ISO
-  lc->add(2);
+  lc->add(inputs ? 1 : 2);
 }
 
 // Slots per iteration of the density and grad-h sweeps: see densityKernel32.
@@ -1333,9 +1333,9 @@ void launchSumDensityFP32(Fields F, Fields32 F32, const int* list, long n, Grid 
 }
 
 void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                     cudaStream_t s, LaunchCounter* lc) {
+                     const PairForm& pf, cudaStream_t s, LaunchCounter* lc) {
   const int L = lanesSweep(n);
-#define SPH_GH(T, LE, MI, K, LA, U) gradhKernel32<T, LE, MI, K, LA, U><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, F32, n, g, nl, t, hp)
+#define SPH_GH(T, LE, MI, K, LA, U) gradhKernel32<T, LE, MI, K, LA, U><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, F32, n, g, nl, t, hp, pf)
   if (!hp.plainSums && (n >= kExactNodes || hp.asph)) {
 #define SPH_GX(LA)                                                    \
   do {                                                                \
@@ -1377,8 +1377,9 @@ void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Neigh
 }
 
 void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
-                                float4* vlo, double dt, int variant, cudaStream_t s, LaunchCounter* lc) {
-  halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, 0.5 * dt, vhi, vlo);
+                                float4* vlo, double dt, int variant, bool half, cudaStream_t s,
+                                LaunchCounter* lc) {
+  if (half) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, HalfStep{vhi, vlo, 0.5 * dt});
   const int L = lanesEnergy(n);
 #define SPH_EN(B, LA)                                                                                                    \
   if (hasMirrors(g)) energyKernel32<true, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt); \
@@ -1394,7 +1395,7 @@ void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, cons
   if (variant == 1) { SPH_ENL(8) } else if (variant == 2) { SPH_ENL(2) } else { SPH_ENL(4) }
 #undef SPH_ENL
 #undef SPH_EN
-  lc->add(2);
+  lc->add(half ? 2 : 1);
 }
 
 void launchDensityDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,

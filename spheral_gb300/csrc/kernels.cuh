@@ -38,15 +38,19 @@ struct StepScratch {
 };
 
 // Reductions ------------------------------------------------------------------
-// out[0] = min hinv, out[1..3] = min x,y,z, out[4..6] = max x,y,z,
-// out[7..9] = (tensor H) max over nodes of sqrt((H^-2)_aa) per axis, else 0
+// sc->bounds: order keys of min hinv; min x,y,z; max x,y,z; (tensor H) max over
+// nodes of (H^-2)_aa per axis, else 0.  NaN is passed over.
 constexpr int kBoundsVals = 10;
-void launchBounds(const Fields& F, long n, bool tensor, double* dScratch, int nScratch, double* dOut, cudaStream_t s,
-                  LaunchCounter* lc);
+void launchBounds(const Fields& F, long n, bool tensor, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 
 // Neighbour build -------------------------------------------------------------
+// Words that the first kernel of the build zeroes for the later ones.
+struct ClearedWords {
+  unsigned* p[2];
+  long long n[2];
+};
 void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
-                    cudaStream_t s, LaunchCounter* lc);   // resets *sc
+                    ClearedWords clear, cudaStream_t s, LaunchCounter* lc);   // resets *sc
 // carriedOnly: move only the state and the derivatives the next step reads
 // before recomputing them (the step rewrites every other field before it
 // returns); otherwise every permuted field.  The same pass writes the cells'
@@ -57,8 +61,7 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
                    bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
                    const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, cudaStream_t s,
                    LaunchCounter* lc);
-// The limited Q's DvDx <- the hydro DvDx; and its FP32 mirror (3 float4 per node).
-void launchCopyQGradient(Fields F, long n, cudaStream_t s, LaunchCounter* lc);
+// FP32 mirror of the limited Q's DvDx (3 float4 per node).
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc);
 // Work items of the group-cooperative search: the chunks of up to `width` (8,
 // 16 or 32) consecutive nodes of a cell, their first nodes, each cell's first
@@ -98,14 +101,31 @@ constexpr int kPairVariantsMax = 4;   // values sphgpu_set_pair_variant takes (a
 constexpr int kRetuneAfter = 2;    // uses between an autotuner's first timing and its one retiming
 constexpr int kPairVariantsTensor = 4;   // of its tensor-H (ASPH) path
 constexpr int kPairVariantsCRK = 2;      // of the mixed CRKSPH pair kernel
+// Form of the isotropic pair sweep's per-node inputs (Fields32::pk, dvq).
+struct PairForm {
+  int on = 0;        // written by the update (and kept current by the grad-h sweep)
+  float Cl = 0.f;
+  int spline = 0;    // times the cubic B-spline's normalisation
+  int limited = 0;   // limited Q: its DvDx too
+  int full = 0;      // all nine components of it
+};
+PairForm pairForm32(long n, const HydroParams& hp);
+// The energy sweep's half-step velocities, written by the pair sweep (hi null:
+// not wanted): v0 + DvDt hdt as hi + lo, hi.w = DepsDt.
+struct HalfStep {
+  float4* hi = nullptr;
+  float4* lo = nullptr;
+  double hdt = 0.0;
+};
+// inputs: pk and dvq are already those of the state being evaluated.
 void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                    HydroParams hp, float* pacc, int variant, cudaStream_t s,
+                    HydroParams hp, float* pacc, int variant, bool inputs, const HalfStep& half, cudaStream_t s,
                     LaunchCounter* lc);
 void launchPrepareFP32(Fields F, Fields32 F32, long n, Grid g, cudaStream_t s, LaunchCounter* lc);
 void launchSumDensityFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                           HydroParams hp, cudaStream_t s, LaunchCounter* lc);
 void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
-                     cudaStream_t s, LaunchCounter* lc);
+                     const PairForm& pf, cudaStream_t s, LaunchCounter* lc);
 void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
                   double maxNperh, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 // Mixed mode: density sum and dt vote fused in one sweep; the vote goes to
@@ -120,8 +140,9 @@ void launchDt(Fields F, const int* list, long n, Grid g, NeighborLists nl, Hydro
 // variant: slots per batch of the sweep, 0 -> 4, 1 -> 8, 2 -> 2 (the same
 // result for every variant; picked by the autotuner).
 constexpr int kEnergyVariants = 3;
+// half: launch the half-step velocities too (else the pair sweep wrote them).
 void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
-                                float4* vlo, double dt, int variant, cudaStream_t s, LaunchCounter* lc);
+                                float4* vlo, double dt, int variant, bool half, cudaStream_t s, LaunchCounter* lc);
 // CRKSPH (crk.cu): the RK volumes (RKCorrections::preStepInitialize), the CRK
 // mass density sum (CRKSPHBase::preStepInitialize), the LinearOrder
 // corrections (RKCorrections::initialize) and the CRKSPH pair loop with the
@@ -154,8 +175,14 @@ void launchRadius0(Fields F, long n, cudaStream_t s, LaunchCounter* lc);
 // timeAdvanceOnly increment with multiplier; else full update (eps
 // already advanced by the compatible-energy sweep when compatible).  mirror:
 // also refresh the FP32 mirrors of the new state (mixed mode), cells of grid g.
-void launchUpdate(Fields F, const int* list, long n, HydroParams hp, double mult,
-                  bool mid, bool gravity, const Fields32* mirror, const Grid& g, cudaStream_t s, LaunchCounter* lc);
+// What the update takes along where the step wants it.
+struct UpdateExtras {
+  PairForm pair;        // half step: the inputs of the mixed pair sweep (pair.on)
+  int copyQ = 0;        // the limited Q's DvDx <- the hydro DvDx
+  StepScratch* end = nullptr;   // full step: walls, state check and bounds (launchEndStep)
+};
+void launchUpdate(Fields F, const int* list, long n, HydroParams hp, double mult, bool mid, bool gravity,
+                  const Fields32* mirror, const Grid& g, const UpdateExtras& ex, cudaStream_t s, LaunchCounter* lc);
 // ASPHSmoothingScale end of step: zeroth moment, IdealH and limits of H
 // (P.posh non-null: the mixed mode's FP32 extents and mirrors are refreshed).
 void launchASPHEnd(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,

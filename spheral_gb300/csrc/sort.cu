@@ -271,14 +271,19 @@ size_t radixSortWorkspaceBytes(long n) {
   return ((size_t)kMaxDigits * 256 + 64 + (size_t)kMaxDigits * nb * 256) * sizeof(unsigned);
 }
 
+size_t radixSortClearedWords(long n, int bits) {
+  const long nb = (n + kSortTile - 1) / kSortTile;
+  return (size_t)kMaxDigits * 256 + 64 + (size_t)((bits + 7) / 8) * nb * 256;
+}
+
 template <typename K>
 void radixSortPairs(K*& keys, int*& vals, K*& keysAlt, int*& valsAlt, long n, int bits, void* workspace, int* timeout,
-                    cudaStream_t s, LaunchCounter* lc) {
+                    bool cleared, cudaStream_t s, LaunchCounter* lc) {
   if (n <= 1) return;
   const long nb = (n + kSortTile - 1) / kSortTile;
   const int digits = (bits + 7) / 8;
   const SortWs w = sortWs(workspace);
-  cudaMemsetAsync(workspace, 0, ((size_t)kMaxDigits * 256 + 64 + (size_t)digits * nb * 256) * sizeof(unsigned), s);
+  if (!cleared) cudaMemsetAsync(workspace, 0, radixSortClearedWords(n, bits) * sizeof(unsigned), s);
   radixCountKernel<K><<<(unsigned)std::min<long>(nb, 1216), kSortThreads, 0, s>>>(keys, n, digits, w.hist);
   for (int d = 0; d < digits; ++d) {
     radixPassKernel<K><<<(unsigned)nb, kSortThreads, 0, s>>>(keys, vals, n, 8 * d, w.hist + 256 * d, w.ticket + d,
@@ -288,9 +293,9 @@ void radixSortPairs(K*& keys, int*& vals, K*& keysAlt, int*& valsAlt, long n, in
   }
   if (lc) lc->add(1 + digits);
 }
-template void radixSortPairs<uint32_t>(uint32_t*&, int*&, uint32_t*&, int*&, long, int, void*, int*, cudaStream_t,
-                                       LaunchCounter*);
-template void radixSortPairs<uint64_t>(uint64_t*&, int*&, uint64_t*&, int*&, long, int, void*, int*, cudaStream_t,
-                                       LaunchCounter*);
+template void radixSortPairs<uint32_t>(uint32_t*&, int*&, uint32_t*&, int*&, long, int, void*, int*, bool,
+                                       cudaStream_t, LaunchCounter*);
+template void radixSortPairs<uint64_t>(uint64_t*&, int*&, uint64_t*&, int*&, long, int, void*, int*, bool,
+                                       cudaStream_t, LaunchCounter*);
 
 }  // namespace sph
