@@ -967,7 +967,7 @@ double step(sphgpu_ctx* c, double maxTime) {
   HalfStep half;
   if (c->fp32() && c->cfg.compatible_energy) {
     c->v12.ensure(c->n * 2 * sizeof(float4));
-    if (!c->hp.crk && !c->xfn) half = HalfStep{c->v12.as<float4>(), c->v12.as<float4>() + c->n, hdt};
+    if (!c->hp.crk && !c->xfn) half = HalfStep{c->v12.as<float4>(), hdt};
   }
   evalDerivs(c, isoPair, half);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
   exchangePoint(c, SPHGPU_EXCHANGE_DERIVS);          // the halo's accelerations and energy rates
@@ -989,8 +989,7 @@ double step(sphgpu_ctx* c, double maxTime) {
         for (int t = 0; t < 2 * kEnergyVariants; ++t) {   // two rounds, best time per variant
           const int v = t % kEnergyVariants;
           CUDA_OK(cudaEventRecord(e0, c->stream));
-          launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(),
-                                     c->v12.as<float4>() + c->n, 0.0, v, !half.hi, c->stream, &c->lc);
+          launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(), 0.0, v, !half.v, c->stream, &c->lc);
           CUDA_OK(cudaEventRecord(e1, c->stream));
           CUDA_OK(cudaEventSynchronize(e1));
           c->check();
@@ -1004,8 +1003,7 @@ double step(sphgpu_ctx* c, double maxTime) {
         c->energyTunedN = c->n;
         c->energyRetuneAt = retune ? -1 : c->energyEvals + kRetuneAfter;
       }
-      launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(),
-                                 c->v12.as<float4>() + c->n, dt, c->energyVariant, !half.hi, c->stream, &c->lc);
+      launchCompatibleEnergyFP32(c->F, c->n, c->grid, c->nl(), c->pacc.as<float>(), c->v12.as<float4>(), dt, c->energyVariant, !half.v, c->stream, &c->lc);
     }
     else {
       c->v12.ensure(c->n * 4 * sizeof(double));

@@ -724,6 +724,19 @@ __device__ __forceinline__ void finalizeNode32(Fields& F, long i, int li, const 
   F.f[F_HIDEAL][i] = fmin(L.hminInv, fmax(L.hmaxInv, hid));
 }
 
+// A 32-byte record in one load (p a multiple of 32 bytes): for a gather half
+// the L1 requests of two 16-byte loads.
+struct Rec32B {
+  float4 a, b;
+};
+__device__ __forceinline__ Rec32B load32B(const float4* p) {
+  Rec32B r;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+      : "l"(p));
+  return r;
+}
+
 // v12 = v0 + a dt/2 of the compatible-energy sweep, formed in FP64 and stored
 // as an unevaluated float pair hi + lo.
 __device__ __forceinline__ void halfStepVelocity(const Fields& F, long i, double ax, double ay, double az, double deps,
@@ -732,8 +745,8 @@ __device__ __forceinline__ void halfStepVelocity(const Fields& F, long i, double
   const double y = F.f[F_VY0][i] + ay * half.hdt;
   const double z = F.f[F_VZ0][i] + az * half.hdt;
   const float hx = (float)x, hy = (float)y, hz = (float)z;
-  half.hi[i] = make_float4(hx, hy, hz, (float)deps);
-  half.lo[i] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.0f);
+  half.v[2 * i] = make_float4(hx, hy, hz, (float)deps);
+  half.v[2 * i + 1] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.0f);
 }
 // Per-node inputs of the isotropic pair sweep: (rho, Omega^-1 P / rho^2, -Cl c,
 // 1 / (2 rho)), once per node instead of once per pair.
@@ -824,7 +837,7 @@ __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSu
   const double deps = a.deps * toDouble(Hdeti * ai);
   F.f[F_DEPSDT][i] =
       hp.totalEnergy ? toDouble(mi) * ((vxi * a.dvx + vyi * a.dvy + vzi * a.dvz) + deps) : deps;
-  if (half.hi) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
+  if (half.v) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
   put(F_MAXQ, rhoi * a.maxE);
   put(F_EFFQ, 2.0f * rhoi * Hdeti * a.ve);
   float xw = a.xw;

@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
 #pragma unroll
   for (int k = 0; k < 9; ++k) { a.D[k] = D[k]; a.M[k] = M[k]; }
   finalizeNode32<false>(F, i, list[i], a, cnt, hp, t.herm);
-  if (half.hi) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
+  if (half.v) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
 }
 // The pair sweep's per-node inputs, where the update has not written them.
 __global__ void pairInputs32(Fields F, Fields32 P, long n, PairForm pf) {
@@ -1092,7 +1092,7 @@ __global__ void halfStepVelocityKernel(Fields F, long n, HalfStep half) {
 // L lanes per node.
 template <bool MIR, int B, int L>
 __global__ void __launch_bounds__(sweepBlock(L)) energyKernel32(Fields F, long n, Grid g, NeighborLists nl,
-                                                      const float4* __restrict__ vhi, const float4* __restrict__ vlo,
+                                                      const float4* __restrict__ v12,
                                                       const float* __restrict__ pacc, double dt) {
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
   const int sub = threadIdx.x % L;
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) energyKernel32(Fields F, long n
   int ci[3];
   unpackCell(nl.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
-  const float4 hi = vhi[i], lo = vlo[i];
+  const float4 hi = v12[2 * i], lo = v12[2 * i + 1];
   const float d0i = hi.w;
   const float feps = (float)DBL_EPSILON;
   float s = 0.0f, c = 0.0f;
@@ -1146,15 +1146,14 @@ __global__ void __launch_bounds__(sweepBlock(L)) energyKernel32(Fields F, long n
   int q = 0;
   for (; q + B <= mine; q += B) {
     uint32_t e[B];
-    float4 H[B], Lo[B];
+    Rec32B v[B];
     float p[B][3];
 #pragma unroll
     for (int u = 0; u < B; ++u) e[u] = en[u];
 #pragma unroll
     for (int u = 0; u < B; ++u) {
       const uint32_t j = e[u] & kIndexMask;
-      H[u] = vhi[j];
-      Lo[u] = vlo[j];
+      v[u] = load32B(v12 + 2 * (size_t)j);
 #pragma unroll
       for (int k = 0; k < 3; ++k) p[u][k] = pa[3 * u * ST + 32 * k];
     }
@@ -1164,12 +1163,13 @@ __global__ void __launch_bounds__(sweepBlock(L)) energyKernel32(Fields F, long n
     for (int u = 0; u < B; ++u)
       if (q + B + u < mine) en[u] = nb[u * ST];
 #pragma unroll
-    for (int u = 0; u < B; ++u) slot(e[u], H[u], Lo[u], p[u][0], p[u][1], p[u][2]);
+    for (int u = 0; u < B; ++u) slot(e[u], v[u].a, v[u].b, p[u][0], p[u][1], p[u][2]);
   }
   for (; q < mine; ++q, nb += ST, pa += 3 * ST) {
     const uint32_t ent = nb[0];
     const uint32_t j = ent & kIndexMask;
-    slot(ent, vhi[j], vlo[j], pa[0], pa[32], pa[64]);
+    const Rec32B v = load32B(v12 + 2 * (size_t)j);
+    slot(ent, v.a, v.b, pa[0], pa[32], pa[64]);
   }
   if (L > 1) {
     laneSumKahan<L>(s, c);
@@ -1245,8 +1245,8 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
       else { if (hp.limitedQ) SPH_PAIR32T(false, false, true); else SPH_PAIR32T(false, false, false); }
     }
 #undef SPH_PAIR32T
-    if (half.hi) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, half);
-    lc->add(half.hi ? 2 : 1);
+    if (half.v) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, half);
+    lc->add(half.v ? 2 : 1);
     return;
   }
   const bool exact = exactPair(n, hp), fast = reducedPair(n, hp);
@@ -1376,14 +1376,14 @@ void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Neigh
   lc->add(2);
 }
 
-void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
-                                float4* vlo, double dt, int variant, bool half, cudaStream_t s,
+void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* v12,
+                                double dt, int variant, bool half, cudaStream_t s,
                                 LaunchCounter* lc) {
-  if (half) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, HalfStep{vhi, vlo, 0.5 * dt});
+  if (half) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, HalfStep{v12, 0.5 * dt});
   const int L = lanesEnergy(n);
 #define SPH_EN(B, LA)                                                                                                    \
-  if (hasMirrors(g)) energyKernel32<true, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt); \
-  else energyKernel32<false, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, vhi, vlo, pacc, dt)
+  if (hasMirrors(g)) energyKernel32<true, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, v12, pacc, dt); \
+  else energyKernel32<false, B, LA><<<gridFor(n * LA, sweepBlock(LA)), sweepBlock(LA), 0, s>>>(F, n, g, nl, v12, pacc, dt)
 #define SPH_ENL(B)                 \
   switch (L) {                     \
     case 1: SPH_EN(B, 1); break;   \

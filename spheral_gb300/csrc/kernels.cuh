@@ -110,11 +110,10 @@ struct PairForm {
   int full = 0;      // all nine components of it
 };
 PairForm pairForm32(long n, const HydroParams& hp);
-// The energy sweep's half-step velocities, written by the pair sweep (hi null:
-// not wanted): v0 + DvDt hdt as hi + lo, hi.w = DepsDt.
+// The energy sweep's half-step velocities v0 + DvDt hdt, written by the pair
+// sweep (v null: not wanted): (hi, DepsDt), (lo, -) per node.
 struct HalfStep {
-  float4* hi = nullptr;
-  float4* lo = nullptr;
+  float4* v = nullptr;
   double hdt = 0.0;
 };
 // inputs: pk and dvq are already those of the state being evaluated.
@@ -141,8 +140,8 @@ void launchDt(Fields F, const int* list, long n, Grid g, NeighborLists nl, Hydro
 // result for every variant; picked by the autotuner).
 constexpr int kEnergyVariants = 3;
 // half: launch the half-step velocities too (else the pair sweep wrote them).
-void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* vhi,
-                                float4* vlo, double dt, int variant, bool half, cudaStream_t s, LaunchCounter* lc);
+void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, const float* pacc, float4* v12,
+                                double dt, int variant, bool half, cudaStream_t s, LaunchCounter* lc);
 // CRKSPH (crk.cu): the RK volumes (RKCorrections::preStepInitialize), the CRK
 // mass density sum (CRKSPHBase::preStepInitialize), the LinearOrder
 // corrections (RKCorrections::initialize) and the CRKSPH pair loop with the
