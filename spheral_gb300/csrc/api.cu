@@ -707,7 +707,7 @@ void settleOmega(sphgpu_ctx* c) {
 void ensureQMirror(sphgpu_ctx* c) {
   if (c->fp32() && c->hp.limitedQ) c->dvq.ensure((size_t)c->n * 3 * sizeof(float4));
 }
-// inputs: the isotropic mixed pair sweep's per-node inputs are already those of
+// inputs: the mixed SPH pair sweep's per-node inputs are already those of
 // this state; half: the energy sweep's half-step velocities, wanted from it.
 void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}) {
   ensurePacc(c);
@@ -947,10 +947,10 @@ double step(sphgpu_ctx* c, double maxTime) {
   // and the pair sweep's per-node inputs; an exchange between them and the pair
   // sweep changes the halo's, so they are then formed at the sweep.
   const Fields32 m32 = c->f32();
-  const bool isoPair = c->fp32() && !c->hp.asph && !c->hp.crk && !c->xfn;
+  const bool formed = c->fp32() && !c->hp.crk && !c->xfn;
   UpdateExtras ex;
   ex.copyQ = c->hp.limitedQ;
-  if (isoPair) ex.pair = pairForm32(c->n, c->hp);
+  if (formed) ex.pair = pairForm32(c->n, c->hp);
   ensureQMirror(c);
   {
     Scope sc(c->prof, "update");   // the half-step update also saves state0
@@ -969,7 +969,7 @@ double step(sphgpu_ctx* c, double maxTime) {
     c->v12.ensure(c->n * 2 * sizeof(float4));
     if (!c->hp.crk && !c->xfn) half = HalfStep{c->v12.as<float4>(), hdt};
   }
-  evalDerivs(c, isoPair, half);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
+  evalDerivs(c, formed, half);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
   exchangePoint(c, SPHGPU_EXCHANGE_DERIVS);          // the halo's accelerations and energy rates
   if (c->cfg.compatible_energy) {
     Scope sc(c->prof, "energy");

@@ -1455,7 +1455,7 @@ __global__ void __launch_bounds__(256) updateKernel(Fields F, const int* __restr
     const float om = toFloatRN(F.f[F_OMEGA][i]);
     const float4 th = make_float4(toFloatRN(rho), toFloatRN(p), cs, om / (om * om + 1.0e-30f));
     P.thermo[i] = th;
-    if (!TENSOR && ex.pair.on) P.pk[i] = pairRecord(th, ex.pair);
+    if (ex.pair.on) P.pk[i] = pairRecord(th, ex.pair);
     if (TENSOR) writeTensorMirror(F, i, P, i);
     if (crk && P.vol) P.vol[i] = toFloatRN(F.f[F_VOL][i]);
   } else {

@@ -756,6 +756,174 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
   finalizeNode32<false>(F, i, list[i], a, cnt, hp, t.herm);
   if (half.v) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
 }
+
+//------------------------------------------------------------------------------
+// The ASPH pair loop (tensor H) of the lean path, in the arithmetic of
+// pairKernelFP32<TENSOR>: the same values in every sum the state reads.  What
+// bounds both is the L1 data pipe: five 16-byte gathers per slot and the table.
+// Here one 16-byte entry per side holds W' (W, which feeds only massDensitySum,
+// normalization and effViscousPressure, is the spline in registers or the
+// second table), and what depends on one node comes formed (Fields32::pk).
+// L lanes per node, U slots per iteration.
+//------------------------------------------------------------------------------
+struct PairRecTensor {
+  float4 p, v, k, a, b;
+};
+template <bool MIR, bool SPLINE, int L, int U, int MINB>
+__global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields32 P, const int* __restrict__ list,
+                                                                long n, Grid g, NeighborLists nl, TableDev t,
+                                                                HydroParams hp, float* __restrict__ pacc,
+                                                                HalfStep half) {
+  __shared__ float4 tg[kTab32];   // (g0, g1, g2, w0)
+  __shared__ float2 tw[SPLINE ? 1 : kTab32];
+  for (int k = threadIdx.x; k <= hp.tableN1 + 1; k += blockDim.x) {
+    const bool in = k <= hp.tableN1;
+    const float4 A = in ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 B = in ? t.p32b[k] : make_float2(0.f, 0.f);
+    tg[k] = make_float4(A.w, B.x, B.y, A.x);
+    if (!SPLINE) tw[k] = make_float2(A.y, A.z);
+  }
+  __syncthreads();
+  const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x % L;
+  const bool live = node < n;
+  if (L == 1 && !live) return;
+  const long i = live ? node : n - 1;
+  const int N1 = hp.tableN1;
+  const float invStep = (float)(1.0 / hp.tableXstep);
+  int ci[3];
+  unpackCell(P.cell[i], ci);
+  const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
+  const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
+  const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i], hi0 = P.hten[2 * i], hi1 = P.hten[2 * i + 1];
+  const float mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w, Hdeti = hi1.z;
+  const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
+  float sw = 0.f, smw = 0.f, sve = 0.f, maxE = 0.f;
+  float sdx = 0.f, cdx = 0.f, sdy = 0.f, cdy = 0.f, sdz = 0.f, cdz = 0.f, se = 0.f, ce = 0.f;
+  float gx = 0.f, gy = 0.f, gz = 0.f, m0 = 0.f, m1x = 0.f, m1y = 0.f, m1z = 0.f;
+  float D[9], M[9], m2[6];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { D[k] = 0.f; M[k] = 0.f; }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) m2[k] = 0.f;
+  const int cnt = live ? nl.count[i] : 0;
+  float* out = pacc + paccSlot(nbSlot(i, 0, nl.cap) + 32 * sub);
+  laneSlots<L, U, PairRecTensor>(
+      nl, i, sub, cnt,
+      [&](uint32_t j, PairRecTensor& r) {
+        r.p = P.posh[j];
+        r.v = P.velm[j];
+        r.k = P.pk[j];
+        r.a = P.hten[2 * j];
+        r.b = P.hten[2 * j + 1];
+      },
+      [&](uint32_t ent, const PairRecTensor& q) {
+        float rx, ry, rz;
+        relSepEntry<MIR>(pi, q.p, ent, mm, cx, cy, cz, rx, ry, rz);
+        float vxj = q.v.x, vyj = q.v.y, vzj = q.v.z;
+        float4 hj0 = q.a, hj1 = q.b;
+        if (MIR) {   // velocity and H_j through the mirrors of the entry
+          const uint32_t mq = (ent >> kIndexBits) & mm;
+          mirrorVel(mq, vxj, vyj, vzj);
+          if (mq) {
+            const float sx = (mq & 3u) ? -1.f : 1.f, sy = (mq & 12u) ? -1.f : 1.f, sz = (mq & 48u) ? -1.f : 1.f;
+            hj0.y *= sx * sy;
+            hj0.z *= sx * sz;
+            hj1.x *= sy * sz;
+          }
+        }
+        const float mj = q.v.w, rhoj = q.k.x, Prhoj = q.k.y, mClcj = q.k.z, hirj = q.k.w;
+        float eix, eiy, eiz, ejx, ejy, ejz;
+        symDot32(hi0, hi1, rx, ry, rz, eix, eiy, eiz);
+        symDot32(hj0, hj1, rx, ry, rz, ejx, ejy, ejz);
+        const float e2i = __fmaf_rn(eiz, eiz, __fmaf_rn(eiy, eiy, __fmul_rn(eix, eix)));
+        const float e2j = __fmaf_rn(ejz, ejz, __fmaf_rn(ejy, ejy, __fmul_rn(ejx, ejx)));
+        const float ri = rsqrtf(fmaxf(e2i, 1.0e-30f)), rj = rsqrtf(fmaxf(e2j, 1.0e-30f));
+        const float etai = __fmul_rn(e2i, ri), etaj = __fmul_rn(e2j, rj);
+        const int ti = min(N1 + 1, (int)(etai * invStep));
+        const float4 Gi = tg[ti], Gj = tg[min(N1 + 1, (int)(etaj * invStep))];
+        const float gi = __fmaf_rn(__fmaf_rn(Gi.z, etai, Gi.y), etai, Gi.x);
+        const float gj = __fmaf_rn(__fmaf_rn(Gj.z, etaj, Gj.y), etaj, Gj.x);
+        float w;
+        if (SPLINE) w = bsplineW(etai);
+        else w = __fmaf_rn(__fmaf_rn(tw[ti].y, etai, tw[ti].x), etai, Gi.w);
+        const float fi = __fmul_rn(__fmul_rn(Hdeti, gi), ri), fj = __fmul_rn(__fmul_rn(hj1.z, gj), rj);
+        float hx, hy, hz;
+        symDot32(hi0, hi1, eix, eiy, eiz, hx, hy, hz);
+        const float gwix = __fmul_rn(fi, hx), gwiy = __fmul_rn(fi, hy), gwiz = __fmul_rn(fi, hz);
+        symDot32(hj0, hj1, ejx, ejy, ejz, hx, hy, hz);
+        const float gwjx = __fmul_rn(fj, hx), gwjy = __fmul_rn(fj, hy), gwjz = __fmul_rn(fj, hz);
+        const float vx = vi.x - vxj, vy = vi.y - vyj, vz = vi.z - vzj;
+        const float mui = __fdividef(__fmaf_rn(vz, eiz, __fmaf_rn(vy, eiy, __fmul_rn(vx, eix))), __fadd_rn(e2i, eps2));
+        const float muj = __fdividef(__fmaf_rn(vz, ejz, __fmaf_rn(vy, ejy, __fmul_rn(vx, ejx))), __fadd_rn(e2j, eps2));
+        const float mni = fminf(0.f, mui), mnj = fminf(0.f, muj);
+        const float ei = __fmaf_rn(Cq, __fmul_rn(mni, mni), __fmul_rn(mClci, mni));
+        const float ej = __fmaf_rn(Cq, __fmul_rn(mnj, mnj), __fmul_rn(mClcj, mnj));
+        const float ci_ = __fadd_rn(Prhoi, __fmul_rn(ei, hiri)), cj_ = __fadd_rn(Prhoj, __fmul_rn(ej, hirj));
+        const float ddx = __fadd_rn(__fmul_rn(ci_, gwix), __fmul_rn(cj_, gwjx));
+        const float ddy = __fadd_rn(__fmul_rn(ci_, gwiy), __fmul_rn(cj_, gwjy));
+        const float ddz = __fadd_rn(__fmul_rn(ci_, gwiz), __fmul_rn(cj_, gwjz));
+        const float pax = __fmul_rn(-mj, ddx), pay = __fmul_rn(-mj, ddy), paz = __fmul_rn(-mj, ddz);
+        out[0] = pax; out[32] = pay; out[64] = paz;
+        out += 96 * L;
+        kahanAdd(sdx, cdx, pax);
+        kahanAdd(sdy, cdy, pay);
+        kahanAdd(sdz, cdz, paz);
+        const float vg = vx * gwix + vy * gwiy + vz * gwiz;
+        kahanAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg));
+        const float mvx = mj * vx, mvy = mj * vy, mvz = mj * vz;
+        D[0] -= mvx * gwix; D[1] -= mvx * gwiy; D[2] -= mvx * gwiz;
+        D[3] -= mvy * gwix; D[4] -= mvy * gwiy; D[5] -= mvy * gwiz;
+        D[6] -= mvz * gwix; D[7] -= mvz * gwiy; D[8] -= mvz * gwiz;
+        const float mrx = mj * rx, mry = mj * ry, mrz = mj * rz;
+        M[0] -= mrx * gwix; M[1] -= mrx * gwiy; M[2] -= mrx * gwiz;
+        M[3] -= mry * gwix; M[4] -= mry * gwiy; M[5] -= mry * gwiz;
+        M[6] -= mrz * gwix; M[7] -= mrz * gwiy; M[8] -= mrz * gwiz;
+        const float gr = mj * (rhoj - rhoi);
+        gx += gr * gwix; gy += gr * gwiy; gz += gr * gwiz;
+        sw += w;
+        smw += mj * w;
+        sve += (mj * hirj) * (ei * w);
+        maxE = fmaxf(maxE, ei);
+        const float wg = fabsf(gi);
+        m0 += wg;
+        m1x -= wg * eix; m1y -= wg * eiy; m1z -= wg * eiz;
+        // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
+        const float ir = rsqrtf(fmaxf(rx * rx + ry * ry + rz * rz, 1.0e-30f));
+        const float ir2 = ir * ir;
+        const float w2 = wg * wg * (ir2 * ir2 * ir);
+        m2[0] += w2 * (rx * rx); m2[1] += w2 * (rx * ry); m2[2] += w2 * (rx * rz);
+        m2[3] += w2 * (ry * ry); m2[4] += w2 * (ry * rz); m2[5] += w2 * (rz * rz);
+      });
+  if (L > 1) {
+    laneSumKahan<L>(sdx, cdx); laneSumKahan<L>(sdy, cdy); laneSumKahan<L>(sdz, cdz); laneSumKahan<L>(se, ce);
+    sw = laneSum<L>(sw); smw = laneSum<L>(smw); sve = laneSum<L>(sve); maxE = laneMax<L>(maxE);
+    gx = laneSum<L>(gx); gy = laneSum<L>(gy); gz = laneSum<L>(gz);
+    m0 = laneSum<L>(m0); m1x = laneSum<L>(m1x); m1y = laneSum<L>(m1y); m1z = laneSum<L>(m1z);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) { D[k] = laneSum<L>(D[k]); M[k] = laneSum<L>(M[k]); }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) m2[k] = laneSum<L>(m2[k]);
+    if (sub != 0 || !live) return;
+  }
+  if (SPLINE) { sw = timesSplineA(sw); smw = timesSplineA(smw); sve = timesSplineA(sve); }
+  NodeAcc32 a;
+  a.rhoSum = Hdeti * smw; a.norm = mi * (2.0f * hiri) * Hdeti * sw;
+  a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
+  a.deps = kahanValue(se, ce);
+  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * Hdeti * sve;
+  a.xw = a.xdx = a.xdy = a.xdz = 0.f;
+  a.m0 = m0; a.m1x = m1x; a.m1y = m1y; a.m1z = m1z;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) { a.D[k] = D[k]; a.M[k] = M[k]; }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) a.m2[k] = m2[k];
+  a.h0 = hi0;
+  a.h1 = hi1;
+  finalizeNode32<true>(F, i, list[i], a, cnt, hp, t.herm);
+  if (half.v) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
+}
+
 // The pair sweep's per-node inputs, where the update has not written them.
 __global__ void pairInputs32(Fields F, Fields32 P, long n, PairForm pf) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -982,7 +1150,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields3
   F.f[F_OMEGA][i] = toDouble(omega);
   const float iom = omega / (omega * omega + 1.0e-30f);
   P.thermo[i].w = iom;
-  if (!TENSOR && pf.on) {
+  if (pf.on) {
     float4 th = P.thermo[i];
     th.w = iom;
     P.pk[i] = pairRecord(th, pf);
@@ -1202,7 +1370,7 @@ PairForm pairForm32(long n, const HydroParams& hp) {
   PairForm f;
   f.on = 1;
   f.Cl = (float)hp.Cl;
-  f.spline = reducedPair(n, hp) ? 1 : 0;
+  f.spline = !hp.asph && reducedPair(n, hp) ? 1 : 0;
   f.limited = hp.limitedQ;
   f.full = exactPair(n, hp) ? 1 : 0;
   return f;
@@ -1229,14 +1397,30 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
     // tensor H: NodeList test at run time; odd variants cap the registers at
     // 128 (4 blocks per SM), even ones at 168 (3); variants 0-1 the pipelined
     // loop, 2-3 (compatible energy, no XSPH, standard Q) two slots per iteration
+    if (leanPair(hp) && !hp.limitedQ) {
+      if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
+#define SPH_TEN(MI, SP, LA, U, MB) \
+  pairKernelTensor32<MI, SP, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
+#define SPH_TENL(MI, LA, U, MB) do { if (hp.cubicSpline) SPH_TEN(MI, true, LA, U, MB); else SPH_TEN(MI, false, LA, U, MB); } while (0)
+#define SPH_TENM(LA, U, MB) do { if (hasMirrors(g)) SPH_TENL(true, LA, U, MB); else SPH_TENL(false, LA, U, MB); } while (0)
+      const int L = n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8));
+      if (L == 1) {
+        if (variant == 1) SPH_TENM(1, 1, 4);
+        else if (variant == 2) SPH_TENM(1, 2, 4);
+        else if (variant == 3) SPH_TENM(1, 3, 2);
+        else SPH_TENM(1, 2, 3);
+      } else if (L == 2) SPH_TENM(2, 2, 3);
+      else if (L == 4) SPH_TENM(4, 2, 3);
+      else SPH_TENM(8, 2, 3);
+#undef SPH_TENM
+#undef SPH_TENL
+#undef SPH_TEN
+      lc->add(inputs ? 1 : 2);
+      return;
+    }
     if (!hp.xsph && hp.compatible && !hp.limitedQ && variant >= 2) {
-      if (lean) {
-        if (variant & 1) pairKernelFP32<false, true, true, 4, 2, false, true, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-        else pairKernelFP32<false, true, true, 3, 2, false, true, 1><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      } else {
-        if (variant & 1) pairKernelFP32<false, true, true, 4, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-        else pairKernelFP32<false, true, true, 3, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      }
+      if (variant & 1) pairKernelFP32<false, true, true, 4, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
+      else pairKernelFP32<false, true, true, 3, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
     } else if (hp.xsph) {
       if (hp.compatible) { if (hp.limitedQ) SPH_PAIR32T(true, true, true); else SPH_PAIR32T(true, true, false); }
       else { if (hp.limitedQ) SPH_PAIR32T(true, false, true); else SPH_PAIR32T(true, false, false); }
