@@ -672,10 +672,12 @@ void prepare32(sphgpu_ctx* c) {
   launchPrepareFP32(c->F, c->f32(), c->n, c->grid, c->stream, &c->lc);
   c->check();
 }
-void sumDensity(sphgpu_ctx* c) {
+// vote (CRKSPH mixed sweep): take the time-step vote along.
+void sumDensity(sphgpu_ctx* c, bool vote = false) {
   Scope sc(c->prof, "sum_density");
   if (c->hp.crk && c->fp32())   // computeCRKSPHSumMassDensity with the current RK volumes
-    launchCRKDensityFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
+    launchCRKDensityFP32(c->F, c->f32(), c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->maxNperh(),
+                         vote ? c->step() : nullptr, c->stream, &c->lc);
   else if (c->hp.crk)
     launchCRKDensity(c->F, c->listp(), c->n, c->grid, c->nl(), c->tableDev(), c->hp, c->stream, &c->lc);
   else if (c->fp32())
@@ -922,7 +924,12 @@ double step(sphgpu_ctx* c, double maxTime) {
         c->check();
         fused = true;
       } else {
-        sumDensity(c);
+        fused = c->hp.crk && c->fp32();
+        if (fused) {
+          setGhostParams(c);
+          if (again) launchDtReset(c->step(), c->stream, &c->lc);
+        }
+        sumDensity(c, fused);
       }
     }
   };

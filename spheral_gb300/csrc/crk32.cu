@@ -86,7 +86,7 @@ __device__ __forceinline__ void loadRKC(const float4* __restrict__ rkc, long j, 
 
 // The sweeps below take L lanes per node and U slots per iteration (their
 // gathers issued together); MIR false: no wall reflects.
-#define SPH_CRK_SETUP()                                                       \
+#define SPH_CRK_SETUP_ALL()                                                       \
   __shared__ float4 ta[kTab32];                                               \
   __shared__ float2 tb[kTab32];                                               \
   loadTable32(ta, tb, t, hp.tableN1);                                         \
@@ -95,7 +95,6 @@ __device__ __forceinline__ void loadRKC(const float4* __restrict__ rkc, long j, 
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;        \
   const int sub = threadIdx.x % L;                                            \
   const bool live = node < n;                                                 \
-  if (L == 1 && !live) return;                                                \
   const long i = live ? node : n - 1;                                         \
   int ci[3];                                                                  \
   unpackCell(P.cell[i], ci);                                                  \
@@ -103,6 +102,9 @@ __device__ __forceinline__ void loadRKC(const float4* __restrict__ rkc, long j, 
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];              \
   const float4 pi = P.posh[i];                                                \
   const int cnt = live ? nl.count[i] : 0
+#define SPH_CRK_SETUP()                                                       \
+  SPH_CRK_SETUP_ALL();                                                        \
+  if (L == 1 && !live) return
 
 //------------------------------------------------------------------------------
 // RKSumVolume: V_i = min(etaVolMax / Hdet_i, 1 / (sum_j W(|H_i r_ij|) + Hdet_i W0)).
@@ -137,14 +139,19 @@ __global__ void __launch_bounds__(sweepBlock(L)) rkSumVolume32(Fields F, Fields3
 // CRK mass density, FP32 sums over the same-NodeList neighbours.
 //------------------------------------------------------------------------------
 struct DensityRec32 {
-  float4 p;
-  float v, m;
+  float4 p, v;
+  float vol;
 };
+// sc: the time-step vote, whose pair limit reads the same neighbours, in the
+// same pass (null: density only).
 template <bool MIR, int L, int U>
 __global__ void __launch_bounds__(sweepBlock(L)) crkDensity32(Fields F, Fields32 P, const int* __restrict__ list,
                                                               long n, Grid g, NeighborLists nl, TableDev t,
-                                                              HydroParams hp) {
-  SPH_CRK_SETUP();
+                                                              HydroParams hp, double maxNperh,
+                                                              StepScratch* __restrict__ sc) {
+  SPH_CRK_SETUP_ALL();
+  const float4 vi = P.velm[i];
+  float worst = 0.f;
   const bool multi = hp.numLists > 1;
   const int li = list[i];
   float sw = 0.f, cw = 0.f, sr = 0.f, cr = 0.f, sv = 0.f, cv = 0.f;
@@ -152,25 +159,31 @@ __global__ void __launch_bounds__(sweepBlock(L)) crkDensity32(Fields F, Fields32
       nl, i, sub, cnt,
       [&](uint32_t j, DensityRec32& r) {
         r.p = P.posh[j];
-        r.v = P.vol[j];
-        r.m = P.velm[j].w;
+        r.vol = P.vol[j];
+        r.v = P.velm[j];
       },
       [&](uint32_t ent, const DensityRec32& r) {
+        float vxj = r.v.x, vyj = r.v.y, vzj = r.v.z;
+        if (MIR) mirrorVel((ent >> kIndexBits) & mm, vxj, vyj, vzj);
+        const float dx = vi.x - vxj, dy = vi.y - vyj, dz = vi.z - vzj;
+        const float aj = r.p.w, am = fmaxf(pi.w, aj);
+        worst = fmaxf(worst, (am * am) * (dx * dx + dy * dy + dz * dz));
         if (multi && list[ent & kIndexMask] != li) return;
         float rx, ry, rz, e2, re;
         relSepEntry<MIR>(pi, r.p, ent, mm, cx, cy, cz, rx, ry, rz);
-        const float aj = r.p.w;
         const float W = T.value(etaMag(aj * rx, aj * ry, aj * rz, e2, re));
         const float Wj = __fmul_rn(__fmul_rn(__fmul_rn(aj, aj), aj), W);
-        const float VW = __fmul_rn(r.v, Wj);
+        const float VW = __fmul_rn(r.vol, Wj);
         kahanAdd(sw, cw, VW);
-        kahanAdd(sr, cr, __fmul_rn(r.m, VW));
-        kahanAdd(sv, cv, __fmul_rn(r.v, VW));
+        kahanAdd(sr, cr, __fmul_rn(r.v.w, VW));
+        kahanAdd(sv, cv, __fmul_rn(r.vol, VW));
       });
   if (L > 1) {
     laneSumKahan<L>(sw, cw); laneSumKahan<L>(sr, cr); laneSumKahan<L>(sv, cv);
-    if (sub != 0 || !live) return;
+    worst = laneMax<L>(worst);
   }
+  const bool owner = live && sub == 0;
+  if (owner) {
   const NodeListParams Li = hp.lists[li];
   const double ai = F.f[F_HINV][i], mi = F.f[F_MASS][i], Vi = F.f[F_VOL][i];
   const double Hdeti = (ai * ai) * ai;
@@ -180,6 +193,9 @@ __global__ void __launch_bounds__(sweepBlock(L)) crkDensity32(Fields F, Fields32
                           fmin(Li.rhoMax, (kahanValue(sr, cr) + mi * Vi * Hdeti * hp.W0) / (wsum * vol1)));
   F.f[F_RHO][i] = rho;
   P.thermo[i].x = (float)rho;
+  }
+  if (sc)
+    voteNode32<false>(F, hp, list, i, owner && !isGhost(hp, i), pi.w, vi, worst, maxNperh, &sc->voteEst, &sc->voteKey);
 }
 
 //------------------------------------------------------------------------------
@@ -581,8 +597,8 @@ void launchRKVolumesFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl,
   }
 }
 void launchCRKDensityFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                          HydroParams hp, cudaStream_t s, LaunchCounter* lc) {
-  SPH_CRK_SWEEP(crkDensity32, 2, F, P, list, n, g, nl, t, hp);
+                          HydroParams hp, double maxNperh, StepScratch* vote, cudaStream_t s, LaunchCounter* lc) {
+  SPH_CRK_SWEEP(crkDensity32, 2, F, P, list, n, g, nl, t, hp, maxNperh, vote);
   lc->add(1);
 }
 void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,

@@ -937,42 +937,6 @@ __global__ void pairInputs32(Fields F, Fields32 P, long n, PairForm pf) {
   }
 }
 
-//------------------------------------------------------------------------------
-// Time-step vote.  The smallest limit travels as one 64-bit word, the bits of
-// a positive double order as integers: the mixed step's FP32 limits carry the
-// reason code in the low mantissa bits that a widened float leaves zero.
-//------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long warpMin64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-    v = w < v ? w : v;
-  }
-  return v;
-}
-__device__ __forceinline__ unsigned long long dtKey(double v, int reason) {
-  return ((unsigned long long)__double_as_longlong(v) & ~7ULL) | (unsigned)reason;
-}
-
-// FP32 node limits of GenericHydro::dt (GenericHydro.cc:113-381): the smallest
-// of them and of the pair limit, with its reason.  Every term is positive.
-__device__ __forceinline__ float nodeDt32(float ns, float cs, float maxQ, float rho, float divv, float vmag,
-                                          float amag, bool velDt, float pairDt, int& reason) {
-  const float tiny = (float)DBL_EPSILON;
-  float best = 3.0e38f;
-  reason = -1;
-  auto vote = [&](float v, int r) {
-    if (v < best) { best = v; reason = r; }
-  };
-  vote(ns / (cs + tiny), 0);
-  vote(ns / (sqrtf(maxQ / rho) + tiny), 1);
-  vote(1.0f / (fabsf(divv) + tiny), 2);
-  vote(0.1f * fmaxf(ns / (vmag + tiny), vmag / (amag + tiny)), 3);
-  if (velDt) vote(ns / (vmag + 1.0e-10f), 4);
-  vote(pairDt, 5);
-  return best;
-}
-
 // H_j through the mirrors of an entry (FP32 tensor mirror): the off-diagonal
 // components flip once per mirrored index.
 __device__ __forceinline__ void mirrorTensor32(uint32_t mq, float4& h0, float4& h1) {
@@ -1192,48 +1156,7 @@ __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const in
         worst = fmaxf(worst, (am * am) * (dx * dx + dy * dy + dz * dz));
       });
   if (L > 1) worst = laneMax<L>(worst);
-  const float bestPair = worst > 0.0f ? rsqrtf(worst) : 3.0e38f;
-  const bool votes = live && sub == 0 && !isGhost(hp, i);
-  float est = 3.0e38f;
-  const NodeListParams Li = hp.lists[list[i]];
-  if (votes) {
-    const float ax = toFloatRN(F.f[F_DVDT_X][i]), ay = toFloatRN(F.f[F_DVDT_Y][i]), az = toFloatRN(F.f[F_DVDT_Z][i]);
-    const float divv = toFloatRN(F.f[F_DVDX_XX][i] + F.f[F_DVDX_YY][i] + F.f[F_DVDX_ZZ][i]);
-    int reason;
-    est = nodeDt32(1.0f / (lmaxi * (float)Li.nPerh), toFloatRN(F.f[F_CS][i]), toFloatRN(F.f[F_MAXQ][i]),
-                   toFloatRN(F.f[F_RHO][i]), divv, sqrtf(vi.x * vi.x + vi.y * vi.y + vi.z * vi.z),
-                   sqrtf(ax * ax + ay * ay + az * az), hp.useVelMagDt != 0, bestPair / (float)maxNperh, reason);
-  }
-  const float wmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(est)));
-  if ((threadIdx.x & 31) == 0 && wmin < 3.0e38f) atomicMin(estOut, __float_as_uint(wmin));
-  const float seen = __uint_as_float(*(volatile unsigned*)estOut);
-  // NaN compares false: a node with a NaN limit takes the FP64 limits too
-  if (votes && !(est > fminf(seen, wmin) * 1.0001f)) {
-    const double tiny = DBL_EPSILON;
-    double best = DBL_MAX;
-    int reason = -1;
-    const double ai = F.f[TENSOR ? F_HLMAX : F_HINV][i];   // largest eigenvalue of H
-    const double nodeScalei = 1.0 / ai / Li.nPerh;
-    const double vxi = F.f[F_VX][i], vyi = F.f[F_VY][i], vzi = F.f[F_VZ][i];
-    const double rhoi = F.f[F_RHO][i];
-    const double csDt = nodeScalei / (F.f[F_CS][i] + tiny);
-    if (csDt < best) { best = csDt; reason = 0; }
-    const double csqDt = nodeScalei / (sqrt(F.f[F_MAXQ][i] / rhoi) + tiny);
-    if (csqDt < best) { best = csqDt; reason = 1; }
-    const double divvDt = 1.0 / (fabs(F.f[F_DVDX_XX][i] + F.f[F_DVDX_YY][i] + F.f[F_DVDX_ZZ][i]) + tiny);
-    if (divvDt < best) { best = divvDt; reason = 2; }
-    const double vmag = sqrt(vxi * vxi + vyi * vyi + vzi * vzi);
-    const double ax = F.f[F_DVDT_X][i], ay = F.f[F_DVDT_Y][i], az = F.f[F_DVDT_Z][i];
-    const double dtAcc = 0.1 * fmax(nodeScalei / (vmag + tiny), vmag / (sqrt(ax * ax + ay * ay + az * az) + tiny));
-    if (dtAcc < best) { best = dtAcc; reason = 3; }
-    if (hp.useVelMagDt) {
-      const double velDt = nodeScalei / (vmag + 1.0e-10);
-      if (velDt < best) { best = velDt; reason = 4; }
-    }
-    const double pairDt = (double)bestPair / maxNperh;
-    if (pairDt < best) { best = pairDt; reason = 5; }
-    if (reason >= 0) atomicMin(dtOut, dtKey(best, reason));
-  }
+  voteNode32<TENSOR>(F, hp, list, i, live && sub == 0 && !isGhost(hp, i), lmaxi, vi, worst, maxNperh, estOut, dtOut);
 }
 
 __global__ void dtInitKernel(StepScratch* __restrict__ sc) {
@@ -1546,6 +1469,10 @@ void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, T
   lc->add(1);
 }
 
+void launchDtReset(StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
+  dtInitKernel<<<1, 1, 0, s>>>(sc);
+  lc->add(1);
+}
 void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
                   double maxNperh, StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
   dtInitKernel<<<1, 1, 0, s>>>(sc);

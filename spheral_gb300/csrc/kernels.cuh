@@ -125,6 +125,7 @@ void launchSumDensityFP32(Fields F, Fields32 F32, const int* list, long n, Grid 
                           HydroParams hp, cudaStream_t s, LaunchCounter* lc);
 void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                      const PairForm& pf, cudaStream_t s, LaunchCounter* lc);
+void launchDtReset(StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, HydroParams hp,
                   double maxNperh, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 // Mixed mode: density sum and dt vote fused in one sweep; the vote goes to
@@ -158,8 +159,9 @@ void launchPairCRK(Fields F, const int* list, long n, Grid g, NeighborLists nl, 
 // per-node completions; the volume and correction mirrors are written too.
 void launchRKVolumesFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                          cudaStream_t s, LaunchCounter* lc);
+// vote: take the time-step vote along (its slots reset; null: density only).
 void launchCRKDensityFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
-                          HydroParams hp, cudaStream_t s, LaunchCounter* lc);
+                          HydroParams hp, double maxNperh, StepScratch* vote, cudaStream_t s, LaunchCounter* lc);
 void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                              cudaStream_t s, LaunchCounter* lc);
 // variant: 0 one neighbour slot per loop iteration, 1 two (autotuned,
