@@ -238,6 +238,7 @@ struct sphgpu_ctx {
     p.hten = cfg.smoothing_scale != SPHGPU_SMOOTHING_SPH ? hten.as<float4>() : nullptr;
     p.vol = vol32.p ? vol32.as<float>() : nullptr;
     p.rkc = rkc32.p ? rkc32.as<float4>() : nullptr;
+    p.stride = n;
     return p;
   }
   // FP64 sweeps with isotropic H (hydro64.cu)

@@ -76,8 +76,8 @@ __device__ __forceinline__ void mirrorRKC(uint32_t mir, float* C) {
   }
 }
 
-__device__ __forceinline__ void loadRKC(const float4* __restrict__ rkc, long j, float* C) {
-  const float4 a = rkc[4 * j], b = rkc[4 * j + 1], c = rkc[4 * j + 2], d = rkc[4 * j + 3];
+__device__ __forceinline__ void loadRKC(const Fields32& P, long j, float* C) {
+  const float4 a = P.rkc[j], b = P.rkc[P.stride + j], c = P.rkc[2 * P.stride + j], d = P.rkc[3 * P.stride + j];
   C[0] = a.x; C[1] = a.y; C[2] = a.z; C[3] = a.w;
   C[4] = b.x; C[5] = b.y; C[6] = b.z; C[7] = b.w;
   C[8] = c.x; C[9] = c.y; C[10] = c.z; C[11] = c.w;
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
   for (int r = 0; r < 4; ++r) {
     piv[r] = r;
 #pragma unroll
-    for (int c2 = 0; c2 < 4; ++c2) A[r][c2] = kahanValue(Ms[symIdx(r, c2)], Mc[symIdx(r, c2)]);
+    for (int c2 = 0; c2 < 4; ++c2) A[r][c2] = toDouble(Ms[symIdx(r, c2)]) - toDouble(Mc[symIdx(r, c2)]);
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
     for (int k = 0; k < 4; ++k) {
       double v = 0.0;
 #pragma unroll
-      for (int l = 0; l < 4; ++l) v += (double)dM[d][symIdx(k, l)] * Ct[l];
+      for (int l = 0; l < 4; ++l) v += toDouble(dM[d][symIdx(k, l)]) * Ct[l];
       rhs[k] = -v;
     }
     solve(rhs, dC);
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(128) rkCorrections32(Fields F, Fields32 P, lon
   for (int k = 0; k < 16; ++k) F.f[F_RKC_0 + k][i] = C[k];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    P.rkc[4 * i + k] = make_float4((float)C[4 * k], (float)C[4 * k + 1], (float)C[4 * k + 2], (float)C[4 * k + 3]);
+    P.rkc[k * P.stride + i] = make_float4((float)C[4 * k], (float)C[4 * k + 1], (float)C[4 * k + 2], (float)C[4 * k + 3]);
 }
 
 //------------------------------------------------------------------------------
@@ -362,13 +362,13 @@ __global__ void __launch_bounds__(128, MINB) pairKernelCRK32(Fields F, Fields32 
   const float ai = pi.w, mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, Vi = thi.w;
   const float invMi = __frcp_rn(mi);
   float Ci[16];
-  loadRKC(P.rkc, i, Ci);
+  loadRKC(P, i, Ci);
   const float Cl = (float)hp.Cl, Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
   const float mClci = __fmul_rn(-Cl, csi);
   const float etaCrit = (float)hp.etaCrit, etaFold = (float)hp.etaFold;
   float DQi[9];
   if (LIMQ) {
-    const float4 d0 = P.dvq[3 * i], d1 = P.dvq[3 * i + 1], d2 = P.dvq[3 * i + 2];
+    const float4 d0 = P.dvq[i], d1 = P.dvq[P.stride + i], d2 = P.dvq[2 * P.stride + i];
     DQi[0] = d0.x; DQi[1] = d0.y; DQi[2] = d0.z; DQi[3] = d0.w;
     DQi[4] = d1.x; DQi[5] = d1.y; DQi[6] = d1.z; DQi[7] = d1.w; DQi[8] = d2.x;
   }
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelCRK32(Fields F, Fields32 
     const float vx = vi.x - vxj, vy = vi.y - vyj, vz = vi.z - vzj;
     float vqx = vx, vqy = vy, vqz = vz;
     if (LIMQ) {
-      const float4 d0 = P.dvq[3 * (long)j], d1 = P.dvq[3 * (long)j + 1], d2 = P.dvq[3 * (long)j + 2];
+      const float4 d0 = P.dvq[j], d1 = P.dvq[P.stride + j], d2 = P.dvq[2 * P.stride + j];
       float Dj[9] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w, d2.x};
       if (MIR && mq) {
         const float sg[3] = {(mq & 3u) ? -1.f : 1.f, (mq & 12u) ? -1.f : 1.f, (mq & 48u) ? -1.f : 1.f};
@@ -491,8 +491,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelCRK32(Fields F, Fields32 
         r.p = P.posh[j];
         r.v = P.velm[j];
         r.t = P.pk[j];
-        const float4* c = P.rkc + 4 * (size_t)j;
-        r.c0 = c[0]; r.c1 = c[1]; r.c2 = c[2]; r.c3 = c[3];
+        r.c0 = P.rkc[j]; r.c1 = P.rkc[P.stride + j]; r.c2 = P.rkc[2 * P.stride + j]; r.c3 = P.rkc[3 * P.stride + j];
       },
       pairSlot);
   if (L > 1) {

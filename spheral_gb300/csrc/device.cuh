@@ -760,15 +760,15 @@ __device__ __forceinline__ float4 pairRecord(const float4& th, const PairForm& p
 // off-diagonal pairs summed), or for the exact form (full) all nine components.
 __device__ __forceinline__ void writeQGradient(const Fields32& P, long i, float* v, const PairForm& pf) {
   if (pf.full) {
-    P.dvq[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
-    P.dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
-    P.dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
+    P.dvq[i] = make_float4(v[0], v[1], v[2], v[3]);
+    P.dvq[P.stride + i] = make_float4(v[4], v[5], v[6], v[7]);
+    P.dvq[2 * P.stride + i] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
     return;
   }
 #pragma unroll
   for (int k = 0; k < 9; ++k) v[k] *= 0.25f;
-  P.dvq[2 * i] = make_float4(v[0], v[4], v[8], v[1] + v[3]);
-  P.dvq[2 * i + 1] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
+  P.dvq[i] = make_float4(v[0], v[4], v[8], v[1] + v[3]);
+  P.dvq[P.stride + i] = make_float4(v[2] + v[6], v[5] + v[7], 0.0f, 0.0f);
 }
 
 // Node completion of the isotropic mixed pair loop: finalizeNode32 in terms

@@ -63,14 +63,19 @@ struct Fields {
 struct Fields32 {
   float4* posh;     // (x - cell origin, y - ..., z - ..., hinv)
   float4* velm;     // (vx, vy, vz, m)
-  float4* thermo;   // (rho, P/rho^2 * Omega^-1, cs, unused)
+  float4* thermo;   // (rho, P, cs, 1/Omega)
   float4* pk;       // isotropic SPH pair loop: (rho, Omega^-1 P / rho^2, -Cl c, 1 / (2 rho))
   uint32_t* cell;   // packed cell coordinates (10 bits per axis)
-  float4* dvq;      // limited Q: DvDx of the Q as 3 float4 per node (xx xy xz yx | yy yz zx zy | zz - - -);
-                    // isotropic SPH: its symmetric part, 2 per node (xx yy zz xy | xz yz - -)
-  float4* hten;     // ASPH: tensor H as 2 float4 per node (xx xy xz yy | yz zz det(H) lambda_max)
+  // Records of several float4 are kept as one array per float4, `stride` nodes
+  // apart: a warp's neighbours are near each other in node order, so a gather
+  // of 16 bytes per lane from a dense array touches half the lines (or a
+  // quarter) of one from 32- or 64-byte records.
+  float4* dvq;      // limited Q: DvDx of the Q as 3 float4 (xx xy xz yx | yy yz zx zy | zz - - -);
+                    // reduced SPH sweep: its symmetric part, 2 (xx yy zz xy | xz yz - -)
+  float4* hten;     // ASPH: tensor H as 2 float4 (xx xy xz yy | yz zz det(H) lambda_max)
   float* vol;       // CRKSPH: RK volume
-  float4* rkc;      // CRKSPH: LinearOrder corrections, 4 float4 per node (C | dC/dx | dC/dy | dC/dz)
+  float4* rkc;      // CRKSPH: LinearOrder corrections, 4 float4 (C | dC/dx | dC/dy | dC/dz)
+  long stride;
 };
 
 }  // namespace sph

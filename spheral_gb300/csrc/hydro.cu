@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128, TENSOR ? 4 : 6) neighborMaskKernel(Fields
   if (!TENSOR) {
     bandGap = bandOf(__fmaf_rn(bandA, pi.w, bandB), bandLo, bandHi);
   } else if (active) {
-    const float4 h0 = P.hten[2 * i], h1 = P.hten[2 * i + 1];
+    const float4 h0 = P.hten[i], h1 = P.hten[P.stride + i];
     bandGap = bandOf(tensorBand(h1.w, pi.w, g), bandLo, bandHi);
     hxx = pack2(h0.x, h0.x); hxy = pack2(h0.y, h0.y); hxz = pack2(h0.z, h0.z);
     hyy = pack2(h0.w, h0.w); hyz = pack2(h1.x, h1.x); hzz = pack2(h1.y, h1.y);
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(128, TENSOR ? 4 : 6) neighborMaskKernel(Fields
       if (lane >= d.y) return;
       const int j = (d.x & kIndexMask) + lane;
       qn = P.posh[j];
-      if (TENSOR) { hn0 = P.hten[2 * j]; hn1 = P.hten[2 * j + 1]; }
+      if (TENSOR) { hn0 = P.hten[j]; hn1 = P.hten[P.stride + j]; }
     };
     if (b0 < b1) ahead(b0);
     for (int b = b0; b < b1; ++b) {
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ ite
   constexpr int NC = TENSOR ? 8 : 4;
   float lo[NC] = {q.x, q.y, q.z, q.w}, hi[4] = {q.x, q.y, q.z, q.w};
   if (TENSOR) {
-    const float4 a = P.hten[2 * (in ? j : s)], b = P.hten[2 * (in ? j : s) + 1];
+    const float4 a = P.hten[in ? j : s], b = P.hten[P.stride + (in ? j : s)];
     const float xy = fabsf(a.x * a.y + a.y * a.w + a.z * b.x), xz = fabsf(a.x * a.z + a.y * b.x + a.z * b.y);
     const float yz = fabsf(a.y * a.z + a.w * b.x + b.x * b.y);
     const float m = 1.0e-5f * (b.w * b.w);
@@ -1621,9 +1621,9 @@ __global__ void qGradient32Kernel(Fields F, float4* __restrict__ dvq, long n) {
   float v[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) v[k] = (float)F.f[F_DVDXQ_XX + k][i];
-  dvq[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
-  dvq[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
-  dvq[3 * i + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
+  dvq[i] = make_float4(v[0], v[1], v[2], v[3]);
+  dvq[n + i] = make_float4(v[4], v[5], v[6], v[7]);
+  dvq[2 * n + i] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
 }
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc) {
   qGradient32Kernel<<<gridFor(n, 256), 256, 0, s>>>(F, dvq, n);

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
   const int li = MULTI ? list[i] : 0;
   const float ai = pi.w, mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, sOi = thi.w;
   float4 hi0 = make_float4(0.f, 0.f, 0.f, 0.f), hi1 = hi0;
-  if (TENSOR) { hi0 = P.hten[2 * i]; hi1 = P.hten[2 * i + 1]; }
+  if (TENSOR) { hi0 = P.hten[i]; hi1 = P.hten[P.stride + i]; }
   const float Hdeti = TENSOR ? hi1.z : ai * ai * ai;
   const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
   const int N1 = hp.tableN1;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
   const float epsT = (float)hp.epsTensile, WnPerh = (float)hp.WnPerh;
   float DQi[9];   // the limited Q's DvDx of node i
   if (LIMQ) {
-    const float4 d0 = P.dvq[3 * i], d1 = P.dvq[3 * i + 1], d2 = P.dvq[3 * i + 2];
+    const float4 d0 = P.dvq[i], d1 = P.dvq[P.stride + i], d2 = P.dvq[2 * P.stride + i];
     DQi[0] = d0.x; DQi[1] = d0.y; DQi[2] = d0.z; DQi[3] = d0.w;
     DQi[4] = d1.x; DQi[5] = d1.y; DQi[6] = d1.z; DQi[7] = d1.w; DQi[8] = d2.x;
   }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       // LimitedMonaghanGingoldViscosity.cc:171-200 in a form symmetric in
       // (i, j): v_q = v_ij - phi (DvDx_i + DvDx_j) x_ij with x_ij = r/2, so
       // the pair force stays bitwise antisymmetric.
-      const float4 d0 = P.dvq[3 * (long)j], d1 = P.dvq[3 * (long)j + 1], d2 = P.dvq[3 * (long)j + 2];
+      const float4 d0 = P.dvq[j], d1 = P.dvq[P.stride + j], d2 = P.dvq[2 * P.stride + j];
       float Dj[9] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w, d2.x};
       const uint32_t mq = (uint32_t)dcode & mm;
       if (mq) {
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       entA = nl.nbr[nbSlot(i, 0, nl.cap)];
       const int j0 = (int)(entA & kIndexMask);
       pjA = P.posh[j0]; vjA = P.velm[j0]; thA = P.thermo[j0];
-      if (TENSOR) { hA0 = P.hten[2 * j0]; hA1 = P.hten[2 * j0 + 1]; }
+      if (TENSOR) { hA0 = P.hten[j0]; hA1 = P.hten[P.stride + j0]; }
     }
     if (cnt > 1) entB = nl.nbr[nbSlot(i, 1, nl.cap)];
     for (int q = 0; q < cnt; ++q) {
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       if (q + 1 < cnt) {
         const int jn = (int)(entB & kIndexMask);
         pjA = P.posh[jn]; vjA = P.velm[jn]; thA = P.thermo[jn];
-        if (TENSOR) { hA0 = P.hten[2 * jn]; hA1 = P.hten[2 * jn + 1]; }
+        if (TENSOR) { hA0 = P.hten[jn]; hA1 = P.hten[P.stride + jn]; }
         entA = entB;
       }
       if (q + 2 < cnt) entB = nl.nbr[nbSlot(i, q + 2, nl.cap)];
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
         const int jj = (int)(e[u] & kIndexMask);
         pp[u] = P.posh[jj]; vv[u] = P.velm[jj]; tt[u] = P.thermo[jj];
         aa[u] = zero4; bb[u] = zero4;
-        if (TENSOR) { aa[u] = P.hten[2 * jj]; bb[u] = P.hten[2 * jj + 1]; }
+        if (TENSOR) { aa[u] = P.hten[jj]; bb[u] = P.hten[P.stride + jj]; }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) slot(e[u], pp[u], vv[u], tt[u], aa[u], bb[u], k0 + 32 * u);
@@ -317,16 +317,16 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       const long long k = nbSlot(i, q, nl.cap);
       const uint32_t ent = nl.nbr[k];
       const int jj = (int)(ent & kIndexMask);
-      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[2 * jj] : zero4,
-           TENSOR ? P.hten[2 * jj + 1] : zero4, k);
+      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[jj] : zero4,
+           TENSOR ? P.hten[P.stride + jj] : zero4, k);
     }
   } else {
     for (int q = 0; q < cnt; ++q) {
       const long long k = nbSlot(i, q, nl.cap);
       const uint32_t ent = nl.nbr[k];
       const int jj = (int)(ent & kIndexMask);
-      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[2 * jj] : zero4,
-           TENSOR ? P.hten[2 * jj + 1] : zero4, k);
+      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[jj] : zero4,
+           TENSOR ? P.hten[P.stride + jj] : zero4, k);
     }
   }
   NodeAcc32 a;
@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   float4 qa = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 qb = make_float2(0.f, 0.f);
   if (LIMQ) {
-    qa = P.dvq[2 * i];
-    const float4 q1 = P.dvq[2 * i + 1];
+    qa = P.dvq[i];
+    const float4 q1 = P.dvq[P.stride + i];
     qb = make_float2(q1.x, q1.y);
   }
   PairSums32 a;
@@ -539,8 +539,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
     for (int u = 0; u < U; ++u) {
       const uint32_t j = e[u] & kIndexMask;
       pp[u] = P.posh[j]; vv[u] = P.velm[j]; kk[u] = P.pk[j];
-      q0[u] = LIMQ ? P.dvq[2 * j] : zero4;
-      q1[u] = LIMQ ? P.dvq[2 * j + 1] : zero4;
+      q0[u] = LIMQ ? P.dvq[j] : zero4;
+      q1[u] = LIMQ ? P.dvq[P.stride + j] : zero4;
     }
     nb += U * ST;
 #pragma unroll
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
     for (int u = 0; u < U - 1; ++u) {
       if (q + u < mine) {
         const uint32_t j = nx[u] & kIndexMask;
-        slot(nx[u], P.posh[j], P.velm[j], P.pk[j], LIMQ ? P.dvq[2 * j] : zero4, LIMQ ? P.dvq[2 * j + 1] : zero4,
+        slot(nx[u], P.posh[j], P.velm[j], P.pk[j], LIMQ ? P.dvq[j] : zero4, LIMQ ? P.dvq[P.stride + j] : zero4,
              out + 3 * u * ST);
       }
     }
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
   const float etaCrit = (float)hp.etaCrit, etaFold = (float)hp.etaFold;
   float DQi[9];   // the limited Q's DvDx of node i
   if (LIMQ) {
-    const float4 d0 = P.dvq[3 * i], d1 = P.dvq[3 * i + 1], d2 = P.dvq[3 * i + 2];
+    const float4 d0 = P.dvq[i], d1 = P.dvq[P.stride + i], d2 = P.dvq[2 * P.stride + i];
     DQi[0] = d0.x; DQi[1] = d0.y; DQi[2] = d0.z; DQi[3] = d0.w;
     DQi[4] = d1.x; DQi[5] = d1.y; DQi[6] = d1.z; DQi[7] = d1.w; DQi[8] = d2.x;
   }
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
         r.p = P.posh[j];
         r.v = P.velm[j];
         r.k = P.pk[j];
-        if (LIMQ) { r.d0 = P.dvq[3 * j]; r.d1 = P.dvq[3 * j + 1]; r.d2 = P.dvq[3 * j + 2]; }
+        if (LIMQ) { r.d0 = P.dvq[j]; r.d1 = P.dvq[P.stride + j]; r.d2 = P.dvq[2 * P.stride + j]; }
       },
       [&](uint32_t ent, const Rec& q) {
         const uint32_t dcode = ent >> kIndexBits;
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
-  const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i], hi0 = P.hten[2 * i], hi1 = P.hten[2 * i + 1];
+  const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i], hi0 = P.hten[i], hi1 = P.hten[P.stride + i];
   const float mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w, Hdeti = hi1.z;
   const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
   float sw = 0.f, smw = 0.f, sve = 0.f, maxE = 0.f;
@@ -814,8 +814,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
         r.p = P.posh[j];
         r.v = P.velm[j];
         r.k = P.pk[j];
-        r.a = P.hten[2 * j];
-        r.b = P.hten[2 * j + 1];
+        r.a = P.hten[j];
+        r.b = P.hten[P.stride + j];
       },
       [&](uint32_t ent, const PairRecTensor& q) {
         float rx, ry, rz;
@@ -983,14 +983,14 @@ __global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Field
   const Kernel32<KERN> K{ta, nullptr, hp.tableN1, (float)(1.0 / hp.tableXstep)};
   float s = 0.f, c = 0.f, worst = 0.0f;
   // the node scale of GenericHydro::dt: 1/h, the largest eigenvalue of H
-  const float lmaxi = TENSOR ? P.hten[2 * i + 1].w : pi.w;
+  const float lmaxi = TENSOR ? P.hten[P.stride + i].w : pi.w;
   const int cnt = live ? nl.count[i] : 0;
   laneSlots<L, U, SweepRec>(
       nl, i, sub, cnt,
       [&](uint32_t j, SweepRec& r) {
         r.p = P.posh[j];
         r.v = P.velm[j];
-        if (TENSOR) { r.h0 = P.hten[2 * j]; r.h1 = P.hten[2 * j + 1]; }
+        if (TENSOR) { r.h0 = P.hten[j]; r.h1 = P.hten[P.stride + j]; }
       },
       [&](uint32_t ent, SweepRec& r) {
         const uint32_t dcode = ent >> kIndexBits;
@@ -1082,7 +1082,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields3
   const float4 pi = P.posh[i];
   const float ai = pi.w;
   float4 hi0 = make_float4(0.f, 0.f, 0.f, 0.f), hi1 = hi0;
-  if (TENSOR) { hi0 = P.hten[2 * i]; hi1 = P.hten[2 * i + 1]; }
+  if (TENSOR) { hi0 = P.hten[i]; hi1 = P.hten[P.stride + i]; }
   float ws = 0.f, wc = 0.f, gs = 0.f, gc = 0.f;
   const int cnt = live ? nl.count[i] : 0;
   laneSlots<L, U, float4>(
@@ -1140,13 +1140,13 @@ __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const in
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
   const float4 vi = P.velm[i];
-  const float lmaxi = TENSOR ? P.hten[2 * i + 1].w : P.posh[i].w;
+  const float lmaxi = TENSOR ? P.hten[P.stride + i].w : P.posh[i].w;
   float worst = 0.0f;
   laneSlots<L, U, float4>(
       nl, i, sub, live ? nl.count[i] : 0,
       [&](uint32_t j, float4& v) {
         v = P.velm[j];
-        v.w = TENSOR ? P.hten[2 * j + 1].w : P.posh[j].w;
+        v.w = TENSOR ? P.hten[P.stride + j].w : P.posh[j].w;
       },
       [&](uint32_t ent, const float4& v) {
         float vxj = v.x, vyj = v.y, vzj = v.z;

@@ -387,14 +387,14 @@ __device__ __forceinline__ Sym incrementASPHHtensor(const Sym& H, const Sym& D, 
 // (xx xy xz yy) (yz zz det(H) lambda_max).
 __device__ __forceinline__ void writeTensorMirror(const Fields& F, long i, const Fields32& P, long k) {
   const Sym h = loadSym(F, F_HT_XX, i);
-  P.hten[2 * k] = make_float4(toFloatRN(h.xx), toFloatRN(h.xy), toFloatRN(h.xz), toFloatRN(h.yy));
-  P.hten[2 * k + 1] = make_float4(toFloatRN(h.yz), toFloatRN(h.zz), toFloatRN(symDet(h)), toFloatRN(F.f[F_HLMAX][i]));
+  P.hten[k] = make_float4(toFloatRN(h.xx), toFloatRN(h.xy), toFloatRN(h.xz), toFloatRN(h.yy));
+  P.hten[P.stride + k] = make_float4(toFloatRN(h.yz), toFloatRN(h.zz), toFloatRN(symDet(h)), toFloatRN(F.f[F_HLMAX][i]));
 }
 // H_j of a neighbour entry from the mirror, seen through the mirror-axis bits
 // mir (dcode layout) of the entry.
 __device__ __forceinline__ void loadTensor32(const Fields32& P, int j, uint32_t mir, float4& a, float4& b) {
-  a = P.hten[2 * j];
-  b = P.hten[2 * j + 1];
+  a = P.hten[j];
+  b = P.hten[P.stride + j];
   if (mir) {
     const float sx = (mir & 3u) ? -1.f : 1.f, sy = (mir & 12u) ? -1.f : 1.f, sz = (mir & 48u) ? -1.f : 1.f;
     a.y *= sx * sy;
