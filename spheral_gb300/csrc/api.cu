@@ -174,6 +174,9 @@ struct sphgpu_ctx {
   double dtMinAcc = 1e300, extraEnergy = 0.0;
   GravityWork* grav = nullptr;
   bool initialized = false;
+  // Gravity runs beside the pair sweep on its own stream (see evalDerivs).
+  cudaStream_t gravStream = nullptr;
+  cudaEvent_t gravReady = nullptr, gravDone = nullptr;
   cudaEvent_t tA = nullptr, tB = nullptr;
   int itemWidth = 32;        // lanes per work item of the neighbour search
   int itemBound = 0;         // upper bound on the number of work items
@@ -710,11 +713,17 @@ void settleOmega(sphgpu_ctx* c) {
 void ensureQMirror(sphgpu_ctx* c) {
   if (c->fp32() && c->hp.limitedQ) c->dvq.ensure((size_t)c->n * 3 * sizeof(float4));
 }
+// Gravity may start from here: the positions it reads are those of now.
+void markPositions(sphgpu_ctx* c) {
+  if (c->cfg.gravity) CUDA_OK(cudaEventRecord(c->gravReady, c->stream));
+}
+// positions: they have been marked.
 // inputs: the mixed SPH pair sweep's per-node inputs are already those of
 // this state; half: the energy sweep's half-step velocities, wanted from it.
-void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}) {
+void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}, bool positions = false) {
   ensurePacc(c);
   ensureQMirror(c);
+  if (!positions) markPositions(c);
   if (c->fp32() && c->hp.limitedQ) {   // FP32 mirror of the Q's DvDx in the current node order
     if (c->hp.asph || c->hp.crk) {   // the isotropic SPH sweep writes its own form
       launchQGradient32(c->F, c->dvq.as<float4>(), c->n, c->stream, &c->lc);
@@ -793,15 +802,25 @@ void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}) {
   }
   c->check();
   if (c->cfg.gravity) {
+    // The octree build is a chain of short, latency-bound launches and the walk
+    // leaves half the issue slots: both run beside the pair sweep just launched,
+    // which reads and writes other fields.  The step's stream waits for the
+    // result; an error drains the gravity stream before it is reported.
     Scope sc(c->prof, "gravity");
     char msg[256] = {0};
     double* d = c->small.as<double>() + 16;
-    const int rc = gravityEvaluate(c->grav, c->F, c->n, c->cfg.G, c->cfg.softening, c->cfg.opening, c->fp32(), d,
-                                   c->stream,
+    cudaStream_t gs = c->gravStream;
+    CUDA_OK(cudaStreamWaitEvent(gs, c->gravReady, 0));
+    const int rc = gravityEvaluate(c->grav, c->F, c->n, c->cfg.G, c->cfg.softening, c->cfg.opening, c->fp32(), d, gs,
                                    &c->lc, msg, sizeof(msg));
-    if (rc != SPHGPU_OK) throw Error(rc, std::string("gravity: ") + msg);
-    CUDA_OK(cudaMemcpyAsync(c->hsmall + 16, d, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_OK(cudaStreamSynchronize(c->stream));
+    if (rc != SPHGPU_OK) {
+      cudaStreamSynchronize(gs);
+      throw Error(rc, std::string("gravity: ") + msg);
+    }
+    CUDA_OK(cudaMemcpyAsync(c->hsmall + 16, d, 2 * sizeof(double), cudaMemcpyDeviceToHost, gs));
+    CUDA_OK(cudaEventRecord(c->gravDone, gs));
+    CUDA_OK(cudaStreamWaitEvent(c->stream, c->gravDone, 0));
+    CUDA_OK(cudaStreamSynchronize(gs));
     c->dtMinAcc = c->hsmall[16];
     c->extraEnergy = c->hsmall[17];
   }
@@ -969,6 +988,7 @@ double step(sphgpu_ctx* c, double maxTime) {
   }
   c->check();
   c->time = t + hdt;
+  markPositions(c);
   if (c->cfg.gradh_correction) gradh(c, ex.pair);    // postStateUpdate (mid)
   c->omegaStale = false;
   if (c->cfg.gradh_correction) exchangePoint(c, SPHGPU_EXCHANGE_OMEGA);
@@ -977,7 +997,7 @@ double step(sphgpu_ctx* c, double maxTime) {
     c->v12.ensure(c->n * 2 * sizeof(float4));
     if (!c->hp.crk && !c->xfn) half = HalfStep{c->v12.as<float4>(), hdt};
   }
-  evalDerivs(c, formed, half);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
+  evalDerivs(c, formed, half, true);                      // derivs.Zero(); evaluateDerivatives(t + dt/2)
   exchangePoint(c, SPHGPU_EXCHANGE_DERIVS);          // the halo's accelerations and energy rates
   if (c->cfg.compatible_energy) {
     Scope sc(c->prof, "energy");
@@ -1258,7 +1278,14 @@ int sphgpu_create(const sphgpu_config* cfg, sphgpu_handle* out) {
     for (int k = 0; k < kMaxNodeLists; ++k)
       c->lists[k] = NodeListParams{1.51, 1e-20, 1e20, 1e-10, 1e10, 5.0 / 3.0, -1.79e308, 1.79e308, 1e20, 1e-20, 0.1};
     c->numLists = 0;
-    if (cfg->gravity) c->grav = gravityCreate();
+    if (cfg->gravity) {
+      c->grav = gravityCreate();
+      int least = 0, greatest = 0;
+      CUDA_OK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      CUDA_OK(cudaStreamCreateWithPriority(&c->gravStream, cudaStreamNonBlocking, greatest));
+      CUDA_OK(cudaEventCreateWithFlags(&c->gravReady, cudaEventDisableTiming));
+      CUDA_OK(cudaEventCreateWithFlags(&c->gravDone, cudaEventDisableTiming));
+    }
     // Build the table of the configured base kernel (TableKernel(BSplineKernel(), n)
     // by default, or TableKernel(NBSplineKernel(order), n)).
     if (cfg->kernel != SPHGPU_KERNEL_BSPLINE && cfg->kernel != SPHGPU_KERNEL_NBSPLINE &&
@@ -1290,6 +1317,7 @@ int sphgpu_create(const sphgpu_config* cfg, sphgpu_handle* out) {
 
 int sphgpu_destroy(sphgpu_handle c) {
   if (!c) return SPHGPU_E_ARG;
+  if (c->gravStream) cudaStreamSynchronize(c->gravStream);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->prof.on = false;
   for (auto& r : c->prof.pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
@@ -1301,6 +1329,9 @@ int sphgpu_destroy(sphgpu_handle c) {
   for (auto* b : bufs) b->release();
   for (int k = 0; k < 2; ++k) { c->orig[k].release(); c->list[k].release(); c->cellc[k].release(); }
   if (c->grav) gravityDestroy(c->grav);
+  if (c->gravReady) cudaEventDestroy(c->gravReady);
+  if (c->gravDone) cudaEventDestroy(c->gravDone);
+  if (c->gravStream) cudaStreamDestroy(c->gravStream);
   if (c->tA) cudaEventDestroy(c->tA);
   if (c->tB) cudaEventDestroy(c->tB);
   if (c->hsmall) cudaFreeHost(c->hsmall);
