@@ -156,6 +156,7 @@ struct sphgpu_ctx {
   long cap = 0;
   // neighbour build
   Grid grid{};
+  bool sortCountsClear = false;   // the sort's digit counts are zero for the next build
   DBuf keys, vals, keysAlt, valsAlt, sortWs, cellRange, counts, nbr, pacc;
   size_t cellSpace = 0;
   long long nnbr = 0;
@@ -566,20 +567,24 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   c->keysAlt.ensure(n * sizeof(uint32_t));
   c->vals.ensure(n * sizeof(int));
   c->valsAlt.ensure(n * sizeof(int));
-  c->sortWs.ensure(radixSortWorkspaceBytes(n));
+  if (radixSortWorkspaceBytes(n) > c->sortWs.bytes) {
+    c->sortWs.ensure(radixSortWorkspaceBytes(n));
+    c->sortCountsClear = false;
+  }
   const size_t space = (size_t)1 << keyBits;
   if (space > c->cellSpace) {
     c->cellRange.release();
     c->cellRange.ensure(2 * space * sizeof(int));
     c->cellSpace = space;
   }
-  // empty cell ranges and the sort's counters, zeroed by the key kernel
-  const ClearedWords clear{{c->sortWs.as<unsigned>(), reinterpret_cast<unsigned*>(c->cellStart())},
-                           {(long long)radixSortClearedWords(n, sortBits), (long long)(c->cellSpace + space)}};
+  const SortPrep prep = radixSortPrep(c->sortWs.p, n, sortBits);
+  if (!c->sortCountsClear)   // a new workspace, or a build that did not finish
+    CUDA_OK(cudaMemsetAsync(c->sortWs.p, 0, c->sortWs.bytes, c->stream));
+  c->sortCountsClear = false;
   {
     Scope sc(c->prof, "cell_keys");
-    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->step(), clear, c->stream,
-                   &c->lc);
+    launchCellKeys(c->F, n, g, c->keys.as<uint32_t>(), c->vals.as<int>(), c->cellp(), c->step(), prep,
+                   reinterpret_cast<unsigned*>(c->cellStart()), (long long)(c->cellSpace + space), c->stream, &c->lc);
   }
   uint32_t* k = c->keys.as<uint32_t>();
   int* v = c->vals.as<int>();
@@ -598,7 +603,8 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
     launchPermute(c->F, c->Falt, v, c->orig[c->cur].as<int>(), c->orig[nx].as<int>(), c->list[c->cur].as<int>(),
                   c->list[nx].as<int>(), c->cellc[c->cur].as<uint32_t>(), c->cellc[nx].as<uint32_t>(), n,
                   inStep, c->hp.asph != 0, c->hp.crk != 0, m, g, c->fp32(), k, (uint32_t)space, c->cellStart(),
-                  c->cellEnd(), c->stream, &c->lc);
+                  c->cellEnd(), prep, c->stream, &c->lc);
+    c->sortCountsClear = true;
     std::swap(c->bankA, c->bankB);
     std::swap(c->F, c->Falt);
     c->cur = nx;
@@ -1883,19 +1889,20 @@ int sphgpu_upload_state(sphgpu_handle c, const double* pos, const double* vel, c
   const bool asph = c->hp.asph != 0;
   const Item items[] = {{pos, F_X, 3, 3}, {vel, F_VX, 3, 3}, {mass, F_MASS, 1, 1}, {rho, F_RHO, 1, 1},
                         {eps, F_EPS, 1, 1}, {H, asph ? (int)F_HT_XX : (int)F_HINV, asph ? 6 : 1, 6}};
+  HostBatch batch;
   size_t off = 0;
   for (const auto& it : items) {
     if (!it.p) continue;
     const size_t bytes = (size_t)n * it.stride * sizeof(double);
     if (const void* dp = mappedHost(it.p, bytes)) {   // pinned: read in place, caller order
-      launchScatterInHost(c->F, invOrder(c), static_cast<const double*>(dp), it.first, it.ncomp, it.stride, n,
-                          c->stream, &c->lc);
+      batch.add(dp, it.first, it.ncomp, it.stride, false);
       continue;
     }
     CUDA_OK(cudaMemcpyAsync(st + off, it.p, bytes, cudaMemcpyHostToDevice, c->stream));
     launchScatterIn(c->F, c->origp(), st + off, it.first, it.ncomp, it.stride, n, c->stream, &c->lc);
     off += (size_t)n * it.stride;
   }
+  if (batch.count) launchScatterInHost(c->F, invOrder(c), batch, n, c->stream, &c->lc);
   if (asph && H) launchTensorExtent(c->F, n, c->stream, &c->lc);
   c->check();
   // The FP32 mirror is not refreshed here: the step rebuilds it with the
@@ -1913,13 +1920,13 @@ int sphgpu_download_state(sphgpu_handle c, double* pos, double* vel, double* rho
   const bool asph = c->hp.asph != 0;
   const Item items[] = {{pos, F_X, 3, 3}, {vel, F_VX, 3, 3}, {rho, F_RHO, 1, 1}, {eps, F_EPS, 1, 1},
                         {H, asph ? (int)F_HT_XX : (int)F_HINV, asph ? 6 : 1, 6}};
+  HostBatch batch;
   size_t off = 0;
   for (const auto& it : items) {
     if (!it.p) continue;
     const size_t bytes = (size_t)n * it.stride * sizeof(double);
     if (void* dp = mappedHost(it.p, bytes)) {   // pinned: written in place, caller order
-      launchGatherOutHost(c->F, invOrder(c), static_cast<double*>(dp), it.first, it.ncomp, it.stride,
-                          it.first == F_HINV && !asph, n, c->stream, &c->lc);
+      batch.add(dp, it.first, it.ncomp, it.stride, it.first == F_HINV && !asph);
       continue;
     }
     if (it.first == F_HINV && !asph) launchGatherOutH(c->F, c->origp(), st + off, F_HINV, n, c->stream, &c->lc);
@@ -1928,6 +1935,7 @@ int sphgpu_download_state(sphgpu_handle c, double* pos, double* vel, double* rho
                             c->stream));
     off += (size_t)n * it.stride;
   }
+  if (batch.count) launchGatherOutHost(c->F, invOrder(c), batch, n, c->stream, &c->lc);
   c->check();
   CUDA_OK(cudaStreamSynchronize(c->stream));
   API_END(c)

@@ -107,14 +107,21 @@ __global__ void __launch_bounds__(256) boundsKernel(Fields F, long n, int tensor
 //------------------------------------------------------------------------------
 // Neighbour build.
 //------------------------------------------------------------------------------
-__global__ void cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ keys, int* __restrict__ vals,
-                              uint32_t* __restrict__ cellc, StepScratch* __restrict__ sc, ClearedWords clear) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i == 0) resetScratch(sc);
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-    for (long long w = i; w < clear.n[k]; w += (long long)gridDim.x * blockDim.x) clear.p[k][w] = 0u;
-  if (i >= n) return;
+__global__ void __launch_bounds__(256) cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ keys,
+                                                     int* __restrict__ vals, uint32_t* __restrict__ cellc,
+                                                     StepScratch* __restrict__ sc, SortPrep prep,
+                                                     unsigned* __restrict__ ranges, long long nranges) {
+  __shared__ unsigned h[4][256];
+  for (int d = 0; d < prep.digits; ++d) h[d][threadIdx.x] = 0u;
+  __syncthreads();
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
+  if (t == 0) resetScratch(sc);
+  for (long long w = t; w < prep.nclear; w += nt) prep.clear[w] = 0u;
+  for (long long w = t; w < nranges; w += nt) ranges[w] = 0u;
+  const int lane = threadIdx.x & 31;
+  for (long b = t - lane; b < n; b += nt) {   // whole warps
+  const long i = b + lane < n ? b + lane : n - 1;
+  const bool live = b + lane < n;
   const double p[3] = {F.f[F_X][i], F.f[F_Y][i], F.f[F_Z][i]};
   uint32_t c[3], f[3];
 #pragma unroll
@@ -137,9 +144,26 @@ __global__ void cellKeyKernel(Fields F, long n, Grid g, uint32_t* __restrict__ k
   // top bits are the cell's Morton key: nodes stay grouped by cell and within
   // a cell they are ordered by octant, so consecutive nodes of a cell (a work
   // chunk or a candidate batch of the neighbour search) sit close together.
-  keys[i] = g.subShift ? cellKey(g, f[0], f[1], f[2], 1) : cellKey(g, c[0], c[1], c[2], 0);
-  vals[i] = (int)i;
-  cellc[i] = c[0] | (c[1] << 10) | (c[2] << 20);
+  const uint32_t key = g.subShift ? cellKey(g, f[0], f[1], f[2], 1) : cellKey(g, c[0], c[1], c[2], 0);
+  if (live) {
+    keys[i] = key;
+    vals[i] = (int)i;
+    cellc[i] = c[0] | (c[1] << 10) | (c[2] << 20);
+  }
+  for (int d = 0; d < prep.digits; ++d) {
+    const unsigned digit = live ? (key >> (8 * d)) & 0xffu : 256u;
+    int all;   // the high digits of a warp are mostly equal
+    __match_all_sync(0xffffffffu, digit, &all);
+    if (all) {
+      if (lane == 0) atomicAdd(&h[d][digit], 32u);
+    } else if (live) {
+      atomicAdd(&h[d][digit], 1u);
+    }
+  }
+  }
+  __syncthreads();
+  for (int d = 0; d < prep.digits; ++d)
+    if (const unsigned c = h[d][threadIdx.x]) atomicAdd(&prep.hist[d * 256 + threadIdx.x], c);
 }
 
 // Gather of the carried fields into the new order, with what the same pass can
@@ -150,7 +174,9 @@ __global__ void permuteKernel(Fields Fin, Fields Fout, const int* __restrict__ p
                               int* __restrict__ origOut, const int* __restrict__ listIn, int* __restrict__ listOut,
                               const uint32_t* __restrict__ cellIn, uint32_t* __restrict__ cellOut, long n,
                               FieldRanges sel, Fields32 P, Grid g, int mirrors, const uint32_t* __restrict__ keys,
-                              uint32_t space, int* __restrict__ cellStart, int* __restrict__ cellEnd) {
+                              uint32_t space, int* __restrict__ cellStart, int* __restrict__ cellEnd, SortPrep prep) {
+  if (blockIdx.x == 0 && blockIdx.y == 0)   // the sort is done with them
+    for (int w = threadIdx.x; w < 256 * prep.digits; w += blockDim.x) prep.hist[w] = 0u;
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int p = (int)min((unsigned)perm[k], (unsigned)(n - 1));
@@ -1562,24 +1588,24 @@ __global__ void inverseOrderKernel(const int* __restrict__ orig, int* __restrict
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k < n) inv[orig[k]] = (int)k;
 }
-__global__ void scatterInHostKernel(Fields F, const int* __restrict__ inv, const double* __restrict__ src, int first,
-                                    int ncomp, int stride, long n) {
+__global__ void scatterInHostKernel(Fields F, const int* __restrict__ inv, HostBatch batch, long n) {
+  const HostBatch::Item it = batch.it[blockIdx.y];
   const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= n * stride) return;
-  const long m = e / stride;
-  const int c = (int)(e - m * stride);
-  if (c < ncomp) F.f[first + c][inv[m]] = src[e];
+  if (e >= n * it.stride) return;
+  const long m = e / it.stride;
+  const int c = (int)(e - m * it.stride);
+  if (c < it.ncomp) F.f[it.first + c][inv[m]] = it.host[e];
 }
-__global__ void gatherOutHostKernel(Fields F, const int* __restrict__ inv, double* __restrict__ dst, int first,
-                                    int ncomp, int stride, int isoH, long n) {
+__global__ void gatherOutHostKernel(Fields F, const int* __restrict__ inv, HostBatch batch, long n) {
+  const HostBatch::Item it = batch.it[blockIdx.y];
   const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= n * stride) return;
-  const long m = e / stride;
-  const int c = (int)(e - m * stride);
+  if (e >= n * it.stride) return;
+  const long m = e / it.stride;
+  const int c = (int)(e - m * it.stride);
   double v;
-  if (isoH) v = (c == 0 || c == 3 || c == 5) ? F.f[first][inv[m]] : 0.0;
-  else v = c < ncomp ? F.f[first + c][inv[m]] : 0.0;
-  dst[e] = v;
+  if (it.isoH) v = (c == 0 || c == 3 || c == 5) ? F.f[it.first][inv[m]] : 0.0;
+  else v = c < it.ncomp ? F.f[it.first + c][inv[m]] : 0.0;
+  it.host[e] = v;
 }
 // H as SymTensor (xx, xy, xz, yy, yz, zz) <-> isotropic hinv.
 __global__ void gatherOutHKernel(Fields F, const int* __restrict__ orig, double* __restrict__ stage, int field,
@@ -1610,8 +1636,9 @@ void launchBounds(const Fields& F, long n, bool tensor, StepScratch* sc, cudaStr
   lc->add(2);
 }
 void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
-                    ClearedWords clear, cudaStream_t s, LaunchCounter* lc) {
-  cellKeyKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, g, keys, vals, cellc, sc, clear);
+                    const SortPrep& prep, unsigned* ranges, long long nranges, cudaStream_t s, LaunchCounter* lc) {
+  // at most 8 blocks per SM: each adds its digit counts to the global ones
+  cellKeyKernel<<<std::min(gridFor(n, 256), 1216u), 256, 0, s>>>(F, n, g, keys, vals, cellc, sc, prep, ranges, nranges);
   lc->add(1);
 }
 // FP32 mirror of the Q's DvDx for the mixed pair sweep.
@@ -1633,8 +1660,8 @@ constexpr long kSplitPermute = 200000;
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
                    bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
-                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, cudaStream_t s,
-                   LaunchCounter* lc) {
+                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
+                   cudaStream_t s, LaunchCounter* lc) {
   // the tensor-H fields (the end of the carried block and of the permuted
   // block) move only in ASPH mode, the RK volume and corrections (the end of
   // the permuted block) only in CRKSPH mode
@@ -1648,7 +1675,7 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
   // a few blocks leave the SMs idle: spread the fields over more
   const dim3 grid(gridFor(n, 256), n < kSplitPermute ? 9 : 1);
   permuteKernel<<<grid, 256, 0, s>>>(Fin, Fout, perm, origIn, origOut, listIn, listOut, cellIn, cellOut, n,
-                                                sel, P, g, mirrors ? 1 : 0, sortedKeys, space, cellStart, cellEnd);
+                                                sel, P, g, mirrors ? 1 : 0, sortedKeys, space, cellStart, cellEnd, prep);
   lc->add(1);
 }
 void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
@@ -1793,14 +1820,14 @@ void launchInverseOrder(const int* orig, int* inv, long n, cudaStream_t s, Launc
   inverseOrderKernel<<<gridFor(n, 256), 256, 0, s>>>(orig, inv, n);
   lc->add(1);
 }
-void launchScatterInHost(Fields F, const int* inv, const double* src, int first, int ncomp, int stride, long n,
-                         cudaStream_t s, LaunchCounter* lc) {
-  scatterInHostKernel<<<gridFor(n * stride, 256), 256, 0, s>>>(F, inv, src, first, ncomp, stride, n);
+void launchScatterInHost(Fields F, const int* inv, const HostBatch& batch, long n, cudaStream_t s, LaunchCounter* lc) {
+  if (batch.count == 0) return;
+  scatterInHostKernel<<<dim3(gridFor(n * batch.maxStride, 256), batch.count), 256, 0, s>>>(F, inv, batch, n);
   lc->add(1);
 }
-void launchGatherOutHost(Fields F, const int* inv, double* dst, int first, int ncomp, int stride, bool isoH, long n,
-                         cudaStream_t s, LaunchCounter* lc) {
-  gatherOutHostKernel<<<gridFor(n * stride, 256), 256, 0, s>>>(F, inv, dst, first, ncomp, stride, isoH ? 1 : 0, n);
+void launchGatherOutHost(Fields F, const int* inv, const HostBatch& batch, long n, cudaStream_t s, LaunchCounter* lc) {
+  if (batch.count == 0) return;
+  gatherOutHostKernel<<<dim3(gridFor(n * batch.maxStride, 256), batch.count), 256, 0, s>>>(F, inv, batch, n);
   lc->add(1);
 }
 void launchGatherOutH(Fields F, const int* orig, double* stage, int field, long n, cudaStream_t s, LaunchCounter* lc) {

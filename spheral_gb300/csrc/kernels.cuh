@@ -44,13 +44,10 @@ constexpr int kBoundsVals = 10;
 void launchBounds(const Fields& F, long n, bool tensor, StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 
 // Neighbour build -------------------------------------------------------------
-// Words that the first kernel of the build zeroes for the later ones.
-struct ClearedWords {
-  unsigned* p[2];
-  long long n[2];
-};
+// The first kernel of the build forms the keys, counts their digits for the
+// sort and zeroes the sort's other counters and the cell ranges.
 void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, uint32_t* cellc, StepScratch* sc,
-                    ClearedWords clear, cudaStream_t s, LaunchCounter* lc);   // resets *sc
+                    const SortPrep& prep, unsigned* ranges, long long nranges, cudaStream_t s, LaunchCounter* lc);   // resets *sc
 // carriedOnly: move only the state and the derivatives the next step reads
 // before recomputing them (the step rewrites every other field before it
 // returns); otherwise every permuted field.  The same pass writes the cells'
@@ -59,8 +56,8 @@ void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, 
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
                    bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
-                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, cudaStream_t s,
-                   LaunchCounter* lc);
+                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
+                   cudaStream_t s, LaunchCounter* lc);   // zeroes prep.hist for the next build
 // FP32 mirror of the limited Q's DvDx (3 float4 per node).
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc);
 // Work items of the group-cooperative search: the chunks of up to `width` (8,
@@ -214,10 +211,21 @@ void launchGatherOutH(Fields F, const int* orig, double* stage, int field, long 
 // caller-order transfers on pinned host arrays addressed in place (inv: the
 // internal index of each caller index)
 void launchInverseOrder(const int* orig, int* inv, long n, cudaStream_t s, LaunchCounter* lc);
-void launchScatterInHost(Fields F, const int* inv, const double* src, int first, int ncomp, int stride, long n,
-                         cudaStream_t s, LaunchCounter* lc);
-void launchGatherOutHost(Fields F, const int* inv, double* dst, int first, int ncomp, int stride, bool isoH, long n,
-                         cudaStream_t s, LaunchCounter* lc);
+// The state fields of one hand-over between the device and mapped host arrays
+// in caller order, in one launch.
+struct HostBatch {
+  int count = 0, maxStride = 0;
+  struct Item {
+    double* host;
+    int first, ncomp, stride, isoH;
+  } it[6];
+  void add(const void* host, int first, int ncomp, int stride, bool isoH) {
+    it[count++] = Item{static_cast<double*>(const_cast<void*>(host)), first, ncomp, stride, isoH ? 1 : 0};
+    if (stride > maxStride) maxStride = stride;
+  }
+};
+void launchScatterInHost(Fields F, const int* inv, const HostBatch& batch, long n, cudaStream_t s, LaunchCounter* lc);
+void launchGatherOutHost(Fields F, const int* inv, const HostBatch& batch, long n, cudaStream_t s, LaunchCounter* lc);
 void launchCountsOut(const int* counts, const int* orig, double* stage, long n, cudaStream_t s, LaunchCounter* lc);
 
 // Gravity (gravity.cu) ---------------------------------------------------------

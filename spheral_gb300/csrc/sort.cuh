@@ -19,15 +19,25 @@ void scanExclusive(const Tin* in, long long* out, long n, void* workspace, long 
                    LaunchCounter* lc);
 
 size_t radixSortWorkspaceBytes(long n);
-// Leading words of the workspace that must be zero before the sort (cleared:
-// the caller has zeroed them in stream order; otherwise the sort does).
-size_t radixSortClearedWords(long n, int bits);
+// A caller whose kernel forms the keys may count their digits there and zero the
+// rest of the workspace, which saves a launch, a clear and a pass over the keys
+// (radixSortPairs with counted): hist[256 d + digit] += 1 for every key and
+// digit place d < digits, on a hist that is zero, and words [0, nclear) of clear
+// set to zero, all in stream order before the sort.  The sort leaves hist as it
+// is; whoever counts clears it for the next time.
+struct SortPrep {
+  unsigned* hist;
+  int digits;
+  unsigned* clear;
+  long long nclear;
+};
+SortPrep radixSortPrep(void* workspace, long n, int bits);
 // Stable sort of (keys, vals) by the low `bits` bits of keys (uint32_t or
 // uint64_t, at most 2^30 pairs).  The pointers are ping-ponged: on return
 // keys/vals point at the sorted data.  *timeout (device) is set when a bounded
 // wait inside the sort ran out; the output is then not sorted.
 template <typename K>
 void radixSortPairs(K*& keys, int*& vals, K*& keysAlt, int*& valsAlt, long n, int bits, void* workspace, int* timeout,
-                    bool cleared, cudaStream_t s, LaunchCounter* lc);
+                    bool counted, cudaStream_t s, LaunchCounter* lc);
 
 }  // namespace sph
