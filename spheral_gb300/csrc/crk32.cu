@@ -605,14 +605,16 @@ void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists
   // several lanes repeat the FP64 solve's issue for fewer nodes per warp: only
   // where one lane per node leaves SMs idle
   const bool mir = hasMirrors(g);
-#define SPH_RKC(MI, LA) rkCorrections32<MI, LA, 2><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp)
+#define SPH_RKC(MI, LA) rkCorrections32<MI, LA, 3><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp)
   if (n >= 40000) { if (mir) SPH_RKC(true, 1); else SPH_RKC(false, 1); }
   else if (n >= 15000) { if (mir) SPH_RKC(true, 2); else SPH_RKC(false, 2); }
   else { if (mir) SPH_RKC(true, 4); else SPH_RKC(false, 4); }
 #undef SPH_RKC
   lc->add(1);
 }
-// variant 0: one slot per iteration, 1: two (compatible energy, no XSPH).
+// Bound by L1 wavefronts (7 gathers per slot) at 8-12 warps per SM.  variant 0:
+// three slots per iteration at two blocks per SM (387,072 nodes: 705 us), 1: two
+// at three (743 us); one at four took 847 us.  With the limited Q one and two.
 void launchPairCRKFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                        HydroParams hp, float* pacc, int variant, cudaStream_t s, LaunchCounter* lc) {
   crkInputs32<<<gridFor(n, 256), 256, 0, s>>>(P, n);
@@ -622,7 +624,7 @@ void launchPairCRKFP32(Fields F, Fields32 P, const int* list, long n, Grid g, Ne
   pairKernelCRK32<X, C, Q, MI, LA, U, MB><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc)
 #define SPH_CRK32L(Q, MI)                                                                                  \
   do {                                                                                                     \
-    if (L == 1) { if (variant & 1) SPH_CRK32(false, true, Q, MI, 1, 2, 2); else SPH_CRK32(false, true, Q, MI, 1, 1, 4); } \
+    if (L == 1) { if (variant & 1) SPH_CRK32(false, true, Q, MI, 1, 2, Q ? 2 : 3); else SPH_CRK32(false, true, Q, MI, 1, Q ? 1 : 3, Q ? 4 : 2); } \
     else if (L == 2) SPH_CRK32(false, true, Q, MI, 2, 1, 4);                                               \
     else SPH_CRK32(false, true, Q, MI, 4, 1, 4);                                                           \
   } while (0)
