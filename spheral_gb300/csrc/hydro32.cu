@@ -589,8 +589,10 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
 // energy; some node of a large run is always that close, so large runs keep
 // these roundings (kExactNodes) and small ones take the cheaper form above.
 // Per-node values (rho, Prho, -Cl c, 1/rho) come from the record, mirror
-// tests and table branches are gone and the accelerations go out in planes:
-// 2.69 -> see launchPairFP32 for the measured times.
+// tests and table branches are gone and the accelerations go out in planes.
+// Bound by the L1 data pipe and issue (64 % of the slots at 12 warps per SM);
+// writes 12 and reads 4 bytes of DRAM per slot, 0.6 ms at 2.1 M nodes of 119.
+// 2.1 M nodes: 2685 -> 2082 us.
 //------------------------------------------------------------------------------
 template <bool LIMQ, bool MIR, bool SPLINE, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32 P, const int* __restrict__ list,
@@ -1299,10 +1301,10 @@ PairForm pairForm32(long n, const HydroParams& hp) {
   return f;
 }
 
-// variant (isotropic, lean path, one lane per node, standard Q): two slots per
-// iteration at 4 blocks per SM (even, <= 128 registers) or 5 (odd, <= 102).
-// At 2.1 M nodes 1741 / 1620 us, the limited Q spills at 102 (180 / 242 us at
-// 104,000 nodes); one slot per iteration ran 1800, four slots at 3 blocks 1890.
+// variant (isotropic, from kExactNodes on, standard Q): five slots per iteration
+// at three blocks per SM (even) or four at two (odd).  Few warps with many
+// gathers each keep the neighbours' lines in L1: 2.1 M nodes 2081 / 2093 us,
+// four at three 2188, six at two 2222.
 void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                     HydroParams hp, float* pacc, int variant, bool inputs, const HalfStep& half, cudaStream_t s,
                     LaunchCounter* lc) {
@@ -1366,8 +1368,8 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
   do {                                                                                                               \
     if (!hp.cubicSpline) pairKernelLean32<Q, MI, false, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
     else if (Q) pairKernelLean32<Q, MI, true, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
-    else if (variant & 1) pairKernelLean32<Q, MI, true, 3, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
-    else pairKernelLean32<Q, MI, true, 4, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half);       \
+    else if (variant & 1) pairKernelLean32<Q, MI, true, 4, 2><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
+    else pairKernelLean32<Q, MI, true, 5, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half);       \
   } while (0)
     if (hasMirrors(g)) { if (hp.limitedQ) SPH_LEAN(true, true); else SPH_LEAN(false, true); }
     else { if (hp.limitedQ) SPH_LEAN(true, false); else SPH_LEAN(false, false); }
