@@ -602,7 +602,7 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
     m.cell = c->cellc[nx].as<uint32_t>();
     launchPermute(c->F, c->Falt, v, c->orig[c->cur].as<int>(), c->orig[nx].as<int>(), c->list[c->cur].as<int>(),
                   c->list[nx].as<int>(), c->cellc[c->cur].as<uint32_t>(), c->cellc[nx].as<uint32_t>(), n,
-                  inStep, c->hp.asph != 0, c->hp.crk != 0, m, g, c->fp32(), k, (uint32_t)space, c->cellStart(),
+                  inStep, c->hp.asph != 0, c->hp.crk != 0, c->hp.limitedQ != 0, m, g, c->fp32(), k, (uint32_t)space, c->cellStart(),
                   c->cellEnd(), prep, c->stream, &c->lc);
     c->sortCountsClear = true;
     std::swap(c->bankA, c->bankB);

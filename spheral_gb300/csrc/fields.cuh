@@ -49,10 +49,10 @@ enum FieldId {
   F_NUM_FIELDS
 };
 
-// Fields a permute moves: up to three index ranges [first, last) of Fields::f.
+// Fields a permute moves: index ranges [first, last) of Fields::f.
 struct FieldRanges {
   int n;
-  int first[3], last[3];
+  int first[6], last[6];
 };
 
 struct Fields {

@@ -1354,7 +1354,7 @@ __global__ void __launch_bounds__(256) endStepKernel(Fields F, long n, Grid g, i
 // IncrementASPHHtensor (fixShape / radialOnly forms) unless FixedH.
 // ex: what the step wants done in the same pass (UpdateExtras); END: its end.
 template <bool TENSOR, bool END>
-__global__ void __launch_bounds__(256) updateKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists,
+__global__ void __launch_bounds__(256, TENSOR ? 4 : 5) updateKernel(Fields F, const int* __restrict__ list, long n, const NodeListParams* __restrict__ lists,
                              double mult, int mid, int gravity, int epsIncrement, int hUpdate, int totalEnergy,
                              int crk, Fields32 P, Grid g, int asphEnd, int fixShape, int radialOnly,
                                                     UpdateExtras ex) {
@@ -1659,16 +1659,26 @@ void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCoun
 constexpr long kSplitPermute = 200000;
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
-                   bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
-                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
+                   bool carriedOnly, bool tensor, bool crk, bool limitedQ, Fields32 P, const Grid& g,
+                   bool mirrors, const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
                    cudaStream_t s, LaunchCounter* lc) {
   // the tensor-H fields (the end of the carried block and of the permuted
   // block) move only in ASPH mode, the RK volume and corrections (the end of
   // the permuted block) only in CRKSPH mode
   FieldRanges sel{};
   auto add = [&](int a, int b) { sel.first[sel.n] = a; sel.last[sel.n] = b; ++sel.n; };
-  add(0, tensor ? (int)F_NUM_CARRIED : (int)F_HT_XX);
-  if (!carriedOnly) {
+  if (carriedOnly) {
+    // of DvDx the vote reads the trace, the limited Q all of it
+    if (limitedQ) {
+      add(0, F_GRAV_X);
+    } else {
+      add(0, F_DVDX_XX + 1);
+      add(F_DVDX_YY, F_DVDX_YY + 1);
+      add(F_DVDX_ZZ, F_DVDX_ZZ + 1);
+    }
+    add(F_GRAV_X, tensor ? (int)F_NUM_CARRIED : (int)F_HT_XX);
+  } else {
+    add(0, tensor ? (int)F_NUM_CARRIED : (int)F_HT_XX);
     add(F_NUM_CARRIED, tensor ? (int)F_VOL : (int)F_HIDEALT_XX);
     if (crk) add(F_VOL, F_NUM_PERMUTED);
   }

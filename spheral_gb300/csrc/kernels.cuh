@@ -55,8 +55,8 @@ void launchCellKeys(const Fields& F, long n, Grid g, uint32_t* keys, int* vals, 
 // (mirrors false: only what the search reads).
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
-                   bool carriedOnly, bool tensor, bool crk, Fields32 P, const Grid& g, bool mirrors,
-                   const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
+                   bool carriedOnly, bool tensor, bool crk, bool limitedQ, Fields32 P, const Grid& g,
+                   bool mirrors, const uint32_t* sortedKeys, uint32_t space, int* cellStart, int* cellEnd, const SortPrep& prep,
                    cudaStream_t s, LaunchCounter* lc);   // zeroes prep.hist for the next build
 // FP32 mirror of the limited Q's DvDx (3 float4 per node).
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc);
