@@ -38,10 +38,10 @@ UNIT = "pair-interactions/s"
 FLOP_PER_PAIR = 456        # algorithmic FLOPs of the reference pair body per unordered pair
 VALUES_PER_NODE = 63       # per-node state read + derivatives written by the pair loop
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unordered pair
-# of one pairKernelFP32 launch, from an ncu --set full capture of
-# kelvin_helmholtz(n1=64) (862 MB for 21.76 M pairs); traffic grows in
+# of one pairKernelLean32 launch, from an ncu capture of
+# kelvin_helmholtz(n1=64) (905 MB for 21.7 M pairs); traffic grows in
 # proportion to the pairs, so it is scaled by the pairs of the launch.
-TRAFFIC_BYTES_PER_PAIR = {"fp32": 39.6}
+TRAFFIC_BYTES_PER_PAIR = {"fp32": 41.7}
 TRAFFIC_SOURCE = "ncu capture at n1=64 scaled by pairs per launch"
 
 
@@ -434,7 +434,7 @@ def run_ours(args, ws, rank, local, dist):
     eng.profile(False)
     ms = max_over_ranks(dist, ms)
     pair_variant = eng.pair_variant()[0] if f32 else None
-    nb_width = eng.neighbor_width()   # lanes per group of the neighbour search (autotuned)
+    nb_width = eng.neighbor_width()   # nodes per work item of the neighbour search
     e1 = eng.conservation()
     energy_err = abs(e1[7] - e0[7]) / abs(e0[7])
     p_scale = float(np.sum(prob.mass * np.linalg.norm(prob.vel, axis=1)))   # sum m |v| of the initial state
@@ -749,7 +749,7 @@ def main():
     ap.add_argument("--cpu1-n1", type=int, default=28, help="lattice of the one-core CPU sample")
     ap.add_argument("--cpu1-steps", type=int, default=2)
     ap.add_argument("--search-width", type=int, default=0, choices=[0, 8, 16, 32],
-                    help="pin the neighbour-search group width (0: autotuned)")
+                    help="pin the neighbour search's item width (0: 32)")
     ap.add_argument("--pair-variant", type=int, default=-1,
                     help="pin the mixed pair kernel's variant (-1: autotuned)")
     args = ap.parse_args()

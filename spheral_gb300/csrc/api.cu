@@ -744,6 +744,12 @@ void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}, b
     ++c->pairEvals;
     const bool retune = c->pairRetuneAt >= 0 && c->pairEvals >= c->pairRetuneAt;
     if (c->pinnedVariant || !(c->pairVariant < 0 || c->tunedN != c->n || retune)) return;
+    if (!pairVariantsDiffer32(c->n, c->hp)) {
+      c->pairVariant = 0;
+      c->tunedN = c->n;
+      c->pairRetuneAt = -1;
+      return;
+    }
     cudaEvent_t e0, e1;
     CUDA_OK(cudaEventCreate(&e0));
     CUDA_OK(cudaEventCreate(&e1));

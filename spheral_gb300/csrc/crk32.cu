@@ -618,7 +618,7 @@ void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists
 void launchPairCRKFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                        HydroParams hp, float* pacc, int variant, cudaStream_t s, LaunchCounter* lc) {
   crkInputs32<<<gridFor(n, 256), 256, 0, s>>>(P, n);
-  const int L = n >= 100000 ? 1 : (n >= 20000 ? 2 : 4);
+  const int L = n >= kCRKOneLane ? 1 : (n >= 20000 ? 2 : 4);
   const bool mir = hasMirrors(g);
 #define SPH_CRK32(X, C, Q, MI, LA, U, MB) \
   pairKernelCRK32<X, C, Q, MI, LA, U, MB><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc)

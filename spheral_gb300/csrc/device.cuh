@@ -167,7 +167,9 @@ __host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 51
 // (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
 // shuffles and the partly filled last slots; the sweeps with light pair bodies
 // gain from two lanes at any size (two list rows per warp access).  Lines set
-// where the measured times cross.
+// where the measured times cross: pair sweep of 103,924 nodes with the limited Q
+// 141 / 148 / 190 us with 2 / 4 / 1 lanes, 3375 nodes 54 us with one, 20 with 16.
+constexpr long kCRKOneLane = 100000;   // from here one lane per node in the CRKSPH pair sweep
 constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
 inline int lanesPair(long n) { return n >= 80000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
 inline int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
@@ -246,44 +248,6 @@ __device__ __forceinline__ void unpackCell(uint32_t cc, int c[3]) {
   c[0] = (int)(cc & 1023u);
   c[1] = (int)((cc >> 10) & 1023u);
   c[2] = (int)((cc >> 20) & 1023u);
-}
-
-// Walk the 27 cells around packed cell cc, resolving periodic wrap and
-// reflecting mirrors; fn(k, dcode) for every candidate slot k in cell order.
-// dcode packs the cell offset per axis (2 bits: 0 -> 0, 1 -> -1, 2 -> +1);
-// together with the home cell it identifies the image (imageCode).
-template <class Fn>
-__device__ __forceinline__ void forEachCandidate(const Grid& g, uint32_t cc, const int* __restrict__ cellStart,
-                                                 const int* __restrict__ cellEnd, Fn fn) {
-  int c[3];
-  unpackCell(cc, c);
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int d[3] = {dx, dy, dz};
-        int cell[3];
-        int dcode = 0;
-        bool ok = true;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          int nn = c[a] + d[a];
-          if (d[a] != 0) dcode |= (d[a] < 0 ? 1 : 2) << (2 * a);
-          if (nn < 0) {
-            if (g.kindLo[a] == AXIS_PERIODIC) nn = g.nc[a] - 1;
-            else if (g.kindLo[a] == AXIS_REFLECT) nn = 0;
-            else ok = false;
-          } else if (nn >= g.nc[a]) {
-            if (g.kindHi[a] == AXIS_PERIODIC) nn = 0;
-            else if (g.kindHi[a] == AXIS_REFLECT) nn = g.nc[a] - 1;
-            else ok = false;
-          }
-          cell[a] = nn;
-        }
-        if (!ok) continue;
-        const uint32_t key = cellKey(g, (uint32_t)cell[0], (uint32_t)cell[1], (uint32_t)cell[2], 0);
-        const int s = cellStart[key], e = cellEnd[key];
-        for (int k = s; k < e; ++k) fn(k, dcode);
-      }
 }
 
 // Image code (2 bits per axis: 0 none, 1 low side, 2 high side) of a

@@ -1291,6 +1291,12 @@ static bool leanPair(const HydroParams& hp) {
 }
 static bool exactPair(long n, const HydroParams& hp) { return leanPair(hp) && n >= kExactNodes; }
 static bool reducedPair(long n, const HydroParams& hp) { return leanPair(hp) && n < kExactNodes && hp.cubicSpline; }
+static int lanesTensor(long n) { return n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8)); }
+bool pairVariantsDiffer32(long n, const HydroParams& hp) {
+  if (hp.crk) return n >= kCRKOneLane && !hp.xsph && hp.compatible;
+  if (hp.asph) return lanesTensor(n) == 1 || !leanPair(hp) || hp.limitedQ;
+  return exactPair(n, hp) && hp.cubicSpline && !hp.limitedQ;
+}
 PairForm pairForm32(long n, const HydroParams& hp) {
   PairForm f;
   f.on = 1;
@@ -1328,7 +1334,7 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
   pairKernelTensor32<MI, SP, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
 #define SPH_TENL(MI, LA, U, MB) do { if (hp.cubicSpline) SPH_TEN(MI, true, LA, U, MB); else SPH_TEN(MI, false, LA, U, MB); } while (0)
 #define SPH_TENM(LA, U, MB) do { if (hasMirrors(g)) SPH_TENL(true, LA, U, MB); else SPH_TENL(false, LA, U, MB); } while (0)
-      const int L = n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8));
+      const int L = lanesTensor(n);
       if (L == 1) {
         if (variant == 1) SPH_TENM(1, 1, 4);
         else if (variant == 2) SPH_TENM(1, 2, 4);

@@ -9,7 +9,8 @@
 //  * with H = a I both kernel gradients lie along the separation, and the
 //    pair reduces to scalars times r (the form of the mixed sweep in
 //    hydro32.cu): ~100 FP64 instructions per ordered pair instead of ~440
-//    (KH slab, 94,500 nodes: pair loop 7.50 -> see the launchers' notes);
+//    (KH slab, 94,500 nodes: pair loop 7.50 -> 2.75 ms, at 88 % of the FP64
+//    unit; density and vote 1.85 -> 0.82 ms at 84 %);
 //  * everything that depends on one node only (1/rho, Prho, Cl c) is formed
 //    once per node into a record, read by aligned 16-byte loads;
 //  * |r| and the viscosity's two quotients come from one reciprocal square

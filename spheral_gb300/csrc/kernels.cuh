@@ -98,6 +98,8 @@ constexpr int kPairVariantsMax = 4;   // values sphgpu_set_pair_variant takes (a
 constexpr int kRetuneAfter = 2;    // uses between an autotuner's first timing and its one retiming
 constexpr int kPairVariantsTensor = 4;   // of its tensor-H (ASPH) path
 constexpr int kPairVariantsCRK = 2;      // of the mixed CRKSPH pair kernel
+// Do the variants differ at this size (else there is nothing to time)?
+bool pairVariantsDiffer32(long n, const HydroParams& hp);
 // Form of the isotropic pair sweep's per-node inputs (Fields32::pk, dvq).
 struct PairForm {
   int on = 0;        // written by the update (and kept current by the grad-h sweep)

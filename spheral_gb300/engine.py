@@ -180,7 +180,7 @@ class Engine:
         return v.value, nv.value
 
     def neighbor_width(self):
-        """Lanes per work group of the neighbour search (autotuned)."""
+        """Nodes per work item of the neighbour search (32 unless pinned)."""
         w = ctypes.c_int()
         self._chk(self.L.sphgpu_get_neighbor_width(self.h, ctypes.byref(w)))
         return w.value
@@ -189,7 +189,7 @@ class Engine:
         self._chk(self.L.sphgpu_set_pair_variant(self.h, v))
 
     def set_neighbor_width(self, w):
-        """Pin the search group width (8, 16 or 32) from the next list build; 0 re-enables the autotuner."""
+        """Pin the search's item width (8, 16 or 32) from the next list build; 0 returns to 32."""
         self._chk(self.L.sphgpu_set_neighbor_width(self.h, w))
 
     def energy_variant(self):

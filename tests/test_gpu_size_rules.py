@@ -119,6 +119,48 @@ def test_elongated_grids(native_lib, oracle_mod, shape):
     assert not bad, bad
 
 
+ASPH_SHAPES = [(30, 20, 19), (30, 20, 21), (45, 32, 27), (45, 32, 28), (60, 48, 34), (60, 48, 35)]
+
+
+@pytest.mark.parametrize("shape,boundaries", [(s, "periodic") for s in ASPH_SHAPES] +
+                         [(s, "reflecting") for s in ASPH_SHAPES[1::2]])
+def test_asph_forms(native_lib, oracle_mod, shape, boundaries):
+    """Tensor H on both sides of 12,000, 40,000 and 100,000 nodes; the bound is
+    the one of the mixed ASPH derivatives.  With walls only the boxes that have
+    no node on one: 1e-9 from a wall, 2e-9 from its own image, the FP32 second
+    moment's |r|^-5 overflows and Hideal falls back to the isotropic one."""
+    p = problems.stretched_box(*shape, seed=sum(shape), boundaries=boundaries)
+    eng, orc = _pair(oracle_mod, p, "fp32")
+    eng.evaluate_derivatives()
+    orc.evaluate_derivatives()
+    bad = compare_fields(eng, orc, ["DvDt", "DepsDt", "DvDx", "massDensitySum", "DHDt", "Hideal", "massZerothMoment",
+                                    "maxViscousPressure"], 2e-5)
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("side", [24, 25, 27, 28, 34, 35, 46, 47, 53, 54])
+def test_crk_forms(native_lib, oracle_mod, side):
+    """CRKSPH on both sides of 15,000, 20,000, 40,000, 100,000 and 150,000 nodes
+    with the standard Q, the limited Q at the odd sides; the bounds are twice
+    those of the mixed CRKSPH evaluation, the vote's the same."""
+    q = dict(viscosity="limited_monaghan_gingold") if side % 2 else dict(viscosity="monaghan_gingold", Cl=1.0, Cq=1.0)
+    p = problems.crksph_box(n_side=side, seed=side, boundaries="reflecting" if side in (25, 46) else "periodic")
+    p.config.update(xsph=False, **q)
+    eng, orc = _pair(oracle_mod, p, "fp32")
+    eng.sum_density()
+    orc.sum_density()
+    eng.evaluate_derivatives()
+    orc.rk_corrections()
+    orc.evaluate_derivatives()
+    bad = compare_fields(eng, orc, ["massDensity", "DvDt", "DepsDt", "DvDx", "Hideal", "massZerothMoment",
+                                    "rkCorrections"], 2e-5)
+    assert not bad, bad
+    dt, ref = eng.dt()[0], orc.hydro_dt()
+    assert abs(dt - ref) <= 1e-6 * ref
+    a, b = eng.step(), orc.step()   # the vote on the density sweep
+    assert abs(a - b) <= 1e-5 * b
+
+
 @pytest.mark.parametrize("n", [2, 3, 7, 8, 9, 31, 33, 127, 1025])
 @pytest.mark.parametrize("softening", [1e-15, 0.01, 30.0])
 def test_gravity_forms(native_lib, oracle_mod, n, softening):
