@@ -1656,6 +1656,8 @@ void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCoun
   qGradient32Kernel<<<gridFor(n, 256), 256, 0, s>>>(F, dvq, n);
   lc->add(1);
 }
+// 3375 nodes 17.9 us in one row of blocks, 10.6 in nine; 2.1 M nodes 292 in one,
+// 303 in four.
 constexpr long kSplitPermute = 200000;
 void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* origIn, int* origOut,
                    const int* listIn, int* listOut, const uint32_t* cellIn, uint32_t* cellOut, long n,
@@ -1710,7 +1712,9 @@ void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, 
 // band used is four times that bound, evaluated with a = a_i >= min(a_i, a_j):
 // delta_i = bandA a_i + bandB.  A node whose delta reaches 1/2 takes the exact
 // test on every candidate.
-constexpr int kWideItems = 2400;   // items below which four warps share one
+// Items below which four warps share one: 30,011 nodes 92 us with four warps,
+// 134 with one; 103,924 nodes 129 us with four, 89 with one.
+constexpr int kWideItems = 2400;
 static void neighborBand(const Grid& g, double ext2, float& bandA, float& bandB) {
   const double u = 1.0 / 16777216.0;
   const double cmax = std::max(g.cell[0], std::max(g.cell[1], g.cell[2]));

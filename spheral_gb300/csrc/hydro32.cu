@@ -27,26 +27,24 @@ __global__ void prepareKernel(Fields F, Fields32 P, long n, Grid g) {
 }
 
 //------------------------------------------------------------------------------
-// SPH pair loop (src/SPH/SPH.cc:294-470) + SPHSmoothingScale moments, FP32.
+// ASPH pair loop (src/SPH/SPH.cc:294-470) + smoothing-scale moments, FP32.
 // Every operation that enters the pair force is deterministic and appears in
 // the same order from both sides of the pair (explicit fma / rn intrinsics,
 // MUFU reciprocal square root and fast division), so slot (j, i) holds the
 // bitwise negation of slot (i, j).
-//------------------------------------------------------------------------------
-// TENSOR (ASPH): H_i, H_j from the FP32 tensor mirror (eta = H r,
+//
+// ASPH: H_i, H_j from the FP32 tensor mirror (eta = H r,
 // grad W = gW H eta^, both in a fixed order so the pair force stays bitwise
 // antisymmetric), the second moment of ASPHClassicSmoothingScale and its
 // FP32 finalize.
 //
-// PF selects the neighbour loop: 0 one slot per iteration, 1 software-
-// pipelined (entry two slots ahead, node data one slot ahead), 2 or 4 that
-// many slots per iteration (their gathers issued together, the next
-// iteration's entries loaded ahead).  Every form evaluates the slots in list
-// order, so all give the same bits.  LEAN (1: compensated sums, 2: plain
-// FP32 sums): the sum type, no tensile correction and the standard Q
-// expansion fixed at compile time (no run-time flag in the loop); 0 reads
-// them from hp.
-template <bool XSPH, bool COMPAT, bool MULTI, int MINB, int PF, bool LIMQ, bool TENSOR, int LEAN = 0>
+// PF selects the neighbour loop: 1 software-pipelined (entry two slots ahead,
+// node data one slot ahead), 2 that many slots per iteration (their gathers
+// issued together, the next iteration's entries loaded ahead).  Every form
+// evaluates the slots in list order, so all give the same bits.  It serves what
+// pairKernelTensor32 does not: XSPH, no compatible energy, the limited Q, several
+// NodeLists, the tensile term, plain sums and the Q's expansion options.
+template <bool XSPH, bool COMPAT, int MINB, int PF, bool LIMQ>
 __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P, const int* __restrict__ list, long n,
                                                       Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                                                       float* __restrict__ pacc) {
@@ -62,11 +60,10 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
   const uint32_t mm = mirrorMask(g, ci);
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
   const float4 pi = P.posh[i], vi = P.velm[i], thi = P.thermo[i];
-  const int li = MULTI ? list[i] : 0;
-  const float ai = pi.w, mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, sOi = thi.w;
-  float4 hi0 = make_float4(0.f, 0.f, 0.f, 0.f), hi1 = hi0;
-  if (TENSOR) { hi0 = P.hten[i]; hi1 = P.hten[P.stride + i]; }
-  const float Hdeti = TENSOR ? hi1.z : ai * ai * ai;
+  const int li = list[i];
+  const float mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, sOi = thi.w;
+  const float4 hi0 = P.hten[i], hi1 = P.hten[P.stride + i];
+  const float Hdeti = hi1.z;
   const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
   const int N1 = hp.tableN1;
   const float Cl = (float)hp.Cl, Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
@@ -102,9 +99,9 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     relSepEntry(pi, pj, ent, mm, cx, cy, cz, rx, ry, rz);
     float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
     mirrorVel((uint32_t)dcode & mm, vxj, vyj, vzj);
-    const float aj = pj.w, mj = vj4.w, rhoj = thj.x, Pj = thj.y, csj = thj.z, sOj = thj.w;
-    const bool same = MULTI ? (list[j] == li) : true;
-    if (TENSOR) {   // H_j through the mirrors of the entry
+    const float mj = vj4.w, rhoj = thj.x, Pj = thj.y, csj = thj.z, sOj = thj.w;
+    const bool same = list[j] == li;
+    {   // H_j through the mirrors of the entry
       const uint32_t mq = (uint32_t)dcode & mm;
       if (mq) {
         const float sx = (mq & 3u) ? -1.f : 1.f, sy = (mq & 12u) ? -1.f : 1.f, sz = (mq & 48u) ? -1.f : 1.f;
@@ -113,17 +110,12 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
         hj1.x *= sy * sz;
       }
     }
-    const float Hdetj = TENSOR ? hj1.z : aj * aj * aj;
+    const float Hdetj = hj1.z;
     const float irj = __frcp_rn(rhoj);
 
     float eix, eiy, eiz, ejx, ejy, ejz;
-    if (TENSOR) {
-      symDot32(hi0, hi1, rx, ry, rz, eix, eiy, eiz);
-      symDot32(hj0, hj1, rx, ry, rz, ejx, ejy, ejz);
-    } else {
-      eix = ai * rx; eiy = ai * ry; eiz = ai * rz;
-      ejx = aj * rx; ejy = aj * ry; ejz = aj * rz;
-    }
+    symDot32(hi0, hi1, rx, ry, rz, eix, eiy, eiz);
+    symDot32(hj0, hj1, rx, ry, rz, ejx, ejy, ejz);
     const float e2i = __fmaf_rn(eiz, eiz, __fmaf_rn(eiy, eiy, __fmul_rn(eix, eix)));
     const float e2j = __fmaf_rn(ejz, ejz, __fmaf_rn(ejy, ejy, __fmul_rn(ejx, ejx)));
     const float ri = rsqrtf(fmaxf(e2i, 1.0e-30f)), rj = rsqrtf(fmaxf(e2j, 1.0e-30f));
@@ -136,20 +128,13 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     Wj *= Hdetj;
     // gradW = gW H eta/|eta|
     float gwix, gwiy, gwiz, gwjx, gwjy, gwjz;
-    if (TENSOR) {
-      const float fi = __fmul_rn(__fmul_rn(Hdeti, gi), ri);
-      const float fj = __fmul_rn(__fmul_rn(Hdetj, gj), rj);
-      float hx, hy, hz;
-      symDot32(hi0, hi1, eix, eiy, eiz, hx, hy, hz);
-      gwix = __fmul_rn(fi, hx); gwiy = __fmul_rn(fi, hy); gwiz = __fmul_rn(fi, hz);
-      symDot32(hj0, hj1, ejx, ejy, ejz, hx, hy, hz);
-      gwjx = __fmul_rn(fj, hx); gwjy = __fmul_rn(fj, hy); gwjz = __fmul_rn(fj, hz);
-    } else {
-      const float fi = __fmul_rn(__fmul_rn(__fmul_rn(Hdeti, gi), ai), ri);
-      const float fj = __fmul_rn(__fmul_rn(__fmul_rn(Hdetj, gj), aj), rj);
-      gwix = fi * eix; gwiy = fi * eiy; gwiz = fi * eiz;
-      gwjx = fj * ejx; gwjy = fj * ejy; gwjz = fj * ejz;
-    }
+    const float fi = __fmul_rn(__fmul_rn(Hdeti, gi), ri);
+    const float fj = __fmul_rn(__fmul_rn(Hdetj, gj), rj);
+    float hx, hy, hz;
+    symDot32(hi0, hi1, eix, eiy, eiz, hx, hy, hz);
+    gwix = __fmul_rn(fi, hx); gwiy = __fmul_rn(fi, hy); gwiz = __fmul_rn(fi, hz);
+    symDot32(hj0, hj1, ejx, ejy, ejz, hx, hy, hz);
+    gwjx = __fmul_rn(fj, hx); gwjy = __fmul_rn(fj, hy); gwjz = __fmul_rn(fj, hz);
 
     if (same) {
       rhoSum += mj * Wi;
@@ -196,10 +181,10 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     const float mui = __fdividef(__fmaf_rn(vqz, eiz, __fmaf_rn(vqy, eiy, __fmul_rn(vqx, eix))), __fadd_rn(e2i, eps2));
     const float muj = __fdividef(__fmaf_rn(vqz, ejz, __fmaf_rn(vqy, ejy, __fmul_rn(vqx, ejx))), __fadd_rn(e2j, eps2));
     const float mni = fminf(0.f, mui), mnj = fminf(0.f, muj);
-    const float li_ = (!LEAN && hp.linearInExpansion) ? mui : mni;
-    const float lj_ = (!LEAN && hp.linearInExpansion) ? muj : mnj;
-    const float qi_ = (!LEAN && hp.quadraticInExpansion) ? -(mui < 0.f ? -1.f : 1.f) * mui * mui : mni * mni;
-    const float qj_ = (!LEAN && hp.quadraticInExpansion) ? -(muj < 0.f ? -1.f : 1.f) * muj * muj : mnj * mnj;
+    const float li_ = hp.linearInExpansion ? mui : mni;
+    const float lj_ = hp.linearInExpansion ? muj : mnj;
+    const float qi_ = hp.quadraticInExpansion ? -(mui < 0.f ? -1.f : 1.f) * mui * mui : mni * mni;
+    const float qj_ = hp.quadraticInExpansion ? -(muj < 0.f ? -1.f : 1.f) * muj * muj : mnj * mnj;
     const float ei = __fmaf_rn(Cq, qi_, __fmul_rn(mClci, li_));
     const float ej = __fmaf_rn(Cq, qj_, __fmul_rn(__fmul_rn(-Cl, csj), lj_));
     const float qai = __fmul_rn(0.5f, __fmul_rn(ei, iri)), qaj = __fmul_rn(0.5f, __fmul_rn(ej, irj));
@@ -207,7 +192,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     maxQ = fmaxf(maxQ, Qi);
     effQ += mj * Qi * Wi * irj;
     float Prhoi = Prhoi0, Prhoj = __fmul_rn(__fmul_rn(__fmul_rn(sOj, Pj), irj), irj);
-    if (!LEAN && epsT != 0.f) {
+    if (epsT != 0.f) {
       const float ti = Wi / (Hdeti * WnPerh), tj = Wj / (Hdetj * WnPerh);
       Prhoi = __fmul_rn(__fmul_rn(__fmul_rn(sOi, Pi + epsT * (ti * ti * ti * ti) * (Pi < 0.f ? -Pi : 0.f)), iri), iri);
       Prhoj = __fmul_rn(__fmul_rn(__fmul_rn(sOj, Pj + epsT * (tj * tj * tj * tj) * (Pj < 0.f ? -Pj : 0.f)), irj), irj);
@@ -218,9 +203,9 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     const float ddy = __fadd_rn(__fmul_rn(ci_, gwiy), __fmul_rn(cj_, gwjy));
     const float ddz = __fadd_rn(__fmul_rn(ci_, gwiz), __fmul_rn(cj_, gwjz));
     const float pax = __fmul_rn(-mj, ddx), pay = __fmul_rn(-mj, ddy), paz = __fmul_rn(-mj, ddz);
-    sumAdd(sdx, cdx, pax, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
-    sumAdd(sdy, cdy, pay, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
-    sumAdd(sdz, cdz, paz, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
+    sumAdd(sdx, cdx, pax, hp.plainSums);
+    sumAdd(sdy, cdy, pay, hp.plainSums);
+    sumAdd(sdz, cdz, paz, hp.plainSums);
     if (COMPAT) {
       float* out = pacc + paccSlot(k);
       out[0] = pax;
@@ -228,7 +213,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       out[64] = paz;
     }
     const float vg = vx * gwix + vy * gwiy + vz * gwiz;
-    sumAdd(se, ce, mj * (Prhoi + qai) * vg, LEAN == 2 ? 1 : (LEAN == 1 ? 0 : hp.plainSums));
+    sumAdd(se, ce, mj * (Prhoi + qai) * vg, hp.plainSums);
     const float mvx = mj * vx, mvy = mj * vy, mvz = mj * vz;
     D[0] -= mvx * gwix; D[1] -= mvx * gwiy; D[2] -= mvx * gwiz;
     D[3] -= mvy * gwix; D[4] -= mvy * gwiy; D[5] -= mvy * gwiz;
@@ -248,7 +233,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
     const float fwW = fw * WSPHi;
     m0 += fwW;
     m1x -= fwW * eix; m1y -= fwW * eiy; m1z -= fwW * eiz;
-    if (TENSOR) {   // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
+    {   // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
       const float ir = rsqrtf(fmaxf(rx * rx + ry * ry + rz * rz, 1.0e-30f));
       const float ir2 = ir * ir;
       const float w = fwW * WSPHi * (ir2 * ir2 * ir);
@@ -267,7 +252,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       entA = nl.nbr[nbSlot(i, 0, nl.cap)];
       const int j0 = (int)(entA & kIndexMask);
       pjA = P.posh[j0]; vjA = P.velm[j0]; thA = P.thermo[j0];
-      if (TENSOR) { hA0 = P.hten[j0]; hA1 = P.hten[P.stride + j0]; }
+      hA0 = P.hten[j0]; hA1 = P.hten[P.stride + j0];
     }
     if (cnt > 1) entB = nl.nbr[nbSlot(i, 1, nl.cap)];
     for (int q = 0; q < cnt; ++q) {
@@ -277,13 +262,13 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       if (q + 1 < cnt) {
         const int jn = (int)(entB & kIndexMask);
         pjA = P.posh[jn]; vjA = P.velm[jn]; thA = P.thermo[jn];
-        if (TENSOR) { hA0 = P.hten[jn]; hA1 = P.hten[P.stride + jn]; }
+        hA0 = P.hten[jn]; hA1 = P.hten[P.stride + jn];
         entA = entB;
       }
       if (q + 2 < cnt) entB = nl.nbr[nbSlot(i, q + 2, nl.cap)];
       slot(ent, pj, vj4, thj, hj0, hj1, nbSlot(i, q, nl.cap));
     }
-  } else if (PF >= 2) {
+  } else {
     // PF slots per iteration (slot q + 1 sits 32 entries after slot q): their
     // gathers are issued together, the next iteration's entries meanwhile
     constexpr int U = PF >= 2 ? PF : 2;
@@ -307,8 +292,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       for (int u = 0; u < U; ++u) {
         const int jj = (int)(e[u] & kIndexMask);
         pp[u] = P.posh[jj]; vv[u] = P.velm[jj]; tt[u] = P.thermo[jj];
-        aa[u] = zero4; bb[u] = zero4;
-        if (TENSOR) { aa[u] = P.hten[jj]; bb[u] = P.hten[P.stride + jj]; }
+        aa[u] = P.hten[jj]; bb[u] = P.hten[P.stride + jj];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) slot(e[u], pp[u], vv[u], tt[u], aa[u], bb[u], k0 + 32 * u);
@@ -317,16 +301,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       const long long k = nbSlot(i, q, nl.cap);
       const uint32_t ent = nl.nbr[k];
       const int jj = (int)(ent & kIndexMask);
-      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[jj] : zero4,
-           TENSOR ? P.hten[P.stride + jj] : zero4, k);
-    }
-  } else {
-    for (int q = 0; q < cnt; ++q) {
-      const long long k = nbSlot(i, q, nl.cap);
-      const uint32_t ent = nl.nbr[k];
-      const int jj = (int)(ent & kIndexMask);
-      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], TENSOR ? P.hten[jj] : zero4,
-           TENSOR ? P.hten[P.stride + jj] : zero4, k);
+      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], P.hten[jj],
+           P.hten[P.stride + jj], k);
     }
   }
   NodeAcc32 a;
@@ -342,7 +318,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
   for (int k = 0; k < 6; ++k) a.m2[k] = m2[k];
   a.h0 = hi0;
   a.h1 = hi1;
-  finalizeNode32<TENSOR>(F, i, MULTI ? li : list[i], a, cnt, hp, t.herm);
+  finalizeNode32<true>(F, i, li, a, cnt, hp, t.herm);
 }
 
 //------------------------------------------------------------------------------
@@ -761,7 +737,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
 
 //------------------------------------------------------------------------------
 // The ASPH pair loop (tensor H) of the lean path, in the arithmetic of
-// pairKernelFP32<TENSOR>: the same values in every sum the state reads.  What
+// pairKernelFP32: the same values in every sum the state reads.  What
 // bounds both is the L1 data pipe: five 16-byte gathers per slot and the table.
 // Here one 16-byte entry per side holds W' (W, which feeds only massDensitySum,
 // normalization and effViscousPressure, is the spline in registers or the
@@ -1315,19 +1291,19 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
                     HydroParams hp, float* pacc, int variant, bool inputs, const HalfStep& half, cudaStream_t s,
                     LaunchCounter* lc) {
   const int b = 128;
-  const bool multi = hp.numLists > 1;
-  // lean forms (no run-time flag in the loop) when the configuration allows
-  const bool lean = hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.plainSums;
   if (hp.asph) {
     const unsigned gb = gridFor(n, b);
 #define SPH_PAIR32T(X, C, LQ)                                                                     \
   do {                                                                                            \
-    if (variant & 1) pairKernelFP32<X, C, true, 4, true, LQ, true><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else pairKernelFP32<X, C, true, 3, true, LQ, true><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);             \
+    if (variant & 1) pairKernelFP32<X, C, 4, 1, LQ><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
+    else pairKernelFP32<X, C, 3, 1, LQ><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);             \
   } while (0)
-    // tensor H: NodeList test at run time; odd variants cap the registers at
-    // 128 (4 blocks per SM), even ones at 168 (3); variants 0-1 the pipelined
-    // loop, 2-3 (compatible energy, no XSPH, standard Q) two slots per iteration
+    // Lean path, one lane per node (303,912 nodes): variants 0 to 3 are two slots
+    // per iteration at three blocks per SM (579 us), one at four (593), two at four
+    // (578), three at two (567); below 100,000 nodes several lanes per node.
+    // Other options: odd variants cap the registers at 128 (four blocks), even
+    // ones at 168 (three); 0-1 the pipelined loop, 2-3 (compatible energy, no
+    // XSPH, standard Q) two slots per iteration.
     if (leanPair(hp) && !hp.limitedQ) {
       if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
 #define SPH_TEN(MI, SP, LA, U, MB) \
@@ -1350,8 +1326,8 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
       return;
     }
     if (!hp.xsph && hp.compatible && !hp.limitedQ && variant >= 2) {
-      if (variant & 1) pairKernelFP32<false, true, true, 4, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      else pairKernelFP32<false, true, true, 3, 2, false, true, 0><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
+      if (variant & 1) pairKernelFP32<false, true, 4, 2, false><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
+      else pairKernelFP32<false, true, 3, 2, false><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
     } else if (hp.xsph) {
       if (hp.compatible) { if (hp.limitedQ) SPH_PAIR32T(true, true, true); else SPH_PAIR32T(true, true, false); }
       else { if (hp.limitedQ) SPH_PAIR32T(true, false, true); else SPH_PAIR32T(true, false, false); }
