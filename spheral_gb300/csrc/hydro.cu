@@ -263,7 +263,7 @@ __device__ __noinline__ bool exactTensorCriterion(const Fields& F, const Grid& g
 //
 // TENSOR (ASPH): h^-1 of the FP32 mirror is the smallest eigenvalue of H, which
 // bounds |H r| from below for the culling, as does a diagonal bound of H^2
-// (itemBoxKernel); the test takes |H_i r|^2 and |H_j r|^2 from the tensor
+// (tensorDiagonal); the test takes |H_i r|^2 and |H_j r|^2 from the tensor
 // mirror, each with its node's band (tensorBand), and a batch that may hold a
 // candidate inside a band repeats its mask with the exact FP64 tensor criterion
 // for those.
@@ -730,8 +730,39 @@ __global__ void itemsKernel(const uint32_t* __restrict__ keys, long n, int shift
 // min z, min a), box[2k+1] = (max x, max y, max z, max a).
 // TENSOR adds what bounds |H r|^2 of all its nodes from below and the widest
 // tensor band: tbox[k] = (d_x, d_y, d_z, band) with H^2 - diag(d) positive
-// semidefinite for every node, d_a = (H^2)_aa - sum_b |(H^2)_ab| (Gershgorin;
-// less a margin for the FP32 products, and not below zero).
+// semidefinite for every node.  Per node (tensorDiagonal) one of two such d, and
+// a chunk takes the smallest of each component, which keeps the property:
+//  * d_a = (H^2)_aa - sum_b |(H^2)_ab| (Gershgorin) where all three are
+//    positive.  With one of them negative it bounds nothing, not even with
+//    that one raised to zero;
+//  * else 1 / (H^-2)_aa on the axis where that is largest and zero on the other
+//    two: r_a is row a of H^-1 times H r, so r_a^2 <= (H^-2)_aa |H r|^2 for any
+//    H.  Axis ratios above 1 + sqrt(2) reach it when the axes are tilted.
+// Both are lowered by more than the FP32 error of their terms (in units of the
+// largest eigenvalue the components are at most 1, their products in the rows
+// and the determinant then carry a few 2^-24 each).
+__device__ __forceinline__ void tensorDiagonal(const float4& a, const float4& b, float& dx, float& dy, float& dz) {
+  const float xy = fabsf(a.x * a.y + a.y * a.w + a.z * b.x), xz = fabsf(a.x * a.z + a.y * b.x + a.z * b.y);
+  const float yz = fabsf(a.y * a.z + a.w * b.x + b.x * b.y);
+  const float l2 = b.w * b.w, m = 1.0e-5f * l2;
+  dx = a.x * a.x + a.y * a.y + a.z * a.z - xy - xz - m;
+  dy = a.y * a.y + a.w * a.w + b.x * b.x - xy - yz - m;
+  dz = a.z * a.z + b.x * b.x + b.y * b.y - xz - yz - m;
+  if (dx >= 0.0f && dy >= 0.0f && dz >= 0.0f) return;
+  // rows of det(H) H^-1 in units of the largest eigenvalue
+  const float i = 1.0f / b.w, u = 5.9604645e-8f;
+  const float xx = a.x * i, hxy = a.y * i, hxz = a.z * i, yy = a.w * i, hyz = b.x * i, zz = b.y * i;
+  const float cxx = yy * zz - hyz * hyz, cxy = hxz * hyz - hxy * zz, cxz = hxy * hyz - hxz * yy;
+  const float cyy = xx * zz - hxz * hxz, cyz = hxy * hxz - xx * hyz, czz = xx * yy - hxy * hxy;
+  const float rx = cxx * cxx + cxy * cxy + cxz * cxz, ry = cxy * cxy + cyy * cyy + cyz * cyz;
+  const float rz = cxz * cxz + cyz * cyz + czz * czz;
+  const float r = fminf(rx, fminf(ry, rz));
+  const float q = fmaxf(0.0f, xx * cxx + hxy * cxy + hxz * cxz - 32.0f * u) / (sqrtf(r) + 32.0f * u);
+  const float d = (q * q) * l2 * (1.0f - 32.0f * u);
+  dx = r == rx ? d : 0.0f;
+  dy = r != rx && r == ry ? d : 0.0f;
+  dz = r != rx && r != ry ? d : 0.0f;
+}
 template <int W, bool TENSOR>
 __global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ items, const StepScratch* __restrict__ sc,
                                                      long n, Grid g, Fields32 P, float4* __restrict__ box,
@@ -747,12 +778,7 @@ __global__ void __launch_bounds__(128) itemBoxKernel(const int* __restrict__ ite
   float lo[NC] = {q.x, q.y, q.z, q.w}, hi[4] = {q.x, q.y, q.z, q.w};
   if (TENSOR) {
     const float4 a = P.hten[in ? j : s], b = P.hten[P.stride + (in ? j : s)];
-    const float xy = fabsf(a.x * a.y + a.y * a.w + a.z * b.x), xz = fabsf(a.x * a.z + a.y * b.x + a.z * b.y);
-    const float yz = fabsf(a.y * a.z + a.w * b.x + b.x * b.y);
-    const float m = 1.0e-5f * (b.w * b.w);
-    lo[4 % NC] = fmaxf(0.0f, a.x * a.x + a.y * a.y + a.z * a.z - xy - xz - m);
-    lo[5 % NC] = fmaxf(0.0f, a.y * a.y + a.w * a.w + b.x * b.x - xy - yz - m);
-    lo[6 % NC] = fmaxf(0.0f, a.z * a.z + b.x * b.x + b.y * b.y - xz - yz - m);
+    tensorDiagonal(a, b, lo[4 % NC], lo[5 % NC], lo[6 % NC]);
     lo[7 % NC] = -tensorBand(b.w, q.w, g);
   }
 #pragma unroll
