@@ -739,7 +739,7 @@ __device__ __forceinline__ void writeQGradient(const Fields32& P, long i, float*
 // of the loop's reduced sums.  The FP32 results go into the FP64 fields by
 // integer conversions (the FP64 pipe is ~1/64 of the FP32 rate).
 struct PairSums32 {
-  float w, mw, ve, g0, m1x, m1y, m1z;      // sum w, m w, (V/2) e w, |g|, |g| r
+  float w, mw, ve, g0, m1x, m1y, m1z;      // sum w, m w, (V/2) e a^3 w, |g|, |g| r
   float D[9], M[6], gx, gy, gz, maxE;      // sum u v r^T, u r r^T (xx xy xz yy yz zz), u (rho_j - rho_i) r; max e
   float xw, xdx, xdy, xdz;                 // XSPH
   double dvx, dvy, dvz, deps;
@@ -759,14 +759,13 @@ __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSu
   }
   put(F_RHOSUM, Hdeti * (a.mw + mi * W0));
   put(F_NORM, mi * irho * Hdeti * (a.w + W0));
-  // gradW_i = a_i^4 g_i r / |r|: the sums carry g_i r / |r|
-  const float f = SPLINE ? -timesSplineA(Hdeti * ai) : -(Hdeti * ai);
+  auto norm = [](float x) { return SPLINE ? timesSplineA(x) : x; };
   float D[9], Mm[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) D[k] = f * a.D[k];
-  Mm[0] = f * a.M[0]; Mm[1] = f * a.M[1]; Mm[2] = f * a.M[2];
-  Mm[3] = Mm[1];      Mm[4] = f * a.M[3]; Mm[5] = f * a.M[4];
-  Mm[6] = Mm[2];      Mm[7] = Mm[5];      Mm[8] = f * a.M[5];
+  for (int k = 0; k < 9; ++k) D[k] = -norm(a.D[k]);
+  Mm[0] = -norm(a.M[0]); Mm[1] = -norm(a.M[1]); Mm[2] = -norm(a.M[2]);
+  Mm[3] = Mm[1];         Mm[4] = -norm(a.M[3]); Mm[5] = -norm(a.M[4]);
+  Mm[6] = Mm[2];         Mm[7] = Mm[5];         Mm[8] = -norm(a.M[5]);
   const float detM = (Mm[0] * Mm[4] * Mm[8] + Mm[1] * Mm[5] * Mm[6] + Mm[2] * Mm[3] * Mm[7] -
                       Mm[0] * Mm[5] * Mm[7] - Mm[1] * Mm[3] * Mm[8] - Mm[2] * Mm[4] * Mm[6]);
   if (hp.correctVelGrad && fabsf(detM) > 1.0e-10f && numNb > 8) {
@@ -790,20 +789,18 @@ __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSu
   }
 #pragma unroll
   for (int k = 0; k < 9; ++k) { put(F_DVDX_XX + k, D[k]); put(F_M_XX + k, Mm[k]); }
-  const float fr = -f * irho;
-  put(F_GRADRHO_X, fr * a.gx); put(F_GRADRHO_Y, fr * a.gy); put(F_GRADRHO_Z, fr * a.gz);
+  put(F_GRADRHO_X, irho * norm(a.gx)); put(F_GRADRHO_Y, irho * norm(a.gy)); put(F_GRADRHO_Z, irho * norm(a.gz));
   const float trace = D[0] + D[4] + D[8];
   put(F_DRHODT, -rhoi * trace);
   const double vxi = F.f[F_VX][i], vyi = F.f[F_VY][i], vzi = F.f[F_VZ][i];
   F.f[F_DVDT_X][i] = a.dvx;
   F.f[F_DVDT_Y][i] = a.dvy;
   F.f[F_DVDT_Z][i] = a.dvz;
-  const double deps = a.deps * toDouble(Hdeti * ai);
   F.f[F_DEPSDT][i] =
-      hp.totalEnergy ? toDouble(mi) * ((vxi * a.dvx + vyi * a.dvy + vzi * a.dvz) + deps) : deps;
+      hp.totalEnergy ? toDouble(mi) * ((vxi * a.dvx + vyi * a.dvy + vzi * a.dvz) + a.deps) : a.deps;
   if (half.v) halfStepVelocity(F, i, a.dvx, a.dvy, a.dvz, F.f[F_DEPSDT][i], half);
   put(F_MAXQ, rhoi * a.maxE);
-  put(F_EFFQ, 2.0f * rhoi * Hdeti * a.ve);
+  put(F_EFFQ, 2.0f * rhoi * a.ve);
   float xw = a.xw;
   if (hp.xsph) {
     xw += Hdeti * mi * irho * W0;

@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
 // moments, FP32.  With H = a I both kernel gradients lie along the separation,
 // grad W = a^4 W'(a |r|) r / |r|, so the pair reduces to scalars times r:
 //
-//   u     = m_j W'_i / |r|              (velocity gradient, M, grad rho)
+//   u     = m_j a_i^4 W'_i / |r|        (velocity gradient, M, grad rho)
 //   mu    = a min(v . r, 0) / (a^2 r^2 + eps2),  e = mu (Cq mu - Cl c)
 //   C     = Prho + e / (2 rho)          (both sides)
 //   g     = -m_j (C_i a_i^4 W'_i + C_j a_j^4 W'_j) / |r|,  a_ij = g r.
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i];
   const int li = MULTI ? list[i] : 0;
   const float ai = pi.w, mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w;
-  const float ai2 = ai * ai, A4i = __fmul_rn(ai2, ai2);
+  const float ai2 = ai * ai, A4i = __fmul_rn(ai2, ai2), Hdeti = ai2 * ai;
   const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
   const float epsT = (float)hp.epsTensile, iWnPerh = 1.0f / (float)hp.WnPerh;
   const float etaCrit = (float)hp.etaCrit, iFold = 1.0f / (float)hp.etaFold;
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
     sumAdd(sdx, cdx, pax, plain);
     sumAdd(sdy, cdy, pay, plain);
     sumAdd(sdz, cdz, paz, plain);
-    const float u = mj * (gi * ir);
+    const float u = (mj * Gi) * ir;   // a^4 first: m r^2 alone leaves FP32 in CGS units of a star
     sumAdd(se, ce, __fmul_rn(Ci, __fmul_rn(u, vr)), plain);
     const float ux = u * rx, uy = u * ry, uz = u * rz;
     a.D[0] += vx * ux; a.D[1] += vx * uy; a.D[2] += vx * uz;
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
       a.w += w;
       a.mw += mj * w;
     }
-    a.ve += (mj * hirj) * (ei * w);
+    a.ve += (mj * hirj) * (ei * (Hdeti * w));
     a.maxE = fmaxf(a.maxE, ei);
     if (XSPH) {
       const float wx = 0.5f * (2.0f * mi * hiri * (ai2 * ai) * w + 2.0f * mj * hirj * (aj2 * aj) * wj);
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
         gx += gr * gwix; gy += gr * gwiy; gz += gr * gwiz;
         sw += w;
         smw += mj * w;
-        sve += (mj * hirj) * (ei * w);
+        sve += (mj * hirj) * (ei * (Hdeti * w));
         maxE = fmaxf(maxE, ei);
         const float wg = fabsf(gi);
         m0 += wg;
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
   a.rhoSum = Hdeti * smw; a.norm = mi * (2.0f * hiri) * Hdeti * sw;
   a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
   a.deps = kahanValue(se, ce);
-  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * Hdeti * sve;
+  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * sve;
   a.xw = a.xdx = a.xdy = a.xdz = 0.f;
   a.m0 = m0; a.m1x = m1x; a.m1y = m1y; a.m1z = m1z;
 #pragma unroll
@@ -861,7 +861,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
         gx += gr * gwix; gy += gr * gwiy; gz += gr * gwiz;
         sw += w;
         smw += mj * w;
-        sve += (mj * hirj) * (ei * w);
+        sve += (mj * hirj) * (ei * (Hdeti * w));
         maxE = fmaxf(maxE, ei);
         const float wg = fabsf(gi);
         m0 += wg;
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
   a.rhoSum = Hdeti * smw; a.norm = mi * (2.0f * hiri) * Hdeti * sw;
   a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
   a.deps = kahanValue(se, ce);
-  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * Hdeti * sve;
+  a.gx = gx; a.gy = gy; a.gz = gz; a.maxQ = rhoi * maxE; a.effQ = 2.0f * rhoi * sve;
   a.xw = a.xdx = a.xdy = a.xdz = 0.f;
   a.m0 = m0; a.m1x = m1x; a.m1y = m1y; a.m1z = m1z;
 #pragma unroll
