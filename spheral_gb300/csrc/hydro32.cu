@@ -440,8 +440,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
     const float di = __fmaf_rn(etai, etai, eps2), dj = __fmaf_rn(etaj, etaj, eps2);
     float ei, ej;
     if (LEAN) {
-      const float vn = fminf(vq, 0.f);
-      const float mni = __fdividef(__fmul_rn(ai, vn), di), mnj = __fdividef(__fmul_rn(aj, vn), dj);
+      // the quotient of coincident nodes is 0/0 with eps2 = 0: fminf makes it 0
+      const float mni = fminf(0.f, __fdividef(__fmul_rn(ai, vq), di)), mnj = fminf(0.f, __fdividef(__fmul_rn(aj, vq), dj));
       ei = __fmul_rn(mni, __fmaf_rn(Cq, mni, mClci));
       ej = __fmul_rn(mnj, __fmaf_rn(Cq, mnj, mClcj));
     } else {

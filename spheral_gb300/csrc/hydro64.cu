@@ -378,7 +378,9 @@ __global__ void __launch_bounds__(128) pair64Kernel(Fields F, const Node64* __re
         const double di = __fma_rn(etai, etai, hp.eps2), dj = __fma_rn(etaj, etaj, hp.eps2);
         const double f = vq * rcp64(di * dj);
         const double mui = (ai * f) * dj, muj = (aj * f) * di;
-        const bool neg = bits(vq) < 0;
+        // strictly negative: coincident nodes have v.r = -0 or +0, and with eps2 = 0 a
+        // quotient of 0/0 that no one-sided mu may take
+        const bool neg = (unsigned long long)bits(vq) > 0x8000000000000000ULL;
         const double mni = neg ? mui : 0.0, mnj = neg ? muj : 0.0;
         double ei, ej;
         if (lin || quad) {
