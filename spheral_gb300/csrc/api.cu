@@ -2010,6 +2010,7 @@ int sphgpu_set_domain(sphgpu_handle c, long n_ghost, sphgpu_exchange_fn fn, void
     throw Error(SPHGPU_E_UNSUPPORTED, "domain decomposition covers the SPH hydro step without gravity");
   c->nGhost = n_ghost;
   c->xfn = fn;
+  c->hp.decomposed = fn ? 1 : 0;
   c->xuser = user;
   API_END(c)
 }

@@ -74,6 +74,7 @@ struct HydroParams {
   // decomposition.  Set by the host just before the dt launches.
   const int* ghostOrig;
   long nOwn;
+  int decomposed;                // one domain of several: the pair sweep's form must not depend on its node count
 };
 __device__ __forceinline__ bool isGhost(const HydroParams& hp, long i) {
   return hp.ghostOrig != nullptr && hp.ghostOrig[i] >= hp.nOwn;

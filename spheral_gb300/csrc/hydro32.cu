@@ -1260,13 +1260,15 @@ void launchPrepareFP32(Fields F, Fields32 F32, long n, Grid g, cudaStream_t s, L
 
 constexpr int kDensU = 2, kGradhU = 4;   // slots per iteration of the density and grad-h sweeps
 // The lean path: one NodeList, compensated sums, the standard Q, no tensile
-// correction, compatible energy, no XSPH.  From kExactNodes on it keeps the
-// earlier arithmetic; below it the reduced one, with the spline in registers.
+// correction, compatible energy, no XSPH.  From kExactNodes on, and in every
+// domain of a decomposed run (the two sides of a pair across a cut are evaluated
+// by domains of different node counts), it keeps the earlier arithmetic; else the
+// reduced one, with the spline in registers.
 static bool leanPair(const HydroParams& hp) {
   return hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.plainSums && !hp.xsph && hp.compatible && hp.numLists == 1;
 }
-static bool exactPair(long n, const HydroParams& hp) { return leanPair(hp) && n >= kExactNodes; }
-static bool reducedPair(long n, const HydroParams& hp) { return leanPair(hp) && n < kExactNodes && hp.cubicSpline; }
+static bool exactPair(long n, const HydroParams& hp) { return leanPair(hp) && (n >= kExactNodes || hp.decomposed); }
+static bool reducedPair(long n, const HydroParams& hp) { return leanPair(hp) && !exactPair(n, hp) && hp.cubicSpline; }
 static int lanesTensor(long n) { return n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8)); }
 bool pairVariantsDiffer32(long n, const HydroParams& hp) {
   if (hp.crk) return n >= kCRKOneLane && !hp.xsph && hp.compatible;
