@@ -508,10 +508,17 @@ void buildGrid(sphgpu_ctx* c) {
 }
 
 int capFor(int m) { return std::max(32, ((m + m / 8 + 16 + 31) / 32) * 32); }
+// After a synchronisation: a node sort that gave up waiting has left empty lists
+// and a state in no order.
+void checkSort(sphgpu_ctx* c) {
+  if (!c->hstep->sortTimeout) return;
+  c->haveNeighbors = c->capCheckPending = false;
+  throw Error(SPHGPU_E_TIMEOUT, "a wait inside the node sort ran out");
+}
 int readMaxCount(sphgpu_ctx* c) {
   fetchScratch(c);
   CUDA_OK(cudaStreamSynchronize(c->stream));
-  if (c->hstep->sortTimeout) throw Error(SPHGPU_E_TIMEOUT, "a wait inside the node sort ran out");
+  checkSort(c);
   return c->hstep->maxCount;
 }
 void searchLists(sphgpu_ctx* c, bool write) {
@@ -625,8 +632,8 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
   {
     Scope sc(c->prof, "neighbor_items");
     launchItems(k, n, g.subShift, (uint32_t)space, c->cellEnd(), c->itemWidth, c->itemBound, g, c->hp.asph != 0,
-                c->f32(), c->items.as<int>(), c->chunkOf.as<int>(), c->itemBox.as<float4>(), c->step(), c->stream,
-                &c->lc);
+                c->f32(), c->items.as<int>(), c->chunkOf.as<int>(), c->counts.as<int>(), c->itemBox.as<float4>(),
+                c->step(), c->stream, &c->lc);
     c->check();
   }
   if (c->nbCapNext > 0) {   // adopt a smaller capacity decided at the previous build
@@ -656,7 +663,7 @@ void buildNeighbors(sphgpu_ctx* c, bool inStep = false) {
 bool resolveNeighbors(sphgpu_ctx* c) {
   if (!c->capCheckPending) return false;
   c->capCheckPending = false;
-  if (c->hstep->sortTimeout) throw Error(SPHGPU_E_TIMEOUT, "a wait inside the node sort ran out");
+  checkSort(c);
   int m = c->hstep->maxCount;
   bool regrown = false;
   while (m > c->nbCap) {   // overflow: enlarge and rewrite
@@ -877,6 +884,7 @@ double packageDt(sphgpu_ctx* c, int* reason, bool fusedDone = false) {
   fetchScratch(c);
   if (!c->fp32()) CUDA_OK(cudaMemcpyAsync(c->hsmall, d, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CUDA_OK(cudaStreamSynchronize(c->stream));
+  if (c->capCheckPending) checkSort(c);   // before the vote of the empty lists is taken for one
   double dt = c->hsmall[0];
   int r = (int)c->hsmall[1];
   if (c->fp32()) readVote(*c->hstep, dt, r);

@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(256) cellKeyKernel(Fields F, long n, Grid g, u
 // Gather of the carried fields into the new order, with what the same pass can
 // take along: the cells' node ranges (from the sorted keys) and the FP32
 // mirrors of the new order.  Indices and keys of a sort that gave up waiting
-// stay in range; the step then fails on the sort's flag.
+// stay in range here, and itemsKernel passes no lists on; the host then fails
+// the call on the sort's flag.
 __global__ void permuteKernel(Fields Fin, Fields Fout, const int* __restrict__ perm, const int* __restrict__ origIn,
                               int* __restrict__ origOut, const int* __restrict__ listIn, int* __restrict__ listOut,
                               const uint32_t* __restrict__ cellIn, uint32_t* __restrict__ cellOut, long n,
@@ -690,10 +691,18 @@ __global__ void __launch_bounds__(128, TENSOR ? 4 : 6) neighborMaskKernel(Fields
 // Work items of the search: every chunk of up to `width` consecutive nodes of
 // a cell, in items[], the chunks of one cell consecutive (their order among
 // cells is free); chunkOf[first node of the cell] = its first chunk.
+// The keys of a sort that gave up waiting are in no order: a cell may come up in
+// several runs, and its chunks would not fit items[].  Then there are no items
+// (the search finds nothing to do) and every list is empty, until the host reads
+// the flag.
 __global__ void itemsKernel(const uint32_t* __restrict__ keys, long n, int shift, uint32_t space,
                             const int* __restrict__ cellEnd, int width, int* __restrict__ items,
-                            int* __restrict__ chunkOf, StepScratch* __restrict__ sc) {
+                            int* __restrict__ chunkOf, int* __restrict__ counts, StepScratch* __restrict__ sc) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (sc->sortTimeout) {   // uniform
+    if (k < n) counts[k] = 0;
+    return;
+  }
   const int lane = threadIdx.x & 31;
   int chunks = 0, first = 0;
   if (k < n) {
@@ -1727,9 +1736,9 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
   lc->add(1);
 }
 void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
-                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, float4* box,
+                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, int* counts, float4* box,
                  StepScratch* sc, cudaStream_t s, LaunchCounter* lc) {
-  itemsKernel<<<gridFor(n, 256), 256, 0, s>>>(sortedKeys, n, shift, space, cellEnd, width, items, chunkOf, sc);
+  itemsKernel<<<gridFor(n, 256), 256, 0, s>>>(sortedKeys, n, shift, space, cellEnd, width, items, chunkOf, counts, sc);
   const unsigned gb = gridFor((long)nItemsBound * width, 128);
 #define SPH_BOX(W, T) itemBoxKernel<W, T><<<gb, 128, 0, s>>>(items, sc, n, g, P, box, box + 2 * n)
 #define SPH_BOXW(T) do { if (width == 8) SPH_BOX(8, T); else if (width == 16) SPH_BOX(16, T); else SPH_BOX(32, T); } while (0)

@@ -62,9 +62,10 @@ void launchPermute(const Fields& Fin, Fields Fout, const int* perm, const int* o
 void launchQGradient32(Fields F, float4* dvq, long n, cudaStream_t s, LaunchCounter* lc);
 // Work items of the group-cooperative search: the chunks of up to `width` (8,
 // 16 or 32) consecutive nodes of a cell, their first nodes, each cell's first
-// chunk and the chunks' bounding boxes; the count goes to sc->items.
+// chunk and the chunks' bounding boxes; the count goes to sc->items.  After a
+// sort that gave up waiting (sc->sortTimeout): no items, and counts[0, n) zero.
 void launchItems(const uint32_t* sortedKeys, long n, int shift, uint32_t space, const int* cellEnd, int width,
-                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, float4* box,
+                 int nItemsBound, Grid g, bool tensor, Fields32 P, int* items, int* chunkOf, int* counts, float4* box,
                  StepScratch* sc, cudaStream_t s, LaunchCounter* lc);
 // nItems: an upper bound on the item count (sizes the grid); sc->items holds
 // the count itself.  The largest count and the sum of all go to *sc.
