@@ -128,7 +128,7 @@ struct sphgpu_ctx {
   bool haveTable = false;
   std::vector<double> tw, tg, tg2, therm, twsum;
   double tmeta[9]{};
-  DBuf dTable;   // w | g | herm (FP64) then w32 | g32
+  DBuf dTable;   // w | g | herm (FP64) then the packed FP32 intervals (p32a | p32b)
 
   // particles
   long n = 0;
@@ -220,10 +220,8 @@ struct sphgpu_ctx {
     t.g = base + nc;
     t.herm = base + 2 * nc;
     float* b32 = reinterpret_cast<float*>(base + 2 * nc + therm.size());
-    t.w32 = b32;
-    t.g32 = b32 + nc;
-    t.p32a = reinterpret_cast<const float4*>(b32 + 2 * nc);
-    t.p32b = reinterpret_cast<const float2*>(b32 + 2 * nc + 4 * (nc / 3));
+    t.p32a = reinterpret_cast<const float4*>(b32);   // 2 nc + 2 hermN doubles in: a multiple of 16 bytes for any nc
+    t.p32b = reinterpret_cast<const float2*>(b32 + 4 * (nc / 3));
     return t;
   }
   StepScratch* step() { return stepScratch.as<StepScratch>(); }
@@ -302,15 +300,14 @@ void setTable(sphgpu_ctx* c, const double* w, const double* g, const double* g2,
   std::copy(c->tw.begin(), c->tw.end(), host.begin());
   std::copy(c->tg.begin(), c->tg.end(), host.begin() + nc);
   std::copy(c->therm.begin(), c->therm.end(), host.begin() + 2 * nc);
-  // FP32: plain copies (2 nc floats), then packed intervals (N1+1) x (w0 w1 w2 g0) and (N1+1) x (g1 g2)
+  // FP32: packed intervals (N1+1) x (w0 w1 w2 g0) and (N1+1) x (g1 g2)
   const size_t nint = (size_t)(N1 + 1);
-  std::vector<float> h32(2 * nc + 4 * nint + 2 * nint);
-  for (size_t k = 0; k < nc; ++k) { h32[k] = (float)c->tw[k]; h32[nc + k] = (float)c->tg[k]; }
+  std::vector<float> h32(4 * nint + 2 * nint);
   for (size_t k = 0; k < nint; ++k) {
-    float* A = &h32[2 * nc + 4 * k];
+    float* A = &h32[4 * k];
     A[0] = (float)c->tw[3 * k]; A[1] = (float)c->tw[3 * k + 1]; A[2] = (float)c->tw[3 * k + 2];
     A[3] = (float)c->tg[3 * k];
-    float* B = &h32[2 * nc + 4 * nint + 2 * k];
+    float* B = &h32[4 * nint + 2 * k];
     B[0] = (float)c->tg[3 * k + 1]; B[1] = (float)c->tg[3 * k + 2];
   }
   const size_t bytes = host.size() * sizeof(double) + h32.size() * sizeof(float);

@@ -10,8 +10,6 @@ struct TableDev {
   const double* w;      // 3*(N1+1) quadratic coefficients of W
   const double* g;      // 3*(N1+1) quadratic coefficients of dW/deta
   const double* herm;   // 2*hermN Hermite knots of the nperh lookup (values, slopes)
-  const float* w32;     // FP32 copies for the FP32 pair loop
-  const float* g32;
   const float4* p32a;   // per interval (w0, w1, w2, g0) in FP32
   const float2* p32b;   // per interval (g1, g2) in FP32
 };
