@@ -221,7 +221,7 @@ struct sphgpu_ctx {
     t.herm = base + 2 * nc;
     float* b32 = reinterpret_cast<float*>(base + 2 * nc + therm.size());
     t.p32a = reinterpret_cast<const float4*>(b32);   // 2 nc + 2 hermN doubles in: a multiple of 16 bytes for any nc
-    t.p32b = reinterpret_cast<const float2*>(b32 + 4 * (nc / 3));
+    t.p32b = reinterpret_cast<const float2*>(b32 + 4 * (size_t)(hp.pack32N1 + 1));
     return t;
   }
   StepScratch* step() { return stepScratch.as<StepScratch>(); }
@@ -300,15 +300,45 @@ void setTable(sphgpu_ctx* c, const double* w, const double* g, const double* g2,
   std::copy(c->tw.begin(), c->tw.end(), host.begin());
   std::copy(c->tg.begin(), c->tg.end(), host.begin() + nc);
   std::copy(c->therm.begin(), c->therm.end(), host.begin() + 2 * nc);
-  // FP32: packed intervals (N1+1) x (w0 w1 w2 g0) and (N1+1) x (g1 g2)
-  const size_t nint = (size_t)(N1 + 1);
+  // FP32: packed intervals (w0 w1 w2 g0) and (g1 g2).  The sweeps take an interval
+  // behind the last as zero, so the intervals have to end at the kernel extent.  A
+  // table over another range (one of another kernel than the configured) is laid
+  // out anew over [0, extent]: the quadratic through each interval's ends and
+  // middle, of the lookup that the FP64 sweeps make below the extent.
+  c->hp.pack32N1 = N1;
+  c->hp.pack32Xstep = meta[1];
+  std::vector<double> pw = c->tw, pg = c->tg;
+  if (std::fabs((N1 + 1) * meta[1] - c->kernelExtent) > 1.0e-9 * c->kernelExtent) {
+    const int nint = kMaxTable / 3;
+    const double step = c->kernelExtent / nint;
+    auto refit = [&](const std::vector<double>& q, std::vector<double>& out) {
+      auto at = [&](double eta) {
+        const size_t i0 = 3u * std::min((size_t)N1, size_t(eta / meta[1]));
+        return q[i0] + (q[i0 + 1] + q[i0 + 2] * eta) * eta;
+      };
+      out.resize(3 * (size_t)nint);
+      for (int k = 0; k < nint; ++k) {
+        const double a = k * step, b = a + step, m = 0.5 * (a + b);
+        const double fa = at(a), fm = at(m), fb = at(b);
+        const double c2 = 2.0 * (fa - 2.0 * fm + fb) / (step * step), c1 = (fb - fa) / step;   // about the middle
+        out[3 * k] = fm - c1 * m + c2 * m * m;
+        out[3 * k + 1] = c1 - 2.0 * c2 * m;
+        out[3 * k + 2] = c2;
+      }
+    };
+    refit(c->tw, pw);
+    refit(c->tg, pg);
+    c->hp.pack32N1 = nint - 1;
+    c->hp.pack32Xstep = step;
+  }
+  const size_t nint = (size_t)(c->hp.pack32N1 + 1);
   std::vector<float> h32(4 * nint + 2 * nint);
   for (size_t k = 0; k < nint; ++k) {
     float* A = &h32[4 * k];
-    A[0] = (float)c->tw[3 * k]; A[1] = (float)c->tw[3 * k + 1]; A[2] = (float)c->tw[3 * k + 2];
-    A[3] = (float)c->tg[3 * k];
+    A[0] = (float)pw[3 * k]; A[1] = (float)pw[3 * k + 1]; A[2] = (float)pw[3 * k + 2];
+    A[3] = (float)pg[3 * k];
     float* B = &h32[4 * nint + 2 * k];
-    B[0] = (float)c->tg[3 * k + 1]; B[1] = (float)c->tg[3 * k + 2];
+    B[0] = (float)pg[3 * k + 1]; B[1] = (float)pg[3 * k + 2];
   }
   const size_t bytes = host.size() * sizeof(double) + h32.size() * sizeof(float);
   c->dTable.ensure(bytes);
@@ -1381,8 +1411,8 @@ int sphgpu_set_kernel_table(sphgpu_handle c, const double* w, const double* grad
   if (!w || !grad || !grad2 || !nperh || !wsum || !meta) throw Error(SPHGPU_E_ARG, "null table pointer");
   // the installed cubic B-spline set again stays the cubic B-spline
   const size_t nc = meta[0] >= 1.0 && meta[0] < kMaxTable ? 3 * ((size_t)meta[0] + 1) : 0;
-  const bool same = c->hp.cubicSpline && nc == c->tw.size() && std::equal(w, w + nc, c->tw.begin()) &&
-                    std::equal(grad, grad + nc, c->tg.begin());
+  const bool same = c->hp.cubicSpline && nc == c->tw.size() && meta[1] == c->tmeta[1] &&
+                    std::equal(w, w + nc, c->tw.begin()) && std::equal(grad, grad + nc, c->tg.begin());
   setTable(c, w, grad, grad2, nperh, wsum, meta, same);
   refreshParams(c);
   API_END(c)

@@ -52,6 +52,8 @@ struct HydroParams {
   int numLists;
   int tableN1;        // N1 of the quadratic table
   double tableXstep;  // interval of the quadratic table
+  int pack32N1;       // the same of the packed FP32 table, whose intervals end at the kernel extent
+  double pack32Xstep;
   double extent;      // kernel extent
   int cubicSpline;    // the table is the built-in cubic B-spline's (fine enough for FP32)
   int hermN;          // Hermite knots of the nperh lookup

@@ -89,9 +89,9 @@ __device__ __forceinline__ void loadRKC(const Fields32& P, long j, float* C) {
 #define SPH_CRK_SETUP_ALL()                                                       \
   __shared__ float4 ta[kTab32];                                               \
   __shared__ float2 tb[kTab32];                                               \
-  loadTable32(ta, tb, t, hp.tableN1);                                         \
+  loadTable32(ta, tb, t, hp.pack32N1);                                         \
   __syncthreads();                                                            \
-  const Kernel32<0> T{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};      \
+  const Kernel32<0> T{ta, tb, hp.pack32N1, (float)(1.0 / hp.pack32Xstep)};      \
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;        \
   const int sub = threadIdx.x % L;                                            \
   const bool live = node < n;                                                 \

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
                                                       float* __restrict__ pacc) {
   __shared__ float4 ta[kMaxTable / 3];
   __shared__ float2 tb[kMaxTable / 3];
-  const int nint = hp.tableN1 + 1;
+  const int nint = hp.pack32N1 + 1;
   for (int k = threadIdx.x; k < nint; k += blockDim.x) { ta[k] = t.p32a[k]; tb[k] = t.p32b[k]; }
   __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -64,8 +64,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
   const float mi = vi.w, rhoi = thi.x, Pi = thi.y, csi = thi.z, sOi = thi.w;
   const float4 hi0 = P.hten[i], hi1 = P.hten[P.stride + i];
   const float Hdeti = hi1.z;
-  const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.tableXstep);
-  const int N1 = hp.tableN1;
+  const float extent = (float)hp.extent, invStep = (float)(1.0 / hp.pack32Xstep);
+  const int N1 = hp.pack32N1;
   const float Cl = (float)hp.Cl, Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
   const float epsT = (float)hp.epsTensile, WnPerh = (float)hp.WnPerh;
   float DQi[9];   // the limited Q's DvDx of node i
@@ -353,14 +353,14 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   constexpr int NT = KERN ? 1 : kTab32;
   __shared__ float4 ta[NT];
   __shared__ float2 tb[NT];
-  if (!KERN) loadTable32(ta, tb, t, hp.tableN1);
+  if (!KERN) loadTable32(ta, tb, t, hp.pack32N1);
   __syncthreads();
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
   const int sub = threadIdx.x % L;
   const bool live = node < n;
   if (L == 1 && !live) return;
   const long i = live ? node : n - 1;   // whole groups run to the shuffles
-  const Kernel32<KERN> K{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};
+  const Kernel32<KERN> K{ta, tb, hp.pack32N1, (float)(1.0 / hp.pack32Xstep)};
   int ci[3];
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
@@ -576,8 +576,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
                                                               HydroParams hp, float* __restrict__ pacc, HalfStep half) {
   __shared__ float4 tg[kTab32];   // (g0, g1, g2, w0)
   __shared__ float2 tw[SPLINE ? 1 : kTab32];
-  for (int k = threadIdx.x; k <= hp.tableN1 + 1; k += blockDim.x) {
-    const bool in = k <= hp.tableN1;
+  for (int k = threadIdx.x; k <= hp.pack32N1 + 1; k += blockDim.x) {
+    const bool in = k <= hp.pack32N1;
     const float4 A = in ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float2 B = in ? t.p32b[k] : make_float2(0.f, 0.f);
     tg[k] = make_float4(A.w, B.x, B.y, A.x);
@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
   __syncthreads();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int N1 = hp.tableN1;
-  const float invStep = (float)(1.0 / hp.tableXstep);
+  const int N1 = hp.pack32N1;
+  const float invStep = (float)(1.0 / hp.pack32Xstep);
   int ci[3];
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
@@ -754,8 +754,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
                                                                 HalfStep half) {
   __shared__ float4 tg[kTab32];   // (g0, g1, g2, w0)
   __shared__ float2 tw[SPLINE ? 1 : kTab32];
-  for (int k = threadIdx.x; k <= hp.tableN1 + 1; k += blockDim.x) {
-    const bool in = k <= hp.tableN1;
+  for (int k = threadIdx.x; k <= hp.pack32N1 + 1; k += blockDim.x) {
+    const bool in = k <= hp.pack32N1;
     const float4 A = in ? t.p32a[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float2 B = in ? t.p32b[k] : make_float2(0.f, 0.f);
     tg[k] = make_float4(A.w, B.x, B.y, A.x);
@@ -767,8 +767,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
   const bool live = node < n;
   if (L == 1 && !live) return;
   const long i = live ? node : n - 1;
-  const int N1 = hp.tableN1;
-  const float invStep = (float)(1.0 / hp.tableXstep);
+  const int N1 = hp.pack32N1;
+  const float invStep = (float)(1.0 / hp.pack32Xstep);
   int ci[3];
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Field
   constexpr int NT = KERN ? 1 : kTab32;
   __shared__ float4 ta[NT];
   __shared__ unsigned long long sv[sweepBlock(L) / 32];
-  if (!KERN) loadTable32(ta, nullptr, t, hp.tableN1);
+  if (!KERN) loadTable32(ta, nullptr, t, hp.pack32N1);
   __syncthreads();
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
   const int sub = threadIdx.x % L;
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Field
   const float4 pi = P.posh[i], vi = P.velm[i];
   const bool multi = !LEAN && hp.numLists > 1;
   const int li = multi ? list[i] : 0;
-  const Kernel32<KERN> K{ta, nullptr, hp.tableN1, (float)(1.0 / hp.tableXstep)};
+  const Kernel32<KERN> K{ta, nullptr, hp.pack32N1, (float)(1.0 / hp.pack32Xstep)};
   float s = 0.f, c = 0.f, worst = 0.0f;
   // the node scale of GenericHydro::dt: 1/h, the largest eigenvalue of H
   const float lmaxi = TENSOR ? P.hten[P.stride + i].w : pi.w;
@@ -1045,14 +1045,14 @@ __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields3
   constexpr int NT = KERN ? 1 : kTab32;
   __shared__ float4 ta[NT];
   __shared__ float2 tb[NT];
-  if (!KERN) loadTable32(ta, tb, t, hp.tableN1);
+  if (!KERN) loadTable32(ta, tb, t, hp.pack32N1);
   __syncthreads();
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
   const int sub = threadIdx.x % L;
   const bool live = node < n;
   if (L == 1 && !live) return;
   const long i = live ? node : n - 1;
-  const Kernel32<KERN> K{ta, tb, hp.tableN1, (float)(1.0 / hp.tableXstep)};
+  const Kernel32<KERN> K{ta, tb, hp.pack32N1, (float)(1.0 / hp.pack32Xstep)};
   int ci[3];
   unpackCell(P.cell[i], ci);
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
