@@ -884,12 +884,19 @@ void setGhostParams(sphgpu_ctx* c) {
 // Blocks of a vote sweep at most (up to 8 lanes per node in the FP64 sweep).
 long voteBlocks(long n) { return (8 * n + 127) / 128; }
 
-// The vote of the mixed sweeps: the value with its low bits as the reason.
+// The vote of the mixed sweeps: FP32 limits with the reason in the low bits, or
+// FP64 limits by reason.
 void readVote(const StepScratch& h, double& v, int& reason) {
-  if (h.voteKey == ~0ULL) { v = std::numeric_limits<double>::max(); reason = -1; return; }
-  const unsigned long long b = h.voteKey & ~7ULL;
-  std::memcpy(&v, &b, sizeof v);
-  reason = (int)(h.voteKey & 7ULL);
+  v = std::numeric_limits<double>::max();
+  reason = -1;
+  auto take = [&](unsigned long long bits, int r) {
+    double x;
+    std::memcpy(&x, &bits, sizeof x);
+    if (x < v) { v = x; reason = r; }
+  };
+  if (h.voteKey != ~0ULL) take(h.voteKey & ~7ULL, (int)(h.voteKey & 7ULL));
+  for (int k = 0; k < kDtReasons; ++k)
+    if (h.votes[k] != ~0ULL) take(h.votes[k], k);
 }
 
 double packageDt(sphgpu_ctx* c, int* reason, bool fusedDone = false) {

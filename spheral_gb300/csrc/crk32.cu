@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) crkDensity32(Fields F, Fields32
   P.thermo[i].x = (float)rho;
   }
   if (sc)
-    voteNode32<false>(F, hp, list, i, owner && !isGhost(hp, i), pi.w, vi, worst, maxNperh, &sc->voteEst, &sc->voteKey);
+    voteNode32<false>(F, hp, list, i, owner && !isGhost(hp, i), pi.w, vi, worst, maxNperh, sc);
 }
 
 //------------------------------------------------------------------------------

@@ -90,13 +90,17 @@ __device__ __forceinline__ float timesSplineA(float x) {
   return __fmaf_rn(x, hi, __fmul_rn(x, lo));
 }
 
+__device__ __forceinline__ void resetVote(StepScratch* sc) {
+  sc->voteKey = ~0ULL;
+  for (int k = 0; k < kDtReasons; ++k) sc->votes[k] = ~0ULL;
+  sc->voteEst = 0x7f7fffffu;   // FLT_MAX
+}
 __device__ __forceinline__ void resetScratch(StepScratch* sc) {
   for (int k = 0; k < 4; ++k) sc->bounds[k] = 0x7fffffffffffffffLL;
   for (int k = 4; k < 10; ++k) sc->bounds[k] = k < 7 ? (long long)0x8000000000000000ULL : 0LL;
   sc->bad = sc->sortTimeout = sc->maxCount = sc->items = 0;
   for (int k = 0; k < kEntrySums; ++k) sc->entries[k] = 0ULL;
-  sc->voteKey = ~0ULL;
-  sc->voteEst = 0x7f7fffffu;   // FLT_MAX
+  resetVote(sc);
 }
 
 __device__ __forceinline__ void lookupPacked(const float4* __restrict__ ta, const float2* __restrict__ tb, int N1,
@@ -830,9 +834,10 @@ __device__ __forceinline__ void finalizePair32(Fields& F, long i, int li, PairSu
 }
 
 //------------------------------------------------------------------------------
-// Time-step vote.  The smallest limit travels as one 64-bit word, the bits of
-// a positive double order as integers: the mixed step's FP32 limits carry the
-// reason code in the low mantissa bits that a widened float leaves zero.
+// Time-step vote; the bits of positive doubles order as integers.  FP32 limits
+// travel as one 64-bit word, the reason code in the low mantissa bits that a
+// widened float leaves zero.  FP64 limits need all their bits: one minimum per
+// reason.
 //------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long warpMin64(unsigned long long v) {
 #pragma unroll
@@ -842,8 +847,8 @@ __device__ __forceinline__ unsigned long long warpMin64(unsigned long long v) {
   }
   return v;
 }
-__device__ __forceinline__ unsigned long long dtKey(double v, int reason) {
-  return ((unsigned long long)__double_as_longlong(v) & ~7ULL) | (unsigned)reason;
+__device__ __forceinline__ unsigned long long dtKey(float v, int reason) {
+  return (unsigned long long)__double_as_longlong(toDouble(v)) | (unsigned)reason;
 }
 
 // FP32 node limits of GenericHydro::dt (GenericHydro.cc:113-381): the smallest
@@ -868,12 +873,12 @@ __device__ __forceinline__ float nodeDt32(float ns, float cs, float maxQ, float 
 // The vote of GenericHydro::dt for one node in the precision of its FP64 limits.
 // Each node first forms all its limits in FP32 (worst: the largest
 // (max(a_i, a_j) |v_ij|)^2 of its pairs); only a node whose FP32 limit is within
-// 1e-4 of the smallest seen so far (estOut, which only falls) can hold the
-// minimum and repeats its node limits in FP64.  Whole warps call it.
+// 1e-4 of the smallest seen so far (voteEst, which only falls) can hold the
+// minimum and repeats its limits in FP64.  Whole warps call it.
 template <bool TENSOR>
 __device__ __forceinline__ void voteNode32(const Fields& F, const HydroParams& hp, const int* __restrict__ list, long i,
                                            bool votes, float lmaxi, const float4& vi, float worst, double maxNperh,
-                                           unsigned* __restrict__ estOut, unsigned long long* __restrict__ dtOut) {
+                                           StepScratch* __restrict__ sc) {
   const float bestPair = worst > 0.0f ? rsqrtf(worst) : 3.0e38f;
   float est = 3.0e38f;
   const NodeListParams Li = hp.lists[list[i]];
@@ -886,8 +891,8 @@ __device__ __forceinline__ void voteNode32(const Fields& F, const HydroParams& h
                    sqrtf(ax * ax + ay * ay + az * az), hp.useVelMagDt != 0, bestPair / (float)maxNperh, reason);
   }
   const float wmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(est)));
-  if ((threadIdx.x & 31) == 0 && wmin < 3.0e38f) atomicMin(estOut, __float_as_uint(wmin));
-  const float seen = __uint_as_float(*(volatile unsigned*)estOut);
+  if ((threadIdx.x & 31) == 0 && wmin < 3.0e38f) atomicMin(&sc->voteEst, __float_as_uint(wmin));
+  const float seen = __uint_as_float(*(volatile unsigned*)&sc->voteEst);
   // NaN compares false: a node with a NaN limit takes the FP64 limits too
   if (votes && !(est > fminf(seen, wmin) * 1.0001f)) {
     const double tiny = DBL_EPSILON;
@@ -911,9 +916,9 @@ __device__ __forceinline__ void voteNode32(const Fields& F, const HydroParams& h
       const double velDt = nodeScalei / (vmag + 1.0e-10);
       if (velDt < best) { best = velDt; reason = 4; }
     }
-    const double pairDt = (double)bestPair / maxNperh;
+    const double pairDt = (worst > 0.0f ? 1.0 / sqrt((double)worst) : 3.0e38) / maxNperh;
     if (pairDt < best) { best = pairDt; reason = 5; }
-    if (reason >= 0) atomicMin(dtOut, dtKey(best, reason));
+    if (reason >= 0) atomicMin(&sc->votes[reason], (unsigned long long)__double_as_longlong(best));
   }
 }
 

@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(sweepBlock(L)) densityKernel32(Fields F, Field
                                   divv, sqrtf(vi.x * vi.x + vi.y * vi.y + vi.z * vi.z),
                                   sqrtf(ax * ax + ay * ay + az * az), hp.useVelMagDt != 0,
                                   (worst > 0.0f ? rsqrtf(worst) : 3.0e38f) / maxNperh, reason);
-      if (reason >= 0) key = dtKey(toDouble(best), reason);
+      if (reason >= 0) key = dtKey(best, reason);
     }
   }
   if (DT) {
@@ -1101,15 +1101,12 @@ __global__ void __launch_bounds__(sweepBlock(L)) gradhKernel32(Fields F, Fields3
 
 //------------------------------------------------------------------------------
 // GenericHydro::dt with the pairwise velocity limit in FP32 and the node
-// limits in FP64.  Each node first forms all its limits in FP32; only a node
-// whose FP32 limit is within 1e-4 of the smallest seen so far (estOut, which
-// only falls) can hold the minimum and repeats its node limits in FP64.
+// limits in FP64 (voteNode32).
 //------------------------------------------------------------------------------
 template <bool TENSOR, bool MIR, int L, int U>
 __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const int* __restrict__ list, long n, Grid g,
                                                   NeighborLists nl, HydroParams hp, double maxNperh,
-                                                  unsigned* __restrict__ estOut,
-                                                  unsigned long long* __restrict__ dtOut) {
+                                                  StepScratch* __restrict__ sc) {
   const long node = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L;
   const int sub = threadIdx.x % L;
   const bool live = node < n;
@@ -1134,13 +1131,10 @@ __global__ void __launch_bounds__(128) dtKernel32(Fields F, Fields32 P, const in
         worst = fmaxf(worst, (am * am) * (dx * dx + dy * dy + dz * dz));
       });
   if (L > 1) worst = laneMax<L>(worst);
-  voteNode32<TENSOR>(F, hp, list, i, live && sub == 0 && !isGhost(hp, i), lmaxi, vi, worst, maxNperh, estOut, dtOut);
+  voteNode32<TENSOR>(F, hp, list, i, live && sub == 0 && !isGhost(hp, i), lmaxi, vi, worst, maxNperh, sc);
 }
 
-__global__ void dtInitKernel(StepScratch* __restrict__ sc) {
-  sc->voteKey = ~0ULL;
-  sc->voteEst = 0x7f7fffffu;   // FLT_MAX
-}
+__global__ void dtInitKernel(StepScratch* __restrict__ sc) { resetVote(sc); }
 
 //------------------------------------------------------------------------------
 // Compatible-energy sweep of the mixed mode (SpecificThermalEnergyPolicy.cc:110-173).
@@ -1465,8 +1459,8 @@ void launchDtFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Neigh
   const int L = lanesSweep(n);
 #define SPH_DT(LA)                                                                                                     \
   do {                                                                                                                 \
-    if (hp.asph) dtKernel32<true, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, &sc->voteEst, &sc->voteKey); \
-    else dtKernel32<false, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, &sc->voteEst, &sc->voteKey);        \
+    if (hp.asph) dtKernel32<true, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, sc); \
+    else dtKernel32<false, true, LA, 2><<<gridFor(n * LA, 128), 128, 0, s>>>(F, F32, list, n, g, nl, hp, maxNperh, sc);        \
   } while (0)
   SPH_BY_LANES(L, SPH_DT)
 #undef SPH_DT

@@ -22,6 +22,7 @@ struct NeighborLists {
 };
 
 constexpr int kEntrySums = 32;
+constexpr int kDtReasons = 6;
 // Values the kernels of a step leave for the host, one per handle.  Reset by
 // the first kernel of a neighbour build.
 struct StepScratch {
@@ -31,8 +32,9 @@ struct StepScratch {
   int maxCount;                // largest neighbour count of the search
   int items;                   // work chunks of the search
   unsigned long long entries[kEntrySums];   // neighbour entries (partial sums)
-  unsigned long long voteKey;  // smallest dtKey of the mixed sweep
-  unsigned voteEst, pad;       // running FP32 estimate of the dt query
+  unsigned long long voteKey;  // time-step vote of FP32 limits: the smallest dtKey
+  unsigned long long votes[kDtReasons];   // of FP64 limits: the smallest of each reason, as bits
+  unsigned voteEst, pad;       // their running FP32 estimate
 };
 
 // Reductions ------------------------------------------------------------------
