@@ -408,14 +408,8 @@ __global__ void cellFinalKernel(TreeCell* __restrict__ cells, long long numCells
     const TreeNode p = tpos[cl.start];
     cl.x = p.x; cl.y = p.y; cl.z = p.z; cl.M = p.m;
   } else {
-    // one reciprocal, each quotient with its residual: a division's rounding but
-    // for rare last-bit cases, at a third of its FP64 operations
-    const double r = fabs(sm.w) > 1.0e-290 ? dev::rcp64(sm.w) : 1.0 / sm.w;
-    auto quotient = [&](double a) {
-      const double q = a * r;
-      return __fma_rn(__fma_rn(-q, sm.w, a), r, q);
-    };
-    cl.x = quotient(sm.x); cl.y = quotient(sm.y); cl.z = quotient(sm.z); cl.M = sm.w;
+    // correctly rounded, as the reference's: the centre decides which cells open
+    cl.x = __ddiv_rn(sm.x, sm.w); cl.y = __ddiv_rn(sm.y, sm.w); cl.z = __ddiv_rn(sm.z, sm.w); cl.M = sm.w;
   }
   // Geometric centre: xmin + (ix + 0.5) * cellsize, cellsize = boxLength / 2^level.
   const uint64_t key = skey[cl.start];
