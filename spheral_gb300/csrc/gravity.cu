@@ -41,10 +41,14 @@
 // (hi + lo) coordinates -- the separation (hi_c - hi_i) + (lo_c - lo_i)
 // carries FP32 relative precision at any distance -- and sums the terms with
 // compensated (Kahan) FP32 accumulators that leave the kernel as the FP64
-// value s - c.  The far/near decision compares the FP32 r^2 with the FP32
-// threshold; inside a guard band of +-4e-6 (far above the FP32 error of both)
-// it is retaken in FP64 with the reference's expression, so the set of far
-// cells and opened leaves is the FP64 walk's.
+// value s - c.
+//
+// Decisions.  Both walks compare an FP32 r^2 with FP32 thresholds and retake the
+// decision in FP64 with the reference's expression inside a guard band, so the
+// set of far cells and opened leaves is the reference's.  The double-float
+// coordinates count from the corner of the bounding box: they are exact to
+// 2^-49 of its length L wherever the system lies, a separation to 2^-46 L, and
+// the band is twice that in r and 4e-6 in r^2 for the FP32 roundings.
 #include "kernels.cuh"
 #include "packed32.cuh"
 #include "recip64.cuh"
@@ -92,8 +96,8 @@ __device__ __forceinline__ TreeNode loadNode(const TreeNode* __restrict__ p) {
   return TreeNode{a.x, a.y, b.x, b.y};
 }
 
-// What a walk reads of a cell it visits: the double-float centre of mass in
-// pairs for the packed operations, the mass, and the decision thresholds.  With
+// What a walk reads of a cell it visits: the double-float centre of mass (from
+// the box corner) in pairs for the packed operations, the mass, and the decision thresholds.  With
 // r2 the FP32 squared separation, r2 > hi: the cell's monopole applies (a far
 // cell, or a one-node leaf, whose monopole is its node); r2 < lo: it does not
 // (an internal cell is opened, a one-node leaf is the node itself); between
@@ -244,8 +248,8 @@ __global__ void treeKeyKernel(Fields F, long n, const double* __restrict__ box, 
 
 // Tree-ordered node data.  Indices of a sort that gave up waiting stay in
 // range; the evaluation then fails on the sort's flag.
-__global__ void treeNodesKernel(Fields F, const int* __restrict__ vals, long n, TreeNode* __restrict__ tpos,
-                                TreeNode32* __restrict__ tpos32) {
+__global__ void treeNodesKernel(Fields F, const int* __restrict__ vals, long n, const double* __restrict__ box,
+                                TreeNode* __restrict__ tpos, TreeNode32* __restrict__ tpos32) {
   const long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int i = (int)min((unsigned)vals[k], (unsigned)(n - 1));
@@ -253,9 +257,9 @@ __global__ void treeNodesKernel(Fields F, const int* __restrict__ vals, long n, 
   tpos[k] = TreeNode{x, y, z, m};
   if (tpos32) {
     TreeNode32 t;
-    splitDF(x, t.xh, t.xl);
-    splitDF(y, t.yh, t.yl);
-    splitDF(z, t.zh, t.zl);
+    splitDF(x - box[0], t.xh, t.xl);
+    splitDF(y - box[1], t.yh, t.yl);
+    splitDF(z - box[2], t.zh, t.zl);
     t.m = (float)m;
     t.pad = 0.0f;
     tpos32[k] = t;
@@ -327,33 +331,40 @@ __global__ void linkKernel(const TreeCell* __restrict__ cells, long long numCell
   pending[c] = m;
 }
 
+// The guard band of the FP32 r^2 around a squared distance d2, in a box of
+// length L: r^2 above hi is above d2, below lo below it.  Values near underflow
+// are left to FP64.
+__device__ __forceinline__ void guardBand(float d2, float L, float& hi, float& lo) {
+  constexpr float kBand = 4.0e-6f, kTiny = 1.0e-30f, kAbs = 2.842171e-14f;   // 2^-45
+  const float d = sqrtf(d2), up = d + kAbs * L, down = fmaxf(d - kAbs * L, 0.0f);
+  hi = fmaxf((up * up) * (1.0f + kBand), kTiny);
+  lo = (down * down) * (1.0f - kBand);
+  if (!(lo > kTiny)) lo = -1.0f;
+}
 // The walks' thresholds (TreeCell32) from the squared opening distance and,
 // for a one-node leaf, the separation limit 1e-10 eps^2 below which the node
-// does not act.  The guard bands (4e-6, and 1e-3 for the limit) are far above
-// the FP32 error of r2; values near underflow are left to FP64.
-__device__ __forceinline__ void setThresholds(TreeCell32& o, double open2, double soft2) {
-  constexpr float kBand = 4.0e-6f, kTiny = 1.0e-30f;
-  const float o2 = (float)open2;
-  float hi = o2 * (1.0f + kBand), lo = o2 * (1.0f - kBand);
+// does not act.
+__device__ __forceinline__ void setThresholds(TreeCell32& o, double open2, double soft2, float L) {
+  guardBand((float)open2, L, o.hi, o.lo);
   if (o.cnt == 1) {
-    const float lim = 1.0e-10f * (float)soft2;
-    hi = fminf(hi, lim * 1.001f);
-    lo = fminf(lo, lim * 0.999f);
+    float hi, lo;
+    guardBand(1.0e-10f * (float)soft2, L, hi, lo);
+    o.hi = fminf(o.hi, hi);
+    o.lo = fminf(o.lo, lo);
   }
-  o.hi = fmaxf(hi, kTiny);
-  o.lo = lo > kTiny ? lo : -1.0f;
 }
 
-__device__ __forceinline__ void cell32(const TreeCell& cl, double thr, double soft2, TreeCell32* __restrict__ out) {
+__device__ __forceinline__ void cell32(const TreeCell& cl, double thr, double soft2, const double* __restrict__ box,
+                                       TreeCell32* __restrict__ out) {
   TreeCell32 o;
-  splitDF(cl.x, o.xh, o.xl);
-  splitDF(cl.y, o.yh, o.yl);
-  splitDF(cl.z, o.zh, o.zl);
+  splitDF(cl.x - box[0], o.xh, o.xl);
+  splitDF(cl.y - box[1], o.yh, o.yl);
+  splitDF(cl.z - box[2], o.zh, o.zl);
   o.M = (float)cl.M;
   o.skip = cl.skip;
   o.start = cl.start;
   o.cnt = (cl.lvl >> 8) ? cl.count : 0;
-  setThresholds(o, __dadd_rn(thr, cl.r2cc), soft2);
+  setThresholds(o, __dadd_rn(thr, cl.r2cc), soft2, (float)box[3]);
   *out = o;
 }
 
@@ -421,7 +432,7 @@ __global__ void cellFinalKernel(TreeCell* __restrict__ cells, long long numCells
   const double dx = __dsub_rn(cl.x, cx), dy = __dsub_rn(cl.y, cy), dz = __dsub_rn(cl.z, cz);
   cl.r2cc = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   cells[c] = cl;
-  cell32(cl, thrLevel[level], soft2, c32 + c);
+  cell32(cl, thrLevel[level], soft2, box, c32 + c);
 }
 
 //------------------------------------------------------------------------------
@@ -500,7 +511,8 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restri
                                                      long n, const double* __restrict__ thrLevel, double soft2,
                                                      double softening, double G, Fields F,
                                                      unsigned long long* __restrict__ dtBits,
-                                                     double* __restrict__ energyPart) {
+                                                     double* __restrict__ energyPart,
+                                                     const double* __restrict__ box) {
   __shared__ double thr[kMaxLevel + 1];
   __shared__ double esum[4];
   __shared__ double dmin[4];
@@ -515,7 +527,7 @@ __global__ void __launch_bounds__(128) treeWalkKernel(const TreeCell32* __restri
     const TreeNode p = tpos[k];
     xi = p.x; yi = p.y; zi = p.z; mi = p.m;
   }
-  const WalkNode me = walkNode(xi, yi, zi);
+  const WalkNode me = walkNode(xi - box[0], yi - box[1], zi - box[2]);
   double ax = 0, ay = 0, az = 0, phi = 0;
   unsigned* queue = queues[threadIdx.x >> 5][(threadIdx.x & 31) / kWalkLanes];
   unsigned head = 0, tail = 0;
@@ -654,7 +666,7 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
     const TreeCell32* __restrict__ c32, const TreeCell* __restrict__ cells, long long numCells,
     const TreeNode32* __restrict__ t32, const TreeNode* __restrict__ tpos, const int* __restrict__ vals, long n,
     const double* __restrict__ thrLevel, double soft2d, double softening, double G, Fields F,
-    unsigned long long* __restrict__ dtBits, double* __restrict__ energyPart) {
+    unsigned long long* __restrict__ dtBits, double* __restrict__ energyPart, const double* __restrict__ box) {
   __shared__ double thr[kMaxLevel + 1];
   __shared__ double esum[4];
   __shared__ double dmin[4];
@@ -667,8 +679,8 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
     const TreeNode p = tpos[k];
     xd = p.x; yd = p.y; zd = p.z; mi = p.m;
   }
-  const WalkNode me = walkNode(xd, yd, zd);
-  const float soft2 = (float)soft2d;
+  const WalkNode me = walkNode(xd - box[0], yd - box[1], zd - box[2]);
+  const float soft2 = (float)soft2d, boxLength = (float)box[3];
   Acc32 acc{0ull, 0ull, 0ull, 0ull};
   unsigned until = valid ? 0u : 0xFFFFFFFFu;
   unsigned c = 1;
@@ -694,7 +706,8 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
         descend = q.q.w == 0;
         if (!descend) until = skip;
         if (q.q.w > 1) {   // nodes that share a deepest cell
-          const float lim = 1.0e-10f * soft2;
+          float limHi, limLo;
+          guardBand(1.0e-10f * soft2, boxLength, limHi, limLo);
           for (int j = q.q.z; j < q.q.z + q.q.w; ++j) {
             const TreeNode32 p = t32[j];
             WalkCell w;
@@ -704,8 +717,8 @@ __global__ void __launch_bounds__(128) treeWalkMixedKernel(
             float ez;
             const float q2 = separation(w, me, exy, ez);
             bool use;
-            if (q2 > lim * 1.001f) use = true;
-            else if (q2 < lim * 0.999f) use = false;
+            if (q2 > limHi) use = true;
+            else if (q2 < limLo) use = false;
             else {   // the reference's r2 / soft2 > 1e-10 in FP64
               const TreeNode pd = tpos[j];
               const double fx = __dsub_rn(pd.x, xd), fy = __dsub_rn(pd.y, yd), fz = __dsub_rn(pd.z, zd);
@@ -862,7 +875,7 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   int* valsAlt = w->vals2.as<int>();
   GCHK(cudaMemsetAsync(w->timeout.p, 0, sizeof(int), s));
   radixSortPairs(skey, vals, skeyAlt, valsAlt, n, 3 * kMaxLevel, w->sortWs.p, w->timeout.as<int>(), false, s, lc);
-  treeNodesKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, vals, n, w->tpos.as<TreeNode>(),
+  treeNodesKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(F, vals, n, w->box.as<double>(), w->tpos.as<TreeNode>(),
                                                              mixed ? w->tpos32.as<TreeNode32>() : nullptr);
   chainCountKernel<<<blocksFor(n, kThreads), kThreads, 0, s>>>(skey, n, w->nc.as<int>());
   lc->add(2);
@@ -901,11 +914,13 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
     treeWalkMixedKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells,
                                                w->tpos32.as<TreeNode32>(), w->tpos.as<TreeNode>(), vals, n,
                                                w->thr.as<double>(), softening * softening, softening, G, F,
-                                               w->dtBits.as<unsigned long long>(), w->energy.as<double>());
+                                               w->dtBits.as<unsigned long long>(), w->energy.as<double>(),
+                                               w->box.as<double>());
   else
     treeWalkKernel<<<nbWalk, 128, 0, s>>>(w->cells32.as<TreeCell32>(), cells, numCells, w->tpos.as<TreeNode>(), vals,
                                           n, w->thr.as<double>(), softening * softening, softening, G, F,
-                                          w->dtBits.as<unsigned long long>(), w->energy.as<double>());
+                                          w->dtBits.as<unsigned long long>(), w->energy.as<double>(),
+                                          w->box.as<double>());
   walkFinalKernel<<<1, 256, 0, s>>>(w->energy.as<double>(), nbWalk, w->dtBits.as<unsigned long long>(), G, dOut);
   lc->add(2);
   GCHK(cudaGetLastError());
