@@ -437,7 +437,9 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
       }
       vq = __fmaf_rn(-2.0f * phi, sum, vr);
     }
-    const float di = __fmaf_rn(etai, etai, eps2), dj = __fmaf_rn(etaj, etaj, eps2);
+    // a (a r^2): eta carries the error of the reciprocal root twice, and a^2 one
+    // rounding that all nodes of the same h share
+    const float di = __fmaf_rn(__fmul_rn(ai, r2), ai, eps2), dj = __fmaf_rn(__fmul_rn(aj, r2), aj, eps2);
     float ei, ej;
     if (LEAN) {
       // the quotient of coincident nodes is 0/0 with eps2 = 0: fminf makes it 0
