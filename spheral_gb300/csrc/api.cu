@@ -61,17 +61,16 @@ struct Profiler {
   std::vector<Rec> pending;
   std::map<std::string, std::pair<long, double>> acc;
   cudaStream_t s = nullptr;
-  void begin(const char* name, cudaEvent_t* a) {
+  void begin(cudaStream_t at, cudaEvent_t* a) {
     if (!on) return;
     CUDA_OK(cudaEventCreate(a));
-    CUDA_OK(cudaEventRecord(*a, s));
-    (void)name;
+    CUDA_OK(cudaEventRecord(*a, at));
   }
-  void end(const char* name, cudaEvent_t a) {
+  void end(const char* name, cudaStream_t at, cudaEvent_t a) {
     if (!on) return;
     cudaEvent_t b;
     CUDA_OK(cudaEventCreate(&b));
-    CUDA_OK(cudaEventRecord(b, s));
+    CUDA_OK(cudaEventRecord(b, at));
     pending.push_back({name, a, b});
   }
   void collect() {
@@ -90,13 +89,16 @@ struct Profiler {
   }
 };
 
+// Times what is launched on stream `at` (the profiler's own by default) during
+// its life.
 struct Scope {
   Profiler& p;
   const char* n;
+  cudaStream_t at;
   cudaEvent_t a{};
-  Scope(Profiler& p_, const char* n_) : p(p_), n(n_) { p.begin(n, &a); }
+  Scope(Profiler& p_, const char* n_, cudaStream_t at_ = nullptr) : p(p_), n(n_), at(at_ ? at_ : p_.s) { p.begin(at, &a); }
   ~Scope() {
-    try { p.end(n, a); } catch (...) {}
+    try { p.end(n, at, a); } catch (...) {}
   }
 };
 
@@ -852,13 +854,16 @@ void evalDerivs(sphgpu_ctx* c, bool inputs = false, const HalfStep& half = {}, b
     // leaves half the issue slots: both run beside the pair sweep just launched,
     // which reads and writes other fields.  The step's stream waits for the
     // result; an error drains the gravity stream before it is reported.
-    Scope sc(c->prof, "gravity");
     char msg[256] = {0};
     double* d = c->small.as<double>() + 16;
     cudaStream_t gs = c->gravStream;
     CUDA_OK(cudaStreamWaitEvent(gs, c->gravReady, 0));
-    const int rc = gravityEvaluate(c->grav, c->F, c->n, c->cfg.G, c->cfg.softening, c->cfg.opening, c->fp32(), d, gs,
-                                   &c->lc, msg, sizeof(msg));
+    int rc;
+    {
+      Scope sc(c->prof, "gravity", gs);
+      rc = gravityEvaluate(c->grav, c->F, c->n, c->cfg.G, c->cfg.softening, c->cfg.opening, c->fp32(), d, gs, &c->lc,
+                           msg, sizeof(msg));
+    }
     if (rc != SPHGPU_OK) {
       cudaStreamSynchronize(gs);
       throw Error(rc, std::string("gravity: ") + msg);
