@@ -38,14 +38,13 @@ __global__ void prepareKernel(Fields F, Fields32 P, long n, Grid g) {
 // antisymmetric), the second moment of ASPHClassicSmoothingScale and its
 // FP32 finalize.
 //
-// PF selects the neighbour loop: 1 software-pipelined (entry two slots ahead,
-// node data one slot ahead), 2 that many slots per iteration (their gathers
-// issued together, the next iteration's entries loaded ahead).  Every form
-// evaluates the slots in list order, so all give the same bits.  It serves what
-// pairKernelTensor32 does not: XSPH, no compatible energy, the limited Q, several
-// NodeLists, the tensile term, plain sums and the Q's expansion options.
-template <bool XSPH, bool COMPAT, int MINB, int PF, bool LIMQ>
-__global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P, const int* __restrict__ list, long n,
+// Two slots per iteration: their gathers are issued together, the next
+// iteration's entries loaded ahead.  It serves what pairKernelTensor32 does not:
+// XSPH, no compatible energy and the limited Q, with any of the other options.
+// 405,224 nodes: XSPH 709 us, limited Q 994 (one slot ahead of another 906 and
+// 1250; three slots at two blocks per SM 837 and 1258; two at four 877 and 1294).
+template <bool XSPH, bool COMPAT, bool LIMQ>
+__global__ void __launch_bounds__(128, 3) pairKernelFP32(Fields F, Fields32 P, const int* __restrict__ list, long n,
                                                       Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                                                       float* __restrict__ pacc) {
   __shared__ float4 ta[kMaxTable / 3];
@@ -241,69 +240,37 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
       m2[3] += w * (ry * ry); m2[4] += w * (ry * rz); m2[5] += w * (rz * rz);
     }
   };
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (PF == 1) {
-    // software pipeline over the neighbour list: the entry two slots ahead
-    // and the node data one slot ahead are loaded while the current pair is
-    // evaluated, so the gathers overlap the arithmetic
-    uint32_t entA = 0u, entB = 0u;
-    float4 pjA = zero4, vjA = zero4, thA = zero4, hA0 = zero4, hA1 = zero4;
-    if (cnt > 0) {
-      entA = nl.nbr[nbSlot(i, 0, nl.cap)];
-      const int j0 = (int)(entA & kIndexMask);
-      pjA = P.posh[j0]; vjA = P.velm[j0]; thA = P.thermo[j0];
-      hA0 = P.hten[j0]; hA1 = P.hten[P.stride + j0];
-    }
-    if (cnt > 1) entB = nl.nbr[nbSlot(i, 1, nl.cap)];
-    for (int q = 0; q < cnt; ++q) {
-      const uint32_t ent = entA;
-      const float4 pj = pjA, vj4 = vjA, thj = thA;
-      const float4 hj0 = hA0, hj1 = hA1;
-      if (q + 1 < cnt) {
-        const int jn = (int)(entB & kIndexMask);
-        pjA = P.posh[jn]; vjA = P.velm[jn]; thA = P.thermo[jn];
-        hA0 = P.hten[jn]; hA1 = P.hten[P.stride + jn];
-        entA = entB;
-      }
-      if (q + 2 < cnt) entB = nl.nbr[nbSlot(i, q + 2, nl.cap)];
-      slot(ent, pj, vj4, thj, hj0, hj1, nbSlot(i, q, nl.cap));
-    }
-  } else {
-    // PF slots per iteration (slot q + 1 sits 32 entries after slot q): their
-    // gathers are issued together, the next iteration's entries meanwhile
-    constexpr int U = PF >= 2 ? PF : 2;
-    uint32_t nx[U];
-    if (U <= cnt) {
+  constexpr int U = 2;
+  uint32_t nx[U];
+  if (U <= cnt) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) nx[u] = nl.nbr[nbSlot(i, u, nl.cap)];
+    for (int u = 0; u < U; ++u) nx[u] = nl.nbr[nbSlot(i, u, nl.cap)];
+  }
+  int q = 0;
+  for (; q + U <= cnt; q += U) {
+    const long long k0 = nbSlot(i, q, nl.cap);
+    uint32_t e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) e[u] = nx[u];
+    if (q + 2 * U <= cnt) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) nx[u] = nl.nbr[k0 + 32 * (U + u)];
     }
-    int q = 0;
-    for (; q + U <= cnt; q += U) {
-      const long long k0 = nbSlot(i, q, nl.cap);
-      uint32_t e[U];
+    float4 pp[U], vv[U], tt[U], aa[U], bb[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = nx[u];
-      if (q + 2 * U <= cnt) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) nx[u] = nl.nbr[k0 + 32 * (U + u)];
-      }
-      float4 pp[U], vv[U], tt[U], aa[U], bb[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int jj = (int)(e[u] & kIndexMask);
-        pp[u] = P.posh[jj]; vv[u] = P.velm[jj]; tt[u] = P.thermo[jj];
-        aa[u] = P.hten[jj]; bb[u] = P.hten[P.stride + jj];
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) slot(e[u], pp[u], vv[u], tt[u], aa[u], bb[u], k0 + 32 * u);
+    for (int u = 0; u < U; ++u) {
+      const int jj = (int)(e[u] & kIndexMask);
+      pp[u] = P.posh[jj]; vv[u] = P.velm[jj]; tt[u] = P.thermo[jj];
+      aa[u] = P.hten[jj]; bb[u] = P.hten[P.stride + jj];
     }
-    for (; q < cnt; ++q) {
-      const long long k = nbSlot(i, q, nl.cap);
-      const uint32_t ent = nl.nbr[k];
-      const int jj = (int)(ent & kIndexMask);
-      slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], P.hten[jj],
-           P.hten[P.stride + jj], k);
-    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) slot(e[u], pp[u], vv[u], tt[u], aa[u], bb[u], k0 + 32 * u);
+  }
+  for (; q < cnt; ++q) {
+    const long long k = nbSlot(i, q, nl.cap);
+    const uint32_t ent = nl.nbr[k];
+    const int jj = (int)(ent & kIndexMask);
+    slot(ent, P.posh[jj], P.velm[jj], P.thermo[jj], P.hten[jj], P.hten[P.stride + jj], k);
   }
   NodeAcc32 a;
   a.rhoSum = rhoSum; a.norm = norm;
@@ -343,10 +310,11 @@ __global__ void __launch_bounds__(128, MINB) pairKernelFP32(Fields F, Fields32 P
 // L lanes per node, U slots per iteration (their gathers issued together, the
 // next iteration's entries loaded ahead).  KERN 1: cubic B-spline in
 // registers, its normalisation A carried by Prho and 1 / (2 rho) (pairInputs32)
-// and applied to the other sums per node; 0: packed table.  LEAN: compensated sums, no tensile correction
-// and the standard Q expansion fixed at compile time; otherwise read from hp.
+// and applied to the other sums per node; 0: packed table.  LEAN 1: one NodeList,
+// compensated sums, no tensile correction and the standard Q expansion fixed at
+// compile time; 2: the same with plain sums; 0: read from hp.
 //------------------------------------------------------------------------------
-template <bool XSPH, bool COMPAT, bool MULTI, bool LIMQ, bool LEAN, bool MIR, int KERN, int L, int U, int MINB>
+template <bool XSPH, bool COMPAT, bool LIMQ, int LEAN, bool MIR, int KERN, int L, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 P, const int* __restrict__ list, long n,
                                                              Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                                                              float* __restrict__ pacc, HalfStep half) {
@@ -366,7 +334,8 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   const uint32_t mm = MIR ? mirrorMask(g, ci) : 0u;
   const float cx = g.cellf[0], cy = g.cellf[1], cz = g.cellf[2];
   const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i];
-  const int li = MULTI ? list[i] : 0;
+  const bool multi = !LEAN && hp.numLists > 1;
+  const int li = multi ? list[i] : 0;
   const float ai = pi.w, mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w;
   const float ai2 = ai * ai, A4i = __fmul_rn(ai2, ai2), Hdeti = ai2 * ai;
   const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
@@ -387,7 +356,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
 #pragma unroll
   for (int k = 0; k < 6; ++k) a.M[k] = 0.f;
   float sdx = 0.f, cdx = 0.f, sdy = 0.f, cdy = 0.f, sdz = 0.f, cdz = 0.f, se = 0.f, ce = 0.f;
-  const int plain = LEAN ? 0 : hp.plainSums;
+  const int plain = LEAN ? LEAN == 2 : hp.plainSums;
 
   auto slot = [&](uint32_t ent, const float4& pj, const float4& vj4, const float4& kj, const float4& q0,
                   const float4& q1, float* out) {
@@ -397,7 +366,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
     float vxj = vj4.x, vyj = vj4.y, vzj = vj4.z;
     if (MIR) mirrorVel(dcode & mm, vxj, vyj, vzj);
     const float aj = pj.w, mj = vj4.w, rhoj = kj.x, Prhoj = kj.y, mClcj = kj.z, hirj = kj.w;
-    const bool same = MULTI ? (list[ent & kIndexMask] == li) : true;
+    const bool same = multi ? (list[ent & kIndexMask] == li) : true;
     const float r2 = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
     const float ir = rsqrtf(fmaxf(r2, 1.0e-36f));
     const float rm = __fmul_rn(r2, ir);
@@ -493,7 +462,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
       a.xdx -= wx * vx; a.xdy -= wx * vy; a.xdz -= wx * vz;
     }
     float wg = fabsf(gi);
-    if (MULTI && !same) wg *= mj * rhoi / (mi * rhoj);
+    if (!same) wg *= mj * rhoi / (mi * rhoj);
     a.g0 += wg;
     a.m1x += wg * rx; a.m1y += wg * ry; a.m1z += wg * rz;
   };
@@ -555,7 +524,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
   }
   a.dvx = kahanValue(sdx, cdx); a.dvy = kahanValue(sdy, cdy); a.dvz = kahanValue(sdz, cdz);
   a.deps = kahanValue(se, ce);
-  finalizePair32<KERN == 1>(F, i, MULTI ? li : list[i], a, ai, mi, rhoi, cnt, hp, t.herm, half);
+  finalizePair32<KERN == 1>(F, i, list[i], a, ai, mi, rhoi, cnt, hp, t.herm, half);
 }
 
 //------------------------------------------------------------------------------
@@ -572,7 +541,7 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
 // writes 12 and reads 4 bytes of DRAM per slot, 0.6 ms at 2.1 M nodes of 119.
 // 2.1 M nodes: 2685 -> 2082 us.
 //------------------------------------------------------------------------------
-template <bool LIMQ, bool MIR, bool SPLINE, int U, int MINB>
+template <bool LIMQ, bool MIR, bool SPLINE, bool PLAIN, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32 P, const int* __restrict__ list,
                                                               long n, Grid g, NeighborLists nl, TableDev t,
                                                               HydroParams hp, float* __restrict__ pacc, HalfStep half) {
@@ -700,11 +669,11 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
         const float pax = __fmul_rn(-mj, ddx), pay = __fmul_rn(-mj, ddy), paz = __fmul_rn(-mj, ddz);
         out[0] = pax; out[32] = pay; out[64] = paz;
         out += 96;
-        kahanAdd(sdx, cdx, pax);
-        kahanAdd(sdy, cdy, pay);
-        kahanAdd(sdz, cdz, paz);
+        sumAdd(sdx, cdx, pax, PLAIN);
+        sumAdd(sdy, cdy, pay, PLAIN);
+        sumAdd(sdz, cdz, paz, PLAIN);
         const float vg = vx * gwix + vy * gwiy + vz * gwiz;
-        kahanAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg));
+        sumAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg), PLAIN);
         const float mvx = mj * vx, mvy = mj * vy, mvz = mj * vz;
         D[0] -= mvx * gwix; D[1] -= mvx * gwiy; D[2] -= mvx * gwiz;
         D[3] -= mvy * gwix; D[4] -= mvy * gwiy; D[5] -= mvy * gwiz;
@@ -744,12 +713,13 @@ __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32
 // Here one 16-byte entry per side holds W' (W, which feeds only massDensitySum,
 // normalization and effViscousPressure, is the spline in registers or the
 // second table), and what depends on one node comes formed (Fields32::pk).
-// L lanes per node, U slots per iteration.
+// L lanes per node, U slots per iteration.  OPT: several NodeLists, plain sums,
+// the tensile correction and the Q's expansion options are read from hp.
 //------------------------------------------------------------------------------
 struct PairRecTensor {
   float4 p, v, k, a, b;
 };
-template <bool MIR, bool SPLINE, int L, int U, int MINB>
+template <bool OPT, bool MIR, bool SPLINE, int L, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields32 P, const int* __restrict__ list,
                                                                 long n, Grid g, NeighborLists nl, TableDev t,
                                                                 HydroParams hp, float* __restrict__ pacc,
@@ -778,6 +748,9 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
   const float4 pi = P.posh[i], vi = P.velm[i], ki = P.pk[i], hi0 = P.hten[i], hi1 = P.hten[P.stride + i];
   const float mi = vi.w, rhoi = ki.x, Prhoi = ki.y, mClci = ki.z, hiri = ki.w, Hdeti = hi1.z;
   const float Cq = (float)hp.Cq, eps2 = (float)hp.eps2;
+  const bool multi = OPT && hp.numLists > 1;
+  const int li = multi ? list[i] : 0, plain = OPT ? hp.plainSums : 0;
+  const float epsT = OPT ? (float)hp.epsTensile : 0.f, iWnPerh = 1.0f / (float)hp.WnPerh;
   float sw = 0.f, smw = 0.f, sve = 0.f, maxE = 0.f;
   float sdx = 0.f, cdx = 0.f, sdy = 0.f, cdy = 0.f, sdz = 0.f, cdz = 0.f, se = 0.f, ce = 0.f;
   float gx = 0.f, gy = 0.f, gz = 0.f, m0 = 0.f, m1x = 0.f, m1y = 0.f, m1z = 0.f;
@@ -837,20 +810,36 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
         const float mui = __fdividef(__fmaf_rn(vz, eiz, __fmaf_rn(vy, eiy, __fmul_rn(vx, eix))), __fadd_rn(e2i, eps2));
         const float muj = __fdividef(__fmaf_rn(vz, ejz, __fmaf_rn(vy, ejy, __fmul_rn(vx, ejx))), __fadd_rn(e2j, eps2));
         const float mni = fminf(0.f, mui), mnj = fminf(0.f, muj);
-        const float ei = __fmaf_rn(Cq, __fmul_rn(mni, mni), __fmul_rn(mClci, mni));
-        const float ej = __fmaf_rn(Cq, __fmul_rn(mnj, mnj), __fmul_rn(mClcj, mnj));
-        const float ci_ = __fadd_rn(Prhoi, __fmul_rn(ei, hiri)), cj_ = __fadd_rn(Prhoj, __fmul_rn(ej, hirj));
+        float lmi = mni, lmj = mnj, qmi = __fmul_rn(mni, mni), qmj = __fmul_rn(mnj, mnj);
+        float pri = Prhoi, prj = Prhoj;
+        if (OPT) {
+          if (hp.linearInExpansion) { lmi = mui; lmj = muj; }
+          if (hp.quadraticInExpansion) {
+            qmi = __fmul_rn(fabsf(mui), -mui);
+            qmj = __fmul_rn(fabsf(muj), -muj);
+          }
+          if (epsT != 0.f) {   // P_eff = P (1 - epsT (W / W(1/nPerh))^4) in tension
+            const int tj = min(N1 + 1, (int)(etaj * invStep));
+            const float wj = __fmaf_rn(__fmaf_rn(tw[tj].y, etaj, tw[tj].x), etaj, Gj.w);
+            const float si = w * iWnPerh, sj = wj * iWnPerh;
+            if (pri < 0.f) pri = __fmul_rn(pri, 1.0f - epsT * ((si * si) * (si * si)));
+            if (prj < 0.f) prj = __fmul_rn(prj, 1.0f - epsT * ((sj * sj) * (sj * sj)));
+          }
+        }
+        const float ei = __fmaf_rn(Cq, qmi, __fmul_rn(mClci, lmi));
+        const float ej = __fmaf_rn(Cq, qmj, __fmul_rn(mClcj, lmj));
+        const float ci_ = __fadd_rn(pri, __fmul_rn(ei, hiri)), cj_ = __fadd_rn(prj, __fmul_rn(ej, hirj));
         const float ddx = __fadd_rn(__fmul_rn(ci_, gwix), __fmul_rn(cj_, gwjx));
         const float ddy = __fadd_rn(__fmul_rn(ci_, gwiy), __fmul_rn(cj_, gwjy));
         const float ddz = __fadd_rn(__fmul_rn(ci_, gwiz), __fmul_rn(cj_, gwjz));
         const float pax = __fmul_rn(-mj, ddx), pay = __fmul_rn(-mj, ddy), paz = __fmul_rn(-mj, ddz);
         out[0] = pax; out[32] = pay; out[64] = paz;
         out += 96 * L;
-        kahanAdd(sdx, cdx, pax);
-        kahanAdd(sdy, cdy, pay);
-        kahanAdd(sdz, cdz, paz);
+        sumAdd(sdx, cdx, pax, plain);
+        sumAdd(sdy, cdy, pay, plain);
+        sumAdd(sdz, cdz, paz, plain);
         const float vg = vx * gwix + vy * gwiy + vz * gwiz;
-        kahanAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg));
+        sumAdd(se, ce, __fmul_rn(__fmul_rn(mj, ci_), vg), plain);
         const float mvx = mj * vx, mvy = mj * vy, mvz = mj * vz;
         D[0] -= mvx * gwix; D[1] -= mvx * gwiy; D[2] -= mvx * gwiz;
         D[3] -= mvy * gwix; D[4] -= mvy * gwiy; D[5] -= mvy * gwiz;
@@ -861,17 +850,21 @@ __global__ void __launch_bounds__(128, MINB) pairKernelTensor32(Fields F, Fields
         M[6] -= mrz * gwix; M[7] -= mrz * gwiy; M[8] -= mrz * gwiz;
         const float gr = mj * (rhoj - rhoi);
         gx += gr * gwix; gy += gr * gwiy; gz += gr * gwiz;
-        sw += w;
-        smw += mj * w;
+        const bool same = multi ? list[ent & kIndexMask] == li : true;
+        if (same) {
+          sw += w;
+          smw += mj * w;
+        }
         sve += (mj * hirj) * (ei * (Hdeti * w));
         maxE = fmaxf(maxE, ei);
-        const float wg = fabsf(gi);
+        const float wf = fabsf(gi);
+        const float wg = same ? wf : wf * (mj * rhoi / (mi * rhoj));
         m0 += wg;
         m1x -= wg * eix; m1y -= wg * eiy; m1z -= wg * eiz;
         // ASPHClassicSmoothingScale second moment: WSPH^2 r r / |r|^5
         const float ir = rsqrtf(fmaxf(rx * rx + ry * ry + rz * rz, 1.0e-30f));
         const float ir2 = ir * ir;
-        const float w2 = wg * wg * (ir2 * ir2 * ir);
+        const float w2 = wg * wf * (ir2 * ir2 * ir);
         m2[0] += w2 * (rx * rx); m2[1] += w2 * (rx * ry); m2[2] += w2 * (rx * rz);
         m2[3] += w2 * (ry * ry); m2[4] += w2 * (ry * rz); m2[5] += w2 * (rz * rz);
       });
@@ -1261,14 +1254,22 @@ constexpr int kDensU = 2, kGradhU = 4;   // slots per iteration of the density a
 // by domains of different node counts), it keeps the earlier arithmetic; else the
 // reduced one, with the spline in registers.
 static bool leanPair(const HydroParams& hp) {
-  return hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.plainSums && !hp.xsph && hp.compatible && hp.numLists == 1;
+  return hp.epsTensile == 0.0 && !hp.linearInExpansion && !hp.quadraticInExpansion && !hp.xsph && hp.compatible && hp.numLists == 1;
 }
 static bool exactPair(long n, const HydroParams& hp) { return leanPair(hp) && (n >= kExactNodes || hp.decomposed); }
 static bool reducedPair(long n, const HydroParams& hp) { return leanPair(hp) && !exactPair(n, hp) && hp.cubicSpline; }
+// and with tensor H: none of the run-time options either
+static bool leanTensor(const HydroParams& hp) { return leanPair(hp) && !hp.plainSums && !hp.limitedQ; }
+// The options read at run time (pairKernelIso32's LEAN 0 and the tensor forms).
+// Isotropic: one lane per node with two slots in flight where its blocks fill
+// their one wave (three blocks of 128 on each of 152 SMs) or several, else four
+// lanes.  The tensile correction at 21,952 / 50,653 / 97,336 / 405,224 nodes:
+// one lane 41 / 52 / 108 / 321 us, four 31 / 67 / 102 / 457.
+static int lanesGeneral(long n) { return n >= kExactNodes || (n >= 40000 && n <= 58368) ? 1 : 4; }
 static int lanesTensor(long n) { return n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8)); }
 bool pairVariantsDiffer32(long n, const HydroParams& hp) {
   if (hp.crk) return n >= kCRKOneLane && !hp.xsph && hp.compatible;
-  if (hp.asph) return lanesTensor(n) == 1 || !leanPair(hp) || hp.limitedQ;
+  if (hp.asph) return !hp.xsph && hp.compatible && !hp.limitedQ && (leanTensor(hp) ? lanesTensor(n) == 1 : n >= 20000);
   return exactPair(n, hp) && hp.cubicSpline && !hp.limitedQ;
 }
 PairForm pairForm32(long n, const HydroParams& hp) {
@@ -1291,25 +1292,24 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
   const int b = 128;
   if (hp.asph) {
     const unsigned gb = gridFor(n, b);
-#define SPH_PAIR32T(X, C, LQ)                                                                     \
-  do {                                                                                            \
-    if (variant & 1) pairKernelFP32<X, C, 4, 1, LQ><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
-    else pairKernelFP32<X, C, 3, 1, LQ><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);             \
-  } while (0)
     // Lean path, one lane per node (303,912 nodes): variants 0 to 3 are two slots
     // per iteration at three blocks per SM (579 us), one at four (593), two at four
-    // (578), three at two (567); below 100,000 nodes several lanes per node.
-    // Other options: odd variants cap the registers at 128 (four blocks), even
-    // ones at 168 (three); 0-1 the pipelined loop, 2-3 (compatible energy, no
-    // XSPH, standard Q) two slots per iteration.
-    if (leanPair(hp) && !hp.limitedQ) {
+    // (578), three at two (567); below 100,000 nodes several lanes per node.  The
+    // run-time options: one lane from 100,000 nodes on, four below.
+    if (!hp.xsph && hp.compatible && !hp.limitedQ) {
       if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
-#define SPH_TEN(MI, SP, LA, U, MB) \
-  pairKernelTensor32<MI, SP, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
-#define SPH_TENL(MI, LA, U, MB) do { if (hp.cubicSpline) SPH_TEN(MI, true, LA, U, MB); else SPH_TEN(MI, false, LA, U, MB); } while (0)
+#define SPH_TEN(OP, MI, SP, LA, U, MB) \
+  pairKernelTensor32<OP, MI, SP, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
+#define SPH_TENL(MI, LA, U, MB) do { if (hp.cubicSpline) SPH_TEN(false, MI, true, LA, U, MB); else SPH_TEN(false, MI, false, LA, U, MB); } while (0)
 #define SPH_TENM(LA, U, MB) do { if (hasMirrors(g)) SPH_TENL(true, LA, U, MB); else SPH_TENL(false, LA, U, MB); } while (0)
       const int L = lanesTensor(n);
-      if (L == 1) {
+      if (!leanTensor(hp)) {
+        if (n < 20000) SPH_TEN(true, true, false, 4, 2, 3);
+        else if (variant == 1) SPH_TEN(true, true, false, 1, 3, 2);
+        else if (variant == 2) SPH_TEN(true, true, false, 1, 2, 4);
+        else if (variant == 3) SPH_TEN(true, true, false, 1, 1, 4);
+        else SPH_TEN(true, true, false, 1, 2, 3);
+      } else if (L == 1) {
         if (variant == 1) SPH_TENM(1, 1, 4);
         else if (variant == 2) SPH_TENM(1, 2, 4);
         else if (variant == 3) SPH_TENM(1, 3, 2);
@@ -1323,17 +1323,14 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
       lc->add(inputs ? 1 : 2);
       return;
     }
-    if (!hp.xsph && hp.compatible && !hp.limitedQ && variant >= 2) {
-      if (variant & 1) pairKernelFP32<false, true, 4, 2, false><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-      else pairKernelFP32<false, true, 3, 2, false><<<gb, b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);
-    } else if (hp.xsph) {
-      if (hp.compatible) { if (hp.limitedQ) SPH_PAIR32T(true, true, true); else SPH_PAIR32T(true, true, false); }
-      else { if (hp.limitedQ) SPH_PAIR32T(true, false, true); else SPH_PAIR32T(true, false, false); }
-    } else {
-      if (hp.compatible) { if (hp.limitedQ) SPH_PAIR32T(false, true, true); else SPH_PAIR32T(false, true, false); }
-      else { if (hp.limitedQ) SPH_PAIR32T(false, false, true); else SPH_PAIR32T(false, false, false); }
-    }
-#undef SPH_PAIR32T
+#define SPH_TENG(X, C)                                                                                          \
+  do {                                                                                                          \
+    if (hp.limitedQ) pairKernelFP32<X, C, true><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc); \
+    else pairKernelFP32<X, C, false><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc);            \
+  } while (0)
+    if (hp.xsph) { if (hp.compatible) SPH_TENG(true, true); else SPH_TENG(true, false); }
+    else { if (hp.compatible) SPH_TENG(false, true); else SPH_TENG(false, false); }
+#undef SPH_TENG
     if (half.v) halfStepVelocityKernel<<<gridFor(n, 256), 256, 0, s>>>(F, n, half);
     lc->add(half.v ? 2 : 1);
     return;
@@ -1341,41 +1338,48 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
   const bool exact = exactPair(n, hp), fast = reducedPair(n, hp);
   if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
   const int L = lanesPair(n);
-#define SPH_ISO(X, C, M, Q, LE, MI, K, LA, U, MB) \
-  pairKernelIso32<X, C, M, Q, LE, MI, K, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
+#define SPH_ISO(X, C, Q, LE, MI, K, LA, U, MB) \
+  pairKernelIso32<X, C, Q, LE, MI, K, LA, U, MB><<<gridFor(n * LA, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
   if (exact) {
-#define SPH_LEAN(Q, MI)                                                                                              \
-  do {                                                                                                               \
-    if (!hp.cubicSpline) pairKernelLean32<Q, MI, false, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
-    else if (Q) pairKernelLean32<Q, MI, true, 2, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
-    else if (variant & 1) pairKernelLean32<Q, MI, true, 4, 2><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half); \
-    else pairKernelLean32<Q, MI, true, 5, 3><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half);       \
+#define SPH_LEAN(Q, MI, SP, PL, U, MB) \
+  pairKernelLean32<Q, MI, SP, PL, U, MB><<<gridFor(n, b), b, 0, s>>>(F, F32, list, n, g, nl, t, hp, pacc, half)
+#define SPH_LEANP(MI, PL)                                                                      \
+  do {                                                                                         \
+    if (hp.limitedQ) { if (hp.cubicSpline) SPH_LEAN(true, MI, true, PL, 2, 3); else SPH_LEAN(true, MI, false, PL, 2, 3); } \
+    else if (!hp.cubicSpline) SPH_LEAN(false, MI, false, PL, 2, 3);                            \
+    else if (variant & 1) SPH_LEAN(false, MI, true, PL, 4, 2);                                 \
+    else SPH_LEAN(false, MI, true, PL, 5, 3);                                                  \
   } while (0)
-    if (hasMirrors(g)) { if (hp.limitedQ) SPH_LEAN(true, true); else SPH_LEAN(false, true); }
-    else { if (hp.limitedQ) SPH_LEAN(true, false); else SPH_LEAN(false, false); }
+    if (hasMirrors(g)) { if (hp.plainSums) SPH_LEANP(true, true); else SPH_LEANP(true, false); }
+    else { if (hp.plainSums) SPH_LEANP(false, true); else SPH_LEANP(false, false); }
+#undef SPH_LEANP
 #undef SPH_LEAN
   } else if (fast) {
-#define SPH_ISOL(Q, MI)                                                                   \
+#define SPH_ISOL(Q, LE, MI)                                                               \
   switch (L) {                                                                            \
-    case 2: SPH_ISO(false, true, false, Q, true, MI, 1, 2, 2, 4); break;                  \
-    case 4: SPH_ISO(false, true, false, Q, true, MI, 1, 4, 2, 4); break;                  \
-    case 8: SPH_ISO(false, true, false, Q, true, MI, 1, 8, 2, 4); break;                  \
-    default: SPH_ISO(false, true, false, Q, true, MI, 1, 16, 2, 4); break;                \
+    case 2: SPH_ISO(false, true, Q, LE, MI, 1, 2, 2, 4); break;                           \
+    case 4: SPH_ISO(false, true, Q, LE, MI, 1, 4, 2, 4); break;                           \
+    case 8: SPH_ISO(false, true, Q, LE, MI, 1, 8, 2, 4); break;                           \
+    default: SPH_ISO(false, true, Q, LE, MI, 1, 16, 2, 4); break;                         \
   }
-    if (hasMirrors(g)) {
-      if (hp.limitedQ) { SPH_ISOL(true, true) } else { SPH_ISOL(false, true) }
+    if (hp.plainSums) {
+      if (hp.limitedQ) { SPH_ISOL(true, 2, true) } else { SPH_ISOL(false, 2, true) }
+    } else if (hasMirrors(g)) {
+      if (hp.limitedQ) { SPH_ISOL(true, 1, true) } else { SPH_ISOL(false, 1, true) }
     } else {
-      if (hp.limitedQ) { SPH_ISOL(true, false) } else { SPH_ISOL(false, false) }
+      if (hp.limitedQ) { SPH_ISOL(true, 1, false) } else { SPH_ISOL(false, 1, false) }
     }
 #undef SPH_ISOL
   } else {
-#define SPH_ISOG(X, C)                                                      \
-  do {                                                                      \
-    if (hp.limitedQ) SPH_ISO(X, C, true, true, false, true, 0, 4, 1, 3);          \
-    else SPH_ISO(X, C, true, false, false, true, 0, 4, 1, 3);                     \
+#define SPH_ISOG(X, C, Q)                                                              \
+  do {                                                                                 \
+    if (lanesGeneral(n) == 1) SPH_ISO(X, C, Q, 0, true, 0, 1, 2, 3);                   \
+    else SPH_ISO(X, C, Q, 0, true, 0, 4, 1, 4);                                        \
   } while (0)
-    if (hp.xsph) { if (hp.compatible) SPH_ISOG(true, true); else SPH_ISOG(true, false); }
-    else { if (hp.compatible) SPH_ISOG(false, true); else SPH_ISOG(false, false); }
+#define SPH_ISOQ(X, C) do { if (hp.limitedQ) SPH_ISOG(X, C, true); else SPH_ISOG(X, C, false); } while (0)
+    if (hp.xsph) { if (hp.compatible) SPH_ISOQ(true, true); else SPH_ISOQ(true, false); }
+    else { if (hp.compatible) SPH_ISOQ(false, true); else SPH_ISOQ(false, false); }
+#undef SPH_ISOQ
 #undef SPH_ISOG
   }
 #undef SPH_ISO
@@ -1407,6 +1411,8 @@ static void launchDensity32(Fields F, Fields32 F32, const int* list, long n, Gri
   } while (0)
     SPH_BY_LANES(L, SPH_DL)
 #undef SPH_DL
+  } else if (L == 1 && !hp.asph) {   // 2,000,376 nodes, two NodeLists: 633 us, four lanes 801; tensor H: 313 against 255
+    if (dt) SPH_DENS(false, true, false, true, 0, 1, 2); else SPH_DENS(false, false, false, true, 0, 1, 2);
   } else if (dt) {
     if (hp.asph) SPH_DENS(true, true, false, true, 0, 4, 1); else SPH_DENS(false, true, false, true, 0, 4, 2);
   } else {
@@ -1444,6 +1450,8 @@ void launchGradhFP32(Fields F, Fields32 F32, long n, Grid g, NeighborLists nl, T
 #undef SPH_GL
   } else if (hp.asph) {
     SPH_GH(true, false, true, 0, 4, 2);
+  } else if (L == 1) {
+    SPH_GH(false, false, true, 0, 1, kGradhU);
   } else {
     SPH_GH(false, false, true, 0, 4, 2);
   }
