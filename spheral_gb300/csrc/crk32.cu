@@ -571,6 +571,10 @@ __global__ void volumeMirrorKernel(Fields F, Fields32 P, long n) {
 
 }  // namespace
 
+// The volume and density sweeps with one / four lanes, us: 57 neighbours, 64,000
+// nodes 26/33 and 39/53, 97,336 37/42 and 65/68, 148,877 37/59 and 66/92; 272
+// neighbours, 97,336 nodes 115/91 and 195/153.  Four lanes up to the line of the
+// SPH sweeps lose less where they lose.
 #define SPH_CRK_SWEEP(KERNEL, U, ...)                                                                              \
   do {                                                                                                             \
     const int L = lanesSweep(n);                                                                                   \
@@ -603,11 +607,12 @@ void launchCRKDensityFP32(Fields F, Fields32 P, const int* list, long n, Grid g,
 void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists nl, TableDev t, HydroParams hp,
                              cudaStream_t s, LaunchCounter* lc) {
   // several lanes repeat the FP64 solve's issue for fewer nodes per warp: only
-  // where one lane per node leaves SMs idle
+  // where one lane per node leaves SMs idle.  us with 1 / 2 / 4 lanes: 5,832 nodes
+  // 40/28/29, 10,648 42/35/39, 21,952 48/44/66, 29,791 48/54/78.
   const bool mir = hasMirrors(g);
 #define SPH_RKC(MI, LA) rkCorrections32<MI, LA, 3><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, n, g, nl, t, hp)
-  if (n >= 40000) { if (mir) SPH_RKC(true, 1); else SPH_RKC(false, 1); }
-  else if (n >= 15000) { if (mir) SPH_RKC(true, 2); else SPH_RKC(false, 2); }
+  if (n >= 25000) { if (mir) SPH_RKC(true, 1); else SPH_RKC(false, 1); }
+  else if (n >= 6000) { if (mir) SPH_RKC(true, 2); else SPH_RKC(false, 2); }
   else { if (mir) SPH_RKC(true, 4); else SPH_RKC(false, 4); }
 #undef SPH_RKC
   lc->add(1);
@@ -615,10 +620,12 @@ void launchRKCorrectionsFP32(Fields F, Fields32 P, long n, Grid g, NeighborLists
 // Bound by L1 wavefronts (7 gathers per slot) at 8-12 warps per SM.  variant 0:
 // three slots per iteration at two blocks per SM (387,072 nodes: 705 us), 1: two
 // at three (743 us); one at four took 847 us.  With the limited Q one and two.
+// Lanes, us with 1 / 2 / 4: 17,576 nodes 39/34/33, 21,952 54/43/50, 29,791 57/56/58,
+// 46,656 99/99/81, 79,507 140/131/121, 125,000 188/180/178 (one lane's variants: 181).
 void launchPairCRKFP32(Fields F, Fields32 P, const int* list, long n, Grid g, NeighborLists nl, TableDev t,
                        HydroParams hp, float* pacc, int variant, cudaStream_t s, LaunchCounter* lc) {
   crkInputs32<<<gridFor(n, 256), 256, 0, s>>>(P, n);
-  const int L = n >= kCRKOneLane ? 1 : (n >= 20000 ? 2 : 4);
+  const int L = n >= kCRKOneLane ? 1 : (n >= 20000 && n < 35000 ? 2 : 4);
   const bool mir = hasMirrors(g);
 #define SPH_CRK32(X, C, Q, MI, LA, U, MB) \
   pairKernelCRK32<X, C, Q, MI, LA, U, MB><<<gridFor(LA * n, 128), 128, 0, s>>>(F, P, list, n, g, nl, t, hp, pacc)

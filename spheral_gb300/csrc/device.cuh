@@ -169,15 +169,19 @@ __host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 51
 
 // Lanes per node.  One lane per node leaves the GPU idle below ~300,000 nodes
 // (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
-// shuffles and the partly filled last slots; the sweeps with light pair bodies
-// gain from two lanes at any size (two list rows per warp access).  Lines set
-// where the measured times cross: pair sweep of 103,924 nodes with the limited Q
-// 141 / 148 / 190 us with 2 / 4 / 1 lanes, 3375 nodes 54 us with one, 20 with 16.
+// shuffles and the partly filled last slots.  The lines lie where the times cross
+// (boxes of 57 neighbours; 115 cross at the same sizes), us with 1 / 2 / 4 / 8 / 16:
+//   pair    2,744 18/16/14/14/16   17,576 20/20/20/30/49   21,952 24/23/28/38/59
+//           97,336 69/68/83/127/227   148,877 97/96/125/194/349
+//   density 4,096 33/23/16/12/12   17,576 36/24/16/14/18   39,304 38/25/18/23/29
+//           97,336 43/29/33/41/55   148,877 43/51/47/57/83
+//   energy  4,096 25/14/10/10/10   17,576 25/14/12/14/20   29,791 25/18/20/25/35
+//           64,000 29/33/37/49/74   148,877 49/55/61/78/121
 constexpr long kCRKOneLane = 100000;   // from here one lane per node in the CRKSPH pair sweep
 constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
-inline int lanesPair(long n) { return n >= 80000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
+inline int lanesPair(long n) { return n >= 20000 ? 2 : 4; }
 inline int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
-inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16))); }
+inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 25000 ? 2 : (n >= 6000 ? 4 : 8)); }
 
 #define SPH_BY_LANES(L, CALL)      \
   switch (L) {                     \

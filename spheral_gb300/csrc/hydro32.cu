@@ -1266,10 +1266,13 @@ static bool leanTensor(const HydroParams& hp) { return leanPair(hp) && !hp.plain
 // lanes.  The tensile correction at 21,952 / 50,653 / 97,336 / 405,224 nodes:
 // one lane 41 / 52 / 108 / 321 us, four 31 / 67 / 102 / 457.
 static int lanesGeneral(long n) { return n >= kExactNodes || (n >= 40000 && n <= 58368) ? 1 : 4; }
-static int lanesTensor(long n) { return n >= 100000 ? 1 : (n >= 40000 ? 2 : (n >= 12000 ? 4 : 8)); }
+// Tensor H, us with 1 / 2 / 4 / 8 lanes: 10,648 nodes 47/39/37/60, 17,576 47/39/62/87,
+// 21,952 55/47/68/107, 29,791 56/72/90/139, 97,336 136/169/231/390.
+static int lanesTensor(long n) { return n >= 25000 ? 1 : (n >= 15000 ? 2 : 4); }
+constexpr long kTensorVariants = 100000;   // from here the variants are worth timing
 bool pairVariantsDiffer32(long n, const HydroParams& hp) {
   if (hp.crk) return n >= kCRKOneLane && !hp.xsph && hp.compatible;
-  if (hp.asph) return !hp.xsph && hp.compatible && !hp.limitedQ && (leanTensor(hp) ? lanesTensor(n) == 1 : n >= 20000);
+  if (hp.asph) return !hp.xsph && hp.compatible && !hp.limitedQ && n >= (leanTensor(hp) ? kTensorVariants : 20000);
   return exactPair(n, hp) && hp.cubicSpline && !hp.limitedQ;
 }
 PairForm pairForm32(long n, const HydroParams& hp) {
@@ -1294,8 +1297,10 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
     const unsigned gb = gridFor(n, b);
     // Lean path, one lane per node (303,912 nodes): variants 0 to 3 are two slots
     // per iteration at three blocks per SM (579 us), one at four (593), two at four
-    // (578), three at two (567); below 100,000 nodes several lanes per node.  The
-    // run-time options: one lane from 100,000 nodes on, four below.
+    // (578), three at two (567); below 100,000 nodes variant 0 (79,507 nodes:
+    // 125 us), and several lanes per node below 25,000.  The run-time options: one
+    // lane from 20,000 nodes on (39,304 nodes, two NodeLists: 87 us, four lanes 97),
+    // four below (10,648: 41, one lane 72).
     if (!hp.xsph && hp.compatible && !hp.limitedQ) {
       if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
 #define SPH_TEN(OP, MI, SP, LA, U, MB) \
@@ -1310,13 +1315,13 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
         else if (variant == 3) SPH_TEN(true, true, false, 1, 1, 4);
         else SPH_TEN(true, true, false, 1, 2, 3);
       } else if (L == 1) {
-        if (variant == 1) SPH_TENM(1, 1, 4);
-        else if (variant == 2) SPH_TENM(1, 2, 4);
-        else if (variant == 3) SPH_TENM(1, 3, 2);
+        const int v = n >= kTensorVariants ? variant : 0;
+        if (v == 1) SPH_TENM(1, 1, 4);
+        else if (v == 2) SPH_TENM(1, 2, 4);
+        else if (v == 3) SPH_TENM(1, 3, 2);
         else SPH_TENM(1, 2, 3);
       } else if (L == 2) SPH_TENM(2, 2, 3);
-      else if (L == 4) SPH_TENM(4, 2, 3);
-      else SPH_TENM(8, 2, 3);
+      else SPH_TENM(4, 2, 3);
 #undef SPH_TENM
 #undef SPH_TENL
 #undef SPH_TEN
@@ -1356,12 +1361,8 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
 #undef SPH_LEAN
   } else if (fast) {
 #define SPH_ISOL(Q, LE, MI)                                                               \
-  switch (L) {                                                                            \
-    case 2: SPH_ISO(false, true, Q, LE, MI, 1, 2, 2, 4); break;                           \
-    case 4: SPH_ISO(false, true, Q, LE, MI, 1, 4, 2, 4); break;                           \
-    case 8: SPH_ISO(false, true, Q, LE, MI, 1, 8, 2, 4); break;                           \
-    default: SPH_ISO(false, true, Q, LE, MI, 1, 16, 2, 4); break;                         \
-  }
+  if (L == 2) SPH_ISO(false, true, Q, LE, MI, 1, 2, 2, 4);                                \
+  else SPH_ISO(false, true, Q, LE, MI, 1, 4, 2, 4);
     if (hp.plainSums) {
       if (hp.limitedQ) { SPH_ISOL(true, 2, true) } else { SPH_ISOL(false, 2, true) }
     } else if (hasMirrors(g)) {
@@ -1374,7 +1375,7 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
 #define SPH_ISOG(X, C, Q)                                                              \
   do {                                                                                 \
     if (lanesGeneral(n) == 1) SPH_ISO(X, C, Q, 0, true, 0, 1, 2, 3);                   \
-    else SPH_ISO(X, C, Q, 0, true, 0, 4, 1, 4);                                        \
+    else SPH_ISO(X, C, Q, 0, true, 0, 4, 1, 3);                                        \
   } while (0)
 #define SPH_ISOQ(X, C) do { if (hp.limitedQ) SPH_ISOG(X, C, true); else SPH_ISOG(X, C, false); } while (0)
     if (hp.xsph) { if (hp.compatible) SPH_ISOQ(true, true); else SPH_ISOQ(true, false); }
@@ -1490,8 +1491,7 @@ void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, cons
     case 1: SPH_EN(B, 1); break;   \
     case 2: SPH_EN(B, 2); break;   \
     case 4: SPH_EN(B, 4); break;   \
-    case 8: SPH_EN(B, 8); break;   \
-    default: SPH_EN(B, 16); break; \
+    default: SPH_EN(B, 8); break;  \
   }
   if (variant == 1) { SPH_ENL(8) } else if (variant == 2) { SPH_ENL(2) } else { SPH_ENL(4) }
 #undef SPH_ENL
