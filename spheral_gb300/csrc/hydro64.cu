@@ -117,12 +117,11 @@ __device__ __forceinline__ double laneMax64(double v) {   // non-negative values
 
 // r = x_i - x_j through the image of the entry; r^2, 1/|r| and |r|.
 __device__ __forceinline__ void separation64(const Grid& g, int code, double xi, double yi, double zi, const double2& xy,
-                                             double z, double& rx, double& ry, double& rz, double& ir, double& rm,
-                                             double& r2) {
+                                             double z, double& rx, double& ry, double& rz, double& ir, double& rm) {
   double xj = xy.x, yj = xy.y, zj = z;
   imagePos(g, code, xj, yj, zj);
   rx = xi - xj; ry = yi - yj; rz = zi - zj;
-  r2 = __fma_rn(rz, rz, __fma_rn(ry, ry, __dmul_rn(rx, rx)));
+  double r2 = __fma_rn(rz, rz, __fma_rn(ry, ry, __dmul_rn(rx, rx)));
   ir = rsqrt64(bits(r2) > bits(1.0e-290) ? r2 : 1.0e-290);   // coincident nodes: |r| = 0, finite 1/|r|
   rm = r2 * ir;
 }
@@ -172,8 +171,8 @@ __global__ void __launch_bounds__(128) density64Kernel(Fields F, const Node64* _
         const int code = imageCode(g, hc, (int)(ent >> kIndexBits));
         const double aj = r.za.y;
         if (DENS) {
-          double rx, ry, rz, ir, rm, r2;
-          separation64(g, code, xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm, r2);
+          double rx, ry, rz, ir, rm;
+          separation64(g, code, xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm);
           const double eta = aj * rm;
           const double w = T.value(T.index(eta), eta);
           const double m = (multi && list[ent & kIndexMask] != li) ? mi : r.vzm.y;
@@ -277,8 +276,8 @@ __global__ void __launch_bounds__(128) gradh64Kernel(Fields F, const Node64* __r
         r.za = rec[j].za;
       },
       [&](uint32_t ent, const Sweep64& r) {
-        double rx, ry, rz, ir, rm, r2;
-        separation64(g, imageCode(g, hc, (int)(ent >> kIndexBits)), xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm, r2);
+        double rx, ry, rz, ir, rm;
+        separation64(g, imageCode(g, hc, (int)(ent >> kIndexBits)), xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm);
         const double eta = ai * rm;
         const int k = T.index(eta);
         wsum += T.value(k, eta);
@@ -338,8 +337,8 @@ __global__ void __launch_bounds__(128) pair64Kernel(Fields F, const Node64* __re
       nl, i, sub, cnt, [&](uint32_t j, Node64& r) { r = rec[j]; },
       [&](uint32_t ent, const Node64& r) {
         const int code = imageCode(g, hc, (int)(ent >> kIndexBits));
-        double rx, ry, rz, ir, rm, r2;
-        separation64(g, code, xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm, r2);
+        double rx, ry, rz, ir, rm;
+        separation64(g, code, xi, yi, zi, r.xy, r.za.x, rx, ry, rz, ir, rm);
         double vxj = r.vxy.x, vyj = r.vxy.y, vzj = r.vzm.x;
         imageVec(g, code, vxj, vyj, vzj);
         const double aj = r.za.y, mj = r.vzm.y, rhoj = r.rp.x, hirj = r.ch.y;
@@ -376,8 +375,7 @@ __global__ void __launch_bounds__(128) pair64Kernel(Fields F, const Node64* __re
           vq = __fma_rn(-2.0 * phi, sum, vr);
         }
         // mu_i = a_i v.r / (eta_i^2 + eps2) and mu_j by one reciprocal
-        const double aj2 = aj * aj;
-        const double di = __fma_rn(ai * ai, r2, hp.eps2), dj = __fma_rn(aj2, r2, hp.eps2);
+        const double di = __fma_rn(etai, etai, hp.eps2), dj = __fma_rn(etaj, etaj, hp.eps2);
         const double f = vq * rcp64(di * dj);
         const double mui = (ai * f) * dj, muj = (aj * f) * di;
         // strictly negative: coincident nodes have v.r = -0 or +0, and with eps2 = 0 a
@@ -402,6 +400,7 @@ __global__ void __launch_bounds__(128) pair64Kernel(Fields F, const Node64* __re
           if (prj < 0.0) prj *= 1.0 - hp.epsTensile * ((tj * tj) * (tj * tj));
         }
         const double Ci = __fma_rn(ei, me.ch.y, pri), Cj = __fma_rn(ej, hirj, prj);
+        const double aj2 = aj * aj;
         const double S = __fma_rn(Ci, A4i * gi, __dmul_rn(Cj, (aj2 * aj2) * gj)) * ir;
         const double gf = -mj * S;
         const double pax = gf * rx, pay = gf * ry, paz = gf * rz;
