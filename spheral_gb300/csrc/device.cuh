@@ -170,18 +170,19 @@ __host__ __device__ constexpr int sweepBlock(int lanes) { return lanes == 1 ? 51
 // Lanes per node.  One lane per node leaves the GPU idle below ~300,000 nodes
 // (152 SMs x 16-20 resident warps of 32 nodes), and several lanes cost the
 // shuffles and the partly filled last slots.  The lines lie where the times cross
-// (boxes of 57 neighbours; 115 cross at the same sizes), us with 1 / 2 / 4 / 8 / 16:
-//   pair    2,744 18/16/14/14/16   17,576 20/20/20/30/49   21,952 24/23/28/38/59
-//           97,336 69/68/83/127/227   148,877 97/96/125/194/349
+// (boxes of 57 and, in brackets, 115 neighbours), us with 1 / 2 / 4 / 8 / 16:
+//   pair    2,744 18/16/14/14/16   13,824 20/20/18/28/39 (26/24/21/34/47)
+//           39,304 36/37/41/57/96 (52/52/52/71/122; with walls or the limited Q
+//           four lanes lead by 1 % of the step)   97,336 69/68/83/127/227 (96/95/109)
 //   density 4,096 33/23/16/12/12   17,576 36/24/16/14/18   39,304 38/25/18/23/29
 //           97,336 43/29/33/41/55   148,877 43/51/47/57/83
-//   energy  4,096 25/14/10/10/10   17,576 25/14/12/14/20   29,791 25/18/20/25/35
-//           64,000 29/33/37/49/74   148,877 49/55/61/78/121
+//   energy  5,832 25/13/10/10/10   13,824 25/14/11/12/19   39,304 27/18/18/25/35
+//           (47/29/27/35/54)   64,000 29/33/37/49/74   148,877 49/55/61/78/121
 constexpr long kCRKOneLane = 100000;   // from here one lane per node in the CRKSPH pair sweep
 constexpr long kExactNodes = 150000;   // node count from which the mixed sweeps keep the earlier arithmetic
-inline int lanesPair(long n) { return n >= 20000 ? 2 : 4; }
+inline int lanesPair(long n) { return n >= 80000 ? 2 : 4; }
 inline int lanesSweep(long n) { return n >= kExactNodes ? 1 : (n >= 20000 ? 4 : (n >= 6000 ? 8 : 16)); }
-inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 25000 ? 2 : (n >= 6000 ? 4 : 8)); }
+inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 : (n >= 6000 ? 4 : 16)); }
 
 #define SPH_BY_LANES(L, CALL)      \
   switch (L) {                     \

@@ -1491,7 +1491,7 @@ void launchCompatibleEnergyFP32(Fields F, long n, Grid g, NeighborLists nl, cons
     case 1: SPH_EN(B, 1); break;   \
     case 2: SPH_EN(B, 2); break;   \
     case 4: SPH_EN(B, 4); break;   \
-    default: SPH_EN(B, 8); break;  \
+    default: SPH_EN(B, 16); break; \
   }
   if (variant == 1) { SPH_ENL(8) } else if (variant == 2) { SPH_ENL(2) } else { SPH_ENL(4) }
 #undef SPH_ENL

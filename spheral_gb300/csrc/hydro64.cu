@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(128) energy64Kernel(Fields F, const Velocity64
 // Lanes per node: enough warps to balance the SMs.  Pair sweep, us with 1 / 2 / 4 / 8:
 // 8,000 nodes 353/189/182/214, 21,952 584/572/490/505, 39,304 835/742/738/854,
 // 64,000 1137/1132/1123/1372, 148,877 2177/2255/2530/3035.
-int lanes64(long n) { return n >= 60000 ? 1 : (n >= 20000 ? 2 : (n >= 8000 ? 4 : 8)); }
+int lanes64(long n) { return n >= 60000 ? 1 : (n >= 30000 ? 2 : (n >= 8000 ? 4 : 8)); }
 
 }  // namespace
 

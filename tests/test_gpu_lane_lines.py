@@ -1,8 +1,8 @@
-"""Both sides of the node counts where the mixed sweeps change their lanes per
-node: the energy sweep (6,000 and 25,000 nodes, seen in a step), the lean tensor
-pair sweep (15,000 and 25,000) and the CRKSPH sweeps (6,000, 25,000 and 35,000),
-against the FP64 oracle within the mixed mode's bounds (2e-5 for
-derivatives, 5e-5 for the state after a step)."""
+"""Both sides of the node counts where the sweeps change their lanes per node.
+FP64: 30,000 nodes.  Mixed: the energy sweep (6,000 and 40,000, seen in a step),
+the lean tensor pair sweep (15,000 and 25,000) and the CRKSPH sweeps (6,000,
+25,000 and 35,000).  Against the FP64 oracle: 1e-12 for FP64 derivatives, 2e-5
+for mixed ones, 5e-5 for the mixed state after a step."""
 import numpy as np
 import pytest
 
@@ -13,22 +13,35 @@ from _parity import compare_fields
 pytestmark = pytest.mark.gpu
 
 
-def _both(oracle_mod, p):
+def _both(oracle_mod, p, precision="fp32"):
     from spheral_gb300.engine import Engine
-    eng, orc = Engine.from_problem(p, precision="fp32"), oracle_mod.Oracle(p)
+    eng, orc = Engine.from_problem(p, precision=precision), oracle_mod.Oracle(p)
     eng.initialize()
     orc.initialize()
     return eng, orc
 
 
-@pytest.mark.parametrize("n", [5999, 6000, 24999, 25000])
-def test_energy_lines(native_lib, oracle_mod, n):
+def _box(n):
     side = int(np.ceil(n ** (1.0 / 3.0)))
     p = problems.random_box(n_side=side, seed=n % 89, nPerh=1.25, boundaries="open")
     keep = np.sort(np.random.default_rng(n).permutation(p.n)[:n])
     for k in ("pos", "vel", "mass", "rho", "eps", "H", "nodelist"):
         setattr(p, k, np.ascontiguousarray(getattr(p, k)[keep]))
-    eng, orc = _both(oracle_mod, p)
+    return p
+
+
+@pytest.mark.parametrize("n", [29999, 30000])
+def test_fp64_line(native_lib, oracle_mod, n):
+    eng, orc = _both(oracle_mod, _box(n), "fp64")
+    eng.evaluate_derivatives()
+    orc.evaluate_derivatives()
+    bad = compare_fields(eng, orc, ["DvDt", "DepsDt", "DvDx", "gradRho", "M", "massZerothMoment", "omegaGradh"], 1e-12)
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("n", [5999, 6000, 39999, 40000])
+def test_energy_lines(native_lib, oracle_mod, n):
+    eng, orc = _both(oracle_mod, _box(n))
     for _ in range(2):
         a, b = eng.step(), orc.step()
         assert abs(a - b) <= 1e-5 * b
