@@ -322,8 +322,9 @@ int sphgpu_timer_stop(sphgpu_handle h, double* ms);
 int sphgpu_neighbor_count(sphgpu_handle h, long* entries);
 /* Mixed-mode pair kernel variant (neighbour slots per iteration and register
  * budget; the count depends on the configured hydro and smoothing scale, and
- * below 100,000 to 150,000 nodes, where several lanes share a node, all are
- * the same kernel).  By default (-1) the fastest is picked by timing each at
+ * below 100,000 nodes, for isotropic SPH 150,000, for ASPH with several
+ * NodeLists, plain sums, tensile correction or expansion options 20,000, all
+ * are the same kernel).  By default (-1) the fastest is picked by timing each at
  * the first evaluation for a problem size and again two evaluations later;
  * sphgpu_set_pair_variant pins one
  * (0 .. *nvariants-1 from sphgpu_get_pair_variant), or -1 to re-enable the

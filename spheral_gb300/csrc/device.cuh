@@ -187,7 +187,6 @@ inline int lanesEnergy(long n) { return n >= kExactNodes ? 1 : (n >= 40000 ? 2 :
 #define SPH_BY_LANES(L, CALL)      \
   switch (L) {                     \
     case 1: CALL(1); break;        \
-    case 2: CALL(2); break;        \
     case 4: CALL(4); break;        \
     case 8: CALL(8); break;        \
     default: CALL(16); break;      \
@@ -317,27 +316,8 @@ __device__ __forceinline__ void writeMirrors(const Fields& F, long i, const Fiel
 
 // FP32 separation r_i - r_j' on cell-relative coordinates: r = (x_i - x_j')
 // - d cell per axis, with x_j' = cell - x_j for a mirror image.  Periodic
-// images need no box arithmetic: the cell offset d carries the wrap.
-__device__ __forceinline__ void relSep(const float4& pi, const float4& pj, int dcode, uint32_t mm, float cx,
-                                       float cy, float cz, float& rx, float& ry, float& rz) {
-  float xj = pj.x, yj = pj.y, zj = pj.z;
-  const uint32_t mir = (uint32_t)dcode & mm;
-  if (mir) {
-    if (mir & 3u) xj = cx - xj;
-    if (mir & 12u) yj = cy - yj;
-    if (mir & 48u) zj = cz - zj;
-  }
-  const int d0 = dcode & 3, d1 = (dcode >> 2) & 3, d2 = (dcode >> 4) & 3;
-  const float ox = d0 == 1 ? cx : (d0 == 2 ? -cx : 0.0f);
-  const float oy = d1 == 1 ? cy : (d1 == 2 ? -cy : 0.0f);
-  const float oz = d2 == 1 ? cz : (d2 == 2 ? -cz : 0.0f);
-  rx = __fadd_rn(__fsub_rn(pi.x, xj), ox);
-  ry = __fadd_rn(__fsub_rn(pi.y, yj), oy);
-  rz = __fadd_rn(__fsub_rn(pi.z, zj), oz);
-}
-
-// relSep from a list entry (bitwise the same result), the cell offset per axis
-// (0, +c, -c for codes 0, 1, 2) by integer selection: the sweeps are bound by
+// images need no box arithmetic: the cell offset d of the list entry carries the
+// wrap.  The offset per axis (0, +c, -c for codes 0, 1, 2) by integer selection: the sweeps are bound by
 // shared-memory / L1 wavefronts (~11 per 16-byte gather), so a table of the
 // offsets in shared memory costs more than these instructions.
 // MIR false: no wall of the grid reflects, so no entry is a mirror image.
@@ -401,21 +381,6 @@ __device__ __forceinline__ double tableEval(const double* c, int i0, double x) {
   return c[i0] + (c[i0 + 1] + c[i0 + 2] * x) * x;
 }
 
-__device__ __forceinline__ double blockMin(double v, double* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if (lane == 0) sm[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sm[lane] : DBL_MAX;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  __syncthreads();
-  return v;
-}
-__device__ __forceinline__ double blockMax(double v, double* sm) { return -blockMin(-v, sm); }
 __device__ __forceinline__ double blockSum(double v, double* sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll

@@ -800,7 +800,6 @@ struct GravityWork {
   GBuf part, box, thr, dtBits, key64, timeout, vals, vals2, sortWs, skey, tpos, nc, off, scanWs, total, cells, mx,
       energy, tpos32, cells32, parent, pending;
   long long* hTotal = nullptr;
-  long long lastCells = 0;
 };
 
 GravityWork* gravityCreate() {
@@ -818,8 +817,6 @@ void gravityDestroy(GravityWork* w) {
   if (w->hTotal) cudaFreeHost(w->hTotal);
   delete w;
 }
-
-long long gravityNumCells(const GravityWork* w) { return w ? w->lastCells : 0; }
 
 int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening, double opening, bool mixed,
                     double* dOut, cudaStream_t s, LaunchCounter* lc, char* err, int errlen) {
@@ -839,7 +836,6 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
   if (n <= 1) {
     zeroGravityKernel<<<blocksFor(n > 0 ? n : 1, kThreads), kThreads, 0, s>>>(F, n, G, dOut);
     lc->add(1);
-    w->lastCells = n;
     GCHK(cudaGetLastError());
     return SPHGPU_OK;
   }
@@ -892,7 +888,6 @@ int gravityEvaluate(GravityWork* w, Fields F, long n, double G, double softening
     std::snprintf(err, errlen, "octree cell count %lld out of range", numCells);
     return SPHGPU_E_OVERFLOW;
   }
-  w->lastCells = numCells;
   GCHK(w->cells.ensure(numCells * sizeof(TreeCell)));
   GCHK(w->mx.ensure(numCells * sizeof(Sums4)));
   TreeCell* cells = w->cells.as<TreeCell>();

@@ -338,6 +338,13 @@ __global__ void __launch_bounds__(128, TENSOR ? 4 : 6) neighborMaskKernel(Fields
   constexpr int G = 4 / CW;                  // items per block
   constexpr int UNROLL = TENSOR ? 1 : 8;     // 35 loads per iteration with TENSOR
   constexpr int NB = CW == 4 ? 8 : 16;       // ring of batches whose masks wait for the writing
+  static_assert(CW == 1 || CW == 4, "one warp or the block's four per item");
+  static_assert(kTile <= 32, "a tile's chunks are listed one per lane");
+  // CW = 4 writes after every tile: a warp stages the candidates of at most
+  // ceil(kTile / 4) chunks of up to 32.  CW = 1 writes when NB - 1 batches wait,
+  // with one more being staged.  `nonempty` has a bit per waiting batch.
+  static_assert(CW == 1 || (kTile + 3) / 4 <= NB, "the ring holds a warp's share of a tile");
+  static_assert(NB >= 3 && NB <= 32, "the ring holds the waiting batches and the two being staged");
   // per warp, 64 slots: the staged candidates' -x, -y, -z and (h^-1)^2; TENSOR:
   // H (xx xy xz yy yz zz) as seen through the mirrors, minus the band's top and
   // its bottom

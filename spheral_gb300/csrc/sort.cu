@@ -115,8 +115,6 @@ void scanExclusive(const Tin* in, long long* out, long n, void* workspace, long 
   if (lc) lc->add(3);
 }
 template void scanExclusive<int>(const int*, long long*, long, void*, long long*, cudaStream_t, LaunchCounter*);
-template void scanExclusive<long long>(const long long*, long long*, long, void*, long long*, cudaStream_t,
-                                       LaunchCounter*);
 
 //------------------------------------------------------------------------------
 // Stable LSD radix sort, 8-bit digits, one kernel per digit.

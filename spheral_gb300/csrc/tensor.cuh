@@ -390,18 +390,6 @@ __device__ __forceinline__ void writeTensorMirror(const Fields& F, long i, const
   P.hten[k] = make_float4(toFloatRN(h.xx), toFloatRN(h.xy), toFloatRN(h.xz), toFloatRN(h.yy));
   P.hten[P.stride + k] = make_float4(toFloatRN(h.yz), toFloatRN(h.zz), toFloatRN(symDet(h)), toFloatRN(F.f[F_HLMAX][i]));
 }
-// H_j of a neighbour entry from the mirror, seen through the mirror-axis bits
-// mir (dcode layout) of the entry.
-__device__ __forceinline__ void loadTensor32(const Fields32& P, int j, uint32_t mir, float4& a, float4& b) {
-  a = P.hten[j];
-  b = P.hten[P.stride + j];
-  if (mir) {
-    const float sx = (mir & 3u) ? -1.f : 1.f, sy = (mir & 12u) ? -1.f : 1.f, sz = (mir & 48u) ? -1.f : 1.f;
-    a.y *= sx * sy;
-    a.z *= sx * sz;
-    b.x *= sy * sz;
-  }
-}
 // H r in FP32 from the mirror (a = xx xy xz yy, b = yz zz . .), fixed order.
 __device__ __forceinline__ void symDot32(const float4& a, const float4& b, float x, float y, float z, float& ox,
                                          float& oy, float& oz) {
