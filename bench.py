@@ -39,9 +39,9 @@ FLOP_PER_PAIR = 456        # algorithmic FLOPs of the reference pair body per un
 VALUES_PER_NODE = 63       # per-node state read + derivatives written by the pair loop
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unordered pair
 # of one pairKernelLean32 launch, from an ncu capture of
-# kelvin_helmholtz(n1=64) (905 MB for 21.7 M pairs); traffic grows in
+# kelvin_helmholtz(n1=64) (902 MB for 21.7 M pairs); traffic grows in
 # proportion to the pairs, so it is scaled by the pairs of the launch.
-TRAFFIC_BYTES_PER_PAIR = {"fp32": 41.7}
+TRAFFIC_BYTES_PER_PAIR = {"fp32": 41.5}
 TRAFFIC_SOURCE = "ncu capture at n1=64 scaled by pairs per launch"
 
 

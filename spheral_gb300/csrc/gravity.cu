@@ -373,7 +373,7 @@ __device__ __forceinline__ void cell32(const TreeCell& cl, double thr, double so
 // daughters in pre-order (so the sums do not depend on who arrives last).  Few
 // lanes of a warp climb far, so only the additions are done here: with the
 // divisions and opening distances it took 232 us at 222,119 cells, without them
-// 67 us and cellFinalKernel 27 us.
+// 67 us and cellFinalKernel 34 us.
 __global__ void momentKernel(const TreeCell* __restrict__ cells, long long numCells,
                              const TreeNode* __restrict__ tpos, const int* __restrict__ parent,
                              int* __restrict__ pending, Sums4* __restrict__ sums) {
@@ -419,7 +419,7 @@ __global__ void cellFinalKernel(TreeCell* __restrict__ cells, long long numCells
     const TreeNode p = tpos[cl.start];
     cl.x = p.x; cl.y = p.y; cl.z = p.z; cl.M = p.m;
   } else {
-    // correctly rounded, as the reference's: the centre decides which cells open
+    // correctly rounded: the centre decides which cells open
     cl.x = __ddiv_rn(sm.x, sm.w); cl.y = __ddiv_rn(sm.y, sm.w); cl.z = __ddiv_rn(sm.z, sm.w); cl.M = sm.w;
   }
   // Geometric centre: xmin + (ix + 0.5) * cellsize, cellsize = boxLength / 2^level.
@@ -660,7 +660,7 @@ __device__ __forceinline__ void addMonopole32Any(float M, dev::f32x2 dxy, float 
 // 150,001 nodes) and the latency of the next cell: the thresholds, the one-node
 // leaves and the next cell's index come with the cell, the separations and
 // compensated sums are packed pairs; ~50 instructions per visit.  150,001 nodes:
-// 893 us.  Loading both cells that may come next ahead of the decision took 89
+// 905 us.  Loading both cells that may come next ahead of the decision took 89
 // registers and 1173 us.
 __global__ void __launch_bounds__(128) treeWalkMixedKernel(
     const TreeCell32* __restrict__ c32, const TreeCell* __restrict__ cells, long long numCells,

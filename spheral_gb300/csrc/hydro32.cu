@@ -537,9 +537,9 @@ __global__ void __launch_bounds__(128, MINB) pairKernelIso32(Fields F, Fields32 
 // these roundings (kExactNodes) and small ones take the cheaper form above.
 // Per-node values (rho, Prho, -Cl c, 1/rho) come from the record, mirror
 // tests and table branches are gone and the accelerations go out in planes.
-// Bound by the L1 data pipe and issue (64 % of the slots at 12 warps per SM);
+// Bound by the L1 data pipe and issue (65 % of the slots at 12 warps per SM);
 // writes 12 and reads 4 bytes of DRAM per slot, 0.6 ms at 2.1 M nodes of 119.
-// 2.1 M nodes: 2685 -> 2082 us.
+// 2.1 M nodes: 2685 -> 2058 us.
 //------------------------------------------------------------------------------
 template <bool LIMQ, bool MIR, bool SPLINE, bool PLAIN, int U, int MINB>
 __global__ void __launch_bounds__(128, MINB) pairKernelLean32(Fields F, Fields32 P, const int* __restrict__ list,
@@ -1299,8 +1299,8 @@ void launchPairFP32(Fields F, Fields32 F32, const int* list, long n, Grid g, Nei
     // per iteration at three blocks per SM (579 us), one at four (593), two at four
     // (578), three at two (567); below 100,000 nodes variant 0 (79,507 nodes:
     // 125 us), and several lanes per node below 25,000.  The run-time options: one
-    // lane from 20,000 nodes on (39,304 nodes, two NodeLists: 87 us, four lanes 97),
-    // four below (10,648: 41, one lane 72).
+    // lane from 20,000 nodes on (two NodeLists, 21,952 nodes: 73 us, four lanes 76;
+    // 50,653: 93 and 145), four below (10,648: 41).
     if (!hp.xsph && hp.compatible && !hp.limitedQ) {
       if (!inputs) pairInputs32<<<gridFor(n, 256), 256, 0, s>>>(F, F32, n, pairForm32(n, hp));
 #define SPH_TEN(OP, MI, SP, LA, U, MB) \
