@@ -315,7 +315,8 @@ void setTable(sphgpu_ctx* c, const double* w, const double* g, const double* g2,
     const double step = c->kernelExtent / nint;
     auto refit = [&](const std::vector<double>& q, std::vector<double>& out) {
       auto at = [&](double eta) {
-        const size_t i0 = 3u * std::min((size_t)N1, size_t(eta / meta[1]));
+        const double k = eta / meta[1];   // any value a caller's interval can give
+        const size_t i0 = 3u * (k >= N1 ? (size_t)N1 : (k > 0.0 ? (size_t)k : 0u));
         return q[i0] + (q[i0 + 1] + q[i0 + 2] * eta) * eta;
       };
       out.resize(3 * (size_t)nint);

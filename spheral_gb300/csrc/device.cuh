@@ -317,8 +317,8 @@ __device__ __forceinline__ void writeMirrors(const Fields& F, long i, const Fiel
 // FP32 separation r_i - r_j' on cell-relative coordinates: r = (x_i - x_j')
 // - d cell per axis, with x_j' = cell - x_j for a mirror image.  Periodic
 // images need no box arithmetic: the cell offset d of the list entry carries the
-// wrap.  The offset per axis (0, +c, -c for codes 0, 1, 2) by integer selection: the sweeps are bound by
-// shared-memory / L1 wavefronts (~11 per 16-byte gather), so a table of the
+// wrap.  The offset per axis (0, +c, -c for codes 0, 1, 2) comes by integer
+// selection: the sweeps are bound by shared-memory / L1 wavefronts (~11 per 16-byte gather), so a table of the
 // offsets in shared memory costs more than these instructions.
 // MIR false: no wall of the grid reflects, so no entry is a mirror image.
 __device__ __forceinline__ float cellOffset(uint32_t ent, int axis, float c) {

@@ -97,8 +97,8 @@ __device__ __forceinline__ TreeNode loadNode(const TreeNode* __restrict__ p) {
 }
 
 // What a walk reads of a cell it visits: the double-float centre of mass (from
-// the box corner) in pairs for the packed operations, the mass, and the decision thresholds.  With
-// r2 the FP32 squared separation, r2 > hi: the cell's monopole applies (a far
+// the box corner) in pairs for the packed operations, the mass, and the decision
+// thresholds.  With r2 the FP32 squared separation, r2 > hi: the cell's monopole applies (a far
 // cell, or a one-node leaf, whose monopole is its node); r2 < lo: it does not
 // (an internal cell is opened, a one-node leaf is the node itself); between
 // them FP64 decides.
